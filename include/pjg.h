@@ -328,7 +328,7 @@ pjg_status pjg_parse_pdb(const char *text, int64_t len, int32_t flags, void *rec
  * stream); the call returns without waiting.
  *
  * It allocates nothing: its scratch is a static device array of
- * PJG_NOALLOC_MAX_ROWS (2^20) row flags (4 MiB) that every GPU loading the
+ * PJG_NOALLOC_MAX_ROWS (2^20) row bits (128 KiB) that every GPU loading the
  * library keeps until the process exits.  More rows than that, or a bad
  * argument, return PJG_ERR_INVALID with a message from
  * pjg_noalloc_last_error().  The first call on each device looks up that

@@ -98,3 +98,43 @@ def test_superpose_noalloc_rejects_oversize():
     st = L.pjg_superpose_noalloc(None, None, (1 << 20) + 1, 9, 2.0, None, None, None, None, count.data_ptr(), None)
     assert st == 1
     assert b"at most" in L.pjg_noalloc_last_error()
+
+
+@pytest.mark.parametrize("rows, atoms", [(0, 3), (1, 3), (31, 32), (32, 12), (33, 2), (64, 5), (65, 1), (1023, 9),
+                                         (1025, 12), (33000, 4)])
+def test_superpose_noalloc_row_edges(rows, atoms):
+    """Row counts around a warp, a block and the compaction's 1,024-row tiles
+    against numpy's SVD fit (FP64, rmsd and rotation within the bounds of the
+    query tests), and the rows under the threshold in row order."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    L = _bind()
+    rng = np.random.default_rng([77, rows, atoms])
+    tpl = rng.normal(scale=4.0, size=(atoms, 3))
+    mol = tpl + rng.normal(size=(rows, atoms, 3)) * rng.uniform(0.1, 2.0, size=(rows, 1, 1))
+    ca, cb = mol.mean(1), tpl.mean(0)
+    u, sv, vt = np.linalg.svd(np.einsum("ni,mnj->mij", tpl - cb, mol - ca[:, None]))
+    sign = np.ones((rows, 3))
+    sign[:, 2] = np.sign(np.linalg.det(u) * np.linalg.det(vt))
+    R = np.einsum("mij,mj,mjk->mik", u, sign, vt)
+    want = np.sqrt((((tpl - cb) - np.einsum("mij,mnj->mni", R, mol - ca[:, None])) ** 2).sum((1, 2)) / atoms)
+    dev = torch.device("cuda")
+    m = max(rows, 1)
+    d = [torch.tensor(mol.reshape(-1), device=dev), torch.tensor(tpl.reshape(-1), device=dev)]
+    rmsd, rot, cen = (torch.zeros(k * m, dtype=torch.float64, device=dev) for k in (1, 9, 6))
+    idx, count = (torch.full((k,), -1, dtype=torch.int32, device=dev) for k in (m, 1))
+    thr = float(np.median(want)) + 1e-7 if rows else 1.0
+    st = L.pjg_superpose_noalloc(d[0].data_ptr(), d[1].data_ptr(), rows, atoms, thr, rmsd.data_ptr(), rot.data_ptr(),
+                                 cen.data_ptr(), idx.data_ptr(), count.data_ptr(), None)
+    assert st == 0, L.pjg_noalloc_last_error()
+    torch.cuda.synchronize()
+    expect = np.flatnonzero(want <= thr) if atoms >= 3 else np.zeros(0, int)  # fewer atoms: no defined rotation
+    k = int(count.item())
+    assert k == len(expect) and np.array_equal(idx.cpu().numpy()[:k], expect)
+    if rows:
+        assert np.abs(rmsd.cpu().numpy() - want).max() <= RMSD_TOL if atoms >= 3 else True
+        assert np.abs(cen.cpu().numpy().reshape(rows, 6)[:, :3] - ca).max() <= 1e-9
+    if rows and atoms >= 4:  # (well separated singular values: a defined rotation)
+        ok = (sv[:, 1] + sign[:, 2] * sv[:, 2]) > 1e-3 * sv[:, 0]
+        assert np.abs(rot.cpu().numpy().reshape(rows, 3, 3) - R)[ok].max() <= ROT_TOL
