@@ -259,7 +259,11 @@ void pjg_results_destroy(pjg_results *r);
  *   leaf_levels    levels (after level 0) whose candidate lists are put in
  *                  kd leaf order before the search; deeper lists when a
  *                  pair first reaches them (default 4; -1 every list up
- *                  front; the plain FP64 mode always orders every list)
+ *                  front; the plain FP64 mode always orders every list).
+ *                  At the default the batched modes search every pair
+ *                  without any order first and order only the lists that
+ *                  tell a pair's rows apart; another value searches every
+ *                  pair in order
  *   block_min      shortest list the search expands one parent at a time
  *                  with block culling (shorter lists: lanes over (parent,
  *                  candidate) pairs) (default 64, 1 .. 65535)

@@ -7,10 +7,17 @@
 //   k_struct_totals               candidate entries per structure
 //   per structure chunk (bounded entry budget):
 //     k_scan_*, k_block_counts    list offsets, culling blocks of CULL_BLK leaves
-//     k_candidates                lists in candidate order
-//     k_demand_levels             requests the lists of the first levels
-//     k_leaf_order, k_leaf_sorted, k_leaf_exact, k_mark_ordered
+//     k_search_free               complete assignments of every pair, in any
+//                                 order; requests the lists that tell a
+//                                 pair's rows apart
+//     k_candidates                lists in candidate order (of the pairs
+//                                 taken in items of seeds), k_search_free on
+//                                 those items
+//     k_leaf_part, k_leaf_sorted, k_leaf_exact, k_mark_ordered
 //                                 requested lists in kd leaf order
+//     k_unit_order                the rows' places in their pair's stream
+//     or, in the plain mode and with explicit leaf levels:
+//     k_demand_levels             requests the lists of the first levels
 //     k_search                    complete assignments, ordered per pair;
 //                                 pairs that reach a list without leaf order
 //                                 request it and are suspended, the lists are
@@ -189,6 +196,14 @@ struct pjg_structures {
     // in nh_pos, which holds every structure's atoms grouped by (bucket,
     // name), each group in ResIndex order
     int32_t *d_nh_off = nullptr, *d_nh_pos = nullptr;
+    // order-free search (FreeView): kinds of the set, per nh_* entry its kind,
+    // points in nh_pos order, atoms in residue order
+    int32_t n_kinds = 0, max_local_kinds = 0;
+    uint32_t *d_kind_name = nullptr, *d_kind_res = nullptr;
+    int32_t *d_nh_kind = nullptr, *d_res_pos = nullptr, *d_res_place = nullptr;
+    float4 *d_kxyz = nullptr;
+    uint16_t *d_res_kind = nullptr;
+    int4 *d_res_range = nullptr;
     int device = 0;
 };
 
@@ -554,6 +569,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
     HostArray<int32_t> sorted((size_t)N);
     HostArray<uint8_t> name_id((size_t)N);
     HostArray<int32_t> nh_pos((size_t)N);
+    HostArray<uint16_t> local_kind((size_t)N);
     std::vector<int32_t> bucket_begin{0}, bucket_lo, bucket_hi;
     std::vector<uint32_t> bucket_name;
     for (int s = 0; s < S; s++) {
@@ -579,11 +595,31 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
         std::vector<uint32_t> hname;  // distinct atom names of each bucket, sorted
         std::vector<int32_t> hcount, hbegin{0};
         std::vector<int32_t> hoff;    // start of each distinct name's atoms in nh_pos (structure-local)
+        std::vector<int32_t> hkind;   // its kind (distinct residue and atom name of the set)
         double radius = 0.0;
         int64_t bad = -1;  // first atom with a non-finite coordinate
     };
     std::vector<Buckets> bk(std::max(S, 0));
-    auto prepare = [&](int s) {
+    // kinds of the set, numbered as the host threads meet them (each thread
+    // keeps the ones it has seen, so the shared table is rarely locked)
+    using KindMap = std::unordered_map<uint64_t, int32_t>;
+    KindMap kinds_all;
+    std::vector<uint32_t> kind_name, kind_res;
+    std::mutex kinds_mutex;
+    auto kind_of = [&](uint32_t res, uint32_t nm, KindMap &seen) -> int32_t {
+        const uint64_t key = ((uint64_t)res << 32) | nm;
+        auto it = seen.find(key);
+        if (it != seen.end()) return it->second;
+        std::lock_guard<std::mutex> g(kinds_mutex);
+        auto ins = kinds_all.emplace(key, (int32_t)kind_name.size());
+        if (ins.second) {
+            kind_name.push_back(nm);
+            kind_res.push_back(res);
+        }
+        seen.emplace(key, ins.first->second);
+        return ins.first->second;
+    };
+    auto prepare = [&](int s, KindMap &seen) {
         const int64_t b0 = base[s];
         const int n = count[s];
         Buckets &B = bk[s];
@@ -665,6 +701,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
                 if (i == 0 || nm[i] != nm[i - 1]) {
                     B.hname.push_back(nm[i]);
                     B.hcount.push_back(0);
+                    B.hkind.push_back(kind_of(B.name[k], nm[i], seen));
                 }
                 B.hcount.back()++;
             }
@@ -682,6 +719,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
                 const size_t id = std::lower_bound(B.hname.begin() + h0, B.hname.end(), name[b0 + a]) -
                                   (B.hname.begin() + h0);
                 name_id[b0 + a] = (uint8_t)std::min<size_t>(id, 255);
+                local_kind[b0 + a] = (uint16_t)std::min<size_t>(h0 + id, 65535);
                 nh_pos[b0 + fill[id]++] = a;
             }
         }
@@ -690,7 +728,8 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
         const int nthreads = (int)std::max<unsigned>(1, std::min<unsigned>(32, std::thread::hardware_concurrency()));
         std::atomic<int> next{0};
         auto worker = [&]() {
-            for (int s; (s = next.fetch_add(1)) < S;) prepare(s);
+            KindMap seen;
+            for (int s; (s = next.fetch_add(1)) < S;) prepare(s, seen);
         };
         std::vector<std::thread> pool;
         for (int i = 1; i < std::min(nthreads, S); i++) pool.emplace_back(worker);
@@ -702,7 +741,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
             delete h;
             return fail(PJG_ERR_INVALID, "structure %d atom %lld: non-finite coordinate", s, (long long)bk[s].bad);
         }
-    std::vector<int32_t> nh_begin{0}, nh_count, nh_off;
+    std::vector<int32_t> nh_begin{0}, nh_count, nh_off, nh_kind;
     std::vector<uint32_t> nh_name;
     for (int s = 0; s < S; s++) {
         const Buckets &B = bk[s];
@@ -710,7 +749,10 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
         nh_name.insert(nh_name.end(), B.hname.begin(), B.hname.end());
         nh_count.insert(nh_count.end(), B.hcount.begin(), B.hcount.end());
         nh_off.insert(nh_off.end(), B.hoff.begin(), B.hoff.end());
+        nh_kind.insert(nh_kind.end(), B.hkind.begin(), B.hkind.end());
+        h->max_local_kinds = std::max(h->max_local_kinds, (int32_t)B.hname.size());
     }
+    h->n_kinds = (int32_t)kind_name.size();
     for (int s = 0; s < S; s++) {
         const Buckets &B = bk[s];
         h->max_radius = std::max(h->max_radius, B.radius);
@@ -739,21 +781,34 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
     if (e == cudaSuccess) e = upload(&h->d_name_id, name_id.p.get(), (size_t)N);
     if (e == cudaSuccess) e = upload(&h->d_nh_off, nh_off);
     if (e == cudaSuccess) e = upload(&h->d_nh_pos, nh_pos.p.get(), (size_t)N);
+    if (e == cudaSuccess) e = upload(&h->d_kind_name, kind_name);
+    if (e == cudaSuccess) e = upload(&h->d_kind_res, kind_res);
+    if (e == cudaSuccess) e = upload(&h->d_nh_kind, nh_kind);
     if (e == cudaSuccess) {
-        // axis ranks of every atom (the leaf-order sorted-axis path)
-        const size_t n3 = 3 * (size_t)std::max<int64_t>(N, 1);
+        // axis ranks of every atom (the leaf-order sorted-axis path), and the
+        // residue order and kind-ordered points of the order-free search
+        const size_t n1 = (size_t)std::max<int64_t>(N, 1), n3 = 3 * n1;
         unsigned long long *tile_key = nullptr;
-        uint16_t *tile_idx = nullptr;
+        uint16_t *tile_idx = nullptr, *d_local_kind = nullptr;
         e = cudaMalloc((void **)&h->d_lrank, n3 * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_urank, n3 * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&tile_key, n3 * sizeof(unsigned long long));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&tile_idx, n3 * sizeof(uint16_t));
+        if (e == cudaSuccess) e = cudaMalloc((void **)&tile_key, 4 * n1 * sizeof(unsigned long long));
+        if (e == cudaSuccess) e = cudaMalloc((void **)&tile_idx, 4 * n1 * sizeof(uint16_t));
+        if (e == cudaSuccess) e = upload(&d_local_kind, local_kind.p.get(), (size_t)N);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_kxyz, n1 * sizeof(float4));
+        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_pos, n1 * sizeof(int32_t));
+        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_place, n1 * sizeof(int32_t));
+        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_kind, n1 * sizeof(uint16_t));
+        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_range, n1 * sizeof(int4));
         if (e == cudaSuccess) {
             launch_axis_ranks(0, S, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key, tile_idx, h->d_lrank,
-                              h->d_urank);
+                              h->d_urank,
+                              ResidueOrder{h->d_xyz32, h->d_nh_pos, d_local_kind, h->d_kxyz, h->d_res_pos,
+                                           h->d_res_kind, h->d_res_range, h->d_sorted, h->d_res_place});
             e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaDeviceSynchronize();
         }
+        if (d_local_kind) cudaFree(d_local_kind);
         if (tile_key) cudaFree(tile_key);
         if (tile_idx) cudaFree(tile_idx);
     }
@@ -772,7 +827,8 @@ void pjg_structures_destroy(pjg_structures *h) {
     void *ptrs[] = {h->d_atom_base, h->d_atom_count, h->d_xyz64, h->d_xyz32, h->d_name, h->d_resname,
                     h->d_sorted, h->d_bucket_begin, h->d_bucket_name, h->d_bucket_lo, h->d_bucket_hi,
                     h->d_lrank, h->d_urank, h->d_nh_begin, h->d_nh_name, h->d_nh_count, h->d_name_id,
-                    h->d_nh_off, h->d_nh_pos};
+                    h->d_nh_off, h->d_nh_pos, h->d_kind_name, h->d_kind_res, h->d_nh_kind, h->d_kxyz,
+                    h->d_res_pos, h->d_res_place, h->d_res_kind, h->d_res_range};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete h;
@@ -950,6 +1006,19 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     cudaStream_t st = nullptr;
     cudaEvent_t ev[8] = {};
     DBuf<AnnulusParam> d_params;
+    // order-free search: kinds of each signature, units of rows, heavy pairs
+    // and their items, frontiers of the items, keys of large units
+    DBuf<uint32_t> d_sig_bits;
+    DBuf<RowUnit> d_units;
+    DBuf<HeavyPair> d_heavy_pairs;
+    DBuf<unsigned long long> d_free_n, d_heavy_stats, d_row_key;
+    DBuf<int2> d_items, d_results;
+    DBuf<int64_t> d_item_base, d_bin_off;
+    DBuf<int32_t> d_bins, d_arena_atom, d_row_scratch, d_item_head, d_large_units, d_long_pairs;
+    DBuf<uint32_t> d_item_branch;
+    DBuf<SpilledEntry> d_spill_a, d_spill_b;
+    DBuf<float4> d_arena_xyz;
+    DBuf<uint16_t> d_arena_parent;
     DBuf<int32_t> d_count, d_scanned, d_cand_atom, d_leaf_atom, d_pair_counter;
     DBuf<int64_t> d_offset, d_totals, d_boff;
     DBuf<int32_t> d_nblk;
@@ -1011,6 +1080,13 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         const char *v = getenv("PJG_LEAF_LEVELS");
         if (v && *v && P->mode != PJG_MODE_PLAIN_FP64) demand_levels = atoi(v);
     }
+    // every pair searched without order first (k_search_free): the batched
+    // modes, unless the levels to order up front are chosen explicitly
+    FreeView fv{sp->n_kinds, (sp->n_kinds + 31) / 32, sp->d_kind_name, sp->d_kind_res, nullptr, sp->d_nh_kind,
+                sp->d_kxyz, sp->d_res_pos, sp->d_res_kind, sp->d_res_range};
+    const bool free_first = P->mode != PJG_MODE_PLAIN_FP64 && demand_levels == TUNING_DEFAULTS.leaf_levels &&
+                            !getenv("PJG_LEAF_LEVELS") && sp->max_local_kinds <= FREE_MAX_KINDS &&
+                            (int64_t)G * fv.kind_words <= (1ll << 28);
     std::vector<int64_t> totals(S);
 
     if (T == 0 || S == 0) {
@@ -1073,7 +1149,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     CUDA_TRY(cudaMemsetAsync(d_counters.p, 0, C_NUM * sizeof(unsigned long long), st));
     CUDA_TRY(dalloc(d_pair_counter, 1, st));
     CUDA_TRY(dalloc(d_ccount, 1, st));
-    CUDA_TRY(dalloc(d_rtotals, 4, st));
+    CUDA_TRY(dalloc(d_rtotals, 5, st));
 
     {
         // pass 1: list lengths for every (structure, signature)
@@ -1091,6 +1167,12 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         launch_candidates(st, std::max(blocks, 1), false, cv, sv, d_count.p, d_scanned.p, nullptr, nullptr);
         k_struct_totals<<<std::max(1, std::min(S, sm_count() * 8)), 256, 0, st>>>(S, G, d_count.p, d_totals.p);
         launches += 2;
+        if (free_first) {
+            CUDA_TRY(dalloc(d_sig_bits, (size_t)G * fv.kind_words, st));
+            fv.sig_bits = d_sig_bits.p;
+            launch_sig_kinds(st, sv, fv, d_sig_bits.p);
+            launches++;
+        }
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(totals.data(), d_totals.p, sizeof(int64_t) * S, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -1275,6 +1357,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             // search rounds) for each deeper list a pair's frontier reaches;
             // a negative value orders every list of the chunk up front
             LeafDemand dm{};
+            bool free_chunk = false;
             const int leaf_blocks =
                 std::max(1, (int)std::min<int64_t>((Wc + LEAF_WARPS - 1) / LEAF_WARPS, (int64_t)sm_count() * 32));
             // room in the leaf arrays for `need` entries (the lists ordered so
@@ -1432,6 +1515,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     status = fail(PJG_ERR_CAPACITY, "too many pairs in one chunk");
                     goto done;
                 }
+                free_chunk = free_first && n_pairs <= INT32_MAX - (1 << 20);
                 // the costliest pairs are searched first (a pair can take
                 // milliseconds; started last, it alone would run on while the
                 // other warps idle): the level demand estimates each pair's
@@ -1442,7 +1526,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 const int64_t per_warp = hw && atoi(hw) > 0 ? atoi(hw) : 2;
                 const int64_t heavy_target = per_warp * 2 * sm_count() * SEARCH_WARPS;
                 const char *hf = getenv("PJG_HEAVY_FIRST");
-                const bool heavy_on = (int64_t)n_pairs >= 8 * heavy_target &&
+                const bool heavy_on = !free_chunk && (int64_t)n_pairs >= 8 * heavy_target &&
                                       (int64_t)n_pairs <= (int64_t)INT32_MAX - heavy_target &&
                                       !(hf && atoi(hf) == 0);
                 dm.pair_cost = nullptr;
@@ -1455,7 +1539,10 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(cudaMemsetAsync(d_hbins.p, 0, 66 * sizeof(unsigned long long), st));
                     dm.pair_cost = d_pcost.p;
                 }
-                launch_demand_levels(st, sm_count() * 16, tv, cd, (int32_t)n_pairs, demand_levels, P->reorder, dm);
+                // (order-free first: only the lists of templates over 32 atoms)
+                if (!free_chunk || !tp->large.empty()) {
+                    launch_demand_levels(st, sm_count() * 16, tv, cd, (int32_t)n_pairs,
+                                         free_chunk ? -1 : demand_levels, P->reorder, dm);
                 if (heavy_on) {
                     launch_heavy_pairs(st, (int32_t)n_pairs, d_pcost.p, d_hbins.p, heavy_target, d_hflag.p,
                                        d_heavy.p);
@@ -1474,6 +1561,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 CUDA_TRY(ensure_leaf((int64_t)used));
                 CUDA_TRY(order_requested());
                 leaf_filled = (int64_t)used;
+                }
             }
             CUDA_TRY(cudaEventRecord(ev[2], st));
             SearchArgs sa;
@@ -1530,7 +1618,9 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 const int64_t bound = n_pairs * ((int64_t)P->max_candidates + 2);
                 const int64_t budget = row_budget();
                 if (bound <= budget) {
-                    want_rows = std::max(want_rows, bound);
+                    // (the items of a pair in flight when its first
+                    // max_candidates + 2 rows are there add to them)
+                    want_rows = std::max(want_rows, free_chunk ? std::min(budget, 2 * bound) : bound);
                 } else if (Sc > 1) {
                     // with the chunk's own lists in memory its bound no
                     // longer fits: take fewer structures before searching
@@ -1566,6 +1656,9 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 dm.resume = nullptr;
                 dm.n_resume = 0;
                 dm.pool_in = nullptr;
+                // units, heavy pairs, their items, (scratch, large units,) spilled entries
+                unsigned long long free_n[6] = {};
+                FreeWork fw{};
                 Suspended *next_out = d_susp_a.p, *spare = d_susp_b.p;
                 unsigned char *pool_next = d_pool_a.p, *pool_spare = d_pool_b.p;
                 for (int round = 0;; round++) {
@@ -1578,8 +1671,25 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         CUDA_TRY(cudaMemsetAsync(d_pool_used.p, 0, sizeof(unsigned long long), st));
                     }
                     CUDA_TRY(cudaEventRecord(ev[6], st));
-                    CUDA_TRY(launch_search(st, grid, wide, fp32, cv, tv, cd, sa, d_pair_counter.p, scn_c, cr,
-                                           d_counters.p, dm));
+                    if (round == 0 && free_chunk) {
+                        CUDA_TRY(dalloc(d_units, (size_t)c_cap, st));
+                        CUDA_TRY(dalloc(d_heavy_pairs, (size_t)n_pairs, st));
+                        CUDA_TRY(dalloc(d_free_n, 6, st));
+                        CUDA_TRY(cudaMemsetAsync(d_free_n.p, 0, 6 * sizeof(unsigned long long), st));
+                        fw.item_seeds = P->max_candidates >= 0 ? FREE_ITEM_CUT : FREE_ITEM;
+                        fw.scratch_used = d_free_n.p + 3;
+                        fw.n_large_units = d_free_n.p + 4;
+                        fw.n_spilled = d_free_n.p + 5;
+                        fw.units = d_units.p;
+                        fw.n_units = d_free_n.p;
+                        fw.heavy = d_heavy_pairs.p;
+                        fw.n_heavy = d_free_n.p + 1;
+                        CUDA_TRY(launch_search_free(st, fp32, cv, tv, cd, fv, sa, d_pair_counter.p, scn_c, cr,
+                                                    d_counters.p, dm, fw));
+                    } else {
+                        CUDA_TRY(launch_search(st, grid, wide, fp32, cv, tv, cd, sa, d_pair_counter.p, scn_c, cr,
+                                               d_counters.p, dm));
+                    }
                     launches++;
                     if (round == 0 && !tp->large.empty()) {
                         // pairs of templates over 32 atoms (every list of
@@ -1592,19 +1702,116 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(cudaEventRecord(ev[7], st));
                     CUDA_TRY(cudaGetLastError());
                     unsigned long long ns = 0, used = 0;
-                    CUDA_TRY(cudaMemcpyAsync(&nc, d_ccount.p, sizeof nc, cudaMemcpyDeviceToHost, st));
-                    if (dm.state) {
-                        CUDA_TRY(cudaMemcpyAsync(&ns, d_nsusp.p, sizeof ns, cudaMemcpyDeviceToHost, st));
-                        CUDA_TRY(cudaMemcpyAsync(&used, d_leaf_used.p, sizeof used, cudaMemcpyDeviceToHost, st));
-                    }
-                    CUDA_TRY(cudaStreamSynchronize(st));
-                    {
+                    auto read_back = [&]() -> cudaError_t {
+                        cudaError_t e = cudaMemcpyAsync(&nc, d_ccount.p, sizeof nc, cudaMemcpyDeviceToHost, st);
+                        if (e == cudaSuccess && dm.state) {
+                            e = cudaMemcpyAsync(&ns, d_nsusp.p, sizeof ns, cudaMemcpyDeviceToHost, st);
+                            if (e == cudaSuccess)
+                                e = cudaMemcpyAsync(&used, d_leaf_used.p, sizeof used, cudaMemcpyDeviceToHost, st);
+                        }
+                        if (e == cudaSuccess && round == 0 && free_chunk)
+                            e = cudaMemcpyAsync(free_n, d_free_n.p, sizeof free_n, cudaMemcpyDeviceToHost, st);
+                        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
                         float m = 0.f;
-                        cudaEventElapsedTime(&m, ev[6], ev[7]);
+                        if (e == cudaSuccess) e = cudaEventElapsedTime(&m, ev[6], ev[7]);
                         ms_search += m;
-                    }
+                        return e;
+                    };
+                    CUDA_TRY(read_back());
                     search_rounds++;
-                    if (ns == 0) break;
+                    if (round == 0 && free_chunk && (free_n[1] || ns)) {
+                        // level-0 lists, in candidate order, of the pairs taken
+                        // in items and of those left to k_search
+                        launch_candidates(st, fill_blocks, true, cv, sv, nullptr, nullptr, d_offset.p, d_cand_atom.p,
+                                          dm.fill_work, dm.n_fill, nullptr, false);
+                        launches++;
+                    }
+                    if (round == 0 && free_chunk && free_n[1]) {
+                        // the heavy pairs in items of seeds, block 0
+                        // of every pair first
+                        const int32_t nh = (int32_t)free_n[1];
+                        const int64_t ni = (int64_t)free_n[2];
+                        const int64_t nbins = (sp->max_atoms + fw.item_seeds - 1) / fw.item_seeds;
+                        if (ni > INT32_MAX) {
+                            status = fail(PJG_ERR_CAPACITY, "too many items in one chunk");
+                            goto done;
+                        }
+                        int64_t warps = 0;
+                        CUDA_TRY(heavy_warps(fp32, ni, &warps));
+                        CUDA_TRY(dalloc(d_bins, 2 * (size_t)nbins, st));
+                        CUDA_TRY(dalloc(d_bin_off, (size_t)nbins, st));
+                        CUDA_TRY(dalloc(d_items, (size_t)ni, st));
+                        CUDA_TRY(dalloc(d_results, (size_t)ni, st));
+                        CUDA_TRY(dalloc(d_item_base, (size_t)ni, st));
+                        CUDA_TRY(dalloc(d_item_head, (size_t)ni, st));
+                        CUDA_TRY(dalloc(d_item_branch, (size_t)ni, st));
+                        CUDA_TRY(dalloc(d_spill_a, SPILL_CAP, st));
+                        CUDA_TRY(dalloc(d_heavy_stats, 4 * (size_t)nh, st));
+                        CUDA_TRY(dalloc(d_arena_xyz, (size_t)warps * HEAVY_CAP, st));
+                        CUDA_TRY(dalloc(d_arena_atom, (size_t)warps * HEAVY_CAP, st));
+                        CUDA_TRY(dalloc(d_arena_parent, 2 * (size_t)warps * HEAVY_CAP, st));
+                        CUDA_TRY(cudaMemsetAsync(d_bins.p, 0, 2 * (size_t)nbins * sizeof(int32_t), st));
+                        CUDA_TRY(cudaMemsetAsync(d_results.p, 0xFF, (size_t)ni * sizeof(int2), st));
+                        CUDA_TRY(cudaMemsetAsync(d_item_head.p, 0xFF, (size_t)ni * sizeof(int32_t), st));
+                        CUDA_TRY(cudaMemsetAsync(d_item_branch.p, 0, (size_t)ni * sizeof(uint32_t), st));
+                        CUDA_TRY(cudaMemsetAsync(d_heavy_stats.p, 0, 4 * (size_t)nh * sizeof(unsigned long long), st));
+                        CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
+                        launch_heavy_bins(st, nh, d_heavy_pairs.p, d_bins.p);
+                        CUDA_TRY(scan_exclusive(d_bins.p, nbins, d_bin_off.p, scan_tmp, st));
+                        launch_heavy_items(st, nh, d_heavy_pairs.p, d_bin_off.p, d_bins.p + nbins, d_items.p);
+                        fw.items = d_items.p;
+                        fw.n_items = (int32_t)ni;
+                        fw.results = d_results.p;
+                        fw.heavy_stats = d_heavy_stats.p;
+                        fw.item_base = d_item_base.p;
+                        fw.arena_xyz = d_arena_xyz.p;
+                        fw.arena_atom = d_arena_atom.p;
+                        fw.arena_parent = d_arena_parent.p;
+                        fw.item_head = d_item_head.p;
+                        fw.item_branch = d_item_branch.p;
+                        fw.spilled_out = d_spill_a.p;
+                        fw.spill_cap = SPILL_CAP;
+                        CUDA_TRY(cudaEventRecord(ev[6], st));
+                        CUDA_TRY(launch_search_heavy(st, fp32, warps, cv, tv, cd, fv, sa, d_pair_counter.p, cr,
+                                                     d_counters.p, dm, fw));
+                        CUDA_TRY(cudaEventRecord(ev[7], st));
+                        launches += 3;
+                        CUDA_TRY(cudaGetLastError());
+                        CUDA_TRY(read_back());
+                        // entries whose children outgrew the frontier, level
+                        // by level at most as deep as a template
+                        for (int pass = 0; free_n[5] > 0; pass++) {
+                            if (pass > 40) {
+                                status = fail(PJG_ERR_CAPACITY, "spilled entries did not converge");
+                                goto done;
+                            }
+                            fw.n_items = (int32_t)free_n[5];
+                            if (pass > 0) std::swap(d_spill_a, d_spill_b);
+                            CUDA_TRY(dalloc(d_spill_b, SPILL_CAP, st));
+                            fw.spilled_in = d_spill_a.p;
+                            fw.spilled_out = d_spill_b.p;
+                            CUDA_TRY(cudaMemsetAsync(fw.n_spilled, 0, sizeof(unsigned long long), st));
+                            CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
+                            CUDA_TRY(heavy_warps(fp32, fw.n_items, &warps));
+                            CUDA_TRY(dalloc(d_arena_xyz, (size_t)warps * HEAVY_CAP, st));
+                            CUDA_TRY(dalloc(d_arena_atom, (size_t)warps * HEAVY_CAP, st));
+                            CUDA_TRY(dalloc(d_arena_parent, 2 * (size_t)warps * HEAVY_CAP, st));
+                            fw.arena_xyz = d_arena_xyz.p;
+                            fw.arena_atom = d_arena_atom.p;
+                            fw.arena_parent = d_arena_parent.p;
+                            CUDA_TRY(cudaEventRecord(ev[6], st));
+                            CUDA_TRY(launch_search_heavy(st, fp32, warps, cv, tv, cd, fv, sa, d_pair_counter.p, cr,
+                                                         d_counters.p, dm, fw));
+                            CUDA_TRY(cudaEventRecord(ev[7], st));
+                            launches++;
+                            CUDA_TRY(cudaGetLastError());
+                            CUDA_TRY(read_back());
+                        }
+                        launch_heavy_rows(st, nh, fw, d_item_base.p, d_pair_rows.p, d_counters.p);
+                        launches++;
+                        CUDA_TRY(cudaGetLastError());
+                    }
+                    if (ns == 0 && (!free_chunk || (int64_t)used <= leaf_filled)) break;
                     if (round > 80) {
                         status = fail(PJG_ERR_CAPACITY, "leaf order on demand did not converge");
                         goto done;
@@ -1614,13 +1821,30 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(ensure_leaf((int64_t)used));
                     CUDA_TRY(order_requested());
                     leaf_filled = (int64_t)used;
+                    if (ns == 0) break;
                     dm.resume = next_out;
                     dm.n_resume = (int32_t)ns;
                     dm.pool_in = pool_next;
                     std::swap(next_out, spare);
                     std::swap(pool_next, pool_spare);
                 }
-                if ((int64_t)nc <= c_cap) break;
+                if ((int64_t)nc <= c_cap) {
+                    if (free_chunk && free_n[0]) {
+                        // the rows found without order, in the reference's
+                        if (free_n[1]) {
+                            CUDA_TRY(dalloc(d_row_key, (size_t)nc, st));
+                            CUDA_TRY(dalloc(d_row_scratch, 5 * (size_t)nc, st));
+                            CUDA_TRY(dalloc(d_large_units, (size_t)free_n[0], st));
+                            fw.row_key = d_row_key.p;
+                            fw.row_scratch = d_row_scratch.p;
+                            fw.large_units = d_large_units.p;
+                        }
+                        launch_unit_order(st, (int64_t)free_n[0], cv, tv, cd, sv, sp->d_res_place, P->reorder, fw, cr);
+                        launches++;
+                        CUDA_TRY(cudaGetLastError());
+                    }
+                    break;
+                }
                 // the row buffer was too small: grow and run the chunk again
                 // (the search counters of the failed attempt are rolled back;
                 // lists ordered meanwhile stay ordered).  Rows beyond the
@@ -1704,10 +1928,17 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     RowResults rr{d_off_q.p, T, d_r_rmsd.p, d_r_nan.p, d_r_rot.p, d_r_cen.p, d_r_src.p};
                     int blocks = (int)std::min<int64_t>((rows + 127) / 128, (int64_t)sm_count() * 24);
                     launch_superpose(st, blocks, cv, tv, cr, rr);
-                    CUDA_TRY(cudaMemsetAsync(d_rtotals.p, 0, 4 * sizeof(unsigned long long), st));
+                    CUDA_TRY(dalloc(d_long_pairs, (size_t)std::min<int64_t>(n_pairs, rows), st));
+                    CUDA_TRY(cudaMemsetAsync(d_rtotals.p, 0, 5 * sizeof(unsigned long long), st));
+                    if (free_chunk) {
+                        // (rows of a pair that k_search took over have no slot)
+                        CUDA_TRY(cudaMemsetAsync(d_r_hit.p, 0, (size_t)rows * sizeof(int32_t), st));
+                        CUDA_TRY(cudaMemsetAsync(d_r_warn.p, 0, (size_t)rows * sizeof(int32_t), st));
+                        CUDA_TRY(cudaMemsetAsync(d_r_hatoms.p, 0, (size_t)rows * sizeof(int32_t), st));
+                    }
                     launch_automaton(st, n_pairs, T, tp->d_atom_begin, d_cnt_q.p, d_off_q.p, rr, P->max_candidates,
                                      P->best_match, P->rmsd_threshold, d_r_hit.p, d_r_warn.p, d_r_hatoms.p,
-                                     d_rtotals.p);
+                                     d_rtotals.p, d_long_pairs.p, d_rtotals.p + 4);
                     CUDA_TRY(scan_exclusive(d_r_hit.p, rows, d_r_hidx.p, scan_tmp, st));
                     CUDA_TRY(scan_exclusive(d_r_warn.p, rows, d_r_widx.p, scan_tmp, st));
                     CUDA_TRY(scan_exclusive(d_r_hatoms.p, rows, d_r_aidx.p, scan_tmp, st));
@@ -1730,7 +1961,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         hs.atoms += (int64_t)tot[2];
                         hs.warns += (int64_t)tot[1];
                     }
-                    launches += 8;
+                    launches += 9;
                 }
                 CUDA_TRY(cudaEventRecord(ev[4], st));
                 float m1 = 0, m2 = 0, m3 = 0;
@@ -1809,6 +2040,12 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
 
 done:
     if (st) {
+        dfree(d_sig_bits, st); dfree(d_units, st); dfree(d_heavy_pairs, st); dfree(d_free_n, st);
+        dfree(d_heavy_stats, st); dfree(d_row_key, st); dfree(d_items, st); dfree(d_results, st);
+        dfree(d_item_base, st); dfree(d_bin_off, st); dfree(d_bins, st); dfree(d_arena_atom, st);
+        dfree(d_row_scratch, st); dfree(d_arena_xyz, st); dfree(d_arena_parent, st); dfree(d_item_head, st);
+        dfree(d_large_units, st); dfree(d_long_pairs, st); dfree(d_item_branch, st); dfree(d_spill_a, st);
+        dfree(d_spill_b, st);
         dfree(d_params, st); dfree(d_count, st); dfree(d_scanned, st); dfree(d_cand_atom, st);
         dfree(d_leaf_atom, st); dfree(d_pair_counter, st); dfree(d_offset, st); dfree(d_totals, st);
         dfree(d_leaf_xyz, st); dfree(d_leaf_atom2, st); dfree(d_leaf_xyz2, st); dfree(d_leaf_off, st);

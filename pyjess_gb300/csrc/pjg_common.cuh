@@ -123,6 +123,26 @@ struct CandView {
     const float4 *blk_hi;           //   consecutive leaves (FP32)
 };
 
+// What the order-free search reads instead of candidate lists.  A kind is a
+// distinct (residue name, atom name) of the structure set; whether an atom
+// joins a signature's list depends on its kind alone.  A structure's local
+// kinds are its distinct names in the nh_* arrays of ChunkView.
+struct FreeView {
+    int32_t n_kinds;
+    int32_t kind_words;             // 32-bit words of a signature's kind bits
+    const uint32_t *kind_name;      // [n_kinds]
+    const uint32_t *kind_res;
+    const uint32_t *sig_bits;       // [G * kind_words] kinds of each signature's list
+    const int32_t *nh_kind;         // kind of each nh_* entry (global index)
+    const float4 *kxyz;             // xyz32 in nh_pos order
+    // atoms by residue: sorted by key (residue number, chainID2), so the
+    // atoms of one residue, and of one residue number, are contiguous
+    const int32_t *res_pos;         // atom at each position (structure-local)
+    const uint16_t *res_kind;       // its local kind
+    const int4 *res_range;          // per atom: first position and count of its
+                                    // key, then of its residue number
+};
+
 // Counters accumulated by the kernels (int64, device).
 enum Counter : int {
     C_PAIRS = 0,

@@ -22,12 +22,19 @@
 //   k_leaf_sorted<M>    kd leaf order by sorted-axis splits, with a qselect
 //                       replay of tied nodes
 //   k_leaf_exact<M>     the literal qselect sequence, for the rest
+//   k_sig_kinds         atom kinds each signature's list takes
+//   k_search_free       every pair without any order (two instances: whole
+//                       pairs, items of seeds of heavy pairs)
+//   k_unit_order, k_unit_order_large
+//                       the rows found without order put in the reference's
 //   k_search            persistent warp per pair, order-preserving
-//                       depth-first-over-tiles frontier expansion
+//                       depth-first-over-tiles frontier expansion: the plain
+//                       mode, explicit leaf levels, and the few pairs the
+//                       order-free search leaves
 //                       (k_search_large: templates over 32 atoms)
 //   k_superpose         thread per complete row, FP64 covariance and
 //                       quaternion eigen-solve
-//   k_order_counts, k_automaton, k_gather_hits
+//   k_order_counts, k_automaton, k_automaton_long, k_gather_hits
 //                       Query.__next__ per pair and compaction of the hits
 //
 // FP64 arithmetic that decides a hit is written with __dadd_rn/__dsub_rn/
@@ -1495,7 +1502,7 @@ __global__ void k_leaf_exact(ChunkView cv, int32_t n_sigs, const int32_t *count,
     for (int64_t i = warp; i < total; i += nwarps) {
         const int64_t w = exact_list[i];
         const int m = count[w];
-        if (m <= MINN || (m > MAXN && MAXN != EXACT_MAX)) continue;
+        if (m <= MINN || (m > MAXN && MAXN != EXACT_LONG)) continue;
         const int s = (int)(w / n_sigs);
         const int64_t o = offset[w];
         const int64_t lo = leaf_offset[w];
@@ -1525,7 +1532,8 @@ __global__ void k_leaf_exact(ChunkView cv, int32_t n_sigs, const int32_t *count,
             st_n[0] = m;
             st_ax[0] = 0;
             // small subtrees collected for the lanes: (lo, n, axis) packed
-            uint32_t small_mine[8];
+            constexpr int SMALL = MAXN / 16 / 32;  // (a subtree has at least 16 points)
+            uint32_t small_mine[SMALL];
             int n_small_mine = 0, n_small = 0;
             while (sp > 0) {
                 sp--;
@@ -1533,10 +1541,10 @@ __global__ void k_leaf_exact(ChunkView cv, int32_t n_sigs, const int32_t *count,
                 if (n <= 1) continue;
                 if (n <= 32) {
                     // lane (n_small % 32) replays this subtree later
-                    if ((n_small & 31) == lane && n_small_mine < 8)
+                    if ((n_small & 31) == lane && n_small_mine < SMALL)
                         small_mine[n_small_mine++] = (uint32_t)lo | ((uint32_t)n << 16) | ((uint32_t)ax << 24);
                     // children of nodes above 32 points have at least 16, so a
-                    // list of EXACT_MAX points has at most 256 such subtrees
+                    // list of MAXN points has at most MAXN / 16 such subtrees
                     n_small++;
                     continue;
                 }
@@ -1599,7 +1607,7 @@ __global__ void k_leaf_exact(ChunkView cv, int32_t n_sigs, const int32_t *count,
                 }
             }
             __syncwarp();
-            if (n_small > 256 && lane == 0) atomicMax(&counters[C_ERROR], 4ull);
+            if (n_small > 32 * SMALL && lane == 0) atomicMax(&counters[C_ERROR], 4ull);
             for (int r = lane; r < m; r += 32) {
                 int e = S.A[m - 1 - r];
                 leaf_atom[lo + r] = ca[e];
@@ -1633,9 +1641,15 @@ __device__ __forceinline__ unsigned long long order_key(double x) {
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
+// a packed (residue number, chainID2) key in the order of its signed value
+__device__ __forceinline__ unsigned long long residue_key(int32_t k) {
+    return (unsigned long long)((uint32_t)k ^ 0x80000000u);
+}
+
 __global__ void __launch_bounds__(RANK_THREADS)
     k_axis_ranks(const int64_t *atom_base, const int32_t *atom_count, const double *xyz64, int64_t n_atoms,
-                 unsigned long long *tile_key, uint16_t *tile_idx, uint32_t *lrank, uint32_t *urank) {
+                 unsigned long long *tile_key, uint16_t *tile_idx, uint32_t *lrank, uint32_t *urank,
+                 ResidueOrder ro) {
     __shared__ unsigned long long key[RANK_TILE];
     __shared__ uint16_t idx[RANK_TILE];
     const int s = blockIdx.x, a = blockIdx.y;
@@ -1644,11 +1658,15 @@ __global__ void __launch_bounds__(RANK_THREADS)
     const int tiles = (n + RANK_TILE - 1) / RANK_TILE;
     unsigned long long *gk = tile_key + a * n_atoms + b0;
     uint16_t *gi = tile_idx + a * n_atoms + b0;
+    // sort key of atom i: its coordinate, or (a == 3) its residue key
+    auto key_of = [&](int i) -> unsigned long long {
+        return a < 3 ? order_key(xyz64[3 * (b0 + i) + a]) : residue_key(__float_as_int(ro.xyz32[b0 + i].w));
+    };
     for (int t = 0; t < tiles; t++) {
         const int t0 = t * RANK_TILE, tn = min(RANK_TILE, n - t0);
         for (int i = threadIdx.x; i < RANK_TILE; i += blockDim.x) {
             if (i < tn) {
-                key[i] = order_key(xyz64[3 * (b0 + t0 + i) + a]);
+                key[i] = key_of(t0 + i);
             } else {
                 key[i] = ~0ull;
             }
@@ -1682,8 +1700,13 @@ __global__ void __launch_bounds__(RANK_THREADS)
         }
         __syncthreads();
     }
+    if (a == 3)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            ro.kxyz[b0 + i] = ro.xyz32[b0 + ro.nh_pos[b0 + i]];
+            ro.res_place[b0 + ro.sorted[b0 + i]] = i;
+        }
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const unsigned long long ki = order_key(xyz64[3 * (b0 + i) + a]);
+        const unsigned long long ki = key_of(i);
         const int ti = i / RANK_TILE;
         const uint16_t li = (uint16_t)(i % RANK_TILE);
         uint32_t lr = 0, ur = 0;
@@ -1718,8 +1741,31 @@ __global__ void __launch_bounds__(RANK_THREADS)
                 ur += lo;
             }
         }
-        lrank[a * n_atoms + b0 + i] = lr;
-        urank[a * n_atoms + b0 + i] = ur;
+        if (a < 3) {
+            lrank[a * n_atoms + b0 + i] = lr;
+            urank[a * n_atoms + b0 + i] = ur;
+        } else {
+            // positions below k over the sorted tiles
+            auto below = [&](unsigned long long k) -> int {
+                int acc = 0;
+                for (int t = 0; t < tiles; t++) {
+                    const unsigned long long *tk = gk + t * RANK_TILE;
+                    int lo = 0, hi = min(RANK_TILE, n - t * RANK_TILE);
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (tk[mid] < k) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    acc += lo;
+                }
+                return acc;
+            };
+            const unsigned long long seq = ki & ~0xFFull;  // first key of the residue number
+            const int r0 = below(seq);
+            ro.res_pos[b0 + ur] = i;
+            ro.res_kind[b0 + ur] = ro.local_kind[b0 + i];
+            ro.res_range[b0 + i] = make_int4((int)lr, below(ki + 1) - (int)lr, r0, below(seq + 256) - r0);
+        }
     }
 }
 
@@ -3906,6 +3952,1029 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Order-free search: warp per (structure, template) pair.
+//
+// The reference's output order (kd leaf order inside every level) only
+// decides the order of a pair's complete rows, and 89% of the pairs of a
+// database search have one row or none; yet putting the lists in that order
+// and walking them is what a search in order spends its time on.  So every
+// pair is searched without any order (the partial assignments of each level
+// are the same set, so the counters are the reference's too), and afterwards
+// the rows of a pair are put in order by the leaf ranks of their atoms, at
+// the levels where rows with the same atoms before them differ
+// (k_unit_order): only those levels' lists are ever put in leaf order.
+//
+// Without an order a level's candidates need no list:
+//   - a template atom of a residue that an earlier level already placed: the
+//     atoms of that residue of the structure (about 8) whose kind the
+//     signature takes, instead of the whole list (about 110 points);
+//   - otherwise the list's atoms, gathered from the structure's atoms
+//     grouped by kind (kxyz: contiguous points), 32 candidates in registers
+//     against every parent in turn.
+// The levels are expanded breadth first, every entry kept until the rows are
+// written (rows are the last level's entries, their atoms the parent chain).
+//
+// Two instances.  The first takes every pair whole, its frontier in shared
+// memory; a pair with more than FREE_CAP / 2 seeds or FREE_CAP entries is
+// passed to the second, which takes pairs in items of fw.item_seeds seeds
+// (consecutive in candidate order, so the items' rows follow each other),
+// many warps a pair, frontiers in global memory; there a level whose
+// children outgrow HEAVY_CAP is expanded some parents at a time, each
+// slice's subtree to its rows before the next (the rows then come in several
+// segments).  Left to k_search: one-atom templates, a single entry with more
+// children than HEAVY_CAP has room for, and points whose decision needs the
+// kd-tree (outside an annulus box by rounding).
+//
+// Bound by issue slots.  Measured on 1,000 structures x 4,000 templates:
+// 68 ms for both instances and 9 ms for the rows' order, with 0.84 M lists put
+// in leaf order; the search in order took 214 ms with 12.6 M lists ordered
+// (whole query 398 -> 131 ms).
+
+template <int CAP>
+struct FreeState {
+    float4 xyz[CAP];            // frontier entries of every level: point and key,
+    int32_t atom[CAP];          //   atom, parent entry
+    uint16_t parent[CAP];
+    uint16_t first[CAP];        // a child that leads to a row (0xFFFF: none)
+    float4 thr[32];             // annulus bounds of the new level to each earlier one
+    int4 rule[32];              // residue / chain rule to it: key bits that must be
+                                //   equal (x), that must differ somewhere (y; z = 1: no such bits)
+    int32_t order[32], tkey[32], sig[32];
+    uint32_t mask[FREE_MAX_KINDS / 32];  // local kinds of the new level's signature
+    int32_t cq[64];             // queued candidates: kxyz or residue-order positions
+    uint16_t pq[64];            //   their parents (residue candidates)
+};
+
+// check_pair as two bit masks over the XOR of two structure keys
+__device__ __forceinline__ int4 residue_rule(int32_t tj, int32_t tn, int ignore) {
+    const bool chain = ((tj ^ tn) & 0xFF) == 0, res = ((tj ^ tn) >> 8) == 0;
+    if (ignore == 0 && !chain) return make_int4(0, 0xFF, 0, 0);
+    if (ignore == 0) return res ? make_int4(-1, 0, 1, 0) : make_int4(0xFF, ~0xFF, 0, 0);
+    if (!res) return make_int4(0, ~0xFF, 0, 0);
+    return ignore == 1 ? make_int4(-1, 0, 1, 0) : make_int4(~0xFF, 0, 1, 0);
+}
+
+// FP64 decision on the levels of `exact` for candidate atom `an` of parent
+// entry p: 0 outside an annulus, 1 inside every one, 2 inside, but outside an
+// annulus box (the kd-tree decides)
+__device__ __noinline__ int free_decide(const int32_t *eatom, const uint16_t *eparent, const int32_t *order,
+                                        unsigned exact, int lev, int p, int32_t an, const double *xyz,
+                                        const AnnulusParam *prm, int n, int qn) {
+    int verdict = 1;
+    for (int j = lev; j >= 0; j--, p = eparent[p]) {
+        if (!((exact >> j) & 1u)) continue;
+        bool inb;
+        if (!annulus64(xyz + 3 * (int64_t)eatom[p], xyz + 3 * (int64_t)an, prm[order[j] * n + qn], &inb)) return 0;
+        if (!inb) verdict = 2;
+    }
+    return verdict;
+}
+
+__global__ void k_sig_kinds(SigView sv, FreeView fv, uint32_t *sig_bits) {
+    const int lane = lane_id();
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t total = (int64_t)sv.n_sigs * fv.kind_words;
+    for (int64_t w = warp; w < total; w += nwarps) {
+        const int g = (int)(w / fv.kind_words);
+        const int k = (int)(w % fv.kind_words) * 32 + lane;
+        bool ok = false;
+        if (k < fv.n_kinds) {
+            const int code = sv.code[g];
+            const uint32_t res = fv.kind_res[k];
+            ok = (code < -1 || code > 8 || in_list(res, sv.resnames, sv.res_begin[g], sv.res_begin[g + 1])) &&
+                 sig_match(sv, g, sv.rule[g], fv.kind_name[k], res);
+        }
+        const unsigned m = __ballot_sync(FULL_MASK, ok);
+        if (lane == 0) sig_bits[w] = m;
+    }
+}
+
+// level order of a pair: this lane's place (stable by list length c)
+__device__ __forceinline__ int level_rank(int n, int c, int reorder) {
+    const int lane = lane_id();
+    if (!reorder) return lane;
+    int rank = 0;
+    for (int j = 0; j < n; j++) {
+        const int cj = __shfl_sync(FULL_MASK, c, j);
+        rank += (cj < c || (cj == c && j < lane)) ? 1 : 0;
+    }
+    return rank;
+}
+
+template <bool FP32, bool HEAVY>
+__global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
+    k_search_free(ChunkView cv, TemplateView tv, CandView cd, FreeView fv, SearchArgs sa, int32_t *item_counter,
+                  const int32_t *scanned, CompleteRows out, unsigned long long *counters, LeafDemand dm,
+                  FreeWork fw) {
+    extern __shared__ __align__(16) unsigned char free_smem[];
+    constexpr int CAP = HEAVY ? HEAVY_CAP : FREE_CAP;
+    using State = FreeState<HEAVY ? 1 : FREE_CAP>;
+    const int lane = lane_id();
+    const unsigned lt = (1u << lane) - 1u;
+    State &st = reinterpret_cast<State *>(free_smem)[threadIdx.x >> 5];
+    const int T = tv.n_templates, G = cd.n_sigs;
+    const int64_t slot = HEAVY ? (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * HEAVY_CAP : 0;
+    float4 *const exyz = HEAVY ? fw.arena_xyz + slot : st.xyz;
+    int32_t *const eatom = HEAVY ? fw.arena_atom + slot : st.atom;
+    uint16_t *const eparent = HEAVY ? fw.arena_parent + 2 * slot : st.parent;
+    uint16_t *const efirst = HEAVY ? fw.arena_parent + 2 * slot + HEAVY_CAP : st.first;
+    // each lane sums its own share of the counters; added up at exit
+    unsigned long long a_pairs = 0, a_cand = 0, a_bcand = 0, a_part = 0, a_comp = 0, a_bexp = 0, a_rech = 0;
+    uint64_t t_start = 0;
+    if (lane == 0) t_start = global_ns();
+    bool timed_out = false;
+    const int n_items = HEAVY ? fw.n_items : sa.n_pairs;
+    int g_next = 0, g_end = 0;
+    while (!timed_out) {
+        if (g_next >= g_end) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(item_counter, sa.pair_grain);
+            g_next = __shfl_sync(FULL_MASK, base, 0);
+            g_end = g_next + sa.pair_grain;
+        }
+        const int item = g_next++;
+        if (item >= n_items) break;
+        HeavyPair hp{};
+        int hidx = -1, blk = 0;
+        const SpilledEntry *sub = nullptr;  // this item: the subtree below one spilled entry
+        if (HEAVY) {
+            if (fw.spilled_in) {
+                sub = fw.spilled_in + item;
+                hidx = sub->heavy;
+                blk = sub->block;
+            } else {
+                const int2 it = fw.items[item];
+                hidx = it.x;
+                blk = it.y;
+            }
+            hp = fw.heavy[hidx];
+            if (hp.failed) continue;
+        }
+        const int pair = HEAVY ? hp.pair : item;
+        const int s = pair / T, t = pair % T;
+        const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
+        if (n <= 0 || n > 32) continue;  // (over 32 atoms: k_search_large)
+        const int64_t abase = cv.atom_base[s];
+        const int64_t wb = (int64_t)s * G;
+
+        // rows of a pair past the max_candidates cut are not wanted: an item
+        // is skipped once the finished items before it hold max_candidates + 2
+        // rows (best_match), or, right before it, that many rows without a
+        // hit among them, or one of them ended the stream
+        if (HEAVY && !sub && sa.max_candidates >= 0 && blk > 0) {
+            const volatile int2 *res = fw.results + hp.first;
+            long long sum = 0;
+            bool end = false;
+            for (int x0 = ((blk - 1) / 32) * 32; x0 >= 0; x0 -= 32) {
+                const int x = x0 + lane;
+                int r = -1, f = 0;
+                if (x < blk) {
+                    r = res[x].x;
+                    f = res[x].y;
+                }
+                const bool done = x < blk && r >= 0;
+                end |= __any_sync(FULL_MASK, done && (f & 2));
+                // the run of finished items without hits that ends at blk - 1
+                // (best_match: every finished item)
+                unsigned use = __ballot_sync(FULL_MASK, done);
+                bool more = true;
+                if (!sa.best_match) {
+                    const unsigned brk = __ballot_sync(FULL_MASK, x < blk && !(done && !(f & 1)));
+                    if (brk) {
+                        use = 31 - __clz(brk) == 31 ? 0u : use & ~((2u << (31 - __clz(brk))) - 1u);
+                        more = false;
+                    }
+                }
+                long long v = (use >> lane) & 1u ? r : 0;
+                for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
+                sum += v;
+                if (!more) break;
+            }
+            if (end || sum >= (long long)sa.max_candidates + 2) {
+                if (lane == 0) fw.results[hp.first + blk] = make_int2(0, 2);
+                continue;
+            }
+        }
+
+        // ---- list lengths, empty lists, statistics
+        int c = INT_MAX, sg = 0;
+        if (lane < n) {
+            sg = tv.sig[ab + lane];
+            c = cd.count[wb + sg];
+        }
+        if (!HEAVY) {
+            const unsigned zero = __ballot_sync(FULL_MASK, lane < n && c == 0);
+            if (lane == 0) a_pairs++;
+            if (lane < n && lane <= (zero ? __ffs(zero) - 1 : n - 1)) {
+                a_bcand += 8ull * scanned[wb + sg] + 16ull * c;
+                a_cand += c;
+            }
+            if (zero) continue;
+        }
+        const int rank = level_rank(n, c, sa.reorder);
+        __syncwarp();
+        if (lane < n) {
+            st.order[rank] = lane;
+            st.sig[rank] = sg;
+            st.tkey[rank] = tv.key[ab + lane];
+        }
+        __syncwarp();
+        // this lane's level: its list and length
+        const int64_t lw = lane < n ? wb + st.sig[lane] : 0;
+        const int llen = __shfl_sync(FULL_MASK, c, lane < n ? st.order[lane] : 0);
+        const AnnulusParam *prm = tv.params + tv.param_begin[t];
+        const double *xyz64 = cv.xyz64 + 3 * abase;
+        const float4 *kx = fv.kxyz + abase;
+        const int q0 = cv.nh_begin[cv.bucket_begin[s]];
+        const int nk = cv.nh_begin[cv.bucket_begin[s + 1]] - q0;  // local kinds
+        const int m0 = __shfl_sync(FULL_MASK, llen, 0);
+
+        // local kinds 32 w .. 32 w + 31 that the list of signature g takes
+        auto kind_bits = [&](int g, int w) -> unsigned {
+            const int q = 32 * w + lane;
+            bool ok = false;
+            if (q < nk) {
+                const int k = fv.nh_kind[q0 + q];
+                ok = (fv.sig_bits[(int64_t)g * fv.kind_words + (k >> 5)] >> (k & 31)) & 1u;
+            }
+            return __ballot_sync(FULL_MASK, ok);
+        };
+
+        bool kd_needed = n == 1;  // (the one-level scanner drops its first candidate: k_search)
+        bool outgrown = !HEAVY && m0 > CAP / 2;
+        int rows = 0, any_hit = 0;
+        // rows written: last segment, its levels at which rows part, segments
+        int seg = -1, seg0 = -1, n_seg = 0;
+        bool spilled = false;
+        unsigned branch = 0;
+        long long F = 0;  // lane l: partial assignments of level l
+        unsigned long long rech = 0;
+        // lane l: entries of level l, the next one to expand, most to expand at once
+        int lbeg = 0, lend = 0, lcur = 0, lmax = CAP;
+        int top = 0, lev = -1;
+        if (HEAVY && sub) {
+            // the entry's chain, one entry a level, all but the last expanded
+            lev = sub->level;
+            if (lane <= lev) {
+                const int32_t a = sub->atom[lane];
+                exyz[lane] = cv.xyz32[abase + a];
+                eatom[lane] = a;
+                eparent[lane] = (uint16_t)(lane > 0 ? lane - 1 : 0);
+                lbeg = lane;
+                lend = lane + 1;
+                lcur = lane < lev ? lane + 1 : lane;
+            }
+            top = lev + 1;
+            __syncwarp();
+        } else if (!kd_needed && !outgrown) {
+            // ---- seeds
+            const int s0 = HEAVY ? blk * fw.item_seeds : 0;
+            const int k0 = HEAVY ? min(fw.item_seeds, m0 - s0) : m0;
+            if (HEAVY) {
+                const int32_t *ca = cd.cand_atom + cd.offset[__shfl_sync(FULL_MASK, lw, 0)] + s0;
+                for (int e = lane; e < k0; e += 32) {
+                    const int32_t a = ca[e];
+                    exyz[e] = cv.xyz32[abase + a];
+                    eatom[e] = a;
+                    eparent[e] = 0;
+                }
+            } else {
+                int at = 0;
+                for (int w = 0; 32 * w < nk && at < k0; w++) {
+                    unsigned bits = kind_bits(st.sig[0], w);
+                    int cnt = 0, off = 0;
+                    if ((bits >> lane) & 1u) {
+                        cnt = cv.nh_count[q0 + 32 * w + lane];
+                        off = cv.nh_off[q0 + 32 * w + lane];
+                    }
+                    while (bits) {
+                        const int b = __ffs(bits) - 1;
+                        bits &= bits - 1;
+                        const int cb = __shfl_sync(FULL_MASK, cnt, b), ob = __shfl_sync(FULL_MASK, off, b);
+                        for (int i = lane; i < cb; i += 32) {
+                            if (at + i >= k0) break;
+                            exyz[at + i] = kx[ob + i];
+                            eatom[at + i] = cv.nh_pos[abase + ob + i];
+                            eparent[at + i] = 0;
+                        }
+                        at += cb;
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) {
+                lend = k0;
+                F = k0;
+            }
+            top = k0;
+            lev = 0;
+        }
+        while (lev >= 0 && !kd_needed && !outgrown) {
+            const int beg = __shfl_sync(FULL_MASK, lcur, lev), lev_end = __shfl_sync(FULL_MASK, lend, lev);
+            if (beg >= lev_end) {
+                // level done: its entries are no longer needed
+                if (!HEAVY) break;  // (the only path down has reached its rows)
+                top = __shfl_sync(FULL_MASK, lbeg, lev);
+                lev--;
+                continue;
+            }
+            if (HEAVY) {
+                int over = 0;
+                if (lane == 0) over = (global_ns() - t_start) > sa.budget_ns;
+                if (__shfl_sync(FULL_MASK, over, 0)) break;
+            }
+            const int end = min(lev_end, beg + __shfl_sync(FULL_MASK, lmax, lev));
+            bool full = false;
+            long long Fc = 0;
+            unsigned long long crech = 0;
+            int nend = top;  // children are appended at the top
+            {
+                const int child = lev + 1;
+                const int qn = st.order[child], g = st.sig[child];
+                int4 myrule = make_int4(0, 0, 1, 0);
+                __syncwarp();
+                if (lane <= lev) {
+                    st.thr[lane] = prm[st.order[lane] * n + qn].thr;
+                    myrule = residue_rule(st.tkey[lane], st.tkey[child], sa.ignore_chain);
+                    st.rule[lane] = myrule;
+                }
+                // the deepest level whose atom shares the new atom's residue
+                const unsigned same = __ballot_sync(FULL_MASK, lane <= lev && (myrule.x & ~0xFF) != 0);
+                __syncwarp();
+                // the lanes' tests at one chain entry
+                auto test = [&](const float4 &e, const float4 &x, const int4 &r, const float4 &th, int j,
+                                unsigned &exact) -> bool {
+                    const int32_t d = __float_as_int(e.w) ^ __float_as_int(x.w);
+                    const float dx = e.x - x.x, dy = e.y - x.y, dz = e.z - x.z;
+                    const float d2 = dx * dx + dy * dy + dz * dz;
+                    const bool ok = (d & r.x) == 0 && ((d & r.y) | r.z) != 0 && !(d2 < th.x || d2 > th.w);
+                    if (!FP32 || !(d2 >= th.y && d2 <= th.z)) exact |= 1u << j;
+                    return ok;
+                };
+                // candidates that passed: inconclusive ones decided in FP64,
+                // the others appended as children
+                auto accept = [&](bool pass, unsigned exact, int p, int32_t an, const float4 &x) {
+                    if (__any_sync(FULL_MASK, pass && exact)) {
+                        int v = 1;
+                        if (pass && exact) {
+                            if (FP32) crech += __popc(exact);
+                            v = free_decide(eatom, eparent, st.order, exact, lev, p, an, xyz64, prm, n, qn);
+                            pass = v != 0;
+                        }
+                        if (__any_sync(FULL_MASK, v == 2)) kd_needed = true;
+                    }
+                    const unsigned m = __ballot_sync(FULL_MASK, pass);
+                    const int np = __popc(m);
+                    if (lane == child) Fc += np;
+                    if (nend + np > CAP) {
+                        full = true;
+                    } else {
+                        if (pass) {
+                            const int e = nend + __popc(m & lt);
+                            exyz[e] = x;
+                            eatom[e] = an;
+                            eparent[e] = (uint16_t)p;
+                        }
+                        nend += np;
+                    }
+                };
+                if (same) {
+                    // ---- the atoms of the placed residue
+                    const int anchor = 31 - __clz(same);
+                    const bool by_number = sa.ignore_chain == 2;
+                    for (int w = 0; 32 * w < nk; w++) {
+                        const unsigned bits = kind_bits(g, w);
+                        if (lane == 0) st.mask[w] = bits;
+                    }
+                    __syncwarp();
+                    int queued = 0;
+                    auto run_batch = [&](int k) {
+                        bool pass = lane < k;
+                        unsigned exact = 0;
+                        const int p = pass ? st.pq[lane] : 0;
+                        int32_t an = 0;
+                        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (pass) {
+                            an = fv.res_pos[abase + st.cq[lane]];
+                            x = cv.xyz32[abase + an];
+                            for (int j = lev, e = p; j >= 0; j--, e = eparent[e])
+                                if (!test(exyz[e], x, st.rule[j], st.thr[j], j, exact)) {
+                                    pass = false;
+                                    break;
+                                }
+                        }
+                        accept(pass, exact, p, an, x);
+                        const int rest = queued - k;
+                        int qc = 0;
+                        uint16_t qp = 0;
+                        if (lane < rest) {
+                            qc = st.cq[k + lane];
+                            qp = st.pq[k + lane];
+                        }
+                        __syncwarp();
+                        if (lane < rest) {
+                            st.cq[lane] = qc;
+                            st.pq[lane] = qp;
+                        }
+                        __syncwarp();
+                        queued = rest;
+                    };
+                    for (int p0 = beg; p0 < end && !full && !kd_needed; p0 += 32) {
+                        const int p = p0 + lane;
+                        int first = 0, cnt = 0;
+                        if (p < end) {
+                            int e = p;
+                            for (int j = lev; j > anchor; j--) e = eparent[e];
+                            const int4 r = fv.res_range[abase + eatom[e]];
+                            first = by_number ? r.z : r.x;
+                            cnt = by_number ? r.w : r.y;
+                        }
+                        const int most = __reduce_max_sync(FULL_MASK, cnt);
+                        for (int i = 0; i < most && !full && !kd_needed; i++) {
+                            bool match = false;
+                            if (i < cnt) {
+                                const int lk = fv.res_kind[abase + first + i];
+                                match = (st.mask[lk >> 5] >> (lk & 31)) & 1u;
+                            }
+                            const unsigned m = __ballot_sync(FULL_MASK, match);
+                            if (match) {
+                                const int qi = queued + __popc(m & lt);
+                                st.cq[qi] = first + i;
+                                st.pq[qi] = (uint16_t)p;
+                            }
+                            queued += __popc(m);
+                            __syncwarp();
+                            if (queued >= 32) run_batch(32);
+                        }
+                    }
+                    if (queued > 0 && !full && !kd_needed) run_batch(queued);
+                } else {
+                    // ---- the whole list, 32 candidates against every parent
+                    const float4 thr_p = st.thr[lev];
+                    const int4 rule_p = st.rule[lev];
+                    int queued = 0;
+                    auto run_batch = [&](int k) {
+                        const int ci = lane < k ? st.cq[lane] : 0;
+                        const float4 x = lane < k ? kx[ci] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        int32_t an = -1;
+                        for (int p = beg; p < end && !full && !kd_needed; p++) {
+                            unsigned exact = 0;
+                            bool pass = lane < k && test(exyz[p], x, rule_p, thr_p, lev, exact);
+                            if (!__any_sync(FULL_MASK, pass)) continue;
+                            int e = p;
+                            for (int j = lev - 1; j >= 0; j--) {
+                                e = eparent[e];
+                                pass = pass && test(exyz[e], x, st.rule[j], st.thr[j], j, exact);
+                                if (!__any_sync(FULL_MASK, pass)) break;
+                            }
+                            if (!__any_sync(FULL_MASK, pass)) continue;
+                            if (an < 0 && lane < k) an = cv.nh_pos[abase + ci];
+                            accept(pass, exact, p, an, x);
+                        }
+                        const int rest = queued - k;
+                        const int qc = lane < rest ? st.cq[k + lane] : 0;
+                        __syncwarp();
+                        if (lane < rest) st.cq[lane] = qc;
+                        __syncwarp();
+                        queued = rest;
+                    };
+                    for (int w = 0; 32 * w < nk && !full && !kd_needed; w++) {
+                        unsigned bits = kind_bits(g, w);
+                        int cnt = 0, off = 0;
+                        if ((bits >> lane) & 1u) {
+                            cnt = cv.nh_count[q0 + 32 * w + lane];
+                            off = cv.nh_off[q0 + 32 * w + lane];
+                        }
+                        while (bits && !full && !kd_needed) {
+                            const int b = __ffs(bits) - 1;
+                            bits &= bits - 1;
+                            const int cb = __shfl_sync(FULL_MASK, cnt, b), ob = __shfl_sync(FULL_MASK, off, b);
+                            for (int i0 = 0; i0 < cb && !full && !kd_needed; i0 += 32) {
+                                const int k = min(32, cb - i0);
+                                if (lane < k) st.cq[queued + lane] = ob + i0 + lane;
+                                queued += k;
+                                __syncwarp();
+                                if (queued >= 32) run_batch(32);
+                            }
+                        }
+                    }
+                    if (queued > 0 && !full && !kd_needed) run_batch(queued);
+                }
+                __syncwarp();
+            }
+            if (kd_needed) break;
+            if (full) {
+                // the whole pair in items; the level's parents as items of
+                // their own (a later launch), or, without room to keep them,
+                // the same parents again, fewer at a time
+                if (!HEAVY) {
+                    outgrown = true;
+                    continue;
+                }
+                if (end - beg == 1) {
+                    kd_needed = true;
+                    continue;
+                }
+                const int np = lev_end - beg;
+                unsigned long long at = ~0ull;
+                if (lane == 0) {
+                    unsigned long long was = *fw.n_spilled, seen;
+                    while (was + np <= (unsigned long long)fw.spill_cap &&
+                           (seen = atomicCAS(fw.n_spilled, was, was + np)) != was)
+                        was = seen;
+                    if (was + np <= (unsigned long long)fw.spill_cap) at = was;
+                }
+                at = __shfl_sync(FULL_MASK, at, 0);
+                if (at != ~0ull) {
+                    for (int i = lane; i < np; i += 32) {
+                        SpilledEntry &r = fw.spilled_out[at + i];
+                        r.heavy = hidx;
+                        r.block = blk;
+                        r.level = lev;
+                        for (int j = lev, e = beg + i; j >= 0; j--, e = eparent[e]) r.atom[j] = eatom[e];
+                    }
+                    __syncwarp();
+                    if (lane == lev) lcur = lend;
+                    spilled = true;
+                } else if (lane == lev) {
+                    lmax = (end - beg) / 2;
+                }
+                continue;
+            }
+            F += Fc;
+            rech += crech;
+            if (lane == lev) lcur = end;
+            if (lev + 1 < n - 1) {
+                if (nend > top) {
+                    lev++;
+                    if (lane == lev) {
+                        lbeg = lcur = top;
+                        lend = nend;
+                    }
+                    top = nend;
+                }
+                continue;
+            }
+            const int crows = nend - top;
+            if (crows == 0) continue;
+            // ---- rows: entries top .. nend - 1 of the last level
+            if (crows > 1) {
+                // levels at which rows with the same atoms before differ
+                for (int e = lane; e < top; e += 32) efirst[e] = 0xFFFF;
+                __syncwarp();
+                for (int l = n - 1; l >= 1; l--) {
+                    const int e0 = l == n - 1 ? top : __shfl_sync(FULL_MASK, lbeg, l);
+                    const int e1 = l == n - 1 ? nend : __shfl_sync(FULL_MASK, lend, l);
+                    for (int e = e0 + lane; e < e1; e += 32)
+                        if (l == n - 1 || efirst[e] != 0xFFFF) efirst[eparent[e]] = (uint16_t)e;
+                    __syncwarp();
+                    bool other = false;
+                    for (int e = e0 + lane; e < e1; e += 32)
+                        if (l == n - 1 || efirst[e] != 0xFFFF) other |= efirst[eparent[e]] != (uint16_t)e;
+                    if (__any_sync(FULL_MASK, other)) branch |= 1u << l;
+                }
+                int live = 0;
+                const int seeds = __shfl_sync(FULL_MASK, lend, 0);
+                for (int e = lane; e < seeds; e += 32) live += efirst[e] != 0xFFFF ? 1 : 0;
+                if (__reduce_add_sync(FULL_MASK, live) > 1) branch |= 1u;
+            }
+            int64_t rb = 0;
+            int ui = -1;
+            if (lane == 0) {
+                rb = (int64_t)atomicAdd(out.count, (unsigned long long)crows);
+                if (HEAVY || crows > 1) ui = (int)atomicAdd(fw.n_units, 1ull);
+            }
+            rb = __shfl_sync(FULL_MASK, rb, 0);
+            const bool room = rb + crows <= out.capacity;
+            if (lane == 0 && ui >= 0 && room && ui < out.capacity) {
+                RowUnit u;
+                u.row_base = rb;
+                u.pair = pair;
+                u.count = crows;
+                u.heavy = hidx;
+                u.item = HEAVY ? hp.first + blk : -1;
+                u.next = seg;
+                u.branch = 0;
+                fw.units[ui] = u;
+            }
+            seg = __shfl_sync(FULL_MASK, ui, 0);
+            if (n_seg++ == 0) seg0 = seg;
+            int hits = 0;
+            for (int i0 = 0; i0 < crows && room; i0 += 32) {
+                const int i = i0 + lane;
+                bool hit = false;
+                if (i < crows) {
+                    int32_t *dst = out.atoms + (rb + i) * out.stride;
+                    for (int j = n - 1, e = top + i; j >= 0; j--, e = eparent[e]) dst[st.order[j]] = eatom[e];
+                    out.pair[rb + i] = pair;
+                    out.ordinal[rb + i] = 0;
+                    if (out.rmsd) {
+                        double rm = -1.0;  // (one item: no cut to decide here)
+                        if (HEAVY) {
+                            rm = lane_rmsd(n, dst, xyz64, tv.pos + 3 * (int64_t)ab);
+                            hit = rm <= sa.rmsd_threshold && n >= 3;
+                        }
+                        out.rmsd[rb + i] = rm;
+                    }
+                }
+                if (HEAVY) hits += __popc(__ballot_sync(FULL_MASK, hit));
+            }
+            rows += crows;
+            any_hit |= hits > 0 || !room;
+            __syncwarp();
+        }
+        if (!kd_needed && !outgrown && rows > 0) {
+            // rows in several segments part anywhere
+            if (n_seg > 1 || spilled || sub) branch = n == 32 ? ~0u : (1u << n) - 1u;
+            request_list_warp(dm, lane >= 1 && lane < n && ((branch >> lane) & 1u), lw, llen);
+        }
+        if (!HEAVY) {
+            if (lane == 0 && seg >= 0 && seg < out.capacity) fw.units[seg].branch = branch;
+        } else if (lane == 0 && seg >= 0) {
+            // the item's segments in one list (its spilled entries add theirs)
+            const int it = hp.first + blk;
+            const int before = atomicExch(&fw.item_head[it], seg);
+            if (seg0 < out.capacity) fw.units[seg0].next = before;
+            atomicOr(&fw.item_branch[it], branch);
+        }
+        // rows without a hit among them that end the stream by themselves
+        const bool ended = HEAVY && !sub && !spilled && sa.max_candidates >= 0 && rows >= sa.max_candidates + 2ll &&
+                           (sa.best_match || !any_hit);
+        if (!HEAVY && outgrown && !kd_needed) {
+            // in items of seeds, its level-0 list in candidate order
+            request_fill_warp(dm, lane == 0, lw);
+            if (lane == 0) {
+                HeavyPair h;
+                h.pair = pair;
+                h.blocks = (m0 + fw.item_seeds - 1) / fw.item_seeds;
+                h.first = (int32_t)atomicAdd(fw.n_heavy + 1, (unsigned long long)h.blocks);
+                h.failed = 0;
+                fw.heavy[atomicAdd(fw.n_heavy, 1ull)] = h;
+            }
+        } else {
+            if (kd_needed) {
+                // every list in kd leaf order (level 0 in candidate order), then k_search
+                int won = 1;
+                if (HEAVY) {
+                    if (lane == 0) won = atomicExch(&fw.heavy[hidx].failed, 1) == 0;
+                    won = __shfl_sync(FULL_MASK, won, 0);
+                }
+                if (won) {
+                    request_fill_warp(dm, lane == 0, lw);
+                    request_list_warp(dm, lane > 0 && lane < n, lw, llen);
+                    if (lane == 0) {
+                        Suspended sp;
+                        sp.pair = pair;
+                        sp.pad = 0;
+                        sp.skip = 0;
+                        sp.state = -1;
+                        dm.suspended[atomicAdd(dm.n_suspended, 1ull)] = sp;
+                    }
+                }
+            }
+            if (!kd_needed || HEAVY) {
+                const long long Fp = __shfl_up_sync(FULL_MASK, F, 1);
+                const unsigned long long bexp =
+                    lane >= 1 && lane < n ? (unsigned long long)(4LL * lane * Fp + (4LL * (lane + 1) + 16) * F) : 0ull;
+                if (HEAVY) {
+                    // per pair: counted unless another item hands the pair to k_search
+                    auto add = [&](int k, unsigned long long v) {
+                        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
+                        if (lane == 0 && v) atomicAdd(&fw.heavy_stats[4 * (int64_t)hidx + k], v);
+                    };
+                    add(0, (unsigned long long)F);
+                    add(1, lane == n - 1 ? (unsigned long long)F : 0ull);
+                    add(2, bexp);
+                    add(3, rech);
+                    if (lane == 0 && sub) atomicAdd(&fw.results[hp.first + blk].x, rows);
+                    if (lane == 0 && !sub)
+                        fw.results[hp.first + blk] = make_int2(rows, (any_hit || spilled ? 1 : 0) | (ended ? 2 : 0));
+                } else {
+                    if (lane == 0 && rows > 0) out.pair_rows[pair] = rows;
+                    a_part += (unsigned long long)F;
+                    if (lane == n - 1) a_comp += (unsigned long long)F;
+                    a_bexp += bexp;
+                    a_rech += rech;
+                }
+            }
+        }
+        int over = 0;
+        if (lane == 0) over = (global_ns() - t_start) > sa.budget_ns;
+        if (__shfl_sync(FULL_MASK, over, 0)) {
+            timed_out = true;
+            if (lane == 0) atomicMax(&counters[C_ERROR], 3ull);
+        }
+        __syncwarp();
+    }
+    if (HEAVY) return;
+    auto add = [&](int which, unsigned long long v) {
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
+        if (lane == 0 && v) atomicAdd(&counters[which], v);
+    };
+    add(C_PAIRS, a_pairs);
+    add(C_CAND, a_cand);
+    add(C_BYTES_CAND, a_bcand);
+    add(C_PARTIALS, a_part);
+    add(C_COMPLETE, a_comp);
+    add(C_BYTES_EXP, a_bexp);
+    add(C_RECHECK, a_rech);
+}
+
+// Items of the pairs in `heavy`: block 0 of every pair, then block 1, ... (so
+// that a pair's earlier items are finished when a later one asks whether it
+// is still wanted).  Pass 1 counts the pairs that have a block b, pass 2
+// (after a scan of the counts) writes the items.
+__global__ void k_heavy_bins(int32_t n_heavy, const HeavyPair *heavy, int32_t *bins) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_heavy; i += gridDim.x * blockDim.x)
+        for (int b = 0; b < heavy[i].blocks; b++) atomicAdd(&bins[b], 1);
+}
+
+__global__ void k_heavy_items(int32_t n_heavy, const HeavyPair *heavy, const int64_t *bin_begin, int32_t *bin_fill,
+                              int2 *items) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_heavy; i += gridDim.x * blockDim.x)
+        for (int b = 0; b < heavy[i].blocks; b++)
+            items[bin_begin[b] + atomicAdd(&bin_fill[b], 1)] = make_int2(i, b);
+}
+
+// Warp per heavy pair: rows before each of its items, the pair's rows and
+// its share of the counters (a pair handed to k_search counts there).
+__global__ void k_heavy_rows(int32_t n_heavy, const HeavyPair *heavy, const int2 *results, int64_t *item_base,
+                             const unsigned long long *heavy_stats, int32_t *pair_rows,
+                             unsigned long long *counters) {
+    const int lane = lane_id();
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    unsigned long long sum = 0;
+    for (int i = warp; i < n_heavy; i += nwarps) {
+        const HeavyPair h = heavy[i];
+        if (h.failed) continue;
+        long long carry = 0;
+        for (int b0 = 0; b0 < h.blocks; b0 += 32) {
+            const int b = b0 + lane;
+            const long long r = b < h.blocks ? max(results[h.first + b].x, 0) : 0;
+            long long incl = r;
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long y = __shfl_up_sync(FULL_MASK, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (b < h.blocks) item_base[h.first + b] = carry + incl - r;
+            carry += __shfl_sync(FULL_MASK, incl, 31);
+        }
+        if (lane == 0) pair_rows[h.pair] = (int32_t)carry;
+        if (lane < 4) sum += heavy_stats[4 * (int64_t)i + lane];
+    }
+    if (lane < 4 && sum)
+        atomicAdd(&counters[lane == 0 ? C_PARTIALS : lane == 1 ? C_COMPLETE : lane == 2 ? C_BYTES_EXP : C_RECHECK],
+                  sum);
+}
+
+// The places of a unit's rows (a pair's, or an item's) in the pair's stream.
+// A row's key is its seed's place in candidate order, then the leaf rank of
+// its atom at every level where rows part (ascending); rows are told apart
+// level by level.  Units of at most UNIT_ROWS rows: a warp each, every row
+// counting the rows with smaller keys; larger ones are listed for
+// k_unit_order_large.
+constexpr int UNIT_ROWS = 192;   // rows whose keys shared memory holds
+constexpr int UNIT_SLOTS = 512;  // hash slots for the atoms of that many rows
+constexpr int UNIT_WARPS = 4;
+constexpr int UNIT_HASH_FROM = 9;  // fewer rows are compared with every leaf
+constexpr int UNIT_LARGE_THREADS = 512;
+
+struct UnitWarp {
+    unsigned long long key[UNIT_ROWS];
+    int32_t cur[UNIT_ROWS], atom[UNIT_ROWS], row[UNIT_ROWS];
+    int32_t slot_atom[UNIT_SLOTS], slot_rank[UNIT_SLOTS];
+    int32_t order[32], sig[32];
+};
+
+// place of atom a in the candidate list of signature g: residue names in the
+// signature's order, then ResIndex order (codes outside -1..8: molecule order)
+__device__ __forceinline__ unsigned long long candidate_place(const ChunkView &cv, const SigView &sv,
+                                                              const int32_t *res_place, int g, int64_t abase,
+                                                              int32_t a) {
+    const int code = sv.code[g];
+    if (code < -1 || code > 8) return (unsigned long long)a;
+    const uint32_t rn = cv.resname[abase + a];
+    int ri = sv.res_begin[g];
+    while (ri < sv.res_begin[g + 1] && sv.resnames[ri] != rn) ri++;
+    return ((unsigned long long)(ri - sv.res_begin[g]) << 32) | (uint32_t)res_place[abase + a];
+}
+
+__global__ void __launch_bounds__(UNIT_WARPS * 32)
+    k_unit_order(ChunkView cv, TemplateView tv, CandView cd, SigView sv, const int32_t *res_place, int32_t reorder,
+                 FreeWork fw, CompleteRows out) {
+    __shared__ UnitWarp sh[UNIT_WARPS];
+    UnitWarp &U = sh[threadIdx.x >> 5];
+    const int lane = lane_id();
+    const int T = tv.n_templates, G = cd.n_sigs;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t total = (int64_t)*fw.n_units;
+    for (int64_t w = warp; w < total; w += nwarps) {
+        const RowUnit u = fw.units[w];
+        if (u.heavy >= 0 && fw.heavy[u.heavy].failed) {
+            for (int i = lane; i < u.count; i += 32) out.pair[u.row_base + i] = -1;  // k_search's rows count
+            continue;
+        }
+        // (a segment that does not lead its unit's list is not a unit)
+        if (u.item >= 0 && fw.item_head[u.item] != (int)w) continue;
+        const int R = u.item >= 0 ? fw.results[u.item].x : u.count;
+        if (R > UNIT_ROWS) {
+            if (lane == 0) fw.large_units[atomicAdd(fw.n_large_units, 1ull)] = (int32_t)w;
+            continue;
+        }
+        const int64_t ord0 = u.item >= 0 ? fw.item_base[u.item] : 0;
+        if (R == 1) {
+            if (lane == 0) out.ordinal[u.row_base] = ord0;
+            continue;
+        }
+        const int s = u.pair / T, t = u.pair % T;
+        const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
+        const int64_t abase = cv.atom_base[s], wb = (int64_t)s * G;
+        int c = INT_MAX, sg = 0;
+        if (lane < n) {
+            sg = tv.sig[ab + lane];
+            c = cd.count[wb + sg];
+        }
+        const int rank = level_rank(n, c, reorder);
+        __syncwarp();
+        if (lane < n) {
+            U.order[rank] = lane;
+            U.sig[rank] = sg;
+        }
+        int at = 0;
+        for (int q = (int)w; q >= 0;) {
+            const RowUnit v = fw.units[q];
+            for (int i = lane; i < v.count; i += 32) U.row[at + i] = (int32_t)(v.row_base + i);
+            at += v.count;
+            q = u.item >= 0 ? v.next : -1;
+        }
+        for (int i = lane; i < R; i += 32) U.cur[i] = 0;
+        __syncwarp();
+        for (unsigned left = u.item >= 0 ? fw.item_branch[u.item] : u.branch; left; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const int k = U.order[l], g = U.sig[l];
+            if (l == 0) {
+                for (int i = lane; i < R; i += 32)
+                    U.key[i] = candidate_place(cv, sv, res_place, g, abase,
+                                               out.atoms[(int64_t)U.row[i] * out.stride + k]);
+            } else {
+                const int m = cd.count[wb + g];
+                const int32_t *la = cd.leaf_atom + cd.leaf_offset[wb + g];
+                const bool hash = R >= UNIT_HASH_FROM;
+                if (hash)
+                    for (int q = lane; q < UNIT_SLOTS; q += 32) U.slot_atom[q] = -1;
+                __syncwarp();
+                auto slot_of = [&](int32_t a) -> int { return (int)(((uint32_t)a * 0x9E3779B1u) >> 23); };
+                static_assert(UNIT_SLOTS == 1 << 9, "slot_of keeps nine bits");
+                for (int i = lane; i < R; i += 32) {
+                    const int32_t a = out.atoms[(int64_t)U.row[i] * out.stride + k];
+                    U.atom[i] = a;
+                    U.key[i] = (unsigned long long)(uint32_t)U.cur[i] << 32;
+                    if (hash)
+                        for (int q = slot_of(a);; q = (q + 1) & (UNIT_SLOTS - 1)) {
+                            const int32_t was = atomicCAS(&U.slot_atom[q], -1, a);
+                            if (was == -1 || was == a) break;
+                        }
+                }
+                __syncwarp();
+                for (int k0 = 0; k0 < m; k0 += 32) {
+                    const int32_t a = k0 + lane < m ? la[k0 + lane] : -2;
+                    if (hash) {
+                        if (a >= 0)
+                            for (int q = slot_of(a);; q = (q + 1) & (UNIT_SLOTS - 1)) {
+                                const int32_t was = U.slot_atom[q];
+                                if (was == a) U.slot_rank[q] = k0 + lane;
+                                if (was == a || was == -1) break;
+                            }
+                    } else {
+                        for (int i = 0; i < R; i++) {
+                            const unsigned f = __ballot_sync(FULL_MASK, a == U.atom[i]);
+                            if (f && lane == 0) U.key[i] |= (unsigned long long)(k0 + __ffs(f) - 1);
+                        }
+                    }
+                }
+                __syncwarp();
+                if (hash)
+                    for (int i = lane; i < R; i += 32) {
+                        int q = slot_of(U.atom[i]);
+                        while (U.slot_atom[q] != U.atom[i]) q = (q + 1) & (UNIT_SLOTS - 1);
+                        U.key[i] |= (unsigned long long)U.slot_rank[q];
+                    }
+            }
+            __syncwarp();
+            for (int i = lane; i < R; i += 32) {
+                const unsigned long long mine = U.key[i];
+                int before = 0;
+                for (int j = 0; j < R; j++) before += U.key[j] < mine ? 1 : 0;
+                U.cur[i] = before;
+            }
+            __syncwarp();
+        }
+        for (int i = lane; i < R; i += 32) out.ordinal[U.row[i]] = ord0 + U.cur[i];
+        __syncwarp();
+    }
+}
+
+// Block per unit of more rows (a seed of a flexible template can have
+// thousands): the rows kept sorted as far as the levels taken tell them
+// apart, row[p] at position p of class cls[p] (the position where its class
+// begins), so a level compares a row with its own class only.
+__global__ void __launch_bounds__(UNIT_LARGE_THREADS)
+    k_unit_order_large(ChunkView cv, TemplateView tv, CandView cd, SigView sv, const int32_t *res_place,
+                       int32_t reorder, FreeWork fw, CompleteRows out) {
+    __shared__ int32_t order[32], sig[32], leaf[UNIT_LARGE_THREADS];
+    __shared__ long long region;
+    const int T = tv.n_templates, G = cd.n_sigs, tid = threadIdx.x;
+    const int64_t total = (int64_t)*fw.n_large_units;
+    for (int64_t x = blockIdx.x; x < total; x += gridDim.x) {
+        const int head = fw.large_units[x];
+        const RowUnit u = fw.units[head];
+        const int R = u.item >= 0 ? fw.results[u.item].x : u.count;
+        const int64_t ord0 = u.item >= 0 ? fw.item_base[u.item] : 0;
+        const int s = u.pair / T, t = u.pair % T;
+        const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
+        const int64_t abase = cv.atom_base[s], wb = (int64_t)s * G;
+        __syncthreads();
+        if (tid < 32) {
+            int c = INT_MAX, sg = 0;
+            if (tid < n) {
+                sg = tv.sig[ab + tid];
+                c = cd.count[wb + sg];
+            }
+            const int rank = level_rank(n, c, reorder);
+            if (tid < n) {
+                order[rank] = tid;
+                sig[rank] = sg;
+            }
+            if (tid == 0) region = (long long)atomicAdd(fw.scratch_used, (unsigned long long)R);
+        }
+        __syncthreads();
+        unsigned long long *key = fw.row_key + region;
+        int32_t *row = fw.row_scratch + 5 * region, *cls = row + R, *row2 = row + 2 * (int64_t)R,
+                *cls2 = row + 3 * (int64_t)R, *fill = row + 4 * (int64_t)R;
+        int at = 0;
+        for (int q = head; q >= 0;) {
+            const RowUnit v = fw.units[q];
+            for (int i = tid; i < v.count; i += blockDim.x) {
+                row[at + i] = (int32_t)(v.row_base + i);
+                cls[at + i] = 0;
+            }
+            at += v.count;
+            q = u.item >= 0 ? v.next : -1;
+        }
+        __syncthreads();
+        for (unsigned left = u.item >= 0 ? fw.item_branch[u.item] : u.branch; left; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const int k = order[l], g = sig[l];
+            const int m = cd.count[wb + g];
+            const int32_t *la = l == 0 ? nullptr : cd.leaf_atom + cd.leaf_offset[wb + g];
+            for (int p = tid; p < R; p += blockDim.x) {
+                const int32_t a = out.atoms[(int64_t)row[p] * out.stride + k];
+                key[p] = l == 0 ? candidate_place(cv, sv, res_place, g, abase, a) : (unsigned long long)(uint32_t)a;
+                fill[p] = 0;
+            }
+            if (l > 0) {
+                // atoms (bit 63 set once replaced) by their leaf ranks, the list
+                // through shared memory
+                for (int k0 = 0; k0 < m; k0 += blockDim.x) {
+                    __syncthreads();
+                    if (k0 + tid < m) leaf[tid] = la[k0 + tid];
+                    __syncthreads();
+                    const int kn = min((int)blockDim.x, m - k0);
+                    for (int p = tid; p < R; p += blockDim.x) {
+                        const unsigned long long a = key[p];
+                        if (a >> 63) continue;
+                        int f = -1;
+                        for (int q = 0; q < kn; q++)
+                            if (leaf[q] == (int32_t)a) f = k0 + q;
+                        if (f >= 0) key[p] = (1ull << 63) | (unsigned long long)f;
+                    }
+                }
+            }
+            __syncthreads();
+            for (int p = tid; p < R; p += blockDim.x) {
+                const int c0 = cls[p];
+                const unsigned long long mine = key[p];
+                int before = 0;
+                for (int q = c0; q < R && cls[q] == c0; q++) before += key[q] < mine ? 1 : 0;
+                const int c1 = c0 + before;
+                const int to = c1 + atomicAdd(&fill[c1], 1);
+                row2[to] = row[p];
+                cls2[to] = c1;
+            }
+            __syncthreads();
+            int32_t *x1 = row, *x2 = cls;
+            row = row2;
+            cls = cls2;
+            row2 = x1;
+            cls2 = x2;
+        }
+        for (int p = tid; p < R; p += blockDim.x) out.ordinal[row[p]] = ord0 + p;
+    }
+}
+
 // Superposition of every complete row, one thread per row (the FP64
 // eigen-solve fills all lanes), written to the row's slot in reference
 // order.
@@ -3917,6 +4986,7 @@ __global__ void k_superpose(ChunkView cv, TemplateView tv, CompleteRows in, RowR
     const int T = tv.n_templates;
     for (int64_t i = tid; i < nrows; i += nthreads) {
         const int pair = in.pair[i];
+        if (pair < 0) continue;  // a row of a pair that k_search took over
         const int s = pair / T, t = pair % T;
         const int ab = tv.atom_begin[t];
         const int n = tv.atom_begin[t + 1] - ab;
@@ -3928,7 +4998,7 @@ __global__ void k_superpose(ChunkView cv, TemplateView tv, CompleteRows in, RowR
         quaternion_fit(S, E0, n, &rmsd, R, &bad);
         // rows whose rmsd already decided the max_candidates cut keep it, so
         // the automaton replays the same decisions
-        if (in.rmsd) rmsd = in.rmsd[i];
+        if (in.rmsd && in.rmsd[i] >= 0.0) rmsd = in.rmsd[i];
         const int64_t d = out.off_q[(int64_t)s * T + (T - 1 - t)] + in.ordinal[i];
         out.rmsd[d] = rmsd;
         out.nan_rot[d] = bad ? 1 : 0;
@@ -3949,24 +5019,35 @@ __global__ void k_order_counts(int64_t n_pairs, int32_t T, const int32_t *pair_r
     cnt_q[q] = pair_rows[s * T + t];
 }
 
-// Query.__next__ (src/pyjess/_jess.pyx:2197-2283) in closed form, one
-// thread per pair, over the pair's rows that pass the rmsd threshold:
+// Query.__next__ (src/pyjess/_jess.pyx:2197-2283) in closed form, over a
+// pair's rows that pass the rmsd threshold:
 //  best_match: over rows with ordinal <= M+1 (M = max_candidates), the
 //    first strict minimum is the hit; a row with an undefined rotation that
 //    would have lowered the minimum raises a warning instead.
 //  otherwise: every passing row is a hit (an undefined rotation: a
 //    warning), but the template's stream ends at the first row whose
 //    ordinal is M+1 past the previous hit (or the template start).
+// A pair of at most AUTOMATON_LANE_ROWS rows by one thread; longer ones are
+// listed for k_automaton_long, a warp each, 32 rows a step (dense pairs have
+// tens of thousands of rows: 60 pairs of 5,000 rows took one thread each
+// 12.3 ms).
+constexpr int AUTOMATON_LANE_ROWS = 16;
+
 __global__ void k_automaton(int64_t n_pairs, int32_t T, const int32_t *atom_begin, const int32_t *cnt_q,
                             const int64_t *off_q, RowResults rr, int32_t M, int32_t best, double thr, int32_t *hit,
-                            int32_t *warn, int32_t *hit_atoms, unsigned long long *totals) {
+                            int32_t *warn, int32_t *hit_atoms, unsigned long long *totals, int32_t *long_pairs,
+                            unsigned long long *n_long) {
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long nh = 0, nw = 0, na = 0, np = 0;
+    int64_t off = 0, cnt = 0;
+    int n = 0;
     if (q < n_pairs) {
         const int t = T - 1 - (int)(q % T);
-        const int n = atom_begin[t + 1] - atom_begin[t];
-        const int64_t off = off_q[q];
-        const int64_t cnt = cnt_q[q];
+        n = atom_begin[t + 1] - atom_begin[t];
+        off = off_q[q];
+        cnt = cnt_q[q];
+    }
+    if (cnt <= AUTOMATON_LANE_ROWS) {
         for (int64_t k = 0; k < cnt; k++) {
             hit[off + k] = 0;
             warn[off + k] = 0;
@@ -4016,6 +5097,113 @@ __global__ void k_automaton(int64_t n_pairs, int32_t T, const int32_t *atom_begi
                 if (M >= 0 && k == base + M + 1) break;
                 if (!nan_rot) base = k + 1;
             }
+        }
+    }
+    if (cnt > AUTOMATON_LANE_ROWS) long_pairs[atomicAdd(n_long, 1ull)] = (int32_t)q;
+    for (int o = 16; o; o >>= 1) {
+        nh += __shfl_xor_sync(FULL_MASK, nh, o);
+        nw += __shfl_xor_sync(FULL_MASK, nw, o);
+        na += __shfl_xor_sync(FULL_MASK, na, o);
+        np += __shfl_xor_sync(FULL_MASK, np, o);
+    }
+    if (lane_id() == 0) {
+        if (nh) atomicAdd(&totals[0], nh);
+        if (nw) atomicAdd(&totals[1], nw);
+        if (na) atomicAdd(&totals[2], na);
+        if (np) atomicAdd(&totals[3], np);
+    }
+}
+
+__global__ void k_automaton_long(int32_t T, const int32_t *atom_begin, const int32_t *cnt_q, const int64_t *off_q,
+                                 RowResults rr, int32_t M, int32_t best, double thr, int32_t *hit, int32_t *warn,
+                                 int32_t *hit_atoms, unsigned long long *totals, const int32_t *long_pairs,
+                                 const unsigned long long *n_long) {
+    const int lane = lane_id();
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t total = (int64_t)*n_long;
+    unsigned long long nh = 0, nw = 0, na = 0, np = 0;
+    for (int64_t w = warp; w < total; w += nwarps) {
+        const int64_t q = long_pairs[w];
+        const int t = T - 1 - (int)(q % T);
+        const int nn = atom_begin[t + 1] - atom_begin[t];
+        const int64_t o = off_q[q], cn = cnt_q[q];
+        int64_t base = 0;       // non-best: row after the last hit
+        double cur = INFINITY;  // best: the minimum so far and its row
+        int64_t b = -1;
+        bool stop = false;
+        for (int64_t k0 = 0; k0 < cn; k0 += 32) {
+            const int64_t k = k0 + lane;
+            const bool valid = k < cn;
+            const double r = valid ? rr.rmsd[o + k] : INFINITY;
+            const bool pass = !stop && valid && r <= thr;
+            const bool nan_rot = pass && rr.nan_rot[o + k] != 0;
+            bool hv = false, wv = false;
+            if (best) {
+                const bool in = pass && (M < 0 || k <= (int64_t)M + 1);
+                // (the first passing row past the cut is counted, then ends it)
+                const unsigned past = __ballot_sync(FULL_MASK, pass && !in);
+                const bool counted = pass && (!past || lane <= __ffs(past) - 1);
+                if (counted) np++;
+                // the minimum before this lane's row, over rows with a rotation
+                double m = in && !nan_rot ? r : INFINITY;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const double y = __shfl_up_sync(FULL_MASK, m, d);
+                    if (lane >= d) m = fmin(m, y);
+                }
+                double ex = __shfl_up_sync(FULL_MASK, m, 1);
+                ex = lane == 0 ? cur : fmin(cur, ex);
+                const bool lowers = in && r < ex;
+                wv = lowers && nan_rot;
+                const unsigned low = __ballot_sync(FULL_MASK, lowers && !nan_rot);
+                if (low) {
+                    const int lastl = 31 - __clz(low);
+                    cur = __shfl_sync(FULL_MASK, r, lastl);
+                    b = k0 + lastl;
+                }
+                if (past) stop = true;
+            } else if (M < 0) {
+                if (pass) np++;
+                hv = pass && !nan_rot;
+                wv = nan_rot;
+            } else {
+                // the passing rows one after the other (the stream may end
+                // at any of them)
+                const unsigned pm = __ballot_sync(FULL_MASK, pass), nm = __ballot_sync(FULL_MASK, nan_rot);
+                for (unsigned left = pm; left && !stop; left &= left - 1) {
+                    const int ln = __ffs(left) - 1;
+                    const int64_t kk = k0 + ln;
+                    if (lane == ln) np++;
+                    if (kk > base + M + 1) {
+                        stop = true;
+                        break;
+                    }
+                    const bool nr = (nm >> ln) & 1u;
+                    if (lane == ln) {
+                        wv = nr;
+                        hv = !nr;
+                    }
+                    if (kk == base + M + 1) stop = true;
+                    if (!nr) base = kk + 1;
+                }
+            }
+            if (valid) {
+                hit[o + k] = hv ? 1 : 0;
+                warn[o + k] = wv ? 1 : 0;
+                hit_atoms[o + k] = hv ? nn : 0;
+            }
+            if (hv) {
+                nh++;
+                na += nn;
+            }
+            if (wv) nw++;
+        }
+        __syncwarp();
+        if (best && b >= 0 && lane == 0) {
+            hit[o + b] = 1;
+            hit_atoms[o + b] = nn;
+            nh++;
+            na += nn;
         }
     }
     for (int o = 16; o; o >>= 1) {
@@ -4213,8 +5401,14 @@ void launch_leaf_order(cudaStream_t st, int blocks, const ChunkView &cv, int32_t
     k_leaf_exact<1024, 0><<<sms * 3, 128, SM1, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom, leaf_offset,
                                                     leaf_atom, leaf_xyz, blk_lo, blk_hi, exact_list, exact_count,
                                                     counters);
-    // longer lists: 64 KB a warp, one warp a block (beyond EXACT_MAX: one
-    // thread replays the list from global memory)
+    // longer lists: 64 KB a warp, one warp a block, then 192 KB (beyond
+    // EXACT_LONG: one thread replays the list from global memory; that took
+    // 35 ms for lists of 5,000 entries)
+    constexpr int SM3 = EXACT_LONG * 16;
+    cudaFuncSetAttribute(k_leaf_exact<EXACT_LONG, EXACT_MAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM3);
+    k_leaf_exact<EXACT_LONG, EXACT_MAX><<<sms, 32, SM3, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom,
+                                                             leaf_offset, leaf_atom, leaf_xyz, blk_lo, blk_hi,
+                                                             exact_list, exact_count, counters);
     constexpr int SM2 = EXACT_MAX * 16;
     cudaFuncSetAttribute(k_leaf_exact<EXACT_MAX, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM2);
     k_leaf_exact<EXACT_MAX, 1024><<<sms * 3, 32, SM2, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom,
@@ -4224,10 +5418,10 @@ void launch_leaf_order(cudaStream_t st, int blocks, const ChunkView &cv, int32_t
 
 void launch_axis_ranks(cudaStream_t st, int32_t n_structures, const int64_t *atom_base, const int32_t *atom_count,
                        const double *xyz64, int64_t n_atoms, unsigned long long *tile_key, uint16_t *tile_idx,
-                       uint32_t *lrank, uint32_t *urank) {
+                       uint32_t *lrank, uint32_t *urank, const ResidueOrder &ro) {
     if (n_structures <= 0) return;
-    k_axis_ranks<<<dim3((unsigned)n_structures, 3), RANK_THREADS, 0, st>>>(atom_base, atom_count, xyz64, n_atoms,
-                                                                          tile_key, tile_idx, lrank, urank);
+    k_axis_ranks<<<dim3((unsigned)n_structures, 4), RANK_THREADS, 0, st>>>(
+        atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, lrank, urank, ro);
 }
 
 void launch_demand_levels(cudaStream_t st, int blocks, const TemplateView &tv, const CandView &cd, int32_t n_pairs,
@@ -4336,6 +5530,87 @@ cudaError_t launch_search(cudaStream_t st, int grid, bool wide, bool fp32, const
     return e;
 }
 
+void launch_sig_kinds(cudaStream_t st, const SigView &sv, const FreeView &fv, uint32_t *sig_bits) {
+    const int64_t warps = (int64_t)sv.n_sigs * fv.kind_words;
+    if (warps > 0)
+        k_sig_kinds<<<(int)std::min<int64_t>((warps + 7) / 8, 152 * 32), 256, 0, st>>>(sv, fv, sig_bits);
+}
+
+// grid of a search_free instance: at most the resident blocks
+static cudaError_t free_grid(const void *kern, int smem, int64_t items, int64_t *grid, int64_t *resident) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0, dev = 0, sms = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, FREE_WARPS * 32, smem);
+    if (e != cudaSuccess) return e;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    *resident = (int64_t)std::max(per_sm, 1) * std::max(sms, 1);
+    *grid = std::max<int64_t>(1, std::min<int64_t>(*resident, (items + FREE_WARPS - 1) / FREE_WARPS));
+    return cudaSuccess;
+}
+
+cudaError_t launch_search_free(cudaStream_t st, bool fp32, const ChunkView &cv, const TemplateView &tv,
+                               const CandView &cd, const FreeView &fv, const SearchArgs &sa, int32_t *item_counter,
+                               const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
+                               const LeafDemand &dm, const FreeWork &fw) {
+    auto kern = fp32 ? k_search_free<true, false> : k_search_free<false, false>;
+    const int smem = (int)sizeof(FreeState<FREE_CAP>) * FREE_WARPS;
+    int64_t grid = 0, resident = 0;
+    cudaError_t e = free_grid((const void *)kern, smem, sa.n_pairs, &grid, &resident);
+    if (e != cudaSuccess) return e;
+    SearchArgs fa = sa;
+    // a pair takes microseconds: several a queue step once every resident
+    // warp has tens of them
+    fa.pair_grain = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, sa.n_pairs / (resident * FREE_WARPS * 16)));
+    kern<<<(int)grid, FREE_WARPS * 32, smem, st>>>(cv, tv, cd, fv, fa, item_counter, scanned, out, counters, dm, fw);
+    return cudaGetLastError();
+}
+
+cudaError_t heavy_warps(bool fp32, int64_t n_items, int64_t *warps) {
+    auto kern = fp32 ? k_search_free<true, true> : k_search_free<false, true>;
+    int64_t grid = 0, resident = 0;
+    cudaError_t e = free_grid((const void *)kern, (int)sizeof(FreeState<1>) * FREE_WARPS, n_items, &grid, &resident);
+    *warps = grid * FREE_WARPS;
+    return e;
+}
+
+cudaError_t launch_search_heavy(cudaStream_t st, bool fp32, int64_t warps, const ChunkView &cv,
+                                const TemplateView &tv, const CandView &cd, const FreeView &fv, const SearchArgs &sa,
+                                int32_t *item_counter, const CompleteRows &out, unsigned long long *counters,
+                                const LeafDemand &dm, const FreeWork &fw) {
+    auto kern = fp32 ? k_search_free<true, true> : k_search_free<false, true>;
+    SearchArgs fa = sa;
+    fa.pair_grain = 1;
+    kern<<<(int)(warps / FREE_WARPS), FREE_WARPS * 32, (int)sizeof(FreeState<1>) * FREE_WARPS, st>>>(
+        cv, tv, cd, fv, fa, item_counter, nullptr, out, counters, dm, fw);
+    return cudaGetLastError();
+}
+
+void launch_heavy_bins(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy, int32_t *bins) {
+    k_heavy_bins<<<(n_heavy + 255) / 256, 256, 0, st>>>(n_heavy, heavy, bins);
+}
+
+void launch_heavy_items(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy, const int64_t *bin_begin,
+                        int32_t *bin_fill, int2 *items) {
+    k_heavy_items<<<(n_heavy + 255) / 256, 256, 0, st>>>(n_heavy, heavy, bin_begin, bin_fill, items);
+}
+
+void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int64_t *item_base, int32_t *pair_rows,
+                       unsigned long long *counters) {
+    k_heavy_rows<<<std::min((n_heavy + 7) / 8, 152 * 8), 256, 0, st>>>(n_heavy, fw.heavy, fw.results, item_base,
+                                                                     fw.heavy_stats, pair_rows, counters);
+}
+
+void launch_unit_order(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
+                       const CandView &cd, const SigView &sv, const int32_t *res_place, int32_t reorder,
+                       const FreeWork &fw, const CompleteRows &out) {
+    const int64_t blocks = std::min<int64_t>((n_units + UNIT_WARPS - 1) / UNIT_WARPS, 152 * 16);
+    k_unit_order<<<(int)blocks, UNIT_WARPS * 32, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
+    if (fw.row_scratch)
+        k_unit_order_large<<<152 * 4, UNIT_LARGE_THREADS, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
+}
+
 cudaError_t launch_search_large(cudaStream_t st, const ChunkView &cv, const TemplateView &tv, const CandView &cd,
                                 const SearchArgs &sa, const int32_t *large, int32_t n_large, int32_t *item_counter,
                                 const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
@@ -4413,11 +5688,14 @@ void launch_order_counts(cudaStream_t st, int64_t n_pairs, int32_t n_templates, 
 void launch_automaton(cudaStream_t st, int64_t n_pairs, int32_t n_templates, const int32_t *atom_begin,
                       const int32_t *cnt_q, const int64_t *off_q, const RowResults &rr, int32_t max_candidates,
                       int32_t best_match, double rmsd_threshold, int32_t *hit, int32_t *warn, int32_t *hit_atoms,
-                      unsigned long long *totals) {
-    if (n_pairs > 0)
-        k_automaton<<<(unsigned)((n_pairs + 127) / 128), 128, 0, st>>>(n_pairs, n_templates, atom_begin, cnt_q,
-                                                                      off_q, rr, max_candidates, best_match,
-                                                                      rmsd_threshold, hit, warn, hit_atoms, totals);
+                      unsigned long long *totals, int32_t *long_pairs, unsigned long long *n_long) {
+    if (n_pairs <= 0) return;
+    k_automaton<<<(unsigned)((n_pairs + 127) / 128), 128, 0, st>>>(
+        n_pairs, n_templates, atom_begin, cnt_q, off_q, rr, max_candidates, best_match, rmsd_threshold, hit, warn,
+        hit_atoms, totals, long_pairs, n_long);
+    k_automaton_long<<<(int)std::min<int64_t>((n_pairs + 3) / 4, 152 * 8), 128, 0, st>>>(
+        n_templates, atom_begin, cnt_q, off_q, rr, max_candidates, best_match, rmsd_threshold, hit, warn, hit_atoms,
+        totals, long_pairs, n_long);
 }
 
 void launch_gather_hits(cudaStream_t st, int64_t n_rows, int32_t n_templates, int32_t structure_base,

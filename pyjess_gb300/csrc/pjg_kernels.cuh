@@ -22,6 +22,25 @@ constexpr int SEARCH_WARPS = PJG_SEARCH_WARPS;  // warps per block of k_search
 #ifndef PJG_SEARCH_MIN_BLOCKS
 #define PJG_SEARCH_MIN_BLOCKS 2
 #endif
+// order-free search: warps per block, resident blocks an SM its registers are
+// sized for, frontier entries a warp holds, most local kinds of a structure
+#ifndef PJG_FREE_WARPS
+#define PJG_FREE_WARPS 8
+#endif
+#ifndef PJG_FREE_MIN_BLOCKS
+#define PJG_FREE_MIN_BLOCKS 3
+#endif
+#ifndef PJG_FREE_CAP
+#define PJG_FREE_CAP 192
+#endif
+constexpr int FREE_WARPS = PJG_FREE_WARPS;
+constexpr int FREE_CAP = PJG_FREE_CAP;
+constexpr int FREE_MAX_KINDS = 1024;
+// seeds of an item of a heavy pair; fewer where max_candidates may make a
+// pair's later items unwanted
+constexpr int FREE_ITEM = 32, FREE_ITEM_CUT = 4;
+constexpr int64_t SPILL_CAP = 1 << 18;  // entries of items kept for a later launch
+constexpr int HEAVY_CAP = 8192;  // frontier entries of an item (16-bit entry numbers)
 // leaves per culling block: k_search tests a parent's join box against the
 // bounding box of each block of CULL_BLK consecutive leaves of a list in kd
 // leaf order, and loads the leaves of the blocks it meets (8, 16 or 32)
@@ -57,7 +76,7 @@ constexpr int LEAF_RANK_MAX = 256;     // default: longest list that instance ta
 constexpr int PART_MAX = PJG_PART_MAX;
 static_assert(PART_MAX == 256 || PART_MAX == 512 || PART_MAX == 1024, "axis partitions up to 256, 512 or 1024");
 // kernels one launch_leaf_order call launches
-constexpr int LEAF_ORDER_LAUNCHES = PJG_LEAF_RANK ? 7 : (PART_MAX >= 1024 ? 8 : PART_MAX >= 512 ? 7 : 6);
+constexpr int LEAF_ORDER_LAUNCHES = PJG_LEAF_RANK ? 8 : (PART_MAX >= 1024 ? 9 : PART_MAX >= 512 ? 8 : 7);
 constexpr int LEAF_LISTS = 5;          // leaf-order worklists: three k_leaf_sorted size
                                        //   classes and two forwarded size classes
 constexpr int LEAF_MID_MAX = 384;      // longest list of the rank method's larger instance
@@ -66,7 +85,8 @@ constexpr int LEAF_SORT_FROM = 64;     // rank method: a level's nodes of this m
 constexpr int LEAF_SORT_WORDS = 128;   // its window (32-bit words)
 constexpr int LEAF_SORTED_MAX = 2048;  // longest list ordered by sorted axes
 constexpr int LEAF_SORT_MAX = 1024;    // longest list ordered by presorted axes
-constexpr int EXACT_MAX = 4096;        // longest list replayed warp-parallel
+constexpr int EXACT_MAX = 4096;        // lists replayed warp-parallel: up to this
+constexpr int EXACT_LONG = 12288;      //   in 64 KB of shared memory, then in 192 KB
 
 // Search profile: event counts and clock64 cycles of k_search's sections,
 // summed over warps.  Compiled only with -DPJG_SEARCH_PROF=1 (a separate
@@ -245,8 +265,69 @@ struct CompleteRows {
     int64_t *ordinal;                  // position in the pair's stream
     int32_t *atoms;                    // [capacity * stride], template order
     double *rmsd;                      // rmsd computed in the search (inline
-                                       // cut mode), else nullptr
+                                       // cut mode; negative: not computed),
+                                       // else nullptr
     int32_t *pair_rows;                // [pairs] complete rows of each pair
+};
+
+// A pair that the order-free search takes in items of FREE_ITEM seeds.
+struct HeavyPair {
+    int32_t pair;
+    int32_t blocks;                    // items
+    int32_t first;                     // its first item in `results`
+    int32_t failed;                    // handed to k_search
+};
+
+// Rows of the order-free search whose order among each other is still to be
+// found: the rows of a pair, or a segment of the rows of an item (of a heavy
+// pair; its segments form a list from item_head on).
+struct RowUnit {
+    int64_t row_base;
+    int32_t pair;
+    int32_t count;
+    int32_t heavy;                     // index of its HeavyPair (-1: none)
+    int32_t item;                      // its item in `results` (-1: none)
+    int32_t next;                      // the item's next segment (-1: none)
+    uint32_t branch;                   // levels at which the pair's rows part
+};
+
+// An entry of an item whose children outgrew the frontier: searched as an
+// item of its own in a later launch.
+struct SpilledEntry {
+    int32_t heavy, block;              // heavy pair and item it belongs to
+    int32_t level;                     // its level; atoms of levels 0 .. level
+    int32_t atom[32];
+};
+
+// Worklists of the order-free search.
+struct FreeWork {
+    RowUnit *units;
+    unsigned long long *n_units;
+    HeavyPair *heavy;
+    unsigned long long *n_heavy;       // [2] heavy pairs, their items
+    const int2 *items;                 // (heavy pair, block), block by block
+    int32_t n_items;
+    int32_t item_seeds;
+    int2 *results;                     // per item: rows (-1: not finished), flags
+                                       //   (1: a hit among them, 2: the stream ends)
+    unsigned long long *heavy_stats;   // [4 * heavy pairs] partials, complete, bytes, rechecks
+    int32_t *item_head;                // per item: its list of segments (-1: no rows)
+    uint32_t *item_branch;             //   levels at which its rows part
+    const int64_t *item_base;          //   rows of the pair before it
+    float4 *arena_xyz;                 // frontiers of the items being searched,
+    int32_t *arena_atom;               //   HEAVY_CAP entries a warp
+    uint16_t *arena_parent;            // [2 * HEAVY_CAP a warp]
+    const SpilledEntry *spilled_in;    // this launch's items (nullptr: `items`)
+    SpilledEntry *spilled_out;         // entries spilled by this launch
+    unsigned long long *n_spilled;
+    int64_t spill_cap;
+    // units of more than UNIT_ROWS rows, and their scratch: a region of as
+    // many entries as rows each, taken from scratch_used
+    int32_t *large_units;
+    unsigned long long *n_large_units;
+    unsigned long long *scratch_used;
+    unsigned long long *row_key;
+    int32_t *row_scratch;              // [5 * rows] (nullptr: no unit can be that large)
 };
 
 // Superposition of every complete row, in reference order: row i of pair
@@ -342,10 +423,49 @@ void launch_heavy_pairs(cudaStream_t st, int32_t n_pairs, const uint8_t *pair_co
 void launch_mark_ordered(cudaStream_t st, int blocks, const LeafDemand &dm);
 
 // per-structure axis ranks (lrank, urank: [3][n_atoms], structure-local
-// values); tile_key / tile_idx: scratch of 3 * n_atoms entries
+// values) and the residue order and kind-ordered points of FreeView;
+// tile_key / tile_idx: scratch of 4 * n_atoms entries
+struct ResidueOrder {
+    const float4 *xyz32;
+    const int32_t *nh_pos;
+    const uint16_t *local_kind;
+    float4 *kxyz;
+    int32_t *res_pos;
+    uint16_t *res_kind;
+    int4 *res_range;
+    const int32_t *sorted;
+    int32_t *res_place;  // per atom: its position in ResIndex order
+};
 void launch_axis_ranks(cudaStream_t st, int32_t n_structures, const int64_t *atom_base, const int32_t *atom_count,
                        const double *xyz64, int64_t n_atoms, unsigned long long *tile_key, uint16_t *tile_idx,
-                       uint32_t *lrank, uint32_t *urank);
+                       uint32_t *lrank, uint32_t *urank, const ResidueOrder &ro);
+
+// sig_bits of FreeView: the kinds of every signature's list
+void launch_sig_kinds(cudaStream_t st, const SigView &sv, const FreeView &fv, uint32_t *sig_bits);
+
+// the order-free search over every pair: rows and units of rows to put in
+// order (fw), pairs to search in items (fw.heavy), and the pairs left to
+// k_search in dm.suspended, with the lists each of them needs requested
+cudaError_t launch_search_free(cudaStream_t st, bool fp32, const ChunkView &cv, const TemplateView &tv,
+                               const CandView &cd, const FreeView &fv, const SearchArgs &sa, int32_t *item_counter,
+                               const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
+                               const LeafDemand &dm, const FreeWork &fw);
+// the items of the heavy pairs: warps to launch (frontiers of HEAVY_CAP
+// entries each), then the search
+cudaError_t heavy_warps(bool fp32, int64_t n_items, int64_t *warps);
+cudaError_t launch_search_heavy(cudaStream_t st, bool fp32, int64_t warps, const ChunkView &cv,
+                                const TemplateView &tv, const CandView &cd, const FreeView &fv, const SearchArgs &sa,
+                                int32_t *item_counter, const CompleteRows &out, unsigned long long *counters,
+                                const LeafDemand &dm, const FreeWork &fw);
+void launch_heavy_bins(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy, int32_t *bins);
+void launch_heavy_items(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy, const int64_t *bin_begin,
+                        int32_t *bin_fill, int2 *items);
+void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int64_t *item_base, int32_t *pair_rows,
+                       unsigned long long *counters);
+// the units' rows in the reference's order (out.ordinal)
+void launch_unit_order(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
+                       const CandView &cd, const SigView &sv, const int32_t *res_place, int32_t reorder,
+                       const FreeWork &fw, const CompleteRows &out);
 
 // culling blocks per list: ceil(count / CULL_BLK)
 void launch_block_counts(cudaStream_t st, int64_t n, const int32_t *count, int32_t *nblk);
@@ -379,11 +499,11 @@ void launch_order_counts(cudaStream_t st, int64_t n_pairs, int32_t n_templates, 
 
 // Query.__next__ per pair over its rows in reference order: hit / warning
 // flags and hit atom counts per row; totals[0..3] += hits, warnings, hit
-// atoms, passing rows
+// atoms, passing rows; long_pairs / n_long (zeroed): pairs of many rows
 void launch_automaton(cudaStream_t st, int64_t n_pairs, int32_t n_templates, const int32_t *atom_begin,
                       const int32_t *cnt_q, const int64_t *off_q, const RowResults &rr, int32_t max_candidates,
                       int32_t best_match, double rmsd_threshold, int32_t *hit, int32_t *warn, int32_t *hit_atoms,
-                      unsigned long long *totals);
+                      unsigned long long *totals, int32_t *long_pairs, unsigned long long *n_long);
 
 // compaction of the flagged rows into a HitSegment (hit_idx, warn_idx,
 // atom_idx: exclusive scans of the flags / hit atom counts)

@@ -1,0 +1,169 @@
+"""The order-free search (k_search_free, k_unit_order) against the oracle.
+
+Each test drives a path of it: residues that are not contiguous in the file
+or share their number, pairs searched in items of seeds, entries spilled to a
+later launch, units of one row up to tens of thousands, structures with more
+atom kinds than it takes (searched in order), and the pairs' streams cut by
+max_candidates.  Bar as in test_gpu_parity.py: identical ordered hits,
+warnings and search counters, RMSD within RMSD_TOL.
+"""
+
+import numpy as np
+import pytest
+
+from test_gpu_parity import compare, gpu_query
+from helpers import hit_keys
+
+pytestmark = pytest.mark.gpu
+
+PARAMS = dict(rmsd_threshold=2.0, distance_cutoff=1.5, max_dynamic_distance=1.5)
+
+
+def _structures(seed, lengths, chains=2):
+    from pyjess_gb300 import workloads as W
+
+    return W.make_structures([np.random.default_rng([seed, i]) for i in range(len(lengths))], lengths,
+                             [chains] * len(lengths))
+
+
+def _templates(seed, structs, n, lo=2, hi=7, **kw):
+    from pyjess_gb300 import workloads as W
+
+    rng = np.random.default_rng([seed, 99])
+    return [W.make_template(rng, structs[int(rng.integers(len(structs)))], int(rng.integers(lo, hi)), **kw)
+            for _ in range(n)]
+
+
+@pytest.mark.parametrize("ignore", [0, 1, 2])
+@pytest.mark.parametrize("mode", ["fp32", "fp64"])
+def test_scattered_residues(mode, ignore):
+    """Atoms in random file order, residue numbers that repeat within and
+    across chains and go below zero: the atoms of a residue are found by key
+    (or by number alone), wherever they stand."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(31, [33, 130, 270, 310])
+    specs = _templates(31, structs, 60)
+    rng = np.random.default_rng(7)
+    for s in structs:
+        s["res_seq"] = ((s["res_seq"] * 7) % 90 - 12).astype(np.int32)
+        order = rng.permutation(len(s["xyz"]))
+        for k in ("xyz", "name", "resname", "res_seq", "chain", "serial"):
+            s[k] = np.ascontiguousarray(s[k][order])
+    _, ref = compare(W.pack_templates(specs), W.pack(structs), mode=mode, ignore_chain=ignore, **PARAMS)
+    assert ref["hits"]["count"] > 0
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(best_match=True), dict(max_candidates=0), dict(max_candidates=5),
+                                dict(max_candidates=300), dict(best_match=True, max_candidates=7),
+                                dict(reorder=False), dict(reorder=False, max_candidates=40)])
+def test_pairs_in_items(kw):
+    """Structures whose lists exceed the first instance's frontier, 2.2 A of
+    play: pairs in items of seeds, units from one row to hundreds, streams cut
+    in the middle."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(32, [900, 1500, 60])
+    specs = _templates(32, structs, 24, hi=5)
+    _, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=1.6, distance_cutoff=2.2,
+                     max_dynamic_distance=2.2, **kw)
+    assert ref["hits"]["count"] > 0
+
+
+@pytest.mark.parametrize("mode", ["fp32", "fp64"])
+@pytest.mark.parametrize("kw", [dict(), dict(max_candidates=20), dict(best_match=True, max_candidates=1000)])
+def test_spilled_entries(mode, kw):
+    """Element-matched templates with 2 A of play in small structures: a few
+    seeds with 100,000 and more partial assignments, so entries are spilled
+    to later launches and a unit has up to 70,000 rows."""
+    from pyjess_gb300 import workloads as W
+
+    for seed in (7, 8):
+        rng = np.random.default_rng(seed)
+        structs = W.make_structures([rng], [60], [1])
+        specs = [W.make_template(rng, structs[0], 6, modes=(3,), mode_p=(1.0,)) for _ in range(2)]
+        compare(W.pack_templates(specs), W.pack(structs), mode=mode, rmsd_threshold=2.0, distance_cutoff=2.0,
+                max_dynamic_distance=2.0, **kw)
+
+
+@pytest.mark.parametrize("residues", [1, 2])
+@pytest.mark.parametrize("kw", [dict(), dict(max_candidates=3), dict(best_match=True),
+                                dict(best_match=True, max_candidates=20)])
+def test_templates_of_one_and_two_atoms(monkeypatch, residues, kw):
+    """One atom (left to the search in order) and two (every rotation
+    undefined: all rows warn), with streams longer than a thread takes: the
+    warnings of the search in order (PJG_LEAF_LEVELS)."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(33, [150, 400])
+    specs = _templates(33, structs, 12, lo=residues, hi=residues + 1, atoms_per_res=1)
+    pt, ps = W.pack_templates(specs), W.pack(structs)
+    free = gpu_query(pt, ps, **PARAMS, **kw)
+    monkeypatch.setenv("PJG_LEAF_LEVELS", "4")
+    ordered = gpu_query(pt, ps, **PARAMS, **kw)
+    assert hit_keys(free.arrays()) == hit_keys(ordered.arrays())
+    a, b = free.warnings(), ordered.warnings()
+    assert len(a[0]) > 0 and np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("kinds", [31, 33, 1023, 1025])
+def test_many_atom_kinds(kinds):
+    """Distinct (residue, atom) names of a structure around a word of kind
+    bits and around the most the order-free search takes."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(34, [220, 90])
+    specs = _templates(34, structs, 30)
+    rng = np.random.default_rng(kinds)
+    for s in structs:
+        have = len(np.unique(np.concatenate([s["resname"], s["name"]], 1), axis=0))
+        if kinds < have:  # keep the most common kinds only
+            both = [bytes(v) for v in np.concatenate([s["resname"], s["name"]], 1)]
+            names, counts = np.unique(both, return_counts=True)
+            keep = np.isin(both, names[np.argsort(-counts, kind="stable")[:kinds]])
+            for k in ("xyz", "name", "resname", "res_seq", "chain", "serial"):
+                s[k] = np.ascontiguousarray(s[k][keep])
+        else:  # ligand atoms of names of their own
+            m = kinds - have
+            extra = {"xyz": s["xyz"][rng.integers(len(s["xyz"]), size=m)] + rng.normal(scale=3.0, size=(m, 3)),
+                     "name": np.frombuffer(b"".join(b"X%03d" % (i % 1000) for i in range(m)), np.uint8).reshape(m, 4),
+                     "resname": np.frombuffer(b"".join(b"L%02d\0" % (i // 100) for i in range(m)),
+                                              np.uint8).reshape(m, 4),
+                     "res_seq": np.arange(900, 900 + m, dtype=np.int32), "chain": np.tile(s["chain"][:1], (m, 1)),
+                     "serial": np.arange(9000, 9000 + m, dtype=np.int32)}
+            for k, v in extra.items():
+                s[k] = np.ascontiguousarray(np.concatenate([s[k], v]))
+    _, ref = compare(W.pack_templates(specs), W.pack(structs), **PARAMS)
+    assert ref["hits"]["count"] > 0 or kinds < 40
+
+
+def test_same_as_search_in_order(monkeypatch):
+    """The same query with the lists ordered up front (PJG_LEAF_LEVELS): every
+    column bit for bit the same."""
+    from pyjess_gb300 import workloads as W
+
+    wl = W.config(3, n_structures=40, n_templates=400)
+    free = gpu_query(wl.templates, wl.structures, **wl.params)
+    monkeypatch.setenv("PJG_LEAF_LEVELS", "4")
+    ordered = gpu_query(wl.templates, wl.structures, **wl.params)
+    a, b = free.arrays(), ordered.arrays()
+    assert hit_keys(a) == hit_keys(b)
+    for k in ("rmsd", "rotation", "centres"):
+        assert np.array_equal(a[k], b[k]), k
+    for k in ("pairs", "candidate_entries", "partials", "complete", "passing", "hits", "fp64_rechecks",
+              "bytes_candidates", "bytes_expansion"):
+        assert free.stats()[k] == ordered.stats()[k], k
+
+
+def test_long_lists_replayed():
+    """Backbone lists of 4,300 entries with ties (the exact replay in 192 KB of
+    shared memory)."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(35, [4300])
+    for s in structs:
+        s["xyz"] = np.round(s["xyz"] / 0.02) * 0.02
+    specs = _templates(35, structs, 2, lo=2, hi=3, permissive=True)
+    res, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=2.0, distance_cutoff=1.0,
+                       max_dynamic_distance=1.0)
+    assert ref["hits"]["count"] > 0 and res.stats()["leaf_exact"] > 0
