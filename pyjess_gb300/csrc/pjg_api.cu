@@ -1014,7 +1014,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     DBuf<unsigned long long> d_free_n, d_heavy_stats, d_row_key;
     DBuf<int2> d_items, d_results;
     DBuf<int64_t> d_item_base, d_bin_off;
-    DBuf<int32_t> d_bins, d_arena_atom, d_row_scratch, d_item_head, d_large_units, d_long_pairs;
+    DBuf<int32_t> d_bins, d_arena_atom, d_row_scratch, d_item_head, d_large_units, d_long_pairs, d_pending;
     DBuf<uint32_t> d_item_branch;
     DBuf<SpilledEntry> d_spill_a, d_spill_b;
     DBuf<float4> d_arena_xyz;
@@ -1388,14 +1388,20 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             // there the leaf offsets are a separate, writable array)
             ListShare ls{};
             bool share_on = false;
-            auto order_requested = [&]() -> cudaError_t {
+            auto order_requested = [&](bool few = false) -> cudaError_t {
                 if (dm.fill_state) {
                     // the requested lists not filled yet
                     launch_candidates(st, fill_blocks, true, cv, sv, nullptr, nullptr, d_offset.p, d_cand_atom.p,
                                       dm.work, dm.n_work, dm.fill_state, true);
                     launches++;
                 }
-                if (share_on) {
+                if (few) {
+                    launch_leaf_order_few(st, cv, G, cnt_c, d_offset.p, d_boff.p, d_cand_atom.p, leaf_off,
+                                          d_leaf_atom.p, d_leaf_xyz.p, d_blk_lo.p, d_blk_hi.p, d_sorted_list.p,
+                                          d_sorted_count.p, d_exact_list.p, d_exact_count.p, d_counters.p, dm.work,
+                                          dm.n_work);
+                    launches += LEAF_FEW_LAUNCHES;
+                } else if (share_on) {
                     // key every requested list, order one list per key, point
                     // the others at its leaves, order those whose atoms differ
                     const cudaError_t e0 = cudaMemsetAsync(ls.n, 0, 3 * sizeof(unsigned long long), st);
@@ -1656,8 +1662,9 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 dm.resume = nullptr;
                 dm.n_resume = 0;
                 dm.pool_in = nullptr;
-                // units, heavy pairs, their items, (scratch, large units,) spilled entries
-                unsigned long long free_n[6] = {};
+                // units, heavy pairs, their items, (scratch, large units,) spilled entries,
+                // units left to the leaf order
+                unsigned long long free_n[7] = {};
                 FreeWork fw{};
                 Suspended *next_out = d_susp_a.p, *spare = d_susp_b.p;
                 unsigned char *pool_next = d_pool_a.p, *pool_spare = d_pool_b.p;
@@ -1674,12 +1681,16 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     if (round == 0 && free_chunk) {
                         CUDA_TRY(dalloc(d_units, (size_t)c_cap, st));
                         CUDA_TRY(dalloc(d_heavy_pairs, (size_t)n_pairs, st));
-                        CUDA_TRY(dalloc(d_free_n, 6, st));
-                        CUDA_TRY(cudaMemsetAsync(d_free_n.p, 0, 6 * sizeof(unsigned long long), st));
-                        fw.item_seeds = P->max_candidates >= 0 ? FREE_ITEM_CUT : FREE_ITEM;
+                        CUDA_TRY(dalloc(d_free_n, 8, st));
+                        CUDA_TRY(cudaMemsetAsync(d_free_n.p, 0, 8 * sizeof(unsigned long long), st));
+                        fw.item_seeds = P->max_candidates >= 0        ? FREE_ITEM_CUT
+                                        : n_pairs <= FREE_FEW_PAIRS ? FREE_ITEM_FEW
+                                                                    : FREE_ITEM;
                         fw.scratch_used = d_free_n.p + 3;
                         fw.n_large_units = d_free_n.p + 4;
                         fw.n_spilled = d_free_n.p + 5;
+                        fw.n_pending = d_free_n.p + 6;
+                        fw.n_long_units = d_free_n.p + 7;
                         fw.units = d_units.p;
                         fw.n_units = d_free_n.p;
                         fw.heavy = d_heavy_pairs.p;
@@ -1811,6 +1822,19 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         launches++;
                         CUDA_TRY(cudaGetLastError());
                     }
+                    if (round == 0 && free_chunk && free_n[0] && (int64_t)nc <= c_cap) {
+                        // the rows found without order, in the reference's;
+                        // units it leaves wait for their lists' leaf order
+                        CUDA_TRY(dalloc(d_pending, 2 * (size_t)free_n[0], st));
+                        fw.pending = d_pending.p;
+                        fw.long_units = d_pending.p + free_n[0];
+                        CUDA_TRY(launch_unit_order_direct(st, (int64_t)free_n[0], cv, tv, cd, sv, fv, sp->d_res_place,
+                                                          P->reorder, fw, cr, dm));
+                        launches += 2;
+                        const double ms0 = ms_search;
+                        CUDA_TRY(read_back());
+                        ms_search = ms0;
+                    }
                     if (ns == 0 && (!free_chunk || (int64_t)used <= leaf_filled)) break;
                     if (round > 80) {
                         status = fail(PJG_ERR_CAPACITY, "leaf order on demand did not converge");
@@ -1819,7 +1843,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     suspensions += (int64_t)ns;
                     // the lists the suspended pairs reached, then those pairs
                     CUDA_TRY(ensure_leaf((int64_t)used));
-                    CUDA_TRY(order_requested());
+                    CUDA_TRY(order_requested(free_chunk && (int64_t)used - leaf_filled <= LEAF_FEW_ENTRIES));
                     leaf_filled = (int64_t)used;
                     if (ns == 0) break;
                     dm.resume = next_out;
@@ -1829,17 +1853,16 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     std::swap(pool_next, pool_spare);
                 }
                 if ((int64_t)nc <= c_cap) {
-                    if (free_chunk && free_n[0]) {
-                        // the rows found without order, in the reference's
+                    if (free_chunk && free_n[6]) {
                         if (free_n[1]) {
                             CUDA_TRY(dalloc(d_row_key, (size_t)nc, st));
                             CUDA_TRY(dalloc(d_row_scratch, 5 * (size_t)nc, st));
-                            CUDA_TRY(dalloc(d_large_units, (size_t)free_n[0], st));
+                            CUDA_TRY(dalloc(d_large_units, (size_t)free_n[6], st));
                             fw.row_key = d_row_key.p;
                             fw.row_scratch = d_row_scratch.p;
                             fw.large_units = d_large_units.p;
                         }
-                        launch_unit_order(st, (int64_t)free_n[0], cv, tv, cd, sv, sp->d_res_place, P->reorder, fw, cr);
+                        launch_unit_order(st, (int64_t)free_n[6], cv, tv, cd, sv, sp->d_res_place, P->reorder, fw, cr);
                         launches++;
                         CUDA_TRY(cudaGetLastError());
                     }
@@ -2044,7 +2067,7 @@ done:
         dfree(d_heavy_stats, st); dfree(d_row_key, st); dfree(d_items, st); dfree(d_results, st);
         dfree(d_item_base, st); dfree(d_bin_off, st); dfree(d_bins, st); dfree(d_arena_atom, st);
         dfree(d_row_scratch, st); dfree(d_arena_xyz, st); dfree(d_arena_parent, st); dfree(d_item_head, st);
-        dfree(d_large_units, st); dfree(d_long_pairs, st); dfree(d_item_branch, st); dfree(d_spill_a, st);
+        dfree(d_large_units, st); dfree(d_long_pairs, st); dfree(d_pending, st); dfree(d_item_branch, st); dfree(d_spill_a, st);
         dfree(d_spill_b, st);
         dfree(d_params, st); dfree(d_count, st); dfree(d_scanned, st); dfree(d_cand_atom, st);
         dfree(d_leaf_atom, st); dfree(d_pair_counter, st); dfree(d_offset, st); dfree(d_totals, st);

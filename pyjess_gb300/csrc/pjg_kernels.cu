@@ -4588,7 +4588,6 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
         if (!kd_needed && !outgrown && rows > 0) {
             // rows in several segments part anywhere
             if (n_seg > 1 || spilled || sub) branch = n == 32 ? ~0u : (1u << n) - 1u;
-            request_list_warp(dm, lane >= 1 && lane < n && ((branch >> lane) & 1u), lw, llen);
         }
         if (!HEAVY) {
             if (lane == 0 && seg >= 0 && seg < out.capacity) fw.units[seg].branch = branch;
@@ -4770,25 +4769,16 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
     const int T = tv.n_templates, G = cd.n_sigs;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t total = (int64_t)*fw.n_units;
-    for (int64_t w = warp; w < total; w += nwarps) {
+    const int64_t total = (int64_t)*fw.n_pending;
+    for (int64_t x = warp; x < total; x += nwarps) {
+        const int w = fw.pending[x];
         const RowUnit u = fw.units[w];
-        if (u.heavy >= 0 && fw.heavy[u.heavy].failed) {
-            for (int i = lane; i < u.count; i += 32) out.pair[u.row_base + i] = -1;  // k_search's rows count
-            continue;
-        }
-        // (a segment that does not lead its unit's list is not a unit)
-        if (u.item >= 0 && fw.item_head[u.item] != (int)w) continue;
         const int R = u.item >= 0 ? fw.results[u.item].x : u.count;
         if (R > UNIT_ROWS) {
-            if (lane == 0) fw.large_units[atomicAdd(fw.n_large_units, 1ull)] = (int32_t)w;
+            if (lane == 0) fw.large_units[atomicAdd(fw.n_large_units, 1ull)] = w;
             continue;
         }
         const int64_t ord0 = u.item >= 0 ? fw.item_base[u.item] : 0;
-        if (R == 1) {
-            if (lane == 0) out.ordinal[u.row_base] = ord0;
-            continue;
-        }
         const int s = u.pair / T, t = u.pair % T;
         const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
         const int64_t abase = cv.atom_base[s], wb = (int64_t)s * G;
@@ -4804,7 +4794,7 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
             U.sig[rank] = sg;
         }
         int at = 0;
-        for (int q = (int)w; q >= 0;) {
+        for (int q = w; q >= 0;) {
             const RowUnit v = fw.units[q];
             for (int i = lane; i < v.count; i += 32) U.row[at + i] = (int32_t)(v.row_base + i);
             at += v.count;
@@ -4873,6 +4863,347 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
             __syncwarp();
         }
         for (int i = lane; i < R; i += 32) out.ordinal[U.row[i]] = ord0 + U.cur[i];
+        __syncwarp();
+    }
+}
+
+// The same without any list in leaf order: the few atoms of a unit's rows at a
+// level are told apart by splitting only the kd nodes that hold two of them,
+// from the root down.  A node's left child is the half with the smaller axis
+// ranks, whatever the rest of the tree looks like: found by a histogram of the
+// rank's high bits for a node of more than 32 atoms; a node of at most 32 is taken apart
+// down to its leaves at once (an atom a lane, per axis the mask of the atoms
+// below it; a lane's place in its node is then a popcount).  A tie at a median
+// boundary, where qselect's arrangement decides, leaves the unit to the leaf
+// order (its lists are requested and the unit listed in fw.pending), and so do
+// large units and long lists with many rows (dense templates: few lists,
+// shared by many units).  Splits along a path halve, so a level costs about
+// two passes over its list.
+//
+// Two instances by list length (shared memory a warp holds): units whose
+// lists have at most DIRECT_MAX entries, and, passed on by the first, lists of
+// up to DIRECT_LONG with at most DIRECT_LONG_ROWS rows.
+// Measured on 1,000 structures x 4,000 templates: 8.8 and 8.9 ms, and 11 ms
+// for the 62,000 lists left to the leaf order, where ordering every such list
+// (0.84 M) and ranking the rows by them took 42 and 9 ms.  With 3,000
+// templates against one protein: 0.35 ms instead of 1.9 ms.
+constexpr int DIRECT_MAX = 512, DIRECT_LONG = 2048;
+constexpr int DIRECT_WARPS = 4, DIRECT_LONG_WARPS = 1;
+constexpr int DIRECT_LONG_ROWS = 32;
+
+template <int MAXM>
+struct DirectWarp {
+    unsigned long long key[UNIT_ROWS];
+    int32_t cur[UNIT_ROWS], atom[UNIT_ROWS], row[UNIT_ROWS];
+    uint32_t code[UNIT_ROWS];  // path from the root: a bit a split, 0 right (reported first)
+    uint16_t node[UNIT_ROWS];  // node the row's atom is in
+    int32_t mem[2][MAXM];      // the nodes' atoms, children in the other buffer
+    uint32_t rk[MAXM];         // ranks of the node being split
+    alignas(16) int32_t bins[128];
+    int32_t order[32], sig[32];
+    int4 stack[32];            // nodes to split: first entry, entries, depth | buffer << 8, number
+};
+
+template <int MAXM, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+    k_unit_order_direct(ChunkView cv, TemplateView tv, CandView cd, SigView sv, FreeView fv, const int32_t *res_place,
+                        int32_t reorder, FreeWork fw, CompleteRows out, LeafDemand dm) {
+    extern __shared__ __align__(16) unsigned char direct_smem[];
+    constexpr bool LONG = MAXM > DIRECT_MAX;
+    DirectWarp<MAXM> &U = reinterpret_cast<DirectWarp<MAXM> *>(direct_smem)[threadIdx.x >> 5];
+    const int lane = lane_id();
+    const unsigned lt = (1u << lane) - 1u;
+    const int T = tv.n_templates, G = cd.n_sigs;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t total = LONG ? (int64_t)*fw.n_long_units : (int64_t)*fw.n_units;
+    for (int64_t x = warp; x < total; x += nwarps) {
+        const int w = LONG ? fw.long_units[x] : (int)x;
+        const RowUnit u = fw.units[w];
+        if (!LONG) {
+            if (u.heavy >= 0 && fw.heavy[u.heavy].failed) {
+                for (int i = lane; i < u.count; i += 32) out.pair[u.row_base + i] = -1;  // k_search's rows count
+                continue;
+            }
+            // (a segment that does not lead its unit's list is not a unit)
+            if (u.item >= 0 && fw.item_head[u.item] != w) continue;
+        }
+        const int R = u.item >= 0 ? fw.results[u.item].x : u.count;
+        const int64_t ord0 = u.item >= 0 ? fw.item_base[u.item] : 0;
+        if (R == 1) {
+            if (lane == 0) out.ordinal[u.row_base] = ord0;
+            continue;
+        }
+        const int s = u.pair / T, t = u.pair % T;
+        const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
+        const int64_t abase = cv.atom_base[s], wb = (int64_t)s * G;
+        // ranks are below the structure's atoms: the shift to 128 bins of them
+        const int shift = max(0, 32 - __clz(cv.atom_count[s]) - 7);
+        const uint32_t branch = u.item >= 0 ? fw.item_branch[u.item] : u.branch;
+        int c = INT_MAX, sg = 0;
+        if (lane < n) {
+            sg = tv.sig[ab + lane];
+            c = cd.count[wb + sg];
+        }
+        const int rank = level_rank(n, c, reorder);
+        const bool parts = lane < n && rank > 0 && ((branch >> rank) & 1u);  // this atom's level parts rows
+        bool pending = R > UNIT_ROWS;
+        if (!LONG && !pending && __any_sync(FULL_MASK, parts && c > DIRECT_MAX)) {
+            if (R <= DIRECT_LONG_ROWS && !__any_sync(FULL_MASK, parts && c > DIRECT_LONG)) {
+                if (lane == 0) fw.long_units[atomicAdd(fw.n_long_units, 1ull)] = w;
+                continue;
+            }
+            pending = true;
+        }
+        __syncwarp();
+        if (lane < n) {
+            U.order[rank] = lane;
+            U.sig[rank] = sg;
+        }
+        if (!pending) {
+            int at = 0;
+            for (int q = w; q >= 0;) {
+                const RowUnit v = fw.units[q];
+                for (int i = lane; i < v.count; i += 32) U.row[at + i] = (int32_t)(v.row_base + i);
+                at += v.count;
+                q = u.item >= 0 ? v.next : -1;
+            }
+            for (int i = lane; i < R; i += 32) U.cur[i] = 0;
+        }
+        __syncwarp();
+        const int q0 = cv.nh_begin[cv.bucket_begin[s]];
+        const int nk = cv.nh_begin[cv.bucket_begin[s + 1]] - q0;
+        for (unsigned left = pending ? 0u : branch; left && !pending; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const int k = U.order[l], g = U.sig[l];
+            if (l == 0) {
+                for (int i = lane; i < R; i += 32)
+                    U.key[i] = candidate_place(cv, sv, res_place, g, abase,
+                                               out.atoms[(int64_t)U.row[i] * out.stride + k]);
+            } else {
+                for (int i = lane; i < R; i += 32) {
+                    U.atom[i] = out.atoms[(int64_t)U.row[i] * out.stride + k];
+                    U.code[i] = 0;
+                    U.node[i] = 0;
+                }
+                // the list's atoms (in any order: splits read sets)
+                int m = 0;
+                for (int w0 = 0; 32 * w0 < nk; w0++) {
+                    const int q = 32 * w0 + lane;
+                    bool ok = false;
+                    if (q < nk) {
+                        const int kd = fv.nh_kind[q0 + q];
+                        ok = (fv.sig_bits[(int64_t)g * fv.kind_words + (kd >> 5)] >> (kd & 31)) & 1u;
+                    }
+                    unsigned bits = __ballot_sync(FULL_MASK, ok);
+                    const int cnt = ok ? cv.nh_count[q0 + q] : 0, off = ok ? cv.nh_off[q0 + q] : 0;
+                    for (; bits; bits &= bits - 1) {
+                        const int b = __ffs(bits) - 1;
+                        const int cb = __shfl_sync(FULL_MASK, cnt, b), ob = __shfl_sync(FULL_MASK, off, b);
+                        for (int i = lane; i < cb; i += 32)
+                            if (m + i < MAXM) U.mem[0][m + i] = cv.nh_pos[abase + ob + i];
+                        m += cb;
+                    }
+                }
+                m = min(m, MAXM);
+                int sp = 1, nodes = 1;
+                if (lane == 0) U.stack[0] = make_int4(0, m, 0, 0);
+                __syncwarp();
+                while (sp > 0) {
+                    const int4 nd = U.stack[--sp];
+                    const int lo = nd.x, nn = nd.y, depth = nd.z & 0xFF, buf = nd.z >> 8, id = nd.w;
+                    const int32_t *src = U.mem[buf] + lo;
+                    if (nn <= 32) {
+                        // an atom a lane: the masks of the atoms below it and of
+                        // those beside it on each axis, then every split of the
+                        // subtree (M: the atoms of the lane's node)
+                        const int32_t a = lane < nn ? src[lane] : -1;
+                        unsigned low[3] = {}, same[3] = {};
+#pragma unroll
+                        for (int ax = 0; ax < 3; ax++) {
+                            const uint32_t v = lane < nn ? cv.lrank[ax * cv.n_atoms + abase + a] : 0u;
+                            for (int j = 0; j < nn; j++) {
+                                const uint32_t y = __shfl_sync(FULL_MASK, v, j);
+                                low[ax] |= y < v ? 1u << j : 0u;
+                                same[ax] |= y == v ? 1u << j : 0u;
+                            }
+                        }
+                        // lanes that hold an atom of the rows
+                        unsigned rows_at = 0;
+                        for (int i0 = 0; i0 < R; i0 += 32) {
+                            const int32_t ra = i0 + lane < R && U.node[i0 + lane] == id ? U.atom[i0 + lane] : -2;
+                            for (int j = 0; j < nn; j++)
+                                if (__any_sync(FULL_MASK, ra == __shfl_sync(FULL_MASK, a, j))) rows_at |= 1u << j;
+                        }
+                        unsigned M = nn == 32 ? FULL_MASK : (1u << nn) - 1u;
+                        if (lane >= nn) M = 0;
+                        uint32_t code = 0;
+                        bool tie = false;
+                        // (down to the nodes that hold one atom of the rows)
+                        for (int d = depth;; d++) {
+                            const unsigned two = M & rows_at;
+                            if (!__any_sync(FULL_MASK, (two & (two - 1)) != 0)) break;
+                            const int ax = d % 3;
+                            const unsigned lw = ax == 0 ? low[0] : ax == 1 ? low[1] : low[2];
+                            const unsigned sm = ax == 0 ? same[0] : ax == 1 ? same[1] : same[2];
+                            const int half = __popc(M) >> 1;
+                            const int strict = __popc(lw & M), place = strict + __popc(sm & M & lt);
+                            const bool lf = place < half;
+                            // the first of the right half beside one of the left
+                            tie |= (two & (two - 1)) != 0 && place == half && strict < half;
+                            const unsigned L = __ballot_sync(FULL_MASK, lf);
+                            if (lf) code |= 0x80000000u >> d;
+                            M &= lf ? L : ~L;
+                        }
+                        if (__any_sync(FULL_MASK, tie)) {
+                            pending = true;
+                            break;
+                        }
+                        for (int i0 = 0; i0 < R; i0 += 32) {
+                            const int i = i0 + lane;
+                            const bool mine = i < R && U.node[i] == id;
+                            const int32_t ra = mine ? U.atom[i] : -2;
+                            uint32_t rc = 0;
+                            for (int j = 0; j < nn; j++) {
+                                const int32_t aj = __shfl_sync(FULL_MASK, a, j);
+                                const uint32_t cj = __shfl_sync(FULL_MASK, code, j);
+                                if (aj == ra) rc = cj;
+                            }
+                            if (mine) U.code[i] |= rc;
+                        }
+                        __syncwarp();
+                        continue;
+                    }
+                    const uint32_t *lr = cv.lrank + (depth % 3) * cv.n_atoms + abase;
+                    int32_t *dst = U.mem[buf ^ 1] + lo;
+#pragma unroll 4
+                    for (int i = lane; i < nn; i += 32) U.rk[i] = lr[src[i]];
+                    // the rank with nn / 2 smaller ones in the node: the bin
+                    // of it among 128 by the ranks' high bits, then its place
+                    // among the bin's
+                    const int half = nn >> 1;
+                    for (int q = lane; q < 128; q += 32) U.bins[q] = 0;
+                    __syncwarp();
+#pragma unroll 4
+                    for (int i = lane; i < nn; i += 32) atomicAdd(&U.bins[U.rk[i] >> shift], 1);
+                    __syncwarp();
+                    const int4 bc = reinterpret_cast<const int4 *>(U.bins)[lane];
+                    int bsum = bc.x + bc.y + bc.z + bc.w;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(FULL_MASK, bsum, o);
+                        if (lane >= o) bsum += y;
+                    }
+                    // first bin with more than nn / 2 atoms up to its end
+                    int bin = 4 * lane, before = bsum - (bc.x + bc.y + bc.z + bc.w), held = bc.x;
+                    if (before + held <= half) before += held, held = bc.y, bin++;
+                    if (before + held <= half) before += held, held = bc.z, bin++;
+                    if (before + held <= half) before += held, held = bc.w, bin++;
+                    const int owner = __ffs(__ballot_sync(FULL_MASK, bsum > half)) - 1;
+                    bin = __shfl_sync(FULL_MASK, bin, owner);
+                    before = __shfl_sync(FULL_MASK, before, owner);
+                    held = __shfl_sync(FULL_MASK, held, owner);
+                    uint32_t vlo = (uint32_t)bin << shift;
+                    int under = before;  // ranks below vlo
+                    if (before < half && held <= 32) {
+                        int at = 0;
+                        for (int i0 = 0; i0 < nn; i0 += 32) {
+                            const uint32_t v = i0 + lane < nn ? U.rk[i0 + lane] : ~0u;
+                            const bool in = v >> shift == (uint32_t)bin;
+                            const unsigned bm = __ballot_sync(FULL_MASK, in);
+                            if (in) U.bins[at + __popc(bm & lt)] = (int32_t)v;
+                            at += __popc(bm);
+                        }
+                        __syncwarp();
+                        const uint32_t v = lane < held ? (uint32_t)U.bins[lane] : ~0u;
+                        int strict = 0;
+                        for (int j = 0; j < held; j++) strict += __shfl_sync(FULL_MASK, v, j) < v ? 1 : 0;
+                        const unsigned first = __ballot_sync(FULL_MASK, lane < held && before + strict == half);
+                        if (first) {
+                            vlo = __shfl_sync(FULL_MASK, v, __ffs(first) - 1);
+                            under = half;
+                        }
+                    } else if (before < half) {
+                        uint32_t vhi = vlo + (1u << shift);
+                        while (vhi - vlo > 1) {
+                            const uint32_t mid = (vlo + vhi) >> 1;
+                            int below = 0;
+                            for (int i = lane; i < nn; i += 32) below += U.rk[i] < mid ? 1 : 0;
+                            below = __reduce_add_sync(FULL_MASK, below);
+                            if (below <= half) {
+                                vlo = mid;
+                                under = below;
+                                if (below == half) break;
+                            } else {
+                                vhi = mid;
+                            }
+                        }
+                    }
+                    if (under != half) {
+                        // equal coordinates on both sides of the boundary
+                        pending = true;
+                        break;
+                    }
+                    int nl = 0, nr = 0;
+                    for (int i0 = 0; i0 < nn; i0 += 32) {
+                        const int i = i0 + lane;
+                        const bool in = i < nn, lf = in && U.rk[i] < vlo;
+                        const unsigned ml = __ballot_sync(FULL_MASK, lf), mr = __ballot_sync(FULL_MASK, in && !lf);
+                        if (in) dst[lf ? nl + __popc(ml & lt) : half + nr + __popc(mr & lt)] = src[i];
+                        nl += __popc(ml);
+                        nr += __popc(mr);
+                    }
+                    // the rows' sides, and whether a side holds two atoms
+                    int32_t lmin = INT_MAX, lmax = -1, rmin = INT_MAX, rmax = -1;
+                    for (int i = lane; i < R; i += 32) {
+                        if (U.node[i] != id) continue;
+                        const int32_t a = U.atom[i];
+                        if (lr[a] < vlo) {
+                            U.code[i] |= 0x80000000u >> depth;
+                            U.node[i] = (uint16_t)nodes;
+                            lmin = min(lmin, a);
+                            lmax = max(lmax, a);
+                        } else {
+                            U.node[i] = (uint16_t)(nodes + 1);
+                            rmin = min(rmin, a);
+                            rmax = max(rmax, a);
+                        }
+                    }
+                    lmin = __reduce_min_sync(FULL_MASK, lmin);
+                    lmax = __reduce_max_sync(FULL_MASK, lmax);
+                    rmin = __reduce_min_sync(FULL_MASK, rmin);
+                    rmax = __reduce_max_sync(FULL_MASK, rmax);
+                    if (lmin < lmax) {
+                        if (lane == 0) U.stack[sp] = make_int4(lo, half, (depth + 1) | ((buf ^ 1) << 8), nodes);
+                        sp++;
+                    }
+                    if (rmin < rmax) {
+                        if (lane == 0)
+                            U.stack[sp] = make_int4(lo + half, nn - half, (depth + 1) | ((buf ^ 1) << 8), nodes + 1);
+                        sp++;
+                    }
+                    nodes += 2;
+                    __syncwarp();
+                }
+                if (pending) break;
+                for (int i = lane; i < R; i += 32)
+                    U.key[i] = ((unsigned long long)(uint32_t)U.cur[i] << 32) | U.code[i];
+            }
+            __syncwarp();
+            for (int i = lane; i < R; i += 32) {
+                const unsigned long long mine = U.key[i];
+                int before = 0;
+                for (int j = 0; j < R; j++) before += U.key[j] < mine ? 1 : 0;
+                U.cur[i] = before;
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+        if (pending) {
+            request_list_warp(dm, parts, wb + sg, c);
+            if (lane == 0) fw.pending[atomicAdd(fw.n_pending, 1ull)] = w;
+        } else {
+            for (int i = lane; i < R; i += 32) out.ordinal[U.row[i]] = ord0 + U.cur[i];
+        }
         __syncwarp();
     }
 }
@@ -5308,6 +5639,71 @@ void leaf_profile_read(unsigned long long *h, cudaStream_t st) {
 }
 #endif
 
+// exact replay of the lists in exact_list, by length: up to 1024 entries
+// 16 KB a warp, 4 warps a block; then 64 KB and 192 KB, one warp a block
+// (beyond EXACT_LONG one thread replays the list from global memory; that
+// took 35 ms for lists of 5,000 entries, 3.7 ms in shared memory)
+static void launch_leaf_exact(cudaStream_t st, int sms, const ChunkView &cv, int32_t n_sigs, const int32_t *count,
+                              const int64_t *offset, const int64_t *blk_offset, const int32_t *cand_atom,
+                              const int64_t *leaf_offset, int32_t *leaf_atom, float4 *leaf_xyz, float4 *blk_lo,
+                              float4 *blk_hi, int64_t *exact_list, unsigned long long *exact_count,
+                              unsigned long long *counters) {
+    auto launch = [&](auto kern, int entries, int warps, int blocks) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, entries * 16 * warps);
+        kern<<<blocks, 32 * warps, entries * 16 * warps, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom,
+                                                              leaf_offset, leaf_atom, leaf_xyz, blk_lo, blk_hi,
+                                                              exact_list, exact_count, counters);
+    };
+    launch(k_leaf_exact<1024, 0>, 1024, 4, sms * 3);
+    launch(k_leaf_exact<EXACT_MAX, 1024>, EXACT_MAX, 1, sms * 3);
+    launch(k_leaf_exact<EXACT_LONG, EXACT_MAX>, EXACT_LONG, 1, sms);
+}
+
+// The requested lists by length, without the tie-free kernels first: those of
+// at most LEAF_SORTED_MAX entries to one worklist, longer ones to the exact
+// replay's.
+__global__ void k_leaf_split(const int32_t *count, const int64_t *work, const unsigned long long *n_work,
+                             int64_t *sorted_list, unsigned long long *sorted_count, int64_t *exact_list,
+                             unsigned long long *exact_count, unsigned long long *counters) {
+    const int64_t n = (int64_t)*n_work;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t w = work[i];
+        const int m = count[w];
+        if (m <= 0) continue;
+        atomicAdd(&counters[C_LEAF_LISTS], 1ull);
+        atomicAdd(&counters[C_LEAF_ENTRIES], (unsigned long long)m);
+        if (m <= LEAF_SORTED_MAX) {
+            atomicAdd(&counters[C_LEAF_SORTED], 1ull);
+            sorted_list[atomicAdd(sorted_count, 1ull)] = w;
+        } else {
+            atomicAdd(&counters[C_LEAF_EXACT], 1ull);
+            exact_list[atomicAdd(exact_count, 1ull)] = w;
+        }
+    }
+}
+
+void launch_leaf_order_few(cudaStream_t st, const ChunkView &cv, int32_t n_sigs, const int32_t *count,
+                           const int64_t *offset, const int64_t *blk_offset, const int32_t *cand_atom,
+                           const int64_t *leaf_offset, int32_t *leaf_atom, float4 *leaf_xyz, float4 *blk_lo,
+                           float4 *blk_hi, int64_t *sorted_list, unsigned long long *sorted_count,
+                           int64_t *exact_list, unsigned long long *exact_count, unsigned long long *counters,
+                           const int64_t *work, const unsigned long long *n_work) {
+    cudaMemsetAsync(sorted_count, 0, LEAF_LISTS * sizeof(unsigned long long), st);
+    cudaMemsetAsync(exact_count, 0, sizeof(unsigned long long), st);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    k_leaf_split<<<32, 256, 0, st>>>(count, work, n_work, sorted_list, sorted_count, exact_list, exact_count,
+                                     counters);
+    constexpr int SS = (int)sizeof(SortedWarp<LEAF_SORTED_MAX>);
+    auto kern = k_leaf_sorted<LEAF_SORTED_MAX, 0, 1>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SS);
+    kern<<<sms * 4, 32, SS, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom, leaf_offset, leaf_atom, leaf_xyz,
+                                 blk_lo, blk_hi, sorted_list, sorted_count, exact_list, exact_count, counters);
+    launch_leaf_exact(st, sms, cv, n_sigs, count, offset, blk_offset, cand_atom, leaf_offset, leaf_atom, leaf_xyz,
+                      blk_lo, blk_hi, exact_list, exact_count, counters);
+}
+
 void launch_leaf_order(cudaStream_t st, int blocks, const ChunkView &cv, int32_t n_sigs, const int32_t *count,
                        const int64_t *offset, const int64_t *blk_offset, const int32_t *cand_atom,
                        const int64_t *leaf_offset, int32_t *leaf_atom, float4 *leaf_xyz, float4 *blk_lo, float4 *blk_hi,
@@ -5395,25 +5791,8 @@ void launch_leaf_order(cudaStream_t st, int blocks, const ChunkView &cv, int32_t
     k_leaf_sorted<LEAF_SORTED_MAX, 1024, 1><<<sms * 4, 32, SS2, st>>>(
         cv, n_sigs, count, offset, blk_offset, cand_atom, leaf_offset, leaf_atom, leaf_xyz, blk_lo, blk_hi,
         sorted_list + 2 * list_cap, sorted_count + 2, exact_list, exact_count, counters);
-    // exact replay: lists up to 1024 entries 16 KB a warp, 4 warps a block
-    constexpr int SM1 = 1024 * 16 * 4;
-    cudaFuncSetAttribute(k_leaf_exact<1024, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM1);
-    k_leaf_exact<1024, 0><<<sms * 3, 128, SM1, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom, leaf_offset,
-                                                    leaf_atom, leaf_xyz, blk_lo, blk_hi, exact_list, exact_count,
-                                                    counters);
-    // longer lists: 64 KB a warp, one warp a block, then 192 KB (beyond
-    // EXACT_LONG: one thread replays the list from global memory; that took
-    // 35 ms for lists of 5,000 entries)
-    constexpr int SM3 = EXACT_LONG * 16;
-    cudaFuncSetAttribute(k_leaf_exact<EXACT_LONG, EXACT_MAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM3);
-    k_leaf_exact<EXACT_LONG, EXACT_MAX><<<sms, 32, SM3, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom,
-                                                             leaf_offset, leaf_atom, leaf_xyz, blk_lo, blk_hi,
-                                                             exact_list, exact_count, counters);
-    constexpr int SM2 = EXACT_MAX * 16;
-    cudaFuncSetAttribute(k_leaf_exact<EXACT_MAX, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM2);
-    k_leaf_exact<EXACT_MAX, 1024><<<sms * 3, 32, SM2, st>>>(cv, n_sigs, count, offset, blk_offset, cand_atom,
-                                                           leaf_offset, leaf_atom, leaf_xyz, blk_lo, blk_hi,
-                                                           exact_list, exact_count, counters);
+    launch_leaf_exact(st, sms, cv, n_sigs, count, offset, blk_offset, cand_atom, leaf_offset, leaf_atom, leaf_xyz,
+                      blk_lo, blk_hi, exact_list, exact_count, counters);
 }
 
 void launch_axis_ranks(cudaStream_t st, int32_t n_structures, const int64_t *atom_base, const int32_t *atom_count,
@@ -5602,10 +5981,35 @@ void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int
                                                                      fw.heavy_stats, pair_rows, counters);
 }
 
-void launch_unit_order(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
+cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
+                                     const CandView &cd, const SigView &sv, const FreeView &fv,
+                                     const int32_t *res_place, int32_t reorder, const FreeWork &fw,
+                                     const CompleteRows &out, const LeafDemand &dm) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    auto launch = [&](auto kern, int smem, int warps, int64_t units) -> cudaError_t {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        int per_sm = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem);
+        if (e != cudaSuccess) return e;
+        const int64_t blocks = std::min<int64_t>((units + warps - 1) / warps, (int64_t)std::max(per_sm * sms, 1) * 4);
+        kern<<<(int)std::max<int64_t>(blocks, 1), warps * 32, smem, st>>>(cv, tv, cd, sv, fv, res_place, reorder, fw,
+                                                                         out, dm);
+        return cudaGetLastError();
+    };
+    cudaError_t e = launch(k_unit_order_direct<DIRECT_MAX, DIRECT_WARPS>,
+                           (int)sizeof(DirectWarp<DIRECT_MAX>) * DIRECT_WARPS, DIRECT_WARPS, n_units);
+    if (e == cudaSuccess)
+        e = launch(k_unit_order_direct<DIRECT_LONG, DIRECT_LONG_WARPS>,
+                   (int)sizeof(DirectWarp<DIRECT_LONG>) * DIRECT_LONG_WARPS, DIRECT_LONG_WARPS, n_units);
+    return e;
+}
+
+void launch_unit_order(cudaStream_t st, int64_t n_pending, const ChunkView &cv, const TemplateView &tv,
                        const CandView &cd, const SigView &sv, const int32_t *res_place, int32_t reorder,
                        const FreeWork &fw, const CompleteRows &out) {
-    const int64_t blocks = std::min<int64_t>((n_units + UNIT_WARPS - 1) / UNIT_WARPS, 152 * 16);
+    const int64_t blocks = std::min<int64_t>((n_pending + UNIT_WARPS - 1) / UNIT_WARPS, 152 * 16);
     k_unit_order<<<(int)blocks, UNIT_WARPS * 32, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
     if (fw.row_scratch)
         k_unit_order_large<<<152 * 4, UNIT_LARGE_THREADS, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);

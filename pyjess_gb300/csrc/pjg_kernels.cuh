@@ -36,9 +36,12 @@ constexpr int SEARCH_WARPS = PJG_SEARCH_WARPS;  // warps per block of k_search
 constexpr int FREE_WARPS = PJG_FREE_WARPS;
 constexpr int FREE_CAP = PJG_FREE_CAP;
 constexpr int FREE_MAX_KINDS = 1024;
-// seeds of an item of a heavy pair; fewer where max_candidates may make a
-// pair's later items unwanted
-constexpr int FREE_ITEM = 32, FREE_ITEM_CUT = 4;
+// seeds of an item of a heavy pair: 32 keep the set-up small (4 M pairs: 22 ms
+// for the items, 38 ms with 8), 8 fill the chip when there are at most
+// FREE_FEW_PAIRS pairs (3,000 pairs: 0.44 ms, 0.79 ms with 32), 4 where
+// max_candidates may make a pair's later items unwanted
+constexpr int64_t FREE_FEW_PAIRS = 1 << 16;
+constexpr int FREE_ITEM = 32, FREE_ITEM_FEW = 8, FREE_ITEM_CUT = 4;
 constexpr int64_t SPILL_CAP = 1 << 18;  // entries of items kept for a later launch
 constexpr int HEAVY_CAP = 8192;  // frontier entries of an item (16-bit entry numbers)
 // leaves per culling block: k_search tests a parent's join box against the
@@ -321,6 +324,10 @@ struct FreeWork {
     SpilledEntry *spilled_out;         // entries spilled by this launch
     unsigned long long *n_spilled;
     int64_t spill_cap;
+    int32_t *long_units;               // units of long lists
+    unsigned long long *n_long_units;
+    int32_t *pending;                  // units left to the leaf order
+    unsigned long long *n_pending;
     // units of more than UNIT_ROWS rows, and their scratch: a region of as
     // many entries as rows each, taken from scratch_used
     int32_t *large_units;
@@ -395,6 +402,20 @@ void launch_leaf_order(cudaStream_t st, int blocks, const ChunkView &cv, int32_t
                        const int64_t *work, const unsigned long long *n_work, int rank_max,
                        uint8_t *part_ok = nullptr, int count_lists = 1);
 
+// the same for few lists (at most LEAF_FEW_ENTRIES entries in all), requested
+// for ties or long units by the order-free search: one launch of the
+// sorted-axis split for every length (as long as its longest list) instead of
+// seven that a tied list would pass through (annotating a protein with 3,000
+// templates, 199 lists: 0.24 ms in 5 launches, 1.0 ms in 19)
+constexpr int64_t LEAF_FEW_ENTRIES = 8 << 20;
+constexpr int LEAF_FEW_LAUNCHES = 5;
+void launch_leaf_order_few(cudaStream_t st, const ChunkView &cv, int32_t n_sigs, const int32_t *count,
+                           const int64_t *offset, const int64_t *blk_offset, const int32_t *cand_atom,
+                           const int64_t *leaf_offset, int32_t *leaf_atom, float4 *leaf_xyz, float4 *blk_lo,
+                           float4 *blk_hi, int64_t *sorted_list, unsigned long long *sorted_count,
+                           int64_t *exact_list, unsigned long long *exact_count, unsigned long long *counters,
+                           const int64_t *work, const unsigned long long *n_work);
+
 // list sharing, around the leaf-order launches of a round: keys of the
 // requested lists into the table (and the lists / entries counters), the
 // split into lists to order and lists sharing another's order, and after
@@ -462,8 +483,14 @@ void launch_heavy_items(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy
                         int32_t *bin_fill, int2 *items);
 void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int64_t *item_base, int32_t *pair_rows,
                        unsigned long long *counters);
-// the units' rows in the reference's order (out.ordinal)
-void launch_unit_order(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
+// the units' rows in the reference's order (out.ordinal): without lists in
+// leaf order where that can be done (the others in fw.pending, their lists
+// requested), then those by their lists' leaf order
+cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
+                                     const CandView &cd, const SigView &sv, const FreeView &fv,
+                                     const int32_t *res_place, int32_t reorder, const FreeWork &fw,
+                                     const CompleteRows &out, const LeafDemand &dm);
+void launch_unit_order(cudaStream_t st, int64_t n_pending, const ChunkView &cv, const TemplateView &tv,
                        const CandView &cd, const SigView &sv, const int32_t *res_place, int32_t reorder,
                        const FreeWork &fw, const CompleteRows &out);
 

@@ -155,6 +155,25 @@ def test_same_as_search_in_order(monkeypatch):
         assert free.stats()[k] == ordered.stats()[k], k
 
 
+@pytest.mark.parametrize("step", [None, 0.05])
+@pytest.mark.parametrize("residues", [31, 32, 33, 65, 511, 512, 513, 2047, 2048, 2049])
+def test_rows_told_apart_in_lists_of(residues, step):
+    """Backbone templates any residue matches (lists of as many entries as
+    residues) around the sizes at which a kd node is taken apart another way,
+    without ties and on a 0.05 A grid."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(36, [residues])
+    if step:
+        for s in structs:
+            s["xyz"] = np.round(s["xyz"] / step) * step
+    specs = _templates(36, structs, 3, lo=2, hi=4, permissive=True)
+    reach = 2.5 if residues < 100 else 1.2 if residues < 600 else 0.9
+    _, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=2.5, distance_cutoff=reach,
+                     max_dynamic_distance=reach)
+    assert ref["hits"]["count"] > 1
+
+
 def test_long_lists_replayed():
     """Backbone lists of 4,300 entries with ties (the exact replay in 192 KB of
     shared memory)."""
