@@ -1008,7 +1008,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     DBuf<AnnulusParam> d_params;
     // order-free search: kinds of each signature, units of rows, heavy pairs
     // and their items, frontiers of the items, keys of large units
-    DBuf<uint32_t> d_sig_bits;
+    DBuf<uint32_t> d_sig_bits, d_kind_masks;
     DBuf<RowUnit> d_units;
     DBuf<HeavyPair> d_heavy_pairs;
     DBuf<unsigned long long> d_free_n, d_heavy_stats, d_row_key;
@@ -1082,8 +1082,9 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     }
     // every pair searched without order first (k_search_free): the batched
     // modes, unless the levels to order up front are chosen explicitly
-    FreeView fv{sp->n_kinds, (sp->n_kinds + 31) / 32, sp->d_kind_name, sp->d_kind_res, nullptr, sp->d_nh_kind,
-                sp->d_kxyz, sp->d_res_pos, sp->d_res_kind, sp->d_res_range};
+    FreeView fv{sp->n_kinds, (sp->n_kinds + 31) / 32, sp->d_kind_name, sp->d_kind_res, nullptr,
+                (sp->max_local_kinds + 31) / 32, nullptr, sp->d_nh_kind, sp->d_kxyz, sp->d_res_pos, sp->d_res_kind,
+                sp->d_res_range};
     const bool free_first = P->mode != PJG_MODE_PLAIN_FP64 && demand_levels == TUNING_DEFAULTS.leaf_levels &&
                             !getenv("PJG_LEAF_LEVELS") && sp->max_local_kinds <= FREE_MAX_KINDS &&
                             (int64_t)G * fv.kind_words <= (1ll << 28);
@@ -1164,15 +1165,19 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         SigView sv{G, tp->d_code, tp->d_rule, tp->d_mainchain, tp->d_name_begin, tp->d_names, tp->d_res_begin,
                    tp->d_resnames, tp->d_partner_begin, tp->d_partner_res, tp->d_partner_name};
         int blocks = (int)std::min<int64_t>((W + 7) / 8, (int64_t)sm_count() * 32);
-        launch_candidates(st, std::max(blocks, 1), false, cv, sv, d_count.p, d_scanned.p, nullptr, nullptr);
-        k_struct_totals<<<std::max(1, std::min(S, sm_count() * 8)), 256, 0, st>>>(S, G, d_count.p, d_totals.p);
-        launches += 2;
         if (free_first) {
             CUDA_TRY(dalloc(d_sig_bits, (size_t)G * fv.kind_words, st));
+            CUDA_TRY(dalloc(d_kind_masks, (size_t)W * fv.mask_words, st));
             fv.sig_bits = d_sig_bits.p;
+            fv.kind_masks = d_kind_masks.p;
             launch_sig_kinds(st, sv, fv, d_sig_bits.p);
+            launch_list_kinds(st, cv, sv, fv, d_count.p, d_scanned.p, d_kind_masks.p);
             launches++;
+        } else {
+            launch_candidates(st, std::max(blocks, 1), false, cv, sv, d_count.p, d_scanned.p, nullptr, nullptr);
         }
+        k_struct_totals<<<std::max(1, std::min(S, sm_count() * 8)), 256, 0, st>>>(S, G, d_count.p, d_totals.p);
+        launches += 2;
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(totals.data(), d_totals.p, sizeof(int64_t) * S, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
@@ -1291,6 +1296,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                        tp->d_resnames, tp->d_partner_begin, tp->d_partner_res, tp->d_partner_name};
             int32_t *cnt_c = d_count.p + (int64_t)s0 * G;
             int32_t *scn_c = d_scanned.p + (int64_t)s0 * G;
+            if (free_first) fv.kind_masks = d_kind_masks.p + (int64_t)s0 * G * fv.mask_words;
             CUDA_TRY(dalloc(d_offset, (size_t)Wc, st));
             CUDA_TRY(cudaEventRecord(ev[1], st));
             CUDA_TRY(scan_exclusive(cnt_c, Wc, d_offset.p, scan_tmp, st));
@@ -1854,14 +1860,12 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 }
                 if ((int64_t)nc <= c_cap) {
                     if (free_chunk && free_n[6]) {
-                        if (free_n[1]) {
-                            CUDA_TRY(dalloc(d_row_key, (size_t)nc, st));
-                            CUDA_TRY(dalloc(d_row_scratch, 5 * (size_t)nc, st));
-                            CUDA_TRY(dalloc(d_large_units, (size_t)free_n[6], st));
-                            fw.row_key = d_row_key.p;
-                            fw.row_scratch = d_row_scratch.p;
-                            fw.large_units = d_large_units.p;
-                        }
+                        CUDA_TRY(dalloc(d_row_key, (size_t)nc, st));
+                        CUDA_TRY(dalloc(d_row_scratch, 5 * (size_t)nc, st));
+                        CUDA_TRY(dalloc(d_large_units, (size_t)free_n[6], st));
+                        fw.row_key = d_row_key.p;
+                        fw.row_scratch = d_row_scratch.p;
+                        fw.large_units = d_large_units.p;
                         launch_unit_order(st, (int64_t)free_n[6], cv, tv, cd, sv, sp->d_res_place, P->reorder, fw, cr);
                         launches++;
                         CUDA_TRY(cudaGetLastError());
@@ -2063,7 +2067,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
 
 done:
     if (st) {
-        dfree(d_sig_bits, st); dfree(d_units, st); dfree(d_heavy_pairs, st); dfree(d_free_n, st);
+        dfree(d_sig_bits, st); dfree(d_kind_masks, st); dfree(d_units, st); dfree(d_heavy_pairs, st); dfree(d_free_n, st);
         dfree(d_heavy_stats, st); dfree(d_row_key, st); dfree(d_items, st); dfree(d_results, st);
         dfree(d_item_base, st); dfree(d_bin_off, st); dfree(d_bins, st); dfree(d_arena_atom, st);
         dfree(d_row_scratch, st); dfree(d_arena_xyz, st); dfree(d_arena_parent, st); dfree(d_item_head, st);

@@ -133,6 +133,8 @@ struct FreeView {
     const uint32_t *kind_name;      // [n_kinds]
     const uint32_t *kind_res;
     const uint32_t *sig_bits;       // [G * kind_words] kinds of each signature's list
+    int32_t mask_words;             // words of the structures' local kinds
+    const uint32_t *kind_masks;     // [lists * mask_words] local kinds of each list
     const int32_t *nh_kind;         // kind of each nh_* entry (global index)
     const float4 *kxyz;             // xyz32 in nh_pos order
     // atoms by residue: sorted by key (residue number, chainID2), so the

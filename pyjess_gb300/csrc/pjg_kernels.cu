@@ -3986,10 +3986,14 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
 // children than HEAVY_CAP has room for, and points whose decision needs the
 // kd-tree (outside an annulus box by rounding).
 //
-// Bound by issue slots.  Measured on 1,000 structures x 4,000 templates:
-// 68 ms for both instances and 9 ms for the rows' order, with 0.84 M lists put
-// in leaf order; the search in order took 214 ms with 12.6 M lists ordered
-// (whole query 398 -> 131 ms).
+// Every test of a chain runs on a full warp: candidates (of a residue, or that
+// passed the parent's own test) are queued with their parents, 32 a batch.
+//
+// Bound by issue slots and the latency of the pair's dependent loads.
+// Measured on 1,000 structures x 4,000 templates: 29 + 13 ms for the two
+// instances (with FREE_CAP 192 26 + 18; without the queue, and with the
+// kinds of a list looked up 32 at a time instead of read as a mask, 44 + 22);
+// the search in order took 214 ms with 12.6 M lists put in leaf order.
 
 template <int CAP>
 struct FreeState {
@@ -4001,9 +4005,10 @@ struct FreeState {
     int4 rule[32];              // residue / chain rule to it: key bits that must be
                                 //   equal (x), that must differ somewhere (y; z = 1: no such bits)
     int32_t order[32], tkey[32], sig[32];
-    uint32_t mask[FREE_MAX_KINDS / 32];  // local kinds of the new level's signature
-    int32_t cq[64];             // queued candidates: kxyz or residue-order positions
-    uint16_t pq[64];            //   their parents (residue candidates)
+    uint32_t mask[FREE_MAX_KINDS / 32];  // local kinds of the new level's list
+    int32_t cq[64];             // queued candidates: atoms
+    uint16_t pq[64];            //   their parents
+    uint16_t sq[32];
 };
 
 // check_pair as two bit masks over the XOR of two structure keys
@@ -4048,6 +4053,108 @@ __global__ void k_sig_kinds(SigView sv, FreeView fv, uint32_t *sig_bits) {
         }
         const unsigned m = __ballot_sync(FULL_MASK, ok);
         if (lane == 0) sig_bits[w] = m;
+    }
+}
+
+// Lists of the order-free search: thread per (structure, signature), the
+// local kinds of the structure that the list takes (a bit each, kind_masks)
+// and the list's length, the sum of their atoms; `scanned` as
+// k_candidate_counts.  The threads of a warp share a structure, so its kinds
+// are read once for all; their signatures' bits are staged in shared memory.
+constexpr int LIST_KINDS_THREADS = 128;
+constexpr int LIST_KINDS_WORDS = 16;  // signature words staged (more: read from global memory)
+
+__global__ void __launch_bounds__(LIST_KINDS_THREADS)
+    k_list_kinds(ChunkView cv, SigView sv, FreeView fv, int32_t *count, int32_t *scanned, uint32_t *masks) {
+    __shared__ uint32_t bits[LIST_KINDS_WORDS][LIST_KINDS_THREADS];
+    const int64_t total = (int64_t)cv.n_structures * sv.n_sigs;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const bool staged = fv.kind_words <= LIST_KINDS_WORDS;
+    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += stride) {
+        const int s = (int)(w / sv.n_sigs), g = (int)(w % sv.n_sigs);
+        const uint32_t *sb = fv.sig_bits + (int64_t)g * fv.kind_words;
+        if (staged)
+            for (int i = 0; i < fv.kind_words; i++) bits[i][threadIdx.x] = sb[i];
+        const int b0 = cv.bucket_begin[s], b1 = cv.bucket_begin[s + 1];
+        const int q0 = cv.nh_begin[b0], nk = cv.nh_begin[b1] - q0;
+        int cnt = 0;
+        for (int i = 0; i < fv.mask_words; i++) {
+            uint32_t m = 0;
+            const int lim = min(32, nk - 32 * i);
+#pragma unroll 4
+            for (int b = 0; b < lim; b++) {
+                const int q = q0 + 32 * i + b, k = fv.nh_kind[q];
+                const uint32_t v = staged ? bits[k >> 5][threadIdx.x] : sb[k >> 5];
+                if ((v >> (k & 31)) & 1u) {
+                    m |= 1u << b;
+                    cnt += cv.nh_count[q];
+                }
+            }
+            masks[w * fv.mask_words + i] = m;
+        }
+        int sc = 0;
+        const int code = sv.code[g];
+        if (code >= -1 && code <= 8) {
+            for (int ri = sv.res_begin[g]; ri < sv.res_begin[g + 1]; ri++) {
+                const uint32_t rn = sv.resnames[ri];
+                int b = b0;
+                while (b < b1 && cv.bucket_name[b] != rn) b++;
+                if (b < b1) sc += cv.bucket_hi[b] - cv.bucket_lo[b];
+            }
+        } else {
+            sc = cv.atom_count[s];
+        }
+        count[w] = cnt;
+        scanned[w] = sc;
+    }
+}
+
+// The atoms of a list 32 at a time, in kind order: `use(valid, pos)` with the
+// lane's position in the structure's kind order (kxyz, nh_pos).  mask: the
+// list's kind_masks; sq: 32 shared entries of the warp.
+template <typename Use>
+__device__ __forceinline__ void for_list(const ChunkView &cv, const uint32_t *mask, int words, int q0, uint16_t *sq,
+                                         Use use) {
+    const int lane = lane_id();
+    const uint32_t mine = lane < words ? mask[lane] : 0u;
+    int pre = __popc(mine);
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL_MASK, pre, o);
+        if (lane >= o) pre += y;
+    }
+    const int nseg = __shfl_sync(FULL_MASK, pre, 31);
+    pre -= __popc(mine);
+    for (int base = 0; base < nseg; base += 32) {
+        // kinds base .. base + 31 of the list, one a lane
+        __syncwarp();
+        int at = pre - base;
+        for (uint32_t m = mine; m && at < 32; m &= m - 1, at++)
+            if (at >= 0) sq[at] = (uint16_t)(32 * lane + __ffs(m) - 1);
+        __syncwarp();
+        const int ns = min(32, nseg - base);
+        int off = 0, cnt = 0;
+        if (lane < ns) {
+            const int q = q0 + sq[lane];
+            off = cv.nh_off[q];
+            cnt = cv.nh_count[q];
+        }
+        int cum = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(FULL_MASK, cum, o);
+            if (lane >= o) cum += y;
+        }
+        const int tot = __shfl_sync(FULL_MASK, cum, 31);
+        cum -= cnt;
+        off -= cum;
+        int started = 0;  // kinds that begin before the window
+        for (int t0 = 0; t0 < tot; t0 += 32) {
+            const unsigned at0 = (unsigned)(cum - t0);
+            const unsigned begins = __reduce_or_sync(FULL_MASK, lane < ns && at0 < 32u ? 1u << at0 : 0u);
+            const int seg = started + __popc(begins & (0xFFFFFFFFu >> (31 - lane))) - 1;
+            const int pos = __shfl_sync(FULL_MASK, off, seg) + t0 + lane;
+            if (!use(t0 + lane < tot, pos)) return;
+            started += __popc(begins);
+        }
     }
 }
 
@@ -4188,19 +4295,10 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
         const double *xyz64 = cv.xyz64 + 3 * abase;
         const float4 *kx = fv.kxyz + abase;
         const int q0 = cv.nh_begin[cv.bucket_begin[s]];
-        const int nk = cv.nh_begin[cv.bucket_begin[s + 1]] - q0;  // local kinds
         const int m0 = __shfl_sync(FULL_MASK, llen, 0);
 
-        // local kinds 32 w .. 32 w + 31 that the list of signature g takes
-        auto kind_bits = [&](int g, int w) -> unsigned {
-            const int q = 32 * w + lane;
-            bool ok = false;
-            if (q < nk) {
-                const int k = fv.nh_kind[q0 + q];
-                ok = (fv.sig_bits[(int64_t)g * fv.kind_words + (k >> 5)] >> (k & 31)) & 1u;
-            }
-            return __ballot_sync(FULL_MASK, ok);
-        };
+        const int mw = fv.mask_words;
+        const uint32_t *masks = fv.kind_masks + wb * mw;
 
         bool kd_needed = n == 1;  // (the one-level scanner drops its first candidate: k_search)
         bool outgrown = !HEAVY && m0 > CAP / 2;
@@ -4242,26 +4340,15 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                 }
             } else {
                 int at = 0;
-                for (int w = 0; 32 * w < nk && at < k0; w++) {
-                    unsigned bits = kind_bits(st.sig[0], w);
-                    int cnt = 0, off = 0;
-                    if ((bits >> lane) & 1u) {
-                        cnt = cv.nh_count[q0 + 32 * w + lane];
-                        off = cv.nh_off[q0 + 32 * w + lane];
+                for_list(cv, masks + (int64_t)st.sig[0] * mw, mw, q0, st.sq, [&](bool valid, int pos) {
+                    if (valid && at + lane < k0) {
+                        exyz[at + lane] = kx[pos];
+                        eatom[at + lane] = cv.nh_pos[abase + pos];
+                        eparent[at + lane] = 0;
                     }
-                    while (bits) {
-                        const int b = __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        const int cb = __shfl_sync(FULL_MASK, cnt, b), ob = __shfl_sync(FULL_MASK, off, b);
-                        for (int i = lane; i < cb; i += 32) {
-                            if (at + i >= k0) break;
-                            exyz[at + i] = kx[ob + i];
-                            eatom[at + i] = cv.nh_pos[abase + ob + i];
-                            eparent[at + i] = 0;
-                        }
-                        at += cb;
-                    }
-                }
+                    at += __popc(__ballot_sync(FULL_MASK, valid));
+                    return true;
+                });
             }
             __syncwarp();
             if (lane == 0) {
@@ -4340,47 +4427,34 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                         nend += np;
                     }
                 };
+                // queued (parent, candidate) pairs in batches of 32, a pair a
+                // lane: the whole chain tested (taken from the queue's end: no
+                // order to keep)
+                int queued = 0;
+                auto run_batch = [&](int k) {
+                    queued -= k;
+                    bool pass = lane < k;
+                    unsigned exact = 0;
+                    const int p = pass ? st.pq[queued + lane] : 0;
+                    const int32_t an = pass ? st.cq[queued + lane] : 0;
+                    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (pass) {
+                        x = cv.xyz32[abase + an];
+                        for (int j = lev, e = p; j >= 0; j--, e = eparent[e])
+                            if (!test(exyz[e], x, st.rule[j], st.thr[j], j, exact)) {
+                                pass = false;
+                                break;
+                            }
+                    }
+                    accept(pass, exact, p, an, x);
+                    __syncwarp();
+                };
                 if (same) {
                     // ---- the atoms of the placed residue
                     const int anchor = 31 - __clz(same);
                     const bool by_number = sa.ignore_chain == 2;
-                    for (int w = 0; 32 * w < nk; w++) {
-                        const unsigned bits = kind_bits(g, w);
-                        if (lane == 0) st.mask[w] = bits;
-                    }
+                    if (lane < mw) st.mask[lane] = masks[(int64_t)g * mw + lane];
                     __syncwarp();
-                    int queued = 0;
-                    auto run_batch = [&](int k) {
-                        bool pass = lane < k;
-                        unsigned exact = 0;
-                        const int p = pass ? st.pq[lane] : 0;
-                        int32_t an = 0;
-                        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (pass) {
-                            an = fv.res_pos[abase + st.cq[lane]];
-                            x = cv.xyz32[abase + an];
-                            for (int j = lev, e = p; j >= 0; j--, e = eparent[e])
-                                if (!test(exyz[e], x, st.rule[j], st.thr[j], j, exact)) {
-                                    pass = false;
-                                    break;
-                                }
-                        }
-                        accept(pass, exact, p, an, x);
-                        const int rest = queued - k;
-                        int qc = 0;
-                        uint16_t qp = 0;
-                        if (lane < rest) {
-                            qc = st.cq[k + lane];
-                            qp = st.pq[k + lane];
-                        }
-                        __syncwarp();
-                        if (lane < rest) {
-                            st.cq[lane] = qc;
-                            st.pq[lane] = qp;
-                        }
-                        __syncwarp();
-                        queued = rest;
-                    };
                     for (int p0 = beg; p0 < end && !full && !kd_needed; p0 += 32) {
                         const int p = p0 + lane;
                         int first = 0, cnt = 0;
@@ -4392,76 +4466,60 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                             cnt = by_number ? r.w : r.y;
                         }
                         const int most = __reduce_max_sync(FULL_MASK, cnt);
-                        for (int i = 0; i < most && !full && !kd_needed; i++) {
-                            bool match = false;
-                            if (i < cnt) {
-                                const int lk = fv.res_kind[abase + first + i];
-                                match = (st.mask[lk >> 5] >> (lk & 31)) & 1u;
+                        for (int i0 = 0; i0 < most; i0 += 32) {
+                            // which of the residue's atoms the list takes
+                            const uint16_t *rk = fv.res_kind + abase + first + i0;
+                            const int lim = min(32, most - i0), ci = cnt - i0;
+                            unsigned match = 0;
+#pragma unroll 4
+                            for (int i = 0; i < lim; i++) {
+                                if (i >= ci) continue;
+                                const int lk = rk[i];
+                                match |= ((st.mask[lk >> 5] >> (lk & 31)) & 1u) << i;
                             }
-                            const unsigned m = __ballot_sync(FULL_MASK, match);
-                            if (match) {
-                                const int qi = queued + __popc(m & lt);
-                                st.cq[qi] = first + i;
-                                st.pq[qi] = (uint16_t)p;
-                            }
-                            queued += __popc(m);
-                            __syncwarp();
-                            if (queued >= 32) run_batch(32);
-                        }
-                    }
-                    if (queued > 0 && !full && !kd_needed) run_batch(queued);
-                } else {
-                    // ---- the whole list, 32 candidates against every parent
-                    const float4 thr_p = st.thr[lev];
-                    const int4 rule_p = st.rule[lev];
-                    int queued = 0;
-                    auto run_batch = [&](int k) {
-                        const int ci = lane < k ? st.cq[lane] : 0;
-                        const float4 x = lane < k ? kx[ci] : make_float4(0.f, 0.f, 0.f, 0.f);
-                        int32_t an = -1;
-                        for (int p = beg; p < end && !full && !kd_needed; p++) {
-                            unsigned exact = 0;
-                            bool pass = lane < k && test(exyz[p], x, rule_p, thr_p, lev, exact);
-                            if (!__any_sync(FULL_MASK, pass)) continue;
-                            int e = p;
-                            for (int j = lev - 1; j >= 0; j--) {
-                                e = eparent[e];
-                                pass = pass && test(exyz[e], x, st.rule[j], st.thr[j], j, exact);
-                                if (!__any_sync(FULL_MASK, pass)) break;
-                            }
-                            if (!__any_sync(FULL_MASK, pass)) continue;
-                            if (an < 0 && lane < k) an = cv.nh_pos[abase + ci];
-                            accept(pass, exact, p, an, x);
-                        }
-                        const int rest = queued - k;
-                        const int qc = lane < rest ? st.cq[k + lane] : 0;
-                        __syncwarp();
-                        if (lane < rest) st.cq[lane] = qc;
-                        __syncwarp();
-                        queued = rest;
-                    };
-                    for (int w = 0; 32 * w < nk && !full && !kd_needed; w++) {
-                        unsigned bits = kind_bits(g, w);
-                        int cnt = 0, off = 0;
-                        if ((bits >> lane) & 1u) {
-                            cnt = cv.nh_count[q0 + 32 * w + lane];
-                            off = cv.nh_off[q0 + 32 * w + lane];
-                        }
-                        while (bits && !full && !kd_needed) {
-                            const int b = __ffs(bits) - 1;
-                            bits &= bits - 1;
-                            const int cb = __shfl_sync(FULL_MASK, cnt, b), ob = __shfl_sync(FULL_MASK, off, b);
-                            for (int i0 = 0; i0 < cb && !full && !kd_needed; i0 += 32) {
-                                const int k = min(32, cb - i0);
-                                if (lane < k) st.cq[queued + lane] = ob + i0 + lane;
-                                queued += k;
+                            // queued one a lane at a time
+                            for (unsigned m; !full && !kd_needed && (m = __ballot_sync(FULL_MASK, match != 0)) != 0;
+                                 match &= match - 1) {
+                                if (match) {
+                                    const int qi = queued + __popc(m & lt);
+                                    st.cq[qi] = fv.res_pos[abase + first + i0 + __ffs(match) - 1];
+                                    st.pq[qi] = (uint16_t)p;
+                                }
+                                queued += __popc(m);
                                 __syncwarp();
                                 if (queued >= 32) run_batch(32);
                             }
                         }
                     }
-                    if (queued > 0 && !full && !kd_needed) run_batch(queued);
+                } else {
+                    // ---- the whole list, 32 candidates against every parent;
+                    // those that pass the parent's own test are queued
+                    const float4 thr_p = st.thr[lev];
+                    const int4 rule_p = st.rule[lev];
+                    for_list(cv, masks + (int64_t)g * mw, mw, q0, st.sq, [&](bool valid, int pos) {
+                        const float4 x = valid ? kx[pos] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        const int32_t an = valid ? cv.nh_pos[abase + pos] : 0;
+                        for (int p = beg; p < end; p++) {
+                            unsigned exact = 0;
+                            const bool near = valid && test(exyz[p], x, rule_p, thr_p, lev, exact);
+                            const unsigned m = __ballot_sync(FULL_MASK, near);
+                            if (!m) continue;
+                            if (near) {
+                                const int qi = queued + __popc(m & lt);
+                                st.cq[qi] = an;
+                                st.pq[qi] = (uint16_t)p;
+                            }
+                            queued += __popc(m);
+                            __syncwarp();
+                            if (queued >= 32) {
+                                run_batch(32);
+                                if (full || kd_needed) return false;
+                            }
+                        }
+                        return true;
+                    });
                 }
+                if (queued > 0 && !full && !kd_needed) run_batch(queued);
                 __syncwarp();
             }
             if (kd_needed) break;
@@ -4734,7 +4792,8 @@ __global__ void k_heavy_rows(int32_t n_heavy, const HeavyPair *heavy, const int2
 // level by level.  Units of at most UNIT_ROWS rows: a warp each, every row
 // counting the rows with smaller keys; larger ones are listed for
 // k_unit_order_large.
-constexpr int UNIT_ROWS = 192;   // rows whose keys shared memory holds
+constexpr int UNIT_ROWS = 256;   // rows whose keys shared memory holds
+static_assert(UNIT_ROWS >= FREE_CAP, "the first instance's units are never large");
 constexpr int UNIT_SLOTS = 512;  // hash slots for the atoms of that many rows
 constexpr int UNIT_WARPS = 4;
 constexpr int UNIT_HASH_FROM = 9;  // fewer rows are compared with every leaf
@@ -4897,6 +4956,7 @@ struct DirectWarp {
     int32_t cur[UNIT_ROWS], atom[UNIT_ROWS], row[UNIT_ROWS];
     uint32_t code[UNIT_ROWS];  // path from the root: a bit a split, 0 right (reported first)
     uint16_t node[UNIT_ROWS];  // node the row's atom is in
+    uint16_t sq[32];
     int32_t mem[2][MAXM];      // the nodes' atoms, children in the other buffer
     uint32_t rk[MAXM];         // ranks of the node being split
     alignas(16) int32_t bins[128];
@@ -4972,7 +5032,6 @@ __global__ void __launch_bounds__(WARPS * 32)
         }
         __syncwarp();
         const int q0 = cv.nh_begin[cv.bucket_begin[s]];
-        const int nk = cv.nh_begin[cv.bucket_begin[s + 1]] - q0;
         for (unsigned left = pending ? 0u : branch; left && !pending; left &= left - 1) {
             const int l = __ffs(left) - 1;
             const int k = U.order[l], g = U.sig[l];
@@ -4988,23 +5047,12 @@ __global__ void __launch_bounds__(WARPS * 32)
                 }
                 // the list's atoms (in any order: splits read sets)
                 int m = 0;
-                for (int w0 = 0; 32 * w0 < nk; w0++) {
-                    const int q = 32 * w0 + lane;
-                    bool ok = false;
-                    if (q < nk) {
-                        const int kd = fv.nh_kind[q0 + q];
-                        ok = (fv.sig_bits[(int64_t)g * fv.kind_words + (kd >> 5)] >> (kd & 31)) & 1u;
-                    }
-                    unsigned bits = __ballot_sync(FULL_MASK, ok);
-                    const int cnt = ok ? cv.nh_count[q0 + q] : 0, off = ok ? cv.nh_off[q0 + q] : 0;
-                    for (; bits; bits &= bits - 1) {
-                        const int b = __ffs(bits) - 1;
-                        const int cb = __shfl_sync(FULL_MASK, cnt, b), ob = __shfl_sync(FULL_MASK, off, b);
-                        for (int i = lane; i < cb; i += 32)
-                            if (m + i < MAXM) U.mem[0][m + i] = cv.nh_pos[abase + ob + i];
-                        m += cb;
-                    }
-                }
+                for_list(cv, fv.kind_masks + (wb + g) * fv.mask_words, fv.mask_words, q0, U.sq,
+                         [&](bool valid, int pos) {
+                             if (valid && m + lane < MAXM) U.mem[0][m + lane] = cv.nh_pos[abase + pos];
+                             m += __popc(__ballot_sync(FULL_MASK, valid));
+                             return true;
+                         });
                 m = min(m, MAXM);
                 int sp = 1, nodes = 1;
                 if (lane == 0) U.stack[0] = make_int4(0, m, 0, 0);
@@ -5929,6 +5977,13 @@ static cudaError_t free_grid(const void *kern, int smem, int64_t items, int64_t 
     return cudaSuccess;
 }
 
+void launch_list_kinds(cudaStream_t st, const ChunkView &cv, const SigView &sv, const FreeView &fv, int32_t *count,
+                       int32_t *scanned, uint32_t *masks) {
+    const int64_t n = (int64_t)cv.n_structures * sv.n_sigs;
+    const int64_t blocks = std::min<int64_t>((n + LIST_KINDS_THREADS - 1) / LIST_KINDS_THREADS, 152 * 64);
+    if (n > 0) k_list_kinds<<<(int)blocks, LIST_KINDS_THREADS, 0, st>>>(cv, sv, fv, count, scanned, masks);
+}
+
 cudaError_t launch_search_free(cudaStream_t st, bool fp32, const ChunkView &cv, const TemplateView &tv,
                                const CandView &cd, const FreeView &fv, const SearchArgs &sa, int32_t *item_counter,
                                const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
@@ -6011,8 +6066,7 @@ void launch_unit_order(cudaStream_t st, int64_t n_pending, const ChunkView &cv, 
                        const FreeWork &fw, const CompleteRows &out) {
     const int64_t blocks = std::min<int64_t>((n_pending + UNIT_WARPS - 1) / UNIT_WARPS, 152 * 16);
     k_unit_order<<<(int)blocks, UNIT_WARPS * 32, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
-    if (fw.row_scratch)
-        k_unit_order_large<<<152 * 4, UNIT_LARGE_THREADS, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
+    k_unit_order_large<<<152 * 4, UNIT_LARGE_THREADS, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
 }
 
 cudaError_t launch_search_large(cudaStream_t st, const ChunkView &cv, const TemplateView &tv, const CandView &cd,

@@ -31,7 +31,7 @@ constexpr int SEARCH_WARPS = PJG_SEARCH_WARPS;  // warps per block of k_search
 #define PJG_FREE_MIN_BLOCKS 3
 #endif
 #ifndef PJG_FREE_CAP
-#define PJG_FREE_CAP 192
+#define PJG_FREE_CAP 256
 #endif
 constexpr int FREE_WARPS = PJG_FREE_WARPS;
 constexpr int FREE_CAP = PJG_FREE_CAP;
@@ -334,7 +334,7 @@ struct FreeWork {
     unsigned long long *n_large_units;
     unsigned long long *scratch_used;
     unsigned long long *row_key;
-    int32_t *row_scratch;              // [5 * rows] (nullptr: no unit can be that large)
+    int32_t *row_scratch;              // [5 * rows]
 };
 
 // Superposition of every complete row, in reference order: row i of pair
@@ -463,6 +463,10 @@ void launch_axis_ranks(cudaStream_t st, int32_t n_structures, const int64_t *ato
 
 // sig_bits of FreeView: the kinds of every signature's list
 void launch_sig_kinds(cudaStream_t st, const SigView &sv, const FreeView &fv, uint32_t *sig_bits);
+
+// kind_masks, lengths and scanned atoms of every list
+void launch_list_kinds(cudaStream_t st, const ChunkView &cv, const SigView &sv, const FreeView &fv, int32_t *count,
+                       int32_t *scanned, uint32_t *masks);
 
 // the order-free search over every pair: rows and units of rows to put in
 // order (fw), pairs to search in items (fw.heavy), and the pairs left to
