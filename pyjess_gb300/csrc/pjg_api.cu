@@ -88,44 +88,255 @@ inline uint32_t pack_upper(const uint8_t *b) {
 
 inline uint32_t pack_lit(const char *s) { return pack_upper((const uint8_t *)s); }
 
+// Small device blocks kept between the queries that share a stream: by power
+// of two from 256 B to 4 MiB, reused in stream order.  A query takes some 60
+// buffers; from the allocator they cost it about 0.2 ms.
+struct BlockCache {
+    static constexpr int CLASSES = 15;
+    std::vector<void *> idle[CLASSES];
+    static int class_of(size_t bytes) {
+        int c = 0;
+        while (c < CLASSES && (size_t(256) << c) < bytes) c++;
+        return c < CLASSES ? c : -1;
+    }
+};
+// the cache of the query running on this thread (nullptr: none)
+thread_local BlockCache *t_cache = nullptr;
+
 // device buffer helper (stream ordered)
 template <typename T>
 struct DBuf {
     T *p = nullptr;
     size_t n = 0;
+    int cls = -1;  // class of a cached block
 };
+
+template <typename T>
+void dfree(DBuf<T> &b, cudaStream_t st) {
+    if (b.p && b.cls >= 0) t_cache->idle[b.cls].push_back(b.p);
+    else if (b.p) cudaFreeAsync(b.p, st);
+    b.p = nullptr;
+    b.n = 0;
+    b.cls = -1;
+}
 
 template <typename T>
 cudaError_t dalloc(DBuf<T> &b, size_t n, cudaStream_t st) {
     if (b.n >= n && b.p) return cudaSuccess;
-    if (b.p) cudaFreeAsync(b.p, st);
-    b.p = nullptr;
-    b.n = 0;
-    size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-    cudaError_t e = cudaMallocAsync((void **)&b.p, bytes, st);
-    if (e == cudaSuccess) b.n = std::max<size_t>(n, 1);
-    return e;
+    dfree(b, st);
+    n = std::max<size_t>(n, 1);
+    const size_t bytes = n * sizeof(T);
+    const int c = t_cache ? BlockCache::class_of(bytes) : -1;
+    if (c >= 0 && !t_cache->idle[c].empty()) {
+        b.p = (T *)t_cache->idle[c].back();
+        t_cache->idle[c].pop_back();
+    } else {
+        cudaError_t e = cudaMallocAsync((void **)&b.p, c >= 0 ? size_t(256) << c : bytes, st);
+        if (e != cudaSuccess) {
+            b.p = nullptr;
+            return e;
+        }
+    }
+    b.n = n;
+    b.cls = c;
+    return cudaSuccess;
 }
 
-template <typename T>
-void dfree(DBuf<T> &b, cudaStream_t st) {
-    if (b.p) cudaFreeAsync(b.p, st);
-    b.p = nullptr;
-    b.n = 0;
+// Keep the stream-ordered pool's memory mapped between calls (up to half the
+// device) instead of returning it at every sync: the next call's buffers then
+// need no new mappings.
+void keep_pool(int device) {
+    static std::mutex m;
+    static bool done[256] = {};
+    std::lock_guard<std::mutex> g(m);
+    if (device < 0 || device >= 256 || done[device]) return;
+    cudaMemPool_t pool;
+    size_t fb = 0, tb = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess && cudaMemGetInfo(&fb, &tb) == cudaSuccess) {
+        uint64_t thr = tb / 2;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
+    }
+    cudaGetLastError();
+    done[device] = true;
 }
 
-template <typename T>
-cudaError_t upload(T **dst, const T *src, size_t n) {
-    cudaError_t e = cudaMalloc((void **)dst, std::max<size_t>(n, 1) * sizeof(T));
-    if (e != cudaSuccess) return e;
-    if (n) e = cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice);
-    return e;
+// What a call on a device needs and the next one can take over: a stream,
+// events, a pinned buffer and the stream's small blocks.  Idle ones are kept
+// (at most IDLE_MAX, with at most CACHE_MAX bytes of blocks each) while any
+// template or structure handle lives; one call has one to itself.  One whose
+// CUDA context has been reset is forgotten.
+struct Scratch {
+    static constexpr size_t PINNED = 1 << 20;
+    int device = 0;
+    unsigned long long ctx = 0;
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev[8] = {};
+    unsigned char *pinned = nullptr;
+    BlockCache cache;
+
+    cudaError_t create(int dev) {
+        device = dev;
+        ctx = current_context_id();
+        cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        for (auto &v : ev)
+            if (e == cudaSuccess) e = cudaEventCreate(&v);
+        if (e == cudaSuccess) e = cudaMallocHost((void **)&pinned, PINNED);
+        return e;
+    }
+    // blocks beyond `most` bytes back to the allocator, the largest first
+    void trim(size_t most) {
+        size_t held = 0;
+        for (int c = 0; c < BlockCache::CLASSES; c++) held += cache.idle[c].size() * (size_t(256) << c);
+        for (int c = BlockCache::CLASSES - 1; c >= 0; c--)
+            while (held > most && !cache.idle[c].empty()) {
+                cudaFreeAsync(cache.idle[c].back(), st);
+                cache.idle[c].pop_back();
+                held -= size_t(256) << c;
+            }
+    }
+    void destroy() {
+        if (st) {
+            trim(0);
+            cudaStreamSynchronize(st);
+            cudaStreamDestroy(st);
+        }
+        for (auto &v : ev)
+            if (v) cudaEventDestroy(v);
+        if (pinned) cudaFreeHost(pinned);
+    }
+};
+
+// a handle's or a result's device block back to its device's pool
+void free_block(void *block, int device) {
+    if (!block) return;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev != device) cudaSetDevice(device);
+    cudaFreeAsync(block, nullptr);
+    if (dev != device) cudaSetDevice(dev);
 }
 
-template <typename T>
-cudaError_t upload(T **dst, const std::vector<T> &v) {
-    return upload(dst, v.data(), v.size());
+constexpr size_t IDLE_MAX = 8, CACHE_MAX = 64 << 20;
+std::mutex g_scratch_mutex;
+std::vector<Scratch *> g_idle;   // guarded by g_scratch_mutex
+int g_handles = 0;               // live template and structure handles (guarded likewise)
+
+// a scratch of the current device, idle; nullptr with *e set on failure
+Scratch *acquire_scratch(int device, cudaError_t *e) {
+    const unsigned long long ctx = current_context_id();
+    *e = cudaSuccess;
+    {
+        std::lock_guard<std::mutex> g(g_scratch_mutex);
+        for (size_t i = g_idle.size(); i-- > 0;) {
+            Scratch *x = g_idle[i];
+            if (x->device != device) continue;
+            g_idle.erase(g_idle.begin() + (long)i);
+            if (ctx != 0 && x->ctx == ctx) return x;
+            delete x;  // its context is gone, its stream and memory with it
+        }
+    }
+    Scratch *x = new Scratch;
+    *e = x->create(device);
+    if (*e == cudaSuccess) return x;
+    x->destroy();
+    delete x;
+    return nullptr;
 }
+
+// back to the idle ones (its stream idle); `reuse` false: after an error
+void release_scratch(Scratch *x, bool reuse) {
+    if (!x) return;
+    if (reuse) {
+        x->trim(CACHE_MAX);
+        std::lock_guard<std::mutex> g(g_scratch_mutex);
+        if (g_handles > 0 && g_idle.size() < IDLE_MAX) {
+            g_idle.push_back(x);
+            return;
+        }
+    }
+    x->destroy();
+    delete x;
+}
+
+void handle_created() {
+    std::lock_guard<std::mutex> g(g_scratch_mutex);
+    g_handles++;
+}
+
+// the last handle gone: the idle scratch is given back
+void handle_destroyed() {
+    std::vector<Scratch *> out;
+    {
+        std::lock_guard<std::mutex> g(g_scratch_mutex);
+        if (--g_handles == 0) out.swap(g_idle);
+    }
+    const unsigned long long ctx = out.empty() ? 0 : current_context_id();
+    int dev = 0;
+    if (!out.empty()) cudaGetDevice(&dev);
+    for (Scratch *x : out) {
+        // (another device's or context's: dropped with its context)
+        if (x->device != dev) {
+            cudaSetDevice(x->device);
+            if (current_context_id() == x->ctx) x->destroy();
+            cudaSetDevice(dev);
+        } else if (x->ctx == ctx) {
+            x->destroy();
+        }
+        delete x;
+    }
+}
+
+// Arrays uploaded into one device block: one allocation, and one copy through
+// the pinned buffer when they fit it.
+struct Upload {
+    struct Item {
+        void **dst;
+        const void *src;  // nullptr: room only
+        size_t bytes, at;
+    };
+    std::vector<Item> items;
+    size_t total = 0;
+
+    template <typename T, typename U>
+    void add(T **dst, const U *src, size_t n) {
+        static_assert(sizeof(T) == sizeof(U), "element size");
+        const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+        items.push_back({(void **)dst, n ? (const void *)src : nullptr, bytes, total});
+        total += (bytes + 255) & ~size_t(255);
+    }
+    template <typename T>
+    void add(T **dst, const std::vector<T> &v) {
+        add(dst, v.data(), v.size());
+    }
+    template <typename T>
+    void room(T **dst, size_t n) {
+        items.push_back({(void **)dst, nullptr, std::max<size_t>(n, 1) * sizeof(T), total});
+        total += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
+    }
+    // allocates *block and fills it on x's stream (arrays with a source
+    // first, so that they share one copy)
+    cudaError_t run(void **block, Scratch *x) {
+        cudaError_t e = cudaMallocAsync(block, std::max<size_t>(total, 1), x->st);
+        if (e != cudaSuccess) {
+            *block = nullptr;
+            return e;
+        }
+        size_t filled = 0;
+        for (const Item &it : items) {
+            *it.dst = (char *)*block + it.at;
+            if (it.src) filled = it.at + it.bytes;
+        }
+        if (filled <= Scratch::PINNED) {
+            for (const Item &it : items)
+                if (it.src) std::memcpy(x->pinned + it.at, it.src, it.bytes);
+            return cudaMemcpyAsync(*block, x->pinned, filled, cudaMemcpyHostToDevice, x->st);
+        }
+        for (const Item &it : items)
+            if (it.src && e == cudaSuccess)
+                e = cudaMemcpyAsync(*it.dst, it.src, it.bytes, cudaMemcpyHostToDevice, x->st);
+        return e;
+    }
+};
 
 // Host staging array of n elements left uninitialised (every element is
 // written before use; a std::vector would zero it first).
@@ -172,6 +383,8 @@ struct pjg_templates {
     // templates of more than 32 atoms (searched by k_search_large)
     std::vector<int32_t> large;
     int32_t *d_large = nullptr;
+    void *block = nullptr;  // the device arrays
+    bool counted = false;   // a live handle
 };
 
 struct pjg_structures {
@@ -205,6 +418,8 @@ struct pjg_structures {
     uint16_t *d_res_kind = nullptr;
     int4 *d_res_range = nullptr;
     int device = 0;
+    void *block = nullptr;  // the device arrays
+    bool counted = false;   // a live handle
 };
 
 // Hits and warnings of a query, on the device: contiguous arrays that grow
@@ -216,44 +431,52 @@ struct HitStore {
     int64_t *ordinal = nullptr, *atom_offset = nullptr, *warn_before = nullptr;
     double *rmsd = nullptr, *rot = nullptr, *centres = nullptr;
 
-    template <typename T>
-    static cudaError_t grow(T **p, int64_t used, int64_t cap, int64_t width, cudaStream_t st) {
-        T *q = nullptr;
-        cudaError_t e = cudaMalloc((void **)&q, (size_t)std::max<int64_t>(cap, 1) * width * sizeof(T));
-        if (e != cudaSuccess) return e;
-        if (*p && used > 0) e = cudaMemcpyAsync(q, *p, (size_t)used * width * sizeof(T), cudaMemcpyDeviceToDevice, st);
-        if (*p) {
-            cudaStreamSynchronize(st);
-            cudaFree(*p);
-        }
-        *p = q;
-        return e;
-    }
+    void *block = nullptr;                            // the arrays
+
     // room for `h` more hits, `a` more atoms, `w` more warnings
     cudaError_t reserve(int64_t h, int64_t a, int64_t w, cudaStream_t st) {
-        cudaError_t e = cudaSuccess;
-        if (hits + h > cap_h) {
-            int64_t c = std::max<int64_t>(hits + h, 2 * cap_h);
-            if (e == cudaSuccess) e = grow(&structure, hits, c, 1, st);
-            if (e == cudaSuccess) e = grow(&tpl, hits, c, 1, st);
-            if (e == cudaSuccess) e = grow(&ordinal, hits, c, 1, st);
-            if (e == cudaSuccess) e = grow(&atom_offset, hits, c + 1, 1, st);
-            if (e == cudaSuccess) e = grow(&rmsd, hits, c, 1, st);
-            if (e == cudaSuccess) e = grow(&rot, hits, c, 9, st);
-            if (e == cudaSuccess) e = grow(&centres, hits, c, 6, st);
-            if (e == cudaSuccess) cap_h = c;
+        if (block && hits + h <= cap_h && atoms + a <= cap_a && warns + w <= cap_w) return cudaSuccess;
+        auto bigger = [](int64_t need, int64_t cap) { return need <= cap ? cap : std::max<int64_t>(need, 2 * cap); };
+        const int64_t nh = bigger(hits + h, cap_h), na = bigger(atoms + a, cap_a), nw = bigger(warns + w, cap_w);
+        HitStore old = *this;
+        Upload lay;
+        lay.room(&structure, (size_t)nh);
+        lay.room(&tpl, (size_t)nh);
+        lay.room(&ordinal, (size_t)nh);
+        lay.room(&rmsd, (size_t)nh);
+        lay.room(&rot, 9 * (size_t)nh);
+        lay.room(&centres, 6 * (size_t)nh);
+        lay.room(&atom_offset, (size_t)nh + 1);
+        lay.room(&atoms_, (size_t)na);
+        lay.room(&warn_structure, (size_t)nw);
+        lay.room(&warn_before, (size_t)nw);
+        void *b = nullptr;
+        cudaError_t e = cudaMallocAsync(&b, std::max<size_t>(lay.total, 1), st);
+        if (e != cudaSuccess) {
+            old.block = nullptr;  // (still this store's)
+            return e;
         }
-        if (atoms + a > cap_a && e == cudaSuccess) {
-            int64_t c = std::max<int64_t>(atoms + a, 2 * cap_a);
-            e = grow(&atoms_, atoms, c, 1, st);
-            if (e == cudaSuccess) cap_a = c;
-        }
-        if (warns + w > cap_w && e == cudaSuccess) {
-            int64_t c = std::max<int64_t>(warns + w, 2 * cap_w);
-            e = grow(&warn_structure, warns, c, 1, st);
-            if (e == cudaSuccess) e = grow(&warn_before, warns, c, 1, st);
-            if (e == cudaSuccess) cap_w = c;
-        }
+        for (const Upload::Item &it : lay.items) *it.dst = (char *)b + it.at;
+        block = b;
+        cap_h = nh;
+        cap_a = na;
+        cap_w = nw;
+        auto keep = [&](void *to, const void *from, int64_t bytes) {
+            if (e == cudaSuccess && from && bytes > 0)
+                e = cudaMemcpyAsync(to, from, (size_t)bytes, cudaMemcpyDeviceToDevice, st);
+        };
+        keep(structure, old.structure, 4 * hits);
+        keep(tpl, old.tpl, 4 * hits);
+        keep(ordinal, old.ordinal, 8 * hits);
+        keep(rmsd, old.rmsd, 8 * hits);
+        keep(rot, old.rot, 72 * hits);
+        keep(centres, old.centres, 48 * hits);
+        keep(atom_offset, old.atom_offset, 8 * hits);
+        keep(atoms_, old.atoms_, 4 * atoms);
+        keep(warn_structure, old.warn_structure, 4 * warns);
+        keep(warn_before, old.warn_before, 8 * warns);
+        if (old.block) cudaFreeAsync(old.block, st);
+        old.block = nullptr;
         return e;
     }
     // the segment view at the current ends
@@ -263,9 +486,7 @@ struct HitStore {
                           warn_before + warns};
     }
     ~HitStore() {
-        void *ptrs[] = {structure, tpl, atoms_, warn_structure, ordinal, atom_offset, warn_before, rmsd, rot, centres};
-        for (void *p : ptrs)
-            if (p) cudaFree(p);
+        if (block) cudaFreeAsync(block, nullptr);
     }
 };
 
@@ -335,6 +556,28 @@ cudaError_t copy_out_all(const std::vector<CopySeg> &segs_in) {
     unsigned hw = std::thread::hardware_concurrency();
     // one thread per MiB, up to 16 (or the host's cores)
     int threads = (int)std::min<size_t>(std::min<unsigned>(hw ? hw : 1, 16u), total >> 20);
+    if (total <= Scratch::PINNED) {
+        // small: every array into the pinned buffer in stream order, one wait
+        cudaError_t e;
+        Scratch *x = acquire_scratch(device, &e);
+        if (x) {
+            size_t at = 0;
+            for (const CopySeg &sg : segs) {
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(x->pinned + at, sg.src, sg.bytes, cudaMemcpyDeviceToHost, x->st);
+                at += sg.bytes;
+            }
+            const cudaError_t e2 = cudaStreamSynchronize(x->st);
+            if (e == cudaSuccess) e = e2;
+            at = 0;
+            for (const CopySeg &sg : segs) {
+                if (e == cudaSuccess) std::memcpy(sg.dst, x->pinned + at, sg.bytes);
+                at += sg.bytes;
+            }
+            release_scratch(x, e == cudaSuccess);
+        }
+        return e;
+    }
     if (threads <= 1) {
         for (const CopySeg &sg : segs) {
             cudaError_t e = cudaMemcpy(sg.dst, sg.src, sg.bytes, cudaMemcpyDeviceToHost);
@@ -507,25 +750,35 @@ pjg_status pjg_templates_create(const pjg_template_set *set, pjg_templates **out
     h->n_params = (int64_t)dist.size();
     if (set->dim) h->dim.assign(set->dim, set->dim + T);
     {
-        cudaError_t e = cudaSuccess;
-        if (e == cudaSuccess) e = upload(&h->d_atom_begin, h->atom_begin);
-        if (e == cudaSuccess) e = upload(&h->d_sig, sig);
-        if (e == cudaSuccess) e = upload(&h->d_key, key);
-        if (e == cudaSuccess) e = upload(&h->d_param_begin, h->param_begin);
-        if (e == cudaSuccess) e = upload(&h->d_pos, pos);
-        if (e == cudaSuccess) e = upload(&h->d_weight, weight);
-        if (e == cudaSuccess) e = upload(&h->d_dist, dist);
-        if (e == cudaSuccess) e = upload(&h->d_code, s_code);
-        if (e == cudaSuccess) e = upload(&h->d_rule, s_rule);
-        if (e == cudaSuccess) e = upload(&h->d_mainchain, s_main);
-        if (e == cudaSuccess) e = upload(&h->d_name_begin, s_nb);
-        if (e == cudaSuccess) e = upload(&h->d_names, s_names);
-        if (e == cudaSuccess) e = upload(&h->d_res_begin, s_rb);
-        if (e == cudaSuccess) e = upload(&h->d_resnames, s_res);
-        if (e == cudaSuccess) e = upload(&h->d_partner_begin, s_pb);
-        if (e == cudaSuccess) e = upload(&h->d_partner_res, s_pres);
-        if (e == cudaSuccess) e = upload(&h->d_partner_name, s_pname);
-        if (e == cudaSuccess && !h->large.empty()) e = upload(&h->d_large, h->large);
+        Upload up;
+        up.add(&h->d_atom_begin, h->atom_begin);
+        up.add(&h->d_sig, sig);
+        up.add(&h->d_key, key);
+        up.add(&h->d_param_begin, h->param_begin);
+        up.add(&h->d_pos, pos);
+        up.add(&h->d_weight, weight);
+        up.add(&h->d_dist, dist);
+        up.add(&h->d_code, s_code);
+        up.add(&h->d_rule, s_rule);
+        up.add(&h->d_mainchain, s_main);
+        up.add(&h->d_name_begin, s_nb);
+        up.add(&h->d_names, s_names);
+        up.add(&h->d_res_begin, s_rb);
+        up.add(&h->d_resnames, s_res);
+        up.add(&h->d_partner_begin, s_pb);
+        up.add(&h->d_partner_res, s_pres);
+        up.add(&h->d_partner_name, s_pname);
+        up.add(&h->d_large, h->large);
+        keep_pool(h->device);
+        cudaError_t e;
+        Scratch *x = acquire_scratch(h->device, &e);
+        if (e == cudaSuccess) e = up.run(&h->block, x);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(x->st);
+        if (e == cudaSuccess) {
+            handle_created();
+            h->counted = true;
+        }
+        release_scratch(x, e == cudaSuccess);
         if (e != cudaSuccess) {
             status = fail(e == cudaErrorMemoryAllocation ? PJG_ERR_OOM : PJG_ERR_CUDA, "template upload: %s",
                           cudaGetErrorString(e));
@@ -539,11 +792,8 @@ pjg_status pjg_templates_create(const pjg_template_set *set, pjg_templates **out
 
 void pjg_templates_destroy(pjg_templates *h) {
     if (!h) return;
-    void *ptrs[] = {h->d_atom_begin, h->d_sig, h->d_key, h->d_param_begin, h->d_pos, h->d_weight, h->d_dist,
-                    h->d_code, h->d_rule, h->d_mainchain, h->d_name_begin, h->d_names, h->d_res_begin,
-                    h->d_resnames, h->d_partner_begin, h->d_partner_res, h->d_partner_name, h->d_large};
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
+    free_block(h->block, h->device);
+    if (h->counted) handle_destroyed();
     delete h;
 }
 
@@ -762,56 +1012,67 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
         bucket_begin.push_back((int32_t)bucket_name.size());
     }
     h->atom_base = base;
-    cudaError_t e = cudaMalloc((void **)&h->d_xyz64, std::max<size_t>(3 * (size_t)N, 1) * sizeof(double));
-    if (e == cudaSuccess && N > 0)
-        e = cudaMemcpy(h->d_xyz64, set->xyz, 3 * (size_t)N * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = upload(&h->d_atom_base, base);
-    if (e == cudaSuccess) e = upload(&h->d_atom_count, count);
-    if (e == cudaSuccess) e = upload(&h->d_xyz32, xyz32.p.get(), (size_t)N);
-    if (e == cudaSuccess) e = upload(&h->d_name, name.p.get(), (size_t)N);
-    if (e == cudaSuccess) e = upload(&h->d_resname, resname.p.get(), (size_t)N);
-    if (e == cudaSuccess) e = upload(&h->d_sorted, sorted.p.get(), (size_t)N);
-    if (e == cudaSuccess) e = upload(&h->d_bucket_begin, bucket_begin);
-    if (e == cudaSuccess) e = upload(&h->d_bucket_name, bucket_name);
-    if (e == cudaSuccess) e = upload(&h->d_bucket_lo, bucket_lo);
-    if (e == cudaSuccess) e = upload(&h->d_bucket_hi, bucket_hi);
-    if (e == cudaSuccess) e = upload(&h->d_nh_begin, nh_begin);
-    if (e == cudaSuccess) e = upload(&h->d_nh_name, nh_name);
-    if (e == cudaSuccess) e = upload(&h->d_nh_count, nh_count);
-    if (e == cudaSuccess) e = upload(&h->d_name_id, name_id.p.get(), (size_t)N);
-    if (e == cudaSuccess) e = upload(&h->d_nh_off, nh_off);
-    if (e == cudaSuccess) e = upload(&h->d_nh_pos, nh_pos.p.get(), (size_t)N);
-    if (e == cudaSuccess) e = upload(&h->d_kind_name, kind_name);
-    if (e == cudaSuccess) e = upload(&h->d_kind_res, kind_res);
-    if (e == cudaSuccess) e = upload(&h->d_nh_kind, nh_kind);
+    const size_t n1 = (size_t)std::max<int64_t>(N, 1);
+    uint16_t *d_local_kind = nullptr;
+    Upload up;
+    up.add(&h->d_xyz64, set->xyz, 3 * (size_t)N);
+    up.add(&h->d_atom_base, base);
+    up.add(&h->d_atom_count, count);
+    up.add(&h->d_xyz32, xyz32.p.get(), (size_t)N);
+    up.add(&h->d_name, name.p.get(), (size_t)N);
+    up.add(&h->d_resname, resname.p.get(), (size_t)N);
+    up.add(&h->d_sorted, sorted.p.get(), (size_t)N);
+    up.add(&h->d_bucket_begin, bucket_begin);
+    up.add(&h->d_bucket_name, bucket_name);
+    up.add(&h->d_bucket_lo, bucket_lo);
+    up.add(&h->d_bucket_hi, bucket_hi);
+    up.add(&h->d_nh_begin, nh_begin);
+    up.add(&h->d_nh_name, nh_name);
+    up.add(&h->d_nh_count, nh_count);
+    up.add(&h->d_name_id, name_id.p.get(), (size_t)N);
+    up.add(&h->d_nh_off, nh_off);
+    up.add(&h->d_nh_pos, nh_pos.p.get(), (size_t)N);
+    up.add(&h->d_kind_name, kind_name);
+    up.add(&h->d_kind_res, kind_res);
+    up.add(&h->d_nh_kind, nh_kind);
+    up.add(&d_local_kind, local_kind.p.get(), (size_t)N);
+    up.room(&h->d_lrank, 3 * n1);
+    up.room(&h->d_urank, 3 * n1);
+    up.room(&h->d_kxyz, n1);
+    up.room(&h->d_res_pos, n1);
+    up.room(&h->d_res_place, n1);
+    up.room(&h->d_res_kind, n1);
+    up.room(&h->d_res_range, n1);
+    keep_pool(h->device);
+    cudaError_t e;
+    Scratch *x = acquire_scratch(h->device, &e);
+    if (e == cudaSuccess) e = up.run(&h->block, x);
     if (e == cudaSuccess) {
         // axis ranks of every atom (the leaf-order sorted-axis path), and the
         // residue order and kind-ordered points of the order-free search
-        const size_t n1 = (size_t)std::max<int64_t>(N, 1), n3 = 3 * n1;
-        unsigned long long *tile_key = nullptr;
-        uint16_t *tile_idx = nullptr, *d_local_kind = nullptr;
-        e = cudaMalloc((void **)&h->d_lrank, n3 * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_urank, n3 * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&tile_key, 4 * n1 * sizeof(unsigned long long));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&tile_idx, 4 * n1 * sizeof(uint16_t));
-        if (e == cudaSuccess) e = upload(&d_local_kind, local_kind.p.get(), (size_t)N);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_kxyz, n1 * sizeof(float4));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_pos, n1 * sizeof(int32_t));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_place, n1 * sizeof(int32_t));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_kind, n1 * sizeof(uint16_t));
-        if (e == cudaSuccess) e = cudaMalloc((void **)&h->d_res_range, n1 * sizeof(int4));
+        DBuf<unsigned long long> tile_key;
+        DBuf<uint16_t> tile_idx;
+        t_cache = &x->cache;
+        e = dalloc(tile_key, 4 * n1, x->st);
+        if (e == cudaSuccess) e = dalloc(tile_idx, 4 * n1, x->st);
         if (e == cudaSuccess) {
-            launch_axis_ranks(0, S, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key, tile_idx, h->d_lrank,
-                              h->d_urank,
+            launch_axis_ranks(x->st, S, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key.p, tile_idx.p,
+                              h->d_lrank, h->d_urank,
                               ResidueOrder{h->d_xyz32, h->d_nh_pos, d_local_kind, h->d_kxyz, h->d_res_pos,
                                            h->d_res_kind, h->d_res_range, h->d_sorted, h->d_res_place});
             e = cudaGetLastError();
-            if (e == cudaSuccess) e = cudaDeviceSynchronize();
         }
-        if (d_local_kind) cudaFree(d_local_kind);
-        if (tile_key) cudaFree(tile_key);
-        if (tile_idx) cudaFree(tile_idx);
+        dfree(tile_key, x->st);
+        dfree(tile_idx, x->st);
+        t_cache = nullptr;
+        const cudaError_t e2 = cudaStreamSynchronize(x->st);
+        if (e == cudaSuccess) e = e2;
     }
+    if (e == cudaSuccess) {
+        handle_created();
+        h->counted = true;
+    }
+    release_scratch(x, e == cudaSuccess);
     if (e != cudaSuccess) {
         pjg_status st = fail(e == cudaErrorMemoryAllocation ? PJG_ERR_OOM : PJG_ERR_CUDA, "structure upload: %s",
                              cudaGetErrorString(e));
@@ -824,13 +1085,8 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
 
 void pjg_structures_destroy(pjg_structures *h) {
     if (!h) return;
-    void *ptrs[] = {h->d_atom_base, h->d_atom_count, h->d_xyz64, h->d_xyz32, h->d_name, h->d_resname,
-                    h->d_sorted, h->d_bucket_begin, h->d_bucket_name, h->d_bucket_lo, h->d_bucket_hi,
-                    h->d_lrank, h->d_urank, h->d_nh_begin, h->d_nh_name, h->d_nh_count, h->d_name_id,
-                    h->d_nh_off, h->d_nh_pos, h->d_kind_name, h->d_kind_res, h->d_nh_kind, h->d_kxyz,
-                    h->d_res_pos, h->d_res_place, h->d_res_kind, h->d_res_range};
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
+    free_block(h->block, h->device);
+    if (h->counted) handle_destroyed();
     delete h;
 }
 
@@ -886,6 +1142,26 @@ cudaError_t scan_exclusive(const T *in, int64_t n, int64_t *out, std::vector<DBu
     }
     return cudaGetLastError();
 }
+
+// places in a query's block of counters: the statistics (Counter), the lists
+// requested in a chunk, then what an attempt at a chunk's search adds up
+enum : int {
+    ZC_LEAF_USED = C_NUM,
+    ZC_NFILL,
+    ZC_ATTEMPT,
+    ZC_ROWS = ZC_ATTEMPT,
+    ZC_FREE,            // units, heavy pairs, their items, scratch, large units,
+                        // spilled entries, units left to the leaf order, long units
+    ZC_NWORK = ZC_FREE + 8,
+    ZC_NSUSP,
+    ZC_POOL,
+    ZC_ITEM,            // the work queue (32 bits)
+    ZC_TOTALS,          // hits, warnings, hit atoms, passing rows, long pairs
+    ZC_LIVE = ZC_TOTALS + 5,
+    ZC_SNAP = ZC_LIVE,  // the statistics before a chunk's search,
+    ZC_CHUNK = ZC_SNAP + C_NUM,  // and before the chunk
+    ZC_END = ZC_CHUNK + C_NUM
+};
 
 #if PJG_SEARCH_PROF
 // Profile builds: append the query's search profile as one JSON line to the
@@ -1004,14 +1280,25 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     const int T = tp->T, S = sp->S, G = tp->G;
     const bool fp32 = P->mode == PJG_MODE_BATCHED_FP32;
     cudaStream_t st = nullptr;
-    cudaEvent_t ev[8] = {};
+    Scratch *scratch = nullptr;
+    cudaEvent_t *ev = nullptr;
+    // the query's counters, in one device block (offsets ZC_*): what a round
+    // adds up is zeroed by one copy and read back by one
+    DBuf<unsigned long long> d_z;
+    unsigned long long *hz = nullptr;  // its host copy (pinned)
+    struct {
+        unsigned long long *p;
+    } d_counters{}, d_ccount{}, d_rtotals{}, d_nwork{}, d_nsusp{}, d_nfill{}, d_pool_used{}, d_leaf_used{}, d_free_n{};
+    struct {
+        int32_t *p;
+    } d_pair_counter{};
     DBuf<AnnulusParam> d_params;
     // order-free search: kinds of each signature, units of rows, heavy pairs
     // and their items, frontiers of the items, keys of large units
     DBuf<uint32_t> d_sig_bits, d_kind_masks;
     DBuf<RowUnit> d_units;
     DBuf<HeavyPair> d_heavy_pairs;
-    DBuf<unsigned long long> d_free_n, d_heavy_stats, d_row_key;
+    DBuf<unsigned long long> d_heavy_stats, d_row_key;
     DBuf<int2> d_items, d_results;
     DBuf<int64_t> d_item_base, d_bin_off;
     DBuf<int32_t> d_bins, d_arena_atom, d_row_scratch, d_item_head, d_large_units, d_long_pairs, d_pending;
@@ -1019,7 +1306,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     DBuf<SpilledEntry> d_spill_a, d_spill_b;
     DBuf<float4> d_arena_xyz;
     DBuf<uint16_t> d_arena_parent;
-    DBuf<int32_t> d_count, d_scanned, d_cand_atom, d_leaf_atom, d_pair_counter;
+    DBuf<int32_t> d_count, d_scanned, d_cand_atom, d_leaf_atom;
     DBuf<int64_t> d_offset, d_totals, d_boff;
     DBuf<int32_t> d_nblk;
     DBuf<int64_t> d_exact_list, d_sorted_list;
@@ -1028,25 +1315,20 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     DBuf<float4> d_leaf_xyz, d_leaf_xyz2;
     DBuf<int32_t> d_leaf_atom2;
     DBuf<int64_t> d_leaf_off;
-    DBuf<unsigned long long> d_leaf_used;
-    DBuf<unsigned long long> d_counters, d_ccount, d_rtotals;
     DBuf<int32_t> d_c_pair, d_c_atoms, d_pair_rows, d_cnt_q;
     DBuf<int64_t> d_c_ord, d_off_q;
     // lists ordered on demand: per-list state, requested lists, suspended pairs
     DBuf<int32_t> d_lstate;
     DBuf<int64_t> d_work;
-    DBuf<unsigned long long> d_nwork, d_nsusp;
     // lists filled on demand
     DBuf<int32_t> d_fill_state;
     DBuf<int64_t> d_fill_work;
-    DBuf<unsigned long long> d_nfill;
     DBuf<Suspended> d_susp_a, d_susp_b;
     DBuf<unsigned char> d_pool_a, d_pool_b;
     // costliest pairs first: cost buckets, heavy flags and list, histogram
     DBuf<uint8_t> d_pcost, d_hflag;
     DBuf<int32_t> d_heavy;
     DBuf<unsigned long long> d_hbins;
-    DBuf<unsigned long long> d_pool_used;
     int64_t pool_cap = 0;
     // requested lists sharing one leaf order (table and worklists)
     DBuf<unsigned long long> d_ls_key, d_ls_n;
@@ -1088,6 +1370,11 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     const bool free_first = P->mode != PJG_MODE_PLAIN_FP64 && demand_levels == TUNING_DEFAULTS.leaf_levels &&
                             !getenv("PJG_LEAF_LEVELS") && sp->max_local_kinds <= FREE_MAX_KINDS &&
                             (int64_t)G * fv.kind_words <= (1ll << 28);
+    // few enough atoms and signatures for one chunk whatever the lists hold:
+    // their total is not read back (order-free search: the lists are filled on
+    // demand, and then their total is)
+    constexpr int64_t LEAST_ENTRIES = 48ll << 20;
+    const bool few_entries = free_first && sp->N * (int64_t)G <= LEAST_ENTRIES && !getenv("PJG_ENTRY_BUDGET");
     std::vector<int64_t> totals(S);
 
     if (T == 0 || S == 0) {
@@ -1102,29 +1389,23 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             return fail(PJG_ERR_INVALID, "templates, structures and the calling thread use different devices");
         }
     }
+    keep_pool(res->device);
     {
-        // keep the stream-ordered pool's memory mapped between queries (up
-        // to half the device) instead of returning it at every sync: the
-        // next query's chunk buffers then need no new mappings
-        static std::mutex m;
-        static bool done[256] = {};
-        std::lock_guard<std::mutex> g(m);
-        if (res->device >= 0 && res->device < 256 && !done[res->device]) {
-            cudaMemPool_t pool;
-            size_t fb = 0, tb = 0;
-            if (cudaDeviceGetDefaultMemPool(&pool, res->device) == cudaSuccess && cudaMemGetInfo(&fb, &tb) == cudaSuccess) {
-                uint64_t thr = tb / 2;
-                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
-            }
-            cudaGetLastError();
-            done[res->device] = true;
+        cudaError_t e;
+        scratch = acquire_scratch(res->device, &e);
+        if (!scratch) {
+            delete res;
+            return fail(e == cudaErrorMemoryAllocation ? PJG_ERR_OOM : PJG_ERR_CUDA, "query set-up: %s",
+                        cudaGetErrorString(e));
         }
+        st = scratch->st;
+        ev = scratch->ev;
+        hz = reinterpret_cast<unsigned long long *>(scratch->pinned);
+        t_cache = &scratch->cache;
     }
-    CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
 #if PJG_SEARCH_PROF
     leaf_profile_reset(st);
 #endif
-    for (auto &e : ev) CUDA_TRY(cudaEventCreate(&e));
     CUDA_TRY(cudaEventRecord(ev[0], st));
 
     {
@@ -1146,11 +1427,18 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         launches++;
         CUDA_TRY(cudaGetLastError());
     }
-    CUDA_TRY(dalloc(d_counters, C_NUM, st));
-    CUDA_TRY(cudaMemsetAsync(d_counters.p, 0, C_NUM * sizeof(unsigned long long), st));
-    CUDA_TRY(dalloc(d_pair_counter, 1, st));
-    CUDA_TRY(dalloc(d_ccount, 1, st));
-    CUDA_TRY(dalloc(d_rtotals, 5, st));
+    CUDA_TRY(dalloc(d_z, ZC_END, st));
+    CUDA_TRY(cudaMemsetAsync(d_z.p, 0, ZC_END * sizeof(unsigned long long), st));
+    d_counters.p = d_z.p;
+    d_leaf_used.p = d_z.p + ZC_LEAF_USED;
+    d_nfill.p = d_z.p + ZC_NFILL;
+    d_ccount.p = d_z.p + ZC_ROWS;
+    d_free_n.p = d_z.p + ZC_FREE;
+    d_nwork.p = d_z.p + ZC_NWORK;
+    d_nsusp.p = d_z.p + ZC_NSUSP;
+    d_pool_used.p = d_z.p + ZC_POOL;
+    d_pair_counter.p = reinterpret_cast<int32_t *>(d_z.p + ZC_ITEM);
+    d_rtotals.p = d_z.p + ZC_TOTALS;
 
     {
         // pass 1: list lengths for every (structure, signature)
@@ -1176,11 +1464,15 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         } else {
             launch_candidates(st, std::max(blocks, 1), false, cv, sv, d_count.p, d_scanned.p, nullptr, nullptr);
         }
-        k_struct_totals<<<std::max(1, std::min(S, sm_count() * 8)), 256, 0, st>>>(S, G, d_count.p, d_totals.p);
-        launches += 2;
+        launches++;
         CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaMemcpyAsync(totals.data(), d_totals.p, sizeof(int64_t) * S, cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
+        if (!few_entries) {
+            k_struct_totals<<<std::max(1, std::min(S, sm_count() * 8)), 256, 0, st>>>(S, G, d_count.p, d_totals.p);
+            launches++;
+            CUDA_TRY(cudaGetLastError());
+            CUDA_TRY(cudaMemcpyAsync(totals.data(), d_totals.p, sizeof(int64_t) * S, cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(cudaStreamSynchronize(st));
+        }
     }
 
     {
@@ -1196,8 +1488,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         // fewer kernel tails and search rounds.  PJG_ENTRY_BUDGET overrides
         // it.
         constexpr double ENTRY_BYTES = 25.0 + 32.0 / CULL_BLK;
-        int64_t ENTRY_BUDGET = 48ll << 20;
-        {
+        int64_t ENTRY_BUDGET = LEAST_ENTRIES;
+        if (!few_entries) {
             size_t free_b = 0, total_b = 0;
             if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
                 cudaMemPool_t pool;
@@ -1283,9 +1575,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             // if it is redone on fewer structures)
             const int search_rounds0 = search_rounds;
             const int64_t suspensions0 = suspensions;
-            unsigned long long chunk_snap[C_NUM];
-            CUDA_TRY(cudaMemcpyAsync(chunk_snap, d_counters.p, sizeof chunk_snap, cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaStreamSynchronize(st));
+            const size_t stats_bytes = C_NUM * sizeof(unsigned long long);
+            CUDA_TRY(cudaMemcpyAsync(d_z.p + ZC_CHUNK, d_counters.p, stats_bytes, cudaMemcpyDeviceToDevice, st));
             const int Sc = s1 - s0;
             const int64_t Wc = (int64_t)Sc * G;
             ChunkView cv{Sc, sp->d_atom_base + s0, sp->d_atom_count + s0, sp->d_xyz64, sp->d_xyz32, sp->d_name,
@@ -1297,73 +1588,25 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             int32_t *cnt_c = d_count.p + (int64_t)s0 * G;
             int32_t *scn_c = d_scanned.p + (int64_t)s0 * G;
             if (free_first) fv.kind_masks = d_kind_masks.p + (int64_t)s0 * G * fv.mask_words;
-            CUDA_TRY(dalloc(d_offset, (size_t)Wc, st));
             CUDA_TRY(cudaEventRecord(ev[1], st));
-            CUDA_TRY(scan_exclusive(cnt_c, Wc, d_offset.p, scan_tmp, st));
-            // culling blocks of CULL_BLK leaves: counts, offsets, total (one
-            // small sync)
-            int64_t nblocks = 0;
-            CUDA_TRY(dalloc(d_nblk, (size_t)Wc, st));
-            CUDA_TRY(dalloc(d_boff, (size_t)Wc, st));
-            launch_block_counts(st, Wc, cnt_c, d_nblk.p);
-            CUDA_TRY(scan_exclusive(d_nblk.p, Wc, d_boff.p, scan_tmp, st));
-            {
-                int64_t lastoff = 0;
-                int32_t lastn = 0;
-                CUDA_TRY(cudaMemcpyAsync(&lastoff, d_boff.p + Wc - 1, 8, cudaMemcpyDeviceToHost, st));
-                CUDA_TRY(cudaMemcpyAsync(&lastn, d_nblk.p + Wc - 1, 4, cudaMemcpyDeviceToHost, st));
-                CUDA_TRY(cudaStreamSynchronize(st));
-                nblocks = lastoff + lastn;
-            }
-            CUDA_TRY(dalloc(d_blk_lo, (size_t)std::max<int64_t>(nblocks, 1), st));
-            CUDA_TRY(dalloc(d_blk_hi, (size_t)std::max<int64_t>(nblocks, 1), st));
-            CUDA_TRY(dalloc(d_cand_atom, (size_t)entries, st));
-            // leaf-order arrays: every entry when every list is ordered up
-            // front, else half of them to start with (grown on demand;
-            // PJG_LEAF_CAPACITY sets the starting size)
-            {
-                int64_t cap0 = demand_levels < 0 ? entries : std::max<int64_t>(entries / 2, 1 << 20);
-                const char *v = getenv("PJG_LEAF_CAPACITY");
-                if (demand_levels >= 0 && v && atoll(v) > 0) {
-                    cap0 = atoll(v);
-                    dfree(d_leaf_atom, st);
-                    dfree(d_leaf_xyz, st);
-                }
-                CUDA_TRY(dalloc(d_leaf_atom, (size_t)cap0, st));
-            }
-            CUDA_TRY(dalloc(d_leaf_xyz, d_leaf_atom.n, st));
+            const int64_t n_pairs = (int64_t)Sc * T;
+            const bool free_chunk = free_first && n_pairs <= INT32_MAX - (1 << 20);
             int64_t leaf_filled = 0;  // leaf entries of the lists ordered so far
             const int fill_blocks = std::max(1, (int)std::min<int64_t>((Wc + 7) / 8, (int64_t)sm_count() * 32));
-            {
-                // every list is filled here when every list is put in leaf
-                // order up front; otherwise only the lists a search reads:
-                // the level-0 list of each pair that can run (queued by
-                // k_demand_levels) and each list put in leaf order (filled
-                // just before it is ordered)
-                if (demand_levels < 0) {
-                    launch_candidates(st, fill_blocks, true, cv, sv, nullptr, nullptr, d_offset.p, d_cand_atom.p);
-                    launches++;
-                }
-                CUDA_TRY(dalloc(d_exact_list, (size_t)Wc, st));
-                CUDA_TRY(dalloc(d_exact_count, 1, st));
-                CUDA_TRY(dalloc(d_sorted_list, (size_t)LEAF_LISTS * (size_t)Wc, st));
-                CUDA_TRY(dalloc(d_sorted_count, LEAF_LISTS, st));
-                launches++;  // block counts
-                CUDA_TRY(cudaGetLastError());
-            }
             TemplateView tv{T, tp->nmax, tp->d_atom_begin, tp->d_sig, tp->d_pos, tp->d_key, tp->d_param_begin,
                             d_params.p};
-            if (demand_levels >= 0) CUDA_TRY(dalloc(d_leaf_off, (size_t)Wc, st));
-            const int64_t *leaf_off = demand_levels < 0 ? d_offset.p : d_leaf_off.p;
-            CandView cd{G, cnt_c, d_offset.p, d_cand_atom.p, leaf_off, d_leaf_atom.p, d_leaf_xyz.p,
-                        d_boff.p, d_blk_lo.p, d_blk_hi.p};
-            const int64_t n_pairs = (int64_t)Sc * T;
+            CandView cd{G, cnt_c, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+            const int64_t *leaf_off = nullptr;
             // kd leaf order: up front for the lists of the first
             // `demand_levels` levels of every pair that can run, later (between
             // search rounds) for each deeper list a pair's frontier reaches;
             // a negative value orders every list of the chunk up front
             LeafDemand dm{};
-            bool free_chunk = false;
+            dm.n_suspended = d_nsusp.p;
+            dm.n_work = d_nwork.p;
+            dm.leaf_used = d_leaf_used.p;
+            dm.n_fill = d_nfill.p;
+            dm.pool_used = d_pool_used.p;
             const int leaf_blocks =
                 std::max(1, (int)std::min<int64_t>((Wc + LEAF_WARPS - 1) / LEAF_WARPS, (int64_t)sm_count() * 32));
             // room in the leaf arrays for `need` entries (the lists ordered so
@@ -1439,70 +1682,111 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 }
                 return cudaGetLastError();
             };
-            if (demand_levels < 0) {
-                CUDA_TRY(order_requested());
-            } else {
-                CUDA_TRY(dalloc(d_lstate, (size_t)Wc, st));
-                CUDA_TRY(dalloc(d_work, (size_t)Wc, st));
-                CUDA_TRY(dalloc(d_nwork, 1, st));
-                CUDA_TRY(dalloc(d_nsusp, 1, st));
-                CUDA_TRY(dalloc(d_susp_a, (size_t)n_pairs, st));
-                CUDA_TRY(dalloc(d_susp_b, (size_t)n_pairs, st));
-                if (pool_cap == 0) {
-                    // saved search states of suspended pairs, one pool per
-                    // round in turn: a sixteenth of the free memory each,
-                    // 64 MiB to 4 GiB (a pair that finds its pool full is
-                    // rerun from its start instead)
-                    size_t free_b = 0, total_b = 0;
-                    int64_t cap = 64ll << 20;
-                    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
-                        cap = std::max<int64_t>(cap, std::min<int64_t>(4ll << 30, (int64_t)(free_b / 16)));
-                    const char *v = getenv("PJG_STATE_POOL");
-                    if (v && atoll(v) >= 0) cap = atoll(v);
-                    pool_cap = std::max<int64_t>(cap, 16);
-                    CUDA_TRY(dalloc(d_pool_a, (size_t)pool_cap, st));
-                    CUDA_TRY(dalloc(d_pool_b, (size_t)pool_cap, st));
-                    CUDA_TRY(dalloc(d_pool_used, 1, st));
+            // the chunk's lists: offsets, culling blocks, room for their atoms
+            // in candidate order and in leaf order, and the state of those
+            // put in leaf order on demand.  The order-free search needs none
+            // of it before a pair is split into items or rows are left to
+            // the leaf order.
+            bool lists_ready = false;
+            auto setup_lists = [&]() -> cudaError_t {
+                if (lists_ready) return cudaSuccess;
+                lists_ready = true;
+                cudaError_t e = cudaSuccess;
+                auto room = [&](auto &buf, int64_t n) {
+                    if (e == cudaSuccess) e = dalloc(buf, (size_t)std::max<int64_t>(n, 1), st);
+                };
+                auto fill = [&](void *p, int v, size_t bytes) {
+                    if (e == cudaSuccess) e = cudaMemsetAsync(p, v, bytes, st);
+                };
+                room(d_offset, Wc);
+                room(d_nblk, Wc);
+                room(d_boff, Wc);
+                if (e == cudaSuccess) e = scan_exclusive(cnt_c, Wc, d_offset.p, scan_tmp, st);
+                if (e != cudaSuccess) return e;
+                // culling blocks of CULL_BLK leaves: counts, offsets, total
+                launch_block_counts(st, Wc, cnt_c, d_nblk.p);
+                launches++;
+                e = scan_exclusive(d_nblk.p, Wc, d_boff.p, scan_tmp, st);
+                int64_t last[3] = {};  // offset and blocks of the last list, its block count and length
+                int32_t lastn[2] = {};
+                auto back = [&](void *to, const void *from, size_t bytes) {
+                    if (e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, st);
+                };
+                back(&last[0], d_offset.p + Wc - 1, 8);
+                back(&last[1], d_boff.p + Wc - 1, 8);
+                back(&lastn[0], cnt_c + Wc - 1, 4);
+                back(&lastn[1], d_nblk.p + Wc - 1, 4);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                const int64_t all = last[0] + lastn[0], nblocks = last[1] + lastn[1];
+                room(d_blk_lo, nblocks);
+                room(d_blk_hi, nblocks);
+                room(d_cand_atom, all);
+                // leaf-order arrays: every entry when every list is ordered
+                // up front, else half of them to start with (order-free
+                // search: few; grown on demand; PJG_LEAF_CAPACITY sets the
+                // starting size)
+                int64_t cap0 = demand_levels < 0 ? all
+                               : free_chunk      ? 1 << 18
+                                                 : std::max<int64_t>(all / 2, 1 << 20);
+                const char *v = getenv("PJG_LEAF_CAPACITY");
+                if (demand_levels >= 0 && v && atoll(v) > 0) {
+                    cap0 = atoll(v);
+                    dfree(d_leaf_atom, st);
+                    dfree(d_leaf_xyz, st);
                 }
-                dm.pool_used = d_pool_used.p;
-                dm.pool_cap = pool_cap;
-                CUDA_TRY(cudaMemsetAsync(d_lstate.p, 0, (size_t)Wc * sizeof(int32_t), st));
-                CUDA_TRY(cudaMemsetAsync(d_nwork.p, 0, sizeof(unsigned long long), st));
+                room(d_leaf_atom, cap0);
+                room(d_leaf_xyz, (int64_t)d_leaf_atom.n);
+                room(d_exact_list, Wc);
+                room(d_exact_count, 1);
+                room(d_sorted_list, (int64_t)LEAF_LISTS * Wc);
+                room(d_sorted_count, LEAF_LISTS);
+                if (demand_levels >= 0) room(d_leaf_off, Wc);
+                if (e != cudaSuccess) return e;
+                leaf_off = demand_levels < 0 ? d_offset.p : d_leaf_off.p;
+                cd = CandView{G, cnt_c, d_offset.p, d_cand_atom.p, leaf_off, d_leaf_atom.p, d_leaf_xyz.p,
+                              d_boff.p, d_blk_lo.p, d_blk_hi.p};
+                if (demand_levels < 0) {
+                    // every list filled and put in leaf order up front
+                    launch_candidates(st, fill_blocks, true, cv, sv, nullptr, nullptr, d_offset.p, d_cand_atom.p);
+                    launches++;
+                    return cudaGetLastError();
+                }
+                // otherwise only the lists a search reads are filled: the
+                // level-0 list of each pair that needs it and each list put in
+                // leaf order (just before it is)
+                room(d_lstate, Wc);
+                room(d_work, Wc);
+                room(d_fill_state, Wc);
+                room(d_fill_work, Wc);
+                fill(d_lstate.p, 0, (size_t)Wc * sizeof(int32_t));
+                fill(d_fill_state.p, 0, (size_t)Wc * sizeof(int32_t));
+                if (e != cudaSuccess) return e;
                 dm.state = d_lstate.p;
                 dm.work = d_work.p;
-                dm.n_work = d_nwork.p;
-                dm.n_suspended = d_nsusp.p;
-                CUDA_TRY(dalloc(d_leaf_used, 1, st));
-                CUDA_TRY(cudaMemsetAsync(d_leaf_used.p, 0, sizeof(unsigned long long), st));
                 dm.leaf_offset = d_leaf_off.p;
-                dm.leaf_used = d_leaf_used.p;
-                CUDA_TRY(dalloc(d_fill_state, (size_t)Wc, st));
-                CUDA_TRY(dalloc(d_fill_work, (size_t)Wc, st));
-                CUDA_TRY(dalloc(d_nfill, 1, st));
-                CUDA_TRY(cudaMemsetAsync(d_fill_state.p, 0, (size_t)Wc * sizeof(int32_t), st));
-                CUDA_TRY(cudaMemsetAsync(d_nfill.p, 0, sizeof(unsigned long long), st));
                 dm.fill_state = d_fill_state.p;
                 dm.fill_work = d_fill_work.p;
-                dm.n_fill = d_nfill.p;
                 {
                     // the list-sharing table: twice the chunk's lists, a power
                     // of two (without the memory, every list is ordered)
                     int64_t cap = 1;
                     while (cap < 2 * Wc) cap <<= 1;
-                    cudaError_t e = dalloc(d_ls_key, (size_t)cap, st);
-                    if (e == cudaSuccess) e = dalloc(d_ls_rep, (size_t)cap, st);
-                    if (e == cudaSuccess) e = dalloc(d_ls_slot, (size_t)Wc, st);
-                    if (e == cudaSuccess) e = dalloc(d_ls_rep_work, (size_t)Wc, st);
-                    if (e == cudaSuccess) e = dalloc(d_ls_dup, (size_t)Wc, st);
-                    if (e == cudaSuccess) e = dalloc(d_ls_left, (size_t)Wc, st);
-                    if (e == cudaSuccess) e = dalloc(d_ls_n, 3, st);
-                    if (e == cudaSuccess) e = dalloc(d_ls_ok, (size_t)Wc, st);
-                    if (e == cudaSuccess) e = cudaMemsetAsync(d_ls_key.p, 0, (size_t)cap * sizeof(unsigned long long), st);
-                    if (e == cudaSuccess) e = cudaMemsetAsync(d_ls_rep.p, 0xFF, (size_t)cap * sizeof(int32_t), st);
-                    if (e == cudaSuccess) e = cudaMemsetAsync(d_ls_ok.p, 0, (size_t)Wc, st);
+                    room(d_ls_key, cap);
+                    room(d_ls_rep, cap);
+                    room(d_ls_slot, Wc);
+                    room(d_ls_rep_work, Wc);
+                    room(d_ls_dup, Wc);
+                    room(d_ls_left, Wc);
+                    room(d_ls_n, 3);
+                    room(d_ls_ok, Wc);
+                    if (e == cudaSuccess) {
+                        fill(d_ls_key.p, 0, (size_t)cap * sizeof(unsigned long long));
+                        fill(d_ls_rep.p, 0xFF, (size_t)cap * sizeof(int32_t));
+                        fill(d_ls_ok.p, 0, (size_t)Wc);
+                    }
                     // PJG_LIST_SHARING=0 orders every list itself
-                    const char *v = getenv("PJG_LIST_SHARING");
-                    share_on = e == cudaSuccess && !(v && v[0] == '0');
+                    const char *w = getenv("PJG_LIST_SHARING");
+                    share_on = e == cudaSuccess && !(w && w[0] == '0');
                     if (e != cudaSuccess) {
                         cudaGetLastError();
                         dfree(d_ls_key, st);
@@ -1523,11 +1807,37 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     ls.n = d_ls_n.p;
                     ls.part_ok = d_ls_ok.p;
                 }
-                if (n_pairs > INT32_MAX) {
-                    status = fail(PJG_ERR_CAPACITY, "too many pairs in one chunk");
-                    goto done;
+                return cudaSuccess;
+            };
+            if (n_pairs > INT32_MAX) {
+                status = fail(PJG_ERR_CAPACITY, "too many pairs in one chunk");
+                goto done;
+            }
+            // (lists requested in this chunk and the attempt's counters)
+            CUDA_TRY(cudaMemsetAsync(d_leaf_used.p, 0, (ZC_LIVE - ZC_LEAF_USED) * sizeof(unsigned long long), st));
+            if (!free_chunk || !tp->large.empty()) CUDA_TRY(setup_lists());
+            if (demand_levels < 0) {
+                CUDA_TRY(order_requested());
+            } else {
+                CUDA_TRY(dalloc(d_susp_a, (size_t)n_pairs, st));
+                if (!free_chunk) CUDA_TRY(dalloc(d_susp_b, (size_t)n_pairs, st));
+                if (pool_cap == 0 && !free_chunk) {
+                    // saved search states of suspended pairs, one pool per
+                    // round in turn: a sixteenth of the free memory each,
+                    // 64 MiB to 4 GiB (a pair that finds its pool full is
+                    // rerun from its start instead; pairs the order-free
+                    // search leaves are never suspended)
+                    size_t free_b = 0, total_b = 0;
+                    int64_t cap = 64ll << 20;
+                    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
+                        cap = std::max<int64_t>(cap, std::min<int64_t>(4ll << 30, (int64_t)(free_b / 16)));
+                    const char *v = getenv("PJG_STATE_POOL");
+                    if (v && atoll(v) >= 0) cap = atoll(v);
+                    pool_cap = std::max<int64_t>(cap, 16);
+                    CUDA_TRY(dalloc(d_pool_a, (size_t)pool_cap, st));
+                    CUDA_TRY(dalloc(d_pool_b, (size_t)pool_cap, st));
                 }
-                free_chunk = free_first && n_pairs <= INT32_MAX - (1 << 20);
+                dm.pool_cap = pool_cap;
                 // the costliest pairs are searched first (a pair can take
                 // milliseconds; started last, it alone would run on while the
                 // other warps idle): the level demand estimates each pair's
@@ -1555,33 +1865,29 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 if (!free_chunk || !tp->large.empty()) {
                     launch_demand_levels(st, sm_count() * 16, tv, cd, (int32_t)n_pairs,
                                          free_chunk ? -1 : demand_levels, P->reorder, dm);
-                if (heavy_on) {
-                    launch_heavy_pairs(st, (int32_t)n_pairs, d_pcost.p, d_hbins.p, heavy_target, d_hflag.p,
-                                       d_heavy.p);
-                    dm.heavy = d_heavy.p;
-                    dm.n_heavy = d_hbins.p + 64;
-                    dm.heavy_flag = d_hflag.p;
+                    if (heavy_on) {
+                        launch_heavy_pairs(st, (int32_t)n_pairs, d_pcost.p, d_hbins.p, heavy_target, d_hflag.p,
+                                           d_heavy.p);
+                        dm.heavy = d_heavy.p;
+                        dm.n_heavy = d_hbins.p + 64;
+                        dm.heavy_flag = d_hflag.p;
+                        launches += 2;
+                    }
+                    // the level-0 lists the pairs read in candidate order
+                    launch_candidates(st, fill_blocks, true, cv, sv, nullptr, nullptr, d_offset.p, d_cand_atom.p,
+                                      dm.fill_work, dm.n_fill, nullptr, false);
                     launches += 2;
-                }
-                // the level-0 lists the pairs read in candidate order
-                launch_candidates(st, fill_blocks, true, cv, sv, nullptr, nullptr, d_offset.p, d_cand_atom.p,
-                                  dm.fill_work, dm.n_fill, nullptr, false);
-                launches += 2;
-                unsigned long long used = 0;
-                CUDA_TRY(cudaMemcpyAsync(&used, d_leaf_used.p, sizeof used, cudaMemcpyDeviceToHost, st));
-                CUDA_TRY(cudaStreamSynchronize(st));
-                CUDA_TRY(ensure_leaf((int64_t)used));
-                CUDA_TRY(order_requested());
-                leaf_filled = (int64_t)used;
+                    unsigned long long used = 0;
+                    CUDA_TRY(cudaMemcpyAsync(&used, d_leaf_used.p, sizeof used, cudaMemcpyDeviceToHost, st));
+                    CUDA_TRY(cudaStreamSynchronize(st));
+                    CUDA_TRY(ensure_leaf((int64_t)used));
+                    CUDA_TRY(order_requested());
+                    leaf_filled = (int64_t)used;
                 }
             }
             CUDA_TRY(cudaEventRecord(ev[2], st));
             SearchArgs sa;
             sa.n_pairs = Sc * T;
-            if (n_pairs > INT32_MAX) {
-                status = fail(PJG_ERR_CAPACITY, "too many pairs in one chunk");
-                goto done;
-            }
             sa.ignore_chain = P->ignore_chain;
             sa.reorder = P->reorder;
             sa.best_match = P->best_match;
@@ -1617,9 +1923,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             }
             bool wide = sp->max_atoms > 65535;
             // counters before this chunk's search, restored if it must rerun
-            unsigned long long snap[C_NUM];
-            CUDA_TRY(cudaMemcpyAsync(snap, d_counters.p, sizeof snap, cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaStreamSynchronize(st));
+            CUDA_TRY(cudaMemcpyAsync(d_z.p + ZC_SNAP, d_counters.p, stats_bytes, cudaMemcpyDeviceToDevice, st));
             CUDA_TRY(dalloc(d_pair_rows, (size_t)n_pairs, st));
             // room before the first attempt (a rerun of the search costs a
             // whole chunk): two complete rows a pair, or, with best_match
@@ -1640,7 +1944,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     bound_cap = std::min(bound_cap, chunk_cap);
                     chunks--;
                     row_splits++;
-                    CUDA_TRY(cudaMemcpyAsync(d_counters.p, chunk_snap, sizeof chunk_snap, cudaMemcpyHostToDevice,
+                    CUDA_TRY(cudaMemcpyAsync(d_counters.p, d_z.p + ZC_CHUNK, stats_bytes, cudaMemcpyDeviceToDevice,
                                              st));
                     continue;
                 }
@@ -1655,8 +1959,11 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             // set when the chunk's complete rows cannot be held: the chunk is
             // redone on half its structures
             bool split = false;
+            bool invalid_rows = false;  // rows of pairs that k_search took over
             for (int attempt = 0; attempt < 8; attempt++) {
-                CUDA_TRY(cudaMemsetAsync(d_ccount.p, 0, sizeof(unsigned long long), st));
+                if (attempt > 0)
+                    CUDA_TRY(cudaMemsetAsync(d_z.p + ZC_ATTEMPT, 0,
+                                             (ZC_LIVE - ZC_ATTEMPT) * sizeof(unsigned long long), st));
                 CUDA_TRY(cudaMemsetAsync(d_pair_rows.p, 0, (size_t)n_pairs * sizeof(int32_t), st));
                 CompleteRows cr{d_ccount.p, c_cap, stride, d_c_pair.p, d_c_ord.p, d_c_atoms.p,
                                 cut_inline ? d_c_rmsd.p : nullptr, d_pair_rows.p};
@@ -1670,25 +1977,22 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 dm.pool_in = nullptr;
                 // units, heavy pairs, their items, (scratch, large units,) spilled entries,
                 // units left to the leaf order
-                unsigned long long free_n[7] = {};
+                unsigned long long free_n[8] = {};
                 FreeWork fw{};
                 Suspended *next_out = d_susp_a.p, *spare = d_susp_b.p;
                 unsigned char *pool_next = d_pool_a.p, *pool_spare = d_pool_b.p;
                 for (int round = 0;; round++) {
-                    CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
-                    if (dm.state) {
-                        dm.suspended = next_out;
-                        dm.pool_out = pool_next;
-                        CUDA_TRY(cudaMemsetAsync(d_nwork.p, 0, sizeof(unsigned long long), st));
-                        CUDA_TRY(cudaMemsetAsync(d_nsusp.p, 0, sizeof(unsigned long long), st));
-                        CUDA_TRY(cudaMemsetAsync(d_pool_used.p, 0, sizeof(unsigned long long), st));
-                    }
+                    dm.suspended = next_out;
+                    dm.pool_out = pool_next;
+                    // requested lists, suspended pairs, pool and work queue
+                    // (the first order-free round: zeroed with the attempt)
+                    if (round > 0 || !free_chunk || !tp->large.empty())
+                        CUDA_TRY(cudaMemsetAsync(d_nwork.p, 0, (ZC_TOTALS - ZC_NWORK) * sizeof(unsigned long long),
+                                                 st));
                     CUDA_TRY(cudaEventRecord(ev[6], st));
                     if (round == 0 && free_chunk) {
                         CUDA_TRY(dalloc(d_units, (size_t)c_cap, st));
                         CUDA_TRY(dalloc(d_heavy_pairs, (size_t)n_pairs, st));
-                        CUDA_TRY(dalloc(d_free_n, 8, st));
-                        CUDA_TRY(cudaMemsetAsync(d_free_n.p, 0, 8 * sizeof(unsigned long long), st));
                         fw.item_seeds = P->max_candidates >= 0        ? FREE_ITEM_CUT
                                         : n_pairs <= FREE_FEW_PAIRS ? FREE_ITEM_FEW
                                                                     : FREE_ITEM;
@@ -1720,15 +2024,14 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(cudaGetLastError());
                     unsigned long long ns = 0, used = 0;
                     auto read_back = [&]() -> cudaError_t {
-                        cudaError_t e = cudaMemcpyAsync(&nc, d_ccount.p, sizeof nc, cudaMemcpyDeviceToHost, st);
-                        if (e == cudaSuccess && dm.state) {
-                            e = cudaMemcpyAsync(&ns, d_nsusp.p, sizeof ns, cudaMemcpyDeviceToHost, st);
-                            if (e == cudaSuccess)
-                                e = cudaMemcpyAsync(&used, d_leaf_used.p, sizeof used, cudaMemcpyDeviceToHost, st);
-                        }
-                        if (e == cudaSuccess && round == 0 && free_chunk)
-                            e = cudaMemcpyAsync(free_n, d_free_n.p, sizeof free_n, cudaMemcpyDeviceToHost, st);
+                        cudaError_t e = cudaMemcpyAsync(hz, d_z.p, ZC_LIVE * sizeof(unsigned long long),
+                                                        cudaMemcpyDeviceToHost, st);
                         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                        nc = hz[ZC_ROWS];
+                        ns = dm.state || free_chunk ? hz[ZC_NSUSP] : 0;
+                        used = hz[ZC_LEAF_USED];
+                        if (round == 0)
+                            for (int i = 0; i < 8; i++) free_n[i] = hz[ZC_FREE + i];
                         float m = 0.f;
                         if (e == cudaSuccess) e = cudaEventElapsedTime(&m, ev[6], ev[7]);
                         ms_search += m;
@@ -1738,7 +2041,12 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     search_rounds++;
                     if (round == 0 && free_chunk && (free_n[1] || ns)) {
                         // level-0 lists, in candidate order, of the pairs taken
-                        // in items and of those left to k_search
+                        // in items and of those left to k_search, whose other
+                        // lists are to be put in leaf order
+                        CUDA_TRY(setup_lists());
+                        launch_free_requests(st, tv, cd, P->reorder, dm, d_heavy_pairs.p, (int32_t)free_n[1],
+                                             dm.suspended, 0, (int32_t)ns);
+                        launches++;
                         launch_candidates(st, fill_blocks, true, cv, sv, nullptr, nullptr, d_offset.p, d_cand_atom.p,
                                           dm.fill_work, dm.n_fill, nullptr, false);
                         launches++;
@@ -1747,6 +2055,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         // the heavy pairs in items of seeds, block 0
                         // of every pair first
                         const int32_t nh = (int32_t)free_n[1];
+                        const int64_t ns1 = (int64_t)ns;
                         const int64_t ni = (int64_t)free_n[2];
                         const int64_t nbins = (sp->max_atoms + fw.item_seeds - 1) / fw.item_seeds;
                         if (ni > INT32_MAX) {
@@ -1826,6 +2135,14 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         }
                         launch_heavy_rows(st, nh, fw, d_item_base.p, d_pair_rows.p, d_counters.p);
                         launches++;
+                        if ((int64_t)ns > ns1) {
+                            // pairs that an item left to k_search (their level-0
+                            // lists are filled)
+                            launch_free_requests(st, tv, cd, P->reorder, dm, nullptr, 0, dm.suspended, (int32_t)ns1,
+                                                 (int32_t)ns);
+                            launches++;
+                            invalid_rows = true;
+                        }
                         CUDA_TRY(cudaGetLastError());
                     }
                     if (round == 0 && free_chunk && free_n[0] && (int64_t)nc <= c_cap) {
@@ -1835,8 +2152,18 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         fw.pending = d_pending.p;
                         fw.long_units = d_pending.p + free_n[0];
                         CUDA_TRY(launch_unit_order_direct(st, (int64_t)free_n[0], cv, tv, cd, sv, fv, sp->d_res_place,
-                                                          P->reorder, fw, cr, dm));
+                                                          P->reorder, fw, cr));
                         launches += 2;
+                        const double ms0 = ms_search;
+                        CUDA_TRY(read_back());
+                        if (free_n[6]) {
+                            CUDA_TRY(setup_lists());
+                            launch_pending_requests(st, (int64_t)free_n[6], tv, cd, P->reorder, dm, fw);
+                            launches++;
+                        }
+                        if (free_n[6] || ns) CUDA_TRY(read_back());
+                        ms_search = ms0;
+                    } else if (round == 0 && free_chunk && ns) {
                         const double ms0 = ms_search;
                         CUDA_TRY(read_back());
                         ms_search = ms0;
@@ -1855,6 +2182,10 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     dm.resume = next_out;
                     dm.n_resume = (int32_t)ns;
                     dm.pool_in = pool_next;
+                    if (!spare) {
+                        CUDA_TRY(dalloc(d_susp_b, (size_t)n_pairs, st));
+                        spare = d_susp_b.p;
+                    }
                     std::swap(next_out, spare);
                     std::swap(pool_next, pool_spare);
                 }
@@ -1898,28 +2229,29 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(eg);
                 }
                 {
-                    unsigned long long cur[C_NUM];
+                    // (the leaf order's statistics and an error stay)
+                    unsigned long long cur[C_NUM], snap[C_NUM];
                     CUDA_TRY(cudaMemcpyAsync(cur, d_counters.p, sizeof cur, cudaMemcpyDeviceToHost, st));
+                    CUDA_TRY(cudaMemcpyAsync(snap, d_z.p + ZC_SNAP, sizeof snap, cudaMemcpyDeviceToHost, st));
                     CUDA_TRY(cudaStreamSynchronize(st));
                     for (int c : {C_LEAF_EXACT, C_LEAF_SORTED, C_LEAF_REPLAY, C_LEAF_LISTS, C_LEAF_ENTRIES, C_LEAF_SHARED, C_ERROR})
                         snap[c] = cur[c];
+                    CUDA_TRY(cudaMemcpyAsync(d_counters.p, snap, sizeof snap, cudaMemcpyHostToDevice, st));
+                    CUDA_TRY(cudaStreamSynchronize(st));
                 }
-                CUDA_TRY(cudaMemcpyAsync(d_counters.p, snap, sizeof snap, cudaMemcpyHostToDevice, st));
             }
             CUDA_TRY(cudaEventRecord(ev[3], st));
             {
                 // superposition of every complete row into its slot in
                 // reference order, Query.__next__ per pair, compaction of
                 // the hits and warnings into this chunk's segment
-                unsigned long long nc = 0;
-                CUDA_TRY(cudaMemcpyAsync(&nc, d_ccount.p, sizeof nc, cudaMemcpyDeviceToHost, st));
-                CUDA_TRY(cudaStreamSynchronize(st));
-                const int64_t rows = (int64_t)nc;
+                const int64_t rows = (int64_t)hz[ZC_ROWS];  // (as read back last)
                 // the per-row stages below hold ~360 + 4 * stride bytes a
                 // complete row: when the chunk's rows need more than 70% of
                 // the memory they may use, or the row buffers could not hold
                 // them, the chunk is redone on half its structures
-                const int64_t budget_now = row_budget();
+                const bool many_rows = split || rows > (1 << 20) || getenv("PJG_ROW_BUDGET");
+                const int64_t budget_now = many_rows ? row_budget() : INT64_MAX;
                 if (Sc > 1 && (split || rows > budget_now)) {
                     // at most half the structures, fewer when the rows seen
                     // say so (rows scale with the structures of a chunk)
@@ -1930,7 +2262,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     search_rounds = search_rounds0;
                     suspensions = suspensions0;
                     ms_search = ms_search_chunk0;
-                    CUDA_TRY(cudaMemcpyAsync(d_counters.p, chunk_snap, sizeof chunk_snap, cudaMemcpyHostToDevice,
+                    CUDA_TRY(cudaMemcpyAsync(d_counters.p, d_z.p + ZC_CHUNK, stats_bytes, cudaMemcpyDeviceToDevice,
                                              st));
                     continue;
                 }
@@ -1956,8 +2288,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     int blocks = (int)std::min<int64_t>((rows + 127) / 128, (int64_t)sm_count() * 24);
                     launch_superpose(st, blocks, cv, tv, cr, rr);
                     CUDA_TRY(dalloc(d_long_pairs, (size_t)std::min<int64_t>(n_pairs, rows), st));
-                    CUDA_TRY(cudaMemsetAsync(d_rtotals.p, 0, 5 * sizeof(unsigned long long), st));
-                    if (free_chunk) {
+                    if (invalid_rows) {
                         // (rows of a pair that k_search took over have no slot)
                         CUDA_TRY(cudaMemsetAsync(d_r_hit.p, 0, (size_t)rows * sizeof(int32_t), st));
                         CUDA_TRY(cudaMemsetAsync(d_r_warn.p, 0, (size_t)rows * sizeof(int32_t), st));
@@ -1969,9 +2300,10 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(scan_exclusive(d_r_hit.p, rows, d_r_hidx.p, scan_tmp, st));
                     CUDA_TRY(scan_exclusive(d_r_warn.p, rows, d_r_widx.p, scan_tmp, st));
                     CUDA_TRY(scan_exclusive(d_r_hatoms.p, rows, d_r_aidx.p, scan_tmp, st));
-                    unsigned long long tot[4] = {};
-                    CUDA_TRY(cudaMemcpyAsync(tot, d_rtotals.p, sizeof tot, cudaMemcpyDeviceToHost, st));
+                    CUDA_TRY(cudaMemcpyAsync(hz, d_z.p, ZC_LIVE * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                             st));
                     CUDA_TRY(cudaStreamSynchronize(st));
+                    const unsigned long long *tot = hz + ZC_TOTALS;
                     passing += (int64_t)tot[3];
                     if (P->count_only) {
                         // counts only: the hits and warnings are not kept
@@ -1992,7 +2324,15 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 }
                 CUDA_TRY(cudaEventRecord(ev[4], st));
                 float m1 = 0, m2 = 0, m3 = 0;
-                CUDA_TRY(cudaEventSynchronize(ev[4]));
+                if (s1 == S) {
+                    // (the last chunk: with the query's end)
+                    CUDA_TRY(cudaMemcpyAsync(hz, d_z.p, ZC_LIVE * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                             st));
+                    CUDA_TRY(cudaEventRecord(ev[5], st));
+                    CUDA_TRY(cudaStreamSynchronize(st));
+                } else {
+                    CUDA_TRY(cudaEventSynchronize(ev[4]));
+                }
                 cudaEventElapsedTime(&m1, ev[1], ev[2]);
                 cudaEventElapsedTime(&m2, ev[2], ev[3]);
                 cudaEventElapsedTime(&m3, ev[3], ev[4]);
@@ -2004,7 +2344,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 // next chunk: as many structures as the row budget takes at
                 // this chunk's rows per structure (a dense chunk early in the
                 // set does not keep every later chunk small)
-                if (rows > 0 && max_chunk > 1) {
+                if (s1 == S) {
+                } else if (rows > 0 && max_chunk > 1) {
                     const double per = (double)rows / (double)Sc;
                     const double fit = 0.8 * (double)row_budget() / per;
                     chunk_cap = (int)std::max(1.0, std::min((double)max_chunk, fit));
@@ -2016,9 +2357,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             s0 = s1;
         }
     }
-    CUDA_TRY(cudaMemcpyAsync(counters, d_counters.p, sizeof counters, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaEventRecord(ev[5], st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    std::memcpy(counters, hz, sizeof counters);
     cudaEventElapsedTime(&ms, ev[0], ev[5]);
     ms_total = ms;
     if (counters[C_ERROR] == 3) {
@@ -2067,35 +2406,35 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
 
 done:
     if (st) {
-        dfree(d_sig_bits, st); dfree(d_kind_masks, st); dfree(d_units, st); dfree(d_heavy_pairs, st); dfree(d_free_n, st);
+        dfree(d_sig_bits, st); dfree(d_kind_masks, st); dfree(d_units, st); dfree(d_heavy_pairs, st);
         dfree(d_heavy_stats, st); dfree(d_row_key, st); dfree(d_items, st); dfree(d_results, st);
         dfree(d_item_base, st); dfree(d_bin_off, st); dfree(d_bins, st); dfree(d_arena_atom, st);
         dfree(d_row_scratch, st); dfree(d_arena_xyz, st); dfree(d_arena_parent, st); dfree(d_item_head, st);
         dfree(d_large_units, st); dfree(d_long_pairs, st); dfree(d_pending, st); dfree(d_item_branch, st); dfree(d_spill_a, st);
         dfree(d_spill_b, st);
         dfree(d_params, st); dfree(d_count, st); dfree(d_scanned, st); dfree(d_cand_atom, st);
-        dfree(d_leaf_atom, st); dfree(d_pair_counter, st); dfree(d_offset, st); dfree(d_totals, st);
+        dfree(d_leaf_atom, st); dfree(d_offset, st); dfree(d_totals, st);
         dfree(d_leaf_xyz, st); dfree(d_leaf_atom2, st); dfree(d_leaf_xyz2, st); dfree(d_leaf_off, st);
-        dfree(d_leaf_used, st); dfree(d_counters, st); dfree(d_ccount, st);
-        dfree(d_rtotals, st); dfree(d_c_pair, st); dfree(d_c_atoms, st); dfree(d_pair_rows, st);
+       
+        dfree(d_c_pair, st); dfree(d_c_atoms, st); dfree(d_pair_rows, st);
         dfree(d_cnt_q, st); dfree(d_c_ord, st); dfree(d_off_q, st); dfree(d_c_rmsd, st); dfree(d_boff, st);
         dfree(d_nblk, st); dfree(d_blk_lo, st); dfree(d_blk_hi, st); dfree(d_exact_list, st);
         dfree(d_exact_count, st); dfree(d_sorted_list, st); dfree(d_sorted_count, st);
         dfree(d_r_rmsd, st); dfree(d_r_rot, st); dfree(d_r_cen, st); dfree(d_r_nan, st); dfree(d_r_hit, st);
         dfree(d_r_warn, st); dfree(d_r_hatoms, st); dfree(d_r_src, st); dfree(d_r_hidx, st); dfree(d_r_widx, st);
-        dfree(d_r_aidx, st); dfree(d_lstate, st); dfree(d_work, st); dfree(d_nwork, st); dfree(d_nsusp, st);
+        dfree(d_r_aidx, st); dfree(d_lstate, st); dfree(d_work, st);
         dfree(d_pcost, st); dfree(d_hflag, st); dfree(d_heavy, st); dfree(d_hbins, st);
-        dfree(d_susp_a, st); dfree(d_susp_b, st); dfree(d_pool_a, st); dfree(d_pool_b, st); dfree(d_pool_used, st);
+        dfree(d_susp_a, st); dfree(d_susp_b, st); dfree(d_pool_a, st); dfree(d_pool_b, st);
         dfree(d_prof, st);
-        dfree(d_fill_state, st); dfree(d_fill_work, st); dfree(d_nfill, st);
+        dfree(d_fill_state, st); dfree(d_fill_work, st);
         dfree(d_ls_key, st); dfree(d_ls_n, st); dfree(d_ls_rep, st); dfree(d_ls_slot, st);
         dfree(d_ls_rep_work, st); dfree(d_ls_dup, st); dfree(d_ls_left, st); dfree(d_ls_ok, st);
+        dfree(d_z, st);
         for (auto &b : scan_tmp) dfree(b, st);
-        cudaStreamSynchronize(st);
-        cudaStreamDestroy(st);
+        t_cache = nullptr;
+        const cudaError_t e = cudaStreamSynchronize(st);
+        release_scratch(scratch, e == cudaSuccess && status != PJG_ERR_CUDA);
     }
-    for (auto &e : ev)
-        if (e) cudaEventDestroy(e);
     if (status != PJG_OK) {
         delete res;
         return status;
@@ -2146,22 +2485,24 @@ pjg_status pjg_results_superposed(const pjg_results *r, const pjg_structures *s,
     int prev = 0;
     cudaGetDevice(&prev);
     if (prev != r->device) cudaSetDevice(r->device);
-    cudaStream_t st = nullptr;
+    const size_t bytes = (size_t)hs.atoms * 3 * sizeof(double);
     double *d_out = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMallocAsync((void **)&d_out, (size_t)hs.atoms * 3 * sizeof(double), st);
+    cudaError_t e;
+    Scratch *x = acquire_scratch(r->device, &e);
+    if (e == cudaSuccess) e = cudaMallocAsync((void **)&d_out, bytes, x->st);
     if (e == cudaSuccess) {
-        launch_superposed_atoms(st, hs.hits, hs.atoms, hs.structure, hs.atom_offset, hs.atoms_, hs.rot, hs.centres,
+        launch_superposed_atoms(x->st, hs.hits, hs.atoms, hs.structure, hs.atom_offset, hs.atoms_, hs.rot, hs.centres,
                                 s->d_atom_base, s->d_xyz64, d_out);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(xyz, d_out, (size_t)hs.atoms * 3 * sizeof(double), cudaMemcpyDeviceToHost, st);
-    if (d_out) cudaFreeAsync(d_out, st);
-    if (st) {
-        cudaError_t e2 = cudaStreamSynchronize(st);
+    if (x) {
+        cudaError_t e2 = cudaStreamSynchronize(x->st);
         if (e == cudaSuccess) e = e2;
-        cudaStreamDestroy(st);
+        if (e == cudaSuccess) e = copy_out(xyz, d_out, bytes);
+        if (d_out) cudaFreeAsync(d_out, x->st);
+        e2 = cudaStreamSynchronize(x->st);
+        if (e == cudaSuccess) e = e2;
+        release_scratch(x, e == cudaSuccess);
     }
     if (prev != r->device) cudaSetDevice(prev);
     if (e != cudaSuccess) return fail(PJG_ERR_CUDA, "superposed atoms: %s", cudaGetErrorString(e));

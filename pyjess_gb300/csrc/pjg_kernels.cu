@@ -4660,8 +4660,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
         const bool ended = HEAVY && !sub && !spilled && sa.max_candidates >= 0 && rows >= sa.max_candidates + 2ll &&
                            (sa.best_match || !any_hit);
         if (!HEAVY && outgrown && !kd_needed) {
-            // in items of seeds, its level-0 list in candidate order
-            request_fill_warp(dm, lane == 0, lw);
+            // in items of seeds
             if (lane == 0) {
                 HeavyPair h;
                 h.pair = pair;
@@ -4672,15 +4671,13 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
             }
         } else {
             if (kd_needed) {
-                // every list in kd leaf order (level 0 in candidate order), then k_search
+                // in order, by k_search
                 int won = 1;
                 if (HEAVY) {
                     if (lane == 0) won = atomicExch(&fw.heavy[hidx].failed, 1) == 0;
                     won = __shfl_sync(FULL_MASK, won, 0);
                 }
                 if (won) {
-                    request_fill_warp(dm, lane == 0, lw);
-                    request_list_warp(dm, lane > 0 && lane < n, lw, llen);
                     if (lane == 0) {
                         Suspended sp;
                         sp.pair = pair;
@@ -4737,6 +4734,58 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
     add(C_COMPLETE, a_comp);
     add(C_BYTES_EXP, a_bexp);
     add(C_RECHECK, a_rech);
+}
+
+// Lists of the pairs that the order-free search passes on, thread per pair:
+// the level-0 list of each (in candidate order), every other list of those in
+// `suspended` (in kd leaf order).
+__global__ void k_free_requests(TemplateView tv, CandView cd, int32_t reorder, LeafDemand dm, const HeavyPair *heavy,
+                                int32_t n_heavy, const Suspended *suspended, int32_t s0, int32_t s1) {
+    const int T = tv.n_templates, G = cd.n_sigs;
+    const int total = n_heavy + s1 - s0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const bool all = i >= n_heavy;
+        const int pair = all ? suspended[s0 + i - n_heavy].pair : heavy[i].pair;
+        const int s = pair / T, t = pair % T;
+        const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
+        const int64_t wb = (int64_t)s * G;
+        int k0 = 0, best = INT_MAX;
+        for (int k = 0; k < n && reorder; k++) {
+            const int c = cd.count[wb + tv.sig[ab + k]];
+            if (c < best) {
+                best = c;
+                k0 = k;
+            }
+        }
+        request_fill(dm, wb + tv.sig[ab + k0]);
+        for (int k = 0; k < n && all; k++) {
+            const int64_t w = wb + tv.sig[ab + k];
+            if (k != k0) request_list(dm, w, cd.count[w]);
+        }
+    }
+}
+
+// Lists of the levels at which the rows of a pending unit part, warp per unit.
+__global__ void k_pending_requests(int64_t n_pending, TemplateView tv, CandView cd, int32_t reorder, LeafDemand dm,
+                                   FreeWork fw) {
+    const int lane = lane_id();
+    const int T = tv.n_templates, G = cd.n_sigs;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t x = warp; x < n_pending; x += nwarps) {
+        const RowUnit u = fw.units[fw.pending[x]];
+        const uint32_t branch = u.item >= 0 ? fw.item_branch[u.item] : u.branch;
+        const int s = u.pair / T, t = u.pair % T;
+        const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
+        int c = INT_MAX;
+        int64_t w = 0;
+        if (lane < n) {
+            w = (int64_t)s * G + tv.sig[ab + lane];
+            c = cd.count[w];
+        }
+        const int rank = level_rank(n, c, reorder);
+        request_list_warp(dm, lane < n && rank > 0 && ((branch >> rank) & 1u), w, c);
+    }
 }
 
 // Items of the pairs in `heavy`: block 0 of every pair, then block 1, ... (so
@@ -4967,7 +5016,7 @@ struct DirectWarp {
 template <int MAXM, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
     k_unit_order_direct(ChunkView cv, TemplateView tv, CandView cd, SigView sv, FreeView fv, const int32_t *res_place,
-                        int32_t reorder, FreeWork fw, CompleteRows out, LeafDemand dm) {
+                        int32_t reorder, FreeWork fw, CompleteRows out) {
     extern __shared__ __align__(16) unsigned char direct_smem[];
     constexpr bool LONG = MAXM > DIRECT_MAX;
     DirectWarp<MAXM> &U = reinterpret_cast<DirectWarp<MAXM> *>(direct_smem)[threadIdx.x >> 5];
@@ -5247,7 +5296,6 @@ __global__ void __launch_bounds__(WARPS * 32)
         }
         __syncwarp();
         if (pending) {
-            request_list_warp(dm, parts, wb + sg, c);
             if (lane == 0) fw.pending[atomicAdd(fw.n_pending, 1ull)] = w;
         } else {
             for (int i = lane; i < R; i += 32) out.ordinal[U.row[i]] = ord0 + U.cur[i];
@@ -6021,6 +6069,21 @@ cudaError_t launch_search_heavy(cudaStream_t st, bool fp32, int64_t warps, const
     return cudaGetLastError();
 }
 
+void launch_free_requests(cudaStream_t st, const TemplateView &tv, const CandView &cd, int32_t reorder,
+                          const LeafDemand &dm, const HeavyPair *heavy, int32_t n_heavy, const Suspended *suspended,
+                          int32_t s0, int32_t s1) {
+    const int64_t n = (int64_t)n_heavy + s1 - s0;
+    if (n > 0)
+        k_free_requests<<<(int)std::min<int64_t>((n + 127) / 128, 152 * 16), 128, 0, st>>>(tv, cd, reorder, dm, heavy,
+                                                                                         n_heavy, suspended, s0, s1);
+}
+
+void launch_pending_requests(cudaStream_t st, int64_t n_pending, const TemplateView &tv, const CandView &cd,
+                             int32_t reorder, const LeafDemand &dm, const FreeWork &fw) {
+    k_pending_requests<<<(int)std::min<int64_t>((n_pending + 7) / 8, 152 * 8), 256, 0, st>>>(n_pending, tv, cd,
+                                                                                           reorder, dm, fw);
+}
+
 void launch_heavy_bins(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy, int32_t *bins) {
     k_heavy_bins<<<(n_heavy + 255) / 256, 256, 0, st>>>(n_heavy, heavy, bins);
 }
@@ -6039,7 +6102,7 @@ void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int
 cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
                                      const CandView &cd, const SigView &sv, const FreeView &fv,
                                      const int32_t *res_place, int32_t reorder, const FreeWork &fw,
-                                     const CompleteRows &out, const LeafDemand &dm) {
+                                     const CompleteRows &out) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -6050,7 +6113,7 @@ cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const Chu
         if (e != cudaSuccess) return e;
         const int64_t blocks = std::min<int64_t>((units + warps - 1) / warps, (int64_t)std::max(per_sm * sms, 1) * 4);
         kern<<<(int)std::max<int64_t>(blocks, 1), warps * 32, smem, st>>>(cv, tv, cd, sv, fv, res_place, reorder, fw,
-                                                                         out, dm);
+                                                                         out);
         return cudaGetLastError();
     };
     cudaError_t e = launch(k_unit_order_direct<DIRECT_MAX, DIRECT_WARPS>,
@@ -6296,12 +6359,7 @@ __global__ void __launch_bounds__(COMPACT_THREADS)
 
 #include "../../include/pjg.h"
 
-namespace {
-std::mutex g_noalloc_mutex;
-void *g_noalloc_ptr[64] = {};                 // device address of g_noalloc_words, per device
-unsigned long long g_noalloc_ctx[64] = {};    // id of the context that address belongs to
-thread_local char g_noalloc_err[256];
-
+namespace pjg {
 // Unique id of the calling thread's current CUDA context (0 if unknown).
 // The driver never reuses an id, so a context destroyed and recreated on
 // the same device (cudaDeviceReset, then new work) gets a new one.  The two
@@ -6333,6 +6391,15 @@ unsigned long long current_context_id() {
     if (!get_current || !get_id || get_current(&ctx) != 0 || !ctx || get_id(ctx, &id) != 0) return 0;
     return id;
 }
+}  // namespace pjg
+
+namespace {
+using pjg::current_context_id;
+std::mutex g_noalloc_mutex;
+void *g_noalloc_ptr[64] = {};                 // device address of g_noalloc_words, per device
+unsigned long long g_noalloc_ctx[64] = {};    // id of the context that address belongs to
+thread_local char g_noalloc_err[256];
+
 }  // namespace
 
 extern "C" const char *pjg_noalloc_last_error(void) { return g_noalloc_err; }

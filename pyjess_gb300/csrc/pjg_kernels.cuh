@@ -364,6 +364,10 @@ struct HitSegment {
     int64_t *warn_before;              // hits of the structure before the warning
 };
 
+// unique id of the calling thread's current CUDA context (0 if unknown; ids
+// are never reused)
+unsigned long long current_context_id();
+
 // bytes of k_search's per-warp pair state (shared memory, before the tiles)
 size_t search_state_bytes();
 
@@ -470,7 +474,7 @@ void launch_list_kinds(cudaStream_t st, const ChunkView &cv, const SigView &sv, 
 
 // the order-free search over every pair: rows and units of rows to put in
 // order (fw), pairs to search in items (fw.heavy), and the pairs left to
-// k_search in dm.suspended, with the lists each of them needs requested
+// k_search in dm.suspended
 cudaError_t launch_search_free(cudaStream_t st, bool fp32, const ChunkView &cv, const TemplateView &tv,
                                const CandView &cd, const FreeView &fv, const SearchArgs &sa, int32_t *item_counter,
                                const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
@@ -488,12 +492,19 @@ void launch_heavy_items(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy
 void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int64_t *item_base, int32_t *pair_rows,
                        unsigned long long *counters);
 // the units' rows in the reference's order (out.ordinal): without lists in
-// leaf order where that can be done (the others in fw.pending, their lists
-// requested), then those by their lists' leaf order
+// leaf order where that can be done (the others in fw.pending), then those by
+// their lists' leaf order
 cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
                                      const CandView &cd, const SigView &sv, const FreeView &fv,
                                      const int32_t *res_place, int32_t reorder, const FreeWork &fw,
-                                     const CompleteRows &out, const LeafDemand &dm);
+                                     const CompleteRows &out);
+// the lists that the pairs passed on by the order-free search, and the
+// pending units, need: heavy pairs and suspended[s0 .. s1)
+void launch_free_requests(cudaStream_t st, const TemplateView &tv, const CandView &cd, int32_t reorder,
+                          const LeafDemand &dm, const HeavyPair *heavy, int32_t n_heavy, const Suspended *suspended,
+                          int32_t s0, int32_t s1);
+void launch_pending_requests(cudaStream_t st, int64_t n_pending, const TemplateView &tv, const CandView &cd,
+                             int32_t reorder, const LeafDemand &dm, const FreeWork &fw);
 void launch_unit_order(cudaStream_t st, int64_t n_pending, const ChunkView &cv, const TemplateView &tv,
                        const CandView &cd, const SigView &sv, const int32_t *res_place, int32_t reorder,
                        const FreeWork &fw, const CompleteRows &out);

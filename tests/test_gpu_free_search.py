@@ -174,6 +174,37 @@ def test_rows_told_apart_in_lists_of(residues, step):
     assert ref["hits"]["count"] > 1
 
 
+def test_concurrent_queries():
+    """Queries from four threads on shared handles (each takes a stream and
+    its kept blocks for itself), structure sets made and dropped meanwhile:
+    the hits of a query alone."""
+    import threading
+
+    from pyjess_gb300 import _native, workloads as W
+    from pyjess_gb300._abi import QueryParams
+
+    wl = W.config(3, n_structures=30, n_templates=300)
+    T, S = _native.Templates(wl.templates), _native.Structures(wl.structures)
+    P = QueryParams(rmsd_threshold=2.0, distance_cutoff=1.5, max_dynamic_distance=1.5, max_candidates=-1,
+                    ignore_chain=0, best_match=0, reorder=1, mode=_native.MODE_BATCHED_FP32)
+    want = _native.query(T, S, P).arrays()
+    bad = []
+
+    def work(i):
+        for k in range(4):
+            s = S if (i + k) % 2 else _native.Structures(wl.structures)
+            a = _native.query(T, s, P).arrays()
+            if any(not np.array_equal(a[c], want[c]) for c in want):
+                bad.append((i, k))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert want["count"] > 0 and not bad
+
+
 def test_long_lists_replayed():
     """Backbone lists of 4,300 entries with ties (the exact replay in 192 KB of
     shared memory)."""
