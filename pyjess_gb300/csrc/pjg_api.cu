@@ -1056,7 +1056,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
         e = dalloc(tile_key, 4 * n1, x->st);
         if (e == cudaSuccess) e = dalloc(tile_idx, 4 * n1, x->st);
         if (e == cudaSuccess) {
-            launch_axis_ranks(x->st, S, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key.p, tile_idx.p,
+            launch_axis_ranks(x->st, S, h->max_atoms, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key.p, tile_idx.p,
                               h->d_lrank, h->d_urank,
                               ResidueOrder{h->d_xyz32, h->d_nh_pos, d_local_kind, h->d_kxyz, h->d_res_pos,
                                            h->d_res_kind, h->d_res_range, h->d_sorted, h->d_res_place});

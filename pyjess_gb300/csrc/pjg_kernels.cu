@@ -1626,14 +1626,17 @@ __global__ void k_leaf_exact(ChunkView cv, int32_t n_sigs, const int32_t *count,
 // coordinate on a is strictly smaller, so lranks compare exactly as the FP64
 // coordinates do (equal coordinates share one); urank = number of atoms
 // before i in (coordinate, index) order, a permutation of 0..n-1
-// (coordinates are finite: pjg_structures_create rejects others).  One
-// block per
-// (structure, axis): the atoms are sorted in tiles of RANK_TILE in shared
-// memory, each tile is stored, and every atom's ranks are sums of binary
-// searches over the sorted tiles.
+// (coordinates are finite: pjg_structures_create rejects others).  A fourth
+// "axis", the residue key, gives the residue order of FreeView.
+//
+// Two kernels, so that one structure spreads over the chip: a block sorts a
+// tile of RANK_TILE atoms of one axis in shared memory, then a thread per
+// (atom, axis) sums binary searches over the sorted tiles.  Bound by their
+// latency for a single structure (8,000 atoms: 310 us with one block an axis
+// and tiles of 2,048, 75 us now).
 
-constexpr int RANK_TILE = 2048;
-constexpr int RANK_THREADS = 512;
+constexpr int RANK_TILE = 512;
+constexpr int RANK_THREADS = 256;
 
 __device__ __forceinline__ unsigned long long order_key(double x) {
     if (x == 0.0) x = 0.0;  // -0 and +0 compare equal
@@ -1646,118 +1649,106 @@ __device__ __forceinline__ unsigned long long residue_key(int32_t k) {
     return (unsigned long long)((uint32_t)k ^ 0x80000000u);
 }
 
+// sort key of atom i (global index): its coordinate on axis a, or (a == 3)
+// its residue key
+__device__ __forceinline__ unsigned long long rank_key(const double *xyz64, const ResidueOrder &ro, int64_t i, int a) {
+    return a < 3 ? order_key(xyz64[3 * i + a]) : residue_key(__float_as_int(ro.xyz32[i].w));
+}
+
 __global__ void __launch_bounds__(RANK_THREADS)
-    k_axis_ranks(const int64_t *atom_base, const int32_t *atom_count, const double *xyz64, int64_t n_atoms,
-                 unsigned long long *tile_key, uint16_t *tile_idx, uint32_t *lrank, uint32_t *urank,
-                 ResidueOrder ro) {
+    k_rank_tiles(const int64_t *atom_base, const int32_t *atom_count, const double *xyz64, int64_t n_atoms,
+                 unsigned long long *tile_key, uint16_t *tile_idx, ResidueOrder ro) {
     __shared__ unsigned long long key[RANK_TILE];
     __shared__ uint16_t idx[RANK_TILE];
     const int s = blockIdx.x, a = blockIdx.y;
     const int64_t b0 = atom_base[s];
     const int n = atom_count[s];
-    const int tiles = (n + RANK_TILE - 1) / RANK_TILE;
-    unsigned long long *gk = tile_key + a * n_atoms + b0;
-    uint16_t *gi = tile_idx + a * n_atoms + b0;
-    // sort key of atom i: its coordinate, or (a == 3) its residue key
-    auto key_of = [&](int i) -> unsigned long long {
-        return a < 3 ? order_key(xyz64[3 * (b0 + i) + a]) : residue_key(__float_as_int(ro.xyz32[b0 + i].w));
-    };
-    for (int t = 0; t < tiles; t++) {
-        const int t0 = t * RANK_TILE, tn = min(RANK_TILE, n - t0);
-        for (int i = threadIdx.x; i < RANK_TILE; i += blockDim.x) {
-            if (i < tn) {
-                key[i] = key_of(t0 + i);
-            } else {
-                key[i] = ~0ull;
-            }
+    for (int t0 = blockIdx.z * RANK_TILE; t0 < n; t0 += gridDim.z * RANK_TILE) {
+        const int tn = min(RANK_TILE, n - t0);
+        for (int i = threadIdx.x; i < RANK_TILE; i += RANK_THREADS) {
+            key[i] = i < tn ? rank_key(xyz64, ro, b0 + t0 + i, a) : ~0ull;
             idx[i] = (uint16_t)i;
         }
         __syncthreads();
-        // bitonic sort by (key, idx)
+        // bitonic sort by (key, idx), a pair a thread
+        static_assert(RANK_TILE == 2 * RANK_THREADS, "one pair a thread");
         for (int k = 2; k <= RANK_TILE; k <<= 1) {
             for (int j = k >> 1; j > 0; j >>= 1) {
-                const int lj = __ffs(j) - 1;
-                for (int q = threadIdx.x; q < RANK_TILE / 2; q += blockDim.x) {
-                    const int i = ((q >> lj) << (lj + 1)) | (q & (j - 1));
-                    const int l = i | j;
-                    const bool asc = (i & k) == 0;
-                    const unsigned long long ki = key[i], kl = key[l];
-                    const uint16_t ii = idx[i], il = idx[l];
-                    const bool gt = ki > kl || (ki == kl && ii > il);
-                    if (gt == asc) {
-                        key[i] = kl;
-                        key[l] = ki;
-                        idx[i] = il;
-                        idx[l] = ii;
-                    }
+                const int q = threadIdx.x, lj = __ffs(j) - 1;
+                const int i = ((q >> lj) << (lj + 1)) | (q & (j - 1));
+                const int l = i | j;
+                const bool asc = (i & k) == 0;
+                const unsigned long long ki = key[i], kl = key[l];
+                const uint16_t ii = idx[i], il = idx[l];
+                const bool gt = ki > kl || (ki == kl && ii > il);
+                if (gt == asc) {
+                    key[i] = kl;
+                    key[l] = ki;
+                    idx[i] = il;
+                    idx[l] = ii;
                 }
                 __syncthreads();
             }
         }
-        for (int i = threadIdx.x; i < tn; i += blockDim.x) {
-            gk[t0 + i] = key[i];
-            gi[t0 + i] = idx[i];
+        for (int i = threadIdx.x; i < tn; i += RANK_THREADS) {
+            tile_key[a * n_atoms + b0 + t0 + i] = key[i];
+            tile_idx[a * n_atoms + b0 + t0 + i] = idx[i];
         }
         __syncthreads();
     }
-    if (a == 3)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            ro.kxyz[b0 + i] = ro.xyz32[b0 + ro.nh_pos[b0 + i]];
-            ro.res_place[b0 + ro.sorted[b0 + i]] = i;
+}
+
+__global__ void __launch_bounds__(RANK_THREADS)
+    k_axis_ranks(const int64_t *atom_base, const int32_t *atom_count, const double *xyz64, int64_t n_atoms,
+                 const unsigned long long *tile_key, const uint16_t *tile_idx, uint32_t *lrank, uint32_t *urank,
+                 ResidueOrder ro) {
+    const int s = blockIdx.x, a = blockIdx.y;
+    const int64_t b0 = atom_base[s];
+    const int n = atom_count[s];
+    const unsigned long long *gk = tile_key + a * n_atoms + b0;
+    const uint16_t *gi = tile_idx + a * n_atoms + b0;
+    // entries of tile t below key k
+    auto lower = [&](int t, unsigned long long k) -> int {
+        const unsigned long long *tk = gk + t * RANK_TILE;
+        int lo = 0, hi = min(RANK_TILE, n - t * RANK_TILE);
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (tk[mid] < k) lo = mid + 1;
+            else hi = mid;
         }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const unsigned long long ki = key_of(i);
+        return lo;
+    };
+    const int tiles = (n + RANK_TILE - 1) / RANK_TILE;
+    for (int i = blockIdx.z * RANK_THREADS + threadIdx.x; i < n; i += gridDim.z * RANK_THREADS) {
+        const unsigned long long ki = rank_key(xyz64, ro, b0 + i, a);
         const int ti = i / RANK_TILE;
         const uint16_t li = (uint16_t)(i % RANK_TILE);
         uint32_t lr = 0, ur = 0;
         for (int t = 0; t < tiles; t++) {
-            const unsigned long long *tk = gk + t * RANK_TILE;
-            const int tn = min(RANK_TILE, n - t * RANK_TILE);
-            int lo = 0, hi = tn;
-            while (lo < hi) {  // first key >= ki
-                const int mid = (lo + hi) >> 1;
-                if (tk[mid] < ki) lo = mid + 1;
-                else hi = mid;
-            }
+            const int lo = lower(t, ki);
             lr += lo;
-            if (t < ti) {  // earlier atoms: equal keys come before i
-                int l2 = lo, h2 = tn;
-                while (l2 < h2) {
-                    const int mid = (l2 + h2) >> 1;
-                    if (tk[mid] <= ki) l2 = mid + 1;
-                    else h2 = mid;
-                }
-                ur += l2;
-            } else if (t == ti) {  // i's own tile: (key, index) order
+            int l2 = lo;
+            if (t < ti) {
+                l2 = lower(t, ki + 1);  // earlier atoms: equal keys come before i
+            } else if (t == ti) {       // i's own tile: (key, index) order
+                const unsigned long long *tk = gk + t * RANK_TILE;
                 const uint16_t *tix = gi + t * RANK_TILE;
-                int l2 = lo, h2 = tn;
+                int h2 = min(RANK_TILE, n - t * RANK_TILE);
                 while (l2 < h2) {
                     const int mid = (l2 + h2) >> 1;
                     if (tk[mid] < ki || (tk[mid] == ki && tix[mid] < li)) l2 = mid + 1;
                     else h2 = mid;
                 }
-                ur += l2;
-            } else {
-                ur += lo;
             }
+            ur += l2;
         }
         if (a < 3) {
             lrank[a * n_atoms + b0 + i] = lr;
             urank[a * n_atoms + b0 + i] = ur;
         } else {
-            // positions below k over the sorted tiles
             auto below = [&](unsigned long long k) -> int {
                 int acc = 0;
-                for (int t = 0; t < tiles; t++) {
-                    const unsigned long long *tk = gk + t * RANK_TILE;
-                    int lo = 0, hi = min(RANK_TILE, n - t * RANK_TILE);
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (tk[mid] < k) lo = mid + 1;
-                        else hi = mid;
-                    }
-                    acc += lo;
-                }
+                for (int t = 0; t < tiles; t++) acc += lower(t, k);
                 return acc;
             };
             const unsigned long long seq = ki & ~0xFFull;  // first key of the residue number
@@ -1765,6 +1756,8 @@ __global__ void __launch_bounds__(RANK_THREADS)
             ro.res_pos[b0 + ur] = i;
             ro.res_kind[b0 + ur] = ro.local_kind[b0 + i];
             ro.res_range[b0 + i] = make_int4((int)lr, below(ki + 1) - (int)lr, r0, below(seq + 256) - r0);
+            ro.kxyz[b0 + i] = ro.xyz32[b0 + ro.nh_pos[b0 + i]];
+            ro.res_place[b0 + ro.sorted[b0 + i]] = i;
         }
     }
 }
@@ -5891,11 +5884,18 @@ void launch_leaf_order(cudaStream_t st, int blocks, const ChunkView &cv, int32_t
                       blk_lo, blk_hi, exact_list, exact_count, counters);
 }
 
-void launch_axis_ranks(cudaStream_t st, int32_t n_structures, const int64_t *atom_base, const int32_t *atom_count,
-                       const double *xyz64, int64_t n_atoms, unsigned long long *tile_key, uint16_t *tile_idx,
+void launch_axis_ranks(cudaStream_t st, int32_t n_structures, int32_t max_atoms, const int64_t *atom_base,
+                       const int32_t *atom_count, const double *xyz64, int64_t n_atoms, unsigned long long *tile_key, uint16_t *tile_idx,
                        uint32_t *lrank, uint32_t *urank, const ResidueOrder &ro) {
     if (n_structures <= 0) return;
-    k_axis_ranks<<<dim3((unsigned)n_structures, 4), RANK_THREADS, 0, st>>>(
+    // enough blocks a structure for the longest one, up to a few waves of the
+    // chip in all
+    const int64_t tiles = ((int64_t)max_atoms + RANK_TILE - 1) / RANK_TILE;
+    const unsigned z = (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>({tiles, 65535, std::max<int64_t>(1, 152 * 64 / ((int64_t)n_structures * 4))}));
+    k_rank_tiles<<<dim3((unsigned)n_structures, 4, z), RANK_THREADS, 0, st>>>(atom_base, atom_count, xyz64, n_atoms,
+                                                                             tile_key, tile_idx, ro);
+    k_axis_ranks<<<dim3((unsigned)n_structures, 4, 2 * z), RANK_THREADS, 0, st>>>(
         atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, lrank, urank, ro);
 }
 

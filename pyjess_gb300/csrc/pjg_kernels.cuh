@@ -461,8 +461,8 @@ struct ResidueOrder {
     const int32_t *sorted;
     int32_t *res_place;  // per atom: its position in ResIndex order
 };
-void launch_axis_ranks(cudaStream_t st, int32_t n_structures, const int64_t *atom_base, const int32_t *atom_count,
-                       const double *xyz64, int64_t n_atoms, unsigned long long *tile_key, uint16_t *tile_idx,
+void launch_axis_ranks(cudaStream_t st, int32_t n_structures, int32_t max_atoms, const int64_t *atom_base,
+                       const int32_t *atom_count, const double *xyz64, int64_t n_atoms, unsigned long long *tile_key, uint16_t *tile_idx,
                        uint32_t *lrank, uint32_t *urank, const ResidueOrder &ro);
 
 // sig_bits of FreeView: the kinds of every signature's list

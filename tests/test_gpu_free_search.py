@@ -205,6 +205,22 @@ def test_concurrent_queries():
     assert want["count"] > 0 and not bad
 
 
+@pytest.mark.parametrize("atoms", [1, 511, 512, 513, 1025])
+def test_structures_around_a_rank_tile(atoms):
+    """Structures cut to sizes around the tiles the axis ranks are sorted in
+    (half of them on a coarse grid: equal coordinates across tiles)."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(37, [160, 160])
+    specs = _templates(37, structs, 20, hi=4)
+    for i, s in enumerate(structs):
+        for k in ("xyz", "name", "resname", "res_seq", "chain", "serial"):
+            s[k] = np.ascontiguousarray(s[k][:atoms])
+        if i:
+            s["xyz"] = np.round(s["xyz"] / 0.25) * 0.25
+    compare(W.pack_templates(specs), W.pack(structs), **PARAMS)
+
+
 def test_long_lists_replayed():
     """Backbone lists of 4,300 entries with ties (the exact replay in 192 KB of
     shared memory)."""
