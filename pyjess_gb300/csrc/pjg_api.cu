@@ -380,9 +380,10 @@ struct pjg_templates {
     uint32_t *d_names = nullptr, *d_resnames = nullptr, *d_partner_res = nullptr, *d_partner_name = nullptr;
     int64_t n_params = 0;
     int device = 0;
-    // templates of more than 32 atoms (searched by k_search_large)
-    std::vector<int32_t> large;
-    int32_t *d_large = nullptr;
+    // templates of more than 32 atoms (k_search_large in the search in order);
+    // of them, those of at most 64 (order-free search) and the larger ones
+    std::vector<int32_t> large, wide, huge;
+    int32_t *d_large = nullptr, *d_wide = nullptr, *d_huge = nullptr;
     void *block = nullptr;  // the device arrays
     bool counted = false;   // a live handle
 };
@@ -657,7 +658,10 @@ pjg_status pjg_templates_create(const pjg_template_set *set, pjg_templates **out
             return fail(PJG_ERR_INVALID, "template %d has %d atoms; at most %d are supported", t, a1 - a0,
                         MAX_TEMPLATE_ATOMS);
         }
-        if (a1 - a0 > 32) h->large.push_back(t);
+        if (a1 - a0 > 32) {
+            h->large.push_back(t);
+            (a1 - a0 <= 64 ? h->wide : h->huge).push_back(t);
+        }
         h->nmax = std::max(h->nmax, a1 - a0);
     }
     for (int a = 0; a < A; a++) {
@@ -769,6 +773,8 @@ pjg_status pjg_templates_create(const pjg_template_set *set, pjg_templates **out
         up.add(&h->d_partner_res, s_pres);
         up.add(&h->d_partner_name, s_pname);
         up.add(&h->d_large, h->large);
+        up.add(&h->d_wide, h->wide);
+        up.add(&h->d_huge, h->huge);
         keep_pool(h->device);
         cudaError_t e;
         Scratch *x = acquire_scratch(h->device, &e);
@@ -1302,7 +1308,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     DBuf<int2> d_items, d_results;
     DBuf<int64_t> d_item_base, d_bin_off;
     DBuf<int32_t> d_bins, d_arena_atom, d_row_scratch, d_item_head, d_large_units, d_long_pairs, d_pending;
-    DBuf<uint32_t> d_item_branch;
+    DBuf<unsigned long long> d_item_branch;
     DBuf<SpilledEntry> d_spill_a, d_spill_b;
     DBuf<float4> d_arena_xyz;
     DBuf<uint16_t> d_arena_parent;
@@ -1815,7 +1821,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             }
             // (lists requested in this chunk and the attempt's counters)
             CUDA_TRY(cudaMemsetAsync(d_leaf_used.p, 0, (ZC_LIVE - ZC_LEAF_USED) * sizeof(unsigned long long), st));
-            if (!free_chunk || !tp->large.empty()) CUDA_TRY(setup_lists());
+            if (!free_chunk || !tp->huge.empty()) CUDA_TRY(setup_lists());
             if (demand_levels < 0) {
                 CUDA_TRY(order_requested());
             } else {
@@ -1861,10 +1867,10 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(cudaMemsetAsync(d_hbins.p, 0, 66 * sizeof(unsigned long long), st));
                     dm.pair_cost = d_pcost.p;
                 }
-                // (order-free first: only the lists of templates over 32 atoms)
-                if (!free_chunk || !tp->large.empty()) {
+                // (order-free first: only the lists of templates over 64 atoms)
+                if (!free_chunk || !tp->huge.empty()) {
                     launch_demand_levels(st, sm_count() * 16, tv, cd, (int32_t)n_pairs,
-                                         free_chunk ? -1 : demand_levels, P->reorder, dm);
+                                         free_chunk ? -1 : demand_levels, P->reorder, free_chunk ? 64 : 32, dm);
                     if (heavy_on) {
                         launch_heavy_pairs(st, (int32_t)n_pairs, d_pcost.p, d_hbins.p, heavy_target, d_hflag.p,
                                            d_heavy.p);
@@ -1986,7 +1992,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     dm.pool_out = pool_next;
                     // requested lists, suspended pairs, pool and work queue
                     // (the first order-free round: zeroed with the attempt)
-                    if (round > 0 || !free_chunk || !tp->large.empty())
+                    if (round > 0 || !free_chunk || !tp->huge.empty())
                         CUDA_TRY(cudaMemsetAsync(d_nwork.p, 0, (ZC_TOTALS - ZC_NWORK) * sizeof(unsigned long long),
                                                  st));
                     CUDA_TRY(cudaEventRecord(ev[6], st));
@@ -2007,17 +2013,30 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         fw.n_heavy = d_free_n.p + 1;
                         CUDA_TRY(launch_search_free(st, fp32, cv, tv, cd, fv, sa, d_pair_counter.p, scn_c, cr,
                                                     d_counters.p, dm, fw));
+                        if (!tp->wide.empty()) {
+                            FreeWork ww = fw;
+                            ww.wide = tp->d_wide;
+                            ww.n_wide = (int32_t)tp->wide.size();
+                            CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
+                            CUDA_TRY(launch_search_free(st, fp32, cv, tv, cd, fv, sa, d_pair_counter.p, scn_c, cr,
+                                                        d_counters.p, dm, ww));
+                            launches++;
+                        }
                     } else {
                         CUDA_TRY(launch_search(st, grid, wide, fp32, cv, tv, cd, sa, d_pair_counter.p, scn_c, cr,
                                                d_counters.p, dm));
                     }
                     launches++;
-                    if (round == 0 && !tp->large.empty()) {
-                        // pairs of templates over 32 atoms (every list of
-                        // theirs was ordered before this round)
+                    // pairs of templates over 32 atoms (over 64: the others
+                    // are searched without order), every list of theirs
+                    // ordered before this round; later, those left to it
+                    const bool left = free_chunk && round > 0;
+                    const auto &big = free_chunk && !left ? tp->huge : tp->large;
+                    if ((round == 0 || left) && !big.empty()) {
                         CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
-                        CUDA_TRY(launch_search_large(st, cv, tv, cd, sa, tp->d_large, (int32_t)tp->large.size(),
-                                                     d_pair_counter.p, scn_c, cr, d_counters.p, dm.state));
+                        CUDA_TRY(launch_search_large(st, cv, tv, cd, sa, free_chunk && !left ? tp->d_huge : tp->d_large,
+                                                     (int32_t)big.size(), d_pair_counter.p, scn_c, cr, d_counters.p,
+                                                     dm.state, left ? dm.resume : nullptr, left ? dm.n_resume : 0));
                         launches++;
                     }
                     CUDA_TRY(cudaEventRecord(ev[7], st));
@@ -2079,7 +2098,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         CUDA_TRY(cudaMemsetAsync(d_bins.p, 0, 2 * (size_t)nbins * sizeof(int32_t), st));
                         CUDA_TRY(cudaMemsetAsync(d_results.p, 0xFF, (size_t)ni * sizeof(int2), st));
                         CUDA_TRY(cudaMemsetAsync(d_item_head.p, 0xFF, (size_t)ni * sizeof(int32_t), st));
-                        CUDA_TRY(cudaMemsetAsync(d_item_branch.p, 0, (size_t)ni * sizeof(uint32_t), st));
+                        CUDA_TRY(cudaMemsetAsync(d_item_branch.p, 0, (size_t)ni * sizeof(unsigned long long), st));
                         CUDA_TRY(cudaMemsetAsync(d_heavy_stats.p, 0, 4 * (size_t)nh * sizeof(unsigned long long), st));
                         CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
                         launch_heavy_bins(st, nh, d_heavy_pairs.p, d_bins.p);
@@ -2097,9 +2116,22 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         fw.item_branch = d_item_branch.p;
                         fw.spilled_out = d_spill_a.p;
                         fw.spill_cap = SPILL_CAP;
+                        // every item, and again for those of wide templates
+                        auto search_items = [&](int64_t w) -> cudaError_t {
+                            cudaError_t e = launch_search_heavy(st, fp32, w, cv, tv, cd, fv, sa, d_pair_counter.p, cr,
+                                                                d_counters.p, dm, fw);
+                            if (e != cudaSuccess || tp->wide.empty()) return e;
+                            FreeWork ww = fw;
+                            ww.wide = tp->d_wide;
+                            ww.n_wide = (int32_t)tp->wide.size();
+                            e = cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st);
+                            if (e != cudaSuccess) return e;
+                            launches++;
+                            return launch_search_heavy(st, fp32, w, cv, tv, cd, fv, sa, d_pair_counter.p, cr,
+                                                       d_counters.p, dm, ww);
+                        };
                         CUDA_TRY(cudaEventRecord(ev[6], st));
-                        CUDA_TRY(launch_search_heavy(st, fp32, warps, cv, tv, cd, fv, sa, d_pair_counter.p, cr,
-                                                     d_counters.p, dm, fw));
+                        CUDA_TRY(search_items(warps));
                         CUDA_TRY(cudaEventRecord(ev[7], st));
                         launches += 3;
                         CUDA_TRY(cudaGetLastError());
@@ -2126,8 +2158,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                             fw.arena_atom = d_arena_atom.p;
                             fw.arena_parent = d_arena_parent.p;
                             CUDA_TRY(cudaEventRecord(ev[6], st));
-                            CUDA_TRY(launch_search_heavy(st, fp32, warps, cv, tv, cd, fv, sa, d_pair_counter.p, cr,
-                                                         d_counters.p, dm, fw));
+                            CUDA_TRY(search_items(warps));
                             CUDA_TRY(cudaEventRecord(ev[7], st));
                             launches++;
                             CUDA_TRY(cudaGetLastError());

@@ -2160,7 +2160,7 @@ __device__ __forceinline__ void request_list_warp(const LeafDemand &dm, bool wan
 // search itself when a pair first reaches them.  Consecutive threads take
 // consecutive templates of one structure.
 __global__ void k_demand_levels(TemplateView tv, CandView cd, int32_t n_pairs, int32_t max_level, int32_t reorder,
-                                LeafDemand dm) {
+                                int32_t whole_over, LeafDemand dm) {
     constexpr int TOP = 8;  // levels requested through the warp-wide path
     const int lane = lane_id();
     const int T = tv.n_templates, G = cd.n_sigs;
@@ -2185,7 +2185,7 @@ __global__ void k_demand_levels(TemplateView tv, CandView cd, int32_t n_pairs, i
             if (cd.count[wb + tv.sig[ab]] > 0) levels = 0;  // its only list, in candidate order
             top[0] = 0;
         } else if (n > 32) {
-            per_thread = true;  // k_search_large: every list, below
+            per_thread = n > whole_over;  // k_search_large: every list, below
         } else if (n >= 2) {
             // the (max_level + 1) smallest (length, index) keys, sorted in
             // registers
@@ -3695,7 +3695,7 @@ __device__ __forceinline__ bool decide_fp64_chain(int levp, const int32_t *catom
 __global__ void __launch_bounds__(LARGE_WARPS * 32)
     k_search_large(ChunkView cv, TemplateView tv, CandView cd, SearchArgs sa, const int32_t *large, int32_t n_large,
                    int32_t *item_counter, const int32_t *scanned, CompleteRows out, unsigned long long *counters,
-                   const int32_t *lstate) {
+                   const int32_t *lstate, const Suspended *left, int32_t n_left) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = lane_id();
     const int nmax = tv.max_atoms;
@@ -3716,17 +3716,20 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
     if (lane == 0) t_start = global_ns();
     bool timed_out = false;
     uint32_t ticks = 0;
-    const int64_t n_items = (int64_t)cv.n_structures * n_large;
+    // every pair of the templates `large`, or those of more than 32 atoms
+    // among the pairs the order-free search left (already counted)
+    const int64_t n_items = left ? n_left : (int64_t)cv.n_structures * n_large;
     for (;;) {
         int64_t item = 0;
         if (lane == 0) item = atomicAdd(item_counter, 1);
         item = __shfl_sync(FULL_MASK, item, 0);
         if (item >= n_items || timed_out) break;
-        const int s = (int)(item / n_large);
-        const int t = large[item % n_large];
+        const int s = left ? left[item].pair / T : (int)(item / n_large);
+        const int t = left ? left[item].pair % T : large[item % n_large];
         const int pair = s * T + t;
         const int ab = tv.atom_begin[t];
         const int n = tv.atom_begin[t + 1] - ab;
+        if (left && n <= 32) continue;
         const int64_t abase = cv.atom_base[s];
         const double *xyz64 = cv.xyz64 + 3 * abase;
         // lengths, empty-set skip and statistics (template atom order), as
@@ -3750,7 +3753,7 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
                 bc += __shfl_xor_sync(FULL_MASK, bc, o);
                 cc += __shfl_xor_sync(FULL_MASK, cc, o);
             }
-            if (lane == 0) {
+            if (lane == 0 && !left) {
                 atomicAdd(&counters[C_PAIRS], 1ull);
                 atomicAdd(&counters[C_BYTES_CAND], (unsigned long long)bc);
                 atomicAdd(&counters[C_CAND], (unsigned long long)cc);
@@ -3987,21 +3990,58 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
 // instances (with FREE_CAP 192 26 + 18; without the queue, and with the
 // kinds of a list looked up 32 at a time instead of read as a mask, 44 + 22);
 // the search in order took 214 ms with 12.6 M lists put in leaf order.
-
-template <int CAP>
+//
+// Templates of 33 to 64 atoms have instances of their own (NL = 64 levels,
+// two a lane); larger ones go to k_search_large (24 structures x 24 such templates in 120: 12 ms in
+// order with every list of theirs ordered up front, 0.6 ms here).
+template <int CAP, int NL>
 struct FreeState {
     float4 xyz[CAP];            // frontier entries of every level: point and key,
     int32_t atom[CAP];          //   atom, parent entry
     uint16_t parent[CAP];
     uint16_t first[CAP];        // a child that leads to a row (0xFFFF: none)
-    float4 thr[32];             // annulus bounds of the new level to each earlier one
-    int4 rule[32];              // residue / chain rule to it: key bits that must be
+    float4 thr[NL];             // annulus bounds of the new level to each earlier one
+    int4 rule[NL];              // residue / chain rule to it: key bits that must be
                                 //   equal (x), that must differ somewhere (y; z = 1: no such bits)
-    int32_t order[32], tkey[32], sig[32];
+    int32_t order[NL], tkey[NL], sig[NL];
     uint32_t mask[FREE_MAX_KINDS / 32];  // local kinds of the new level's list
     int32_t cq[64];             // queued candidates: atoms
     uint16_t pq[64];            //   their parents
     uint16_t sq[32];
+};
+
+// a value a level, lane l holding levels l, l + 32, ...
+template <typename V, int W>
+struct PerLevel {
+    V v[W];
+    __device__ __forceinline__ void fill(V x) {
+        for (int w = 0; w < W; w++) v[w] = x;
+    }
+    __device__ __forceinline__ V get(int l) const {  // by every lane, l uniform
+        V x = __shfl_sync(FULL_MASK, v[0], l & 31);
+        for (int w = 1; w < W; w++) {
+            const V y = __shfl_sync(FULL_MASK, v[w], l & 31);
+            if (l >= 32 * w) x = y;
+        }
+        return x;
+    }
+    __device__ __forceinline__ void set(int l, V x) {
+        for (int w = 0; w < W; w++)
+            if (lane_id() + 32 * w == l) v[w] = x;
+    }
+    __device__ __forceinline__ void add(int l, V x) {
+        for (int w = 0; w < W; w++)
+            if (lane_id() + 32 * w == l) v[w] += x;
+    }
+};
+// a bit a level
+template <int W>
+struct LevelMask {
+    using T = unsigned;
+};
+template <>
+struct LevelMask<2> {
+    using T = unsigned long long;
 };
 
 // check_pair as two bit masks over the XOR of two structure keys
@@ -4017,7 +4057,7 @@ __device__ __forceinline__ int4 residue_rule(int32_t tj, int32_t tn, int ignore)
 // entry p: 0 outside an annulus, 1 inside every one, 2 inside, but outside an
 // annulus box (the kd-tree decides)
 __device__ __noinline__ int free_decide(const int32_t *eatom, const uint16_t *eparent, const int32_t *order,
-                                        unsigned exact, int lev, int p, int32_t an, const double *xyz,
+                                        unsigned long long exact, int lev, int p, int32_t an, const double *xyz,
                                         const AnnulusParam *prm, int n, int qn) {
     int verdict = 1;
     for (int j = lev; j >= 0; j--, p = eparent[p]) {
@@ -4151,26 +4191,73 @@ __device__ __forceinline__ void for_list(const ChunkView &cv, const uint32_t *ma
     }
 }
 
-// level order of a pair: this lane's place (stable by list length c)
-__device__ __forceinline__ int level_rank(int n, int c, int reorder) {
-    const int lane = lane_id();
-    if (!reorder) return lane;
-    int rank = 0;
-    for (int j = 0; j < n; j++) {
-        const int cj = __shfl_sync(FULL_MASK, c, j);
-        rank += (cj < c || (cj == c && j < lane)) ? 1 : 0;
+// template atoms a lane holds (lane, lane + 32, ..): their signatures and list
+// lengths; rank: the level of each (by length, ties by index)
+template <int W>
+struct PairLists {
+    int c[W], sg[W];
+    __device__ __forceinline__ PairLists(const TemplateView &tv, const CandView &cd, int ab, int n, int64_t wb) {
+        for (int w = 0; w < W; w++) {
+            const int k = lane_id() + 32 * w;
+            c[w] = INT_MAX;
+            sg[w] = 0;
+            if (k < n) {
+                sg[w] = tv.sig[ab + k];
+                c[w] = cd.count[wb + sg[w]];
+            }
+        }
     }
-    return rank;
+    __device__ __forceinline__ void levels(int n, int reorder, int (&rank)[W]) const {
+        for (int w = 0; w < W; w++) rank[w] = reorder ? 0 : lane_id() + 32 * w;
+        if (!reorder) return;
+        for (int v = 0; v < W; v++)
+            for (int j = 32 * v; j < min(n, 32 * v + 32); j++) {
+                const int cj = __shfl_sync(FULL_MASK, c[v], j & 31);
+                for (int w = 0; w < W; w++)
+                    rank[w] += (cj < c[w] || (cj == c[w] && j < lane_id() + 32 * w)) ? 1 : 0;
+            }
+    }
+    __device__ __forceinline__ int shortest() const {
+        int m = c[0];
+        for (int w = 1; w < W; w++) m = min(m, c[w]);
+        return __reduce_min_sync(FULL_MASK, m);
+    }
+};
+
+// levels of a pair of up to 64 atoms: the template atom of each, its signature
+__device__ __forceinline__ void level_order(const TemplateView &tv, const CandView &cd, int ab, int n, int64_t wb,
+                                            int reorder, int32_t *order, int32_t *sig) {
+    const int lane = lane_id();
+    if (n <= 32) {
+        const PairLists<1> pl(tv, cd, ab, n, wb);
+        int rank[1];
+        pl.levels(n, reorder, rank);
+        if (lane < n) {
+            order[rank[0]] = lane;
+            sig[rank[0]] = pl.sg[0];
+        }
+    } else {
+        const PairLists<2> pl(tv, cd, ab, n, wb);
+        int rank[2];
+        pl.levels(n, reorder, rank);
+        for (int w = 0; w < 2; w++) {
+            if (lane + 32 * w >= n) continue;
+            order[rank[w]] = lane + 32 * w;
+            sig[rank[w]] = pl.sg[w];
+        }
+    }
 }
 
-template <bool FP32, bool HEAVY>
-__global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
+template <bool FP32, bool HEAVY, int NL>
+__global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCKS : 2)
     k_search_free(ChunkView cv, TemplateView tv, CandView cd, FreeView fv, SearchArgs sa, int32_t *item_counter,
                   const int32_t *scanned, CompleteRows out, unsigned long long *counters, LeafDemand dm,
                   FreeWork fw) {
     extern __shared__ __align__(16) unsigned char free_smem[];
     constexpr int CAP = HEAVY ? HEAVY_CAP : FREE_CAP;
-    using State = FreeState<HEAVY ? 1 : FREE_CAP>;
+    using State = FreeState<HEAVY ? 1 : FREE_CAP, NL>;
+    constexpr int W = NL / 32;
+    using Mask = typename LevelMask<W>::T;
     const int lane = lane_id();
     const unsigned lt = (1u << lane) - 1u;
     State &st = reinterpret_cast<State *>(free_smem)[threadIdx.x >> 5];
@@ -4185,7 +4272,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
     uint64_t t_start = 0;
     if (lane == 0) t_start = global_ns();
     bool timed_out = false;
-    const int n_items = HEAVY ? fw.n_items : sa.n_pairs;
+    const int n_items = HEAVY ? fw.n_items : NL == 32 ? sa.n_pairs : cv.n_structures * fw.n_wide;
     int g_next = 0, g_end = 0;
     while (!timed_out) {
         if (g_next >= g_end) {
@@ -4212,10 +4299,12 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
             hp = fw.heavy[hidx];
             if (hp.failed) continue;
         }
-        const int pair = HEAVY ? hp.pair : item;
+        const int pair = HEAVY      ? hp.pair
+                         : NL == 32 ? item
+                                    : item / fw.n_wide * T + fw.wide[item % fw.n_wide];
         const int s = pair / T, t = pair % T;
         const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
-        if (n <= 0 || n > 32) continue;  // (over 32 atoms: k_search_large)
+        if (n <= (NL == 32 ? 0 : 32) || n > NL) continue;  // (another instance's)
         const int64_t abase = cv.atom_base[s];
         const int64_t wb = (int64_t)s * G;
 
@@ -4259,36 +4348,37 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
         }
 
         // ---- list lengths, empty lists, statistics
-        int c = INT_MAX, sg = 0;
-        if (lane < n) {
-            sg = tv.sig[ab + lane];
-            c = cd.count[wb + sg];
-        }
+        const PairLists<W> pl(tv, cd, ab, n, wb);
         if (!HEAVY) {
-            const unsigned zero = __ballot_sync(FULL_MASK, lane < n && c == 0);
+            int first_zero = n;
             if (lane == 0) a_pairs++;
-            if (lane < n && lane <= (zero ? __ffs(zero) - 1 : n - 1)) {
-                a_bcand += 8ull * scanned[wb + sg] + 16ull * c;
-                a_cand += c;
+            for (int w = 0; w < W && first_zero == n; w++) {
+                const int k = lane + 32 * w;
+                const unsigned zero = __ballot_sync(FULL_MASK, k < n && pl.c[w] == 0);
+                if (zero) first_zero = 32 * w + __ffs(zero) - 1;
+                if (k < n && k <= first_zero) {
+                    a_bcand += 8ull * scanned[wb + pl.sg[w]] + 16ull * pl.c[w];
+                    a_cand += pl.c[w];
+                }
             }
-            if (zero) continue;
+            if (first_zero < n) continue;
         }
-        const int rank = level_rank(n, c, sa.reorder);
+        int rank[W];
+        pl.levels(n, sa.reorder, rank);
         __syncwarp();
-        if (lane < n) {
-            st.order[rank] = lane;
-            st.sig[rank] = sg;
-            st.tkey[rank] = tv.key[ab + lane];
+        for (int w = 0; w < W; w++) {
+            const int k = lane + 32 * w;
+            if (k >= n) continue;
+            st.order[rank[w]] = k;
+            st.sig[rank[w]] = pl.sg[w];
+            st.tkey[rank[w]] = tv.key[ab + k];
         }
         __syncwarp();
-        // this lane's level: its list and length
-        const int64_t lw = lane < n ? wb + st.sig[lane] : 0;
-        const int llen = __shfl_sync(FULL_MASK, c, lane < n ? st.order[lane] : 0);
         const AnnulusParam *prm = tv.params + tv.param_begin[t];
         const double *xyz64 = cv.xyz64 + 3 * abase;
         const float4 *kx = fv.kxyz + abase;
         const int q0 = cv.nh_begin[cv.bucket_begin[s]];
-        const int m0 = __shfl_sync(FULL_MASK, llen, 0);
+        const int m0 = sa.reorder ? pl.shortest() : __shfl_sync(FULL_MASK, pl.c[0], 0);
 
         const int mw = fv.mask_words;
         const uint32_t *masks = fv.kind_masks + wb * mw;
@@ -4299,23 +4389,30 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
         // rows written: last segment, its levels at which rows part, segments
         int seg = -1, seg0 = -1, n_seg = 0;
         bool spilled = false;
-        unsigned branch = 0;
-        long long F = 0;  // lane l: partial assignments of level l
+        Mask branch = 0;
+        PerLevel<long long, W> F;  // partial assignments
+        F.fill(0);
         unsigned long long rech = 0;
-        // lane l: entries of level l, the next one to expand, most to expand at once
-        int lbeg = 0, lend = 0, lcur = 0, lmax = CAP;
+        // entries of each level, the next one to expand, most to expand at once
+        PerLevel<int, W> lbeg, lend, lcur, lmax;
+        lbeg.fill(0);
+        lend.fill(0);
+        lcur.fill(0);
+        lmax.fill(CAP);
         int top = 0, lev = -1;
         if (HEAVY && sub) {
             // the entry's chain, one entry a level, all but the last expanded
             lev = sub->level;
-            if (lane <= lev) {
-                const int32_t a = sub->atom[lane];
-                exyz[lane] = cv.xyz32[abase + a];
-                eatom[lane] = a;
-                eparent[lane] = (uint16_t)(lane > 0 ? lane - 1 : 0);
-                lbeg = lane;
-                lend = lane + 1;
-                lcur = lane < lev ? lane + 1 : lane;
+            for (int w = 0; w < W; w++) {
+                const int j = lane + 32 * w;
+                if (j > lev) continue;
+                const int32_t a = sub->atom[j];
+                exyz[j] = cv.xyz32[abase + a];
+                eatom[j] = a;
+                eparent[j] = (uint16_t)(j > 0 ? j - 1 : 0);
+                lbeg.v[w] = j;
+                lend.v[w] = j + 1;
+                lcur.v[w] = j < lev ? j + 1 : j;
             }
             top = lev + 1;
             __syncwarp();
@@ -4324,7 +4421,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
             const int s0 = HEAVY ? blk * fw.item_seeds : 0;
             const int k0 = HEAVY ? min(fw.item_seeds, m0 - s0) : m0;
             if (HEAVY) {
-                const int32_t *ca = cd.cand_atom + cd.offset[__shfl_sync(FULL_MASK, lw, 0)] + s0;
+                const int32_t *ca = cd.cand_atom + cd.offset[wb + st.sig[0]] + s0;
                 for (int e = lane; e < k0; e += 32) {
                     const int32_t a = ca[e];
                     exyz[e] = cv.xyz32[abase + a];
@@ -4344,19 +4441,17 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                 });
             }
             __syncwarp();
-            if (lane == 0) {
-                lend = k0;
-                F = k0;
-            }
+            lend.set(0, k0);
+            F.set(0, k0);
             top = k0;
             lev = 0;
         }
         while (lev >= 0 && !kd_needed && !outgrown) {
-            const int beg = __shfl_sync(FULL_MASK, lcur, lev), lev_end = __shfl_sync(FULL_MASK, lend, lev);
+            const int beg = lcur.get(lev), lev_end = lend.get(lev);
             if (beg >= lev_end) {
                 // level done: its entries are no longer needed
                 if (!HEAVY) break;  // (the only path down has reached its rows)
-                top = __shfl_sync(FULL_MASK, lbeg, lev);
+                top = lbeg.get(lev);
                 lev--;
                 continue;
             }
@@ -4365,41 +4460,42 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                 if (lane == 0) over = (global_ns() - t_start) > sa.budget_ns;
                 if (__shfl_sync(FULL_MASK, over, 0)) break;
             }
-            const int end = min(lev_end, beg + __shfl_sync(FULL_MASK, lmax, lev));
+            const int end = min(lev_end, beg + lmax.get(lev));
             bool full = false;
-            long long Fc = 0;
-            unsigned long long crech = 0;
+            int Fc = 0;
+            unsigned crech = 0;
             int nend = top;  // children are appended at the top
             {
                 const int child = lev + 1;
                 const int qn = st.order[child], g = st.sig[child];
-                int4 myrule = make_int4(0, 0, 1, 0);
+                // the deepest level whose atom shares the new atom's residue (-1: none)
+                int anchor = -1;
                 __syncwarp();
-                if (lane <= lev) {
-                    st.thr[lane] = prm[st.order[lane] * n + qn].thr;
-                    myrule = residue_rule(st.tkey[lane], st.tkey[child], sa.ignore_chain);
-                    st.rule[lane] = myrule;
+                for (int j = lane; j <= lev; j += 32) {
+                    st.thr[j] = prm[st.order[j] * n + qn].thr;
+                    const int4 rule = residue_rule(st.tkey[j], st.tkey[child], sa.ignore_chain);
+                    st.rule[j] = rule;
+                    if ((rule.x & ~0xFF) != 0) anchor = j;
                 }
-                // the deepest level whose atom shares the new atom's residue
-                const unsigned same = __ballot_sync(FULL_MASK, lane <= lev && (myrule.x & ~0xFF) != 0);
+                anchor = __reduce_max_sync(FULL_MASK, anchor);
                 __syncwarp();
                 // the lanes' tests at one chain entry
                 auto test = [&](const float4 &e, const float4 &x, const int4 &r, const float4 &th, int j,
-                                unsigned &exact) -> bool {
+                                Mask &exact) -> bool {
                     const int32_t d = __float_as_int(e.w) ^ __float_as_int(x.w);
                     const float dx = e.x - x.x, dy = e.y - x.y, dz = e.z - x.z;
                     const float d2 = dx * dx + dy * dy + dz * dz;
                     const bool ok = (d & r.x) == 0 && ((d & r.y) | r.z) != 0 && !(d2 < th.x || d2 > th.w);
-                    if (!FP32 || !(d2 >= th.y && d2 <= th.z)) exact |= 1u << j;
+                    if (!FP32 || !(d2 >= th.y && d2 <= th.z)) exact |= Mask(1) << j;
                     return ok;
                 };
                 // candidates that passed: inconclusive ones decided in FP64,
                 // the others appended as children
-                auto accept = [&](bool pass, unsigned exact, int p, int32_t an, const float4 &x) {
+                auto accept = [&](bool pass, Mask exact, int p, int32_t an, const float4 &x) {
                     if (__any_sync(FULL_MASK, pass && exact)) {
                         int v = 1;
                         if (pass && exact) {
-                            if (FP32) crech += __popc(exact);
+                            if (FP32) crech += __popcll((unsigned long long)exact);
                             v = free_decide(eatom, eparent, st.order, exact, lev, p, an, xyz64, prm, n, qn);
                             pass = v != 0;
                         }
@@ -4407,7 +4503,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                     }
                     const unsigned m = __ballot_sync(FULL_MASK, pass);
                     const int np = __popc(m);
-                    if (lane == child) Fc += np;
+                    Fc += np;
                     if (nend + np > CAP) {
                         full = true;
                     } else {
@@ -4427,7 +4523,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                 auto run_batch = [&](int k) {
                     queued -= k;
                     bool pass = lane < k;
-                    unsigned exact = 0;
+                    Mask exact = 0;
                     const int p = pass ? st.pq[queued + lane] : 0;
                     const int32_t an = pass ? st.cq[queued + lane] : 0;
                     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -4442,9 +4538,8 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                     accept(pass, exact, p, an, x);
                     __syncwarp();
                 };
-                if (same) {
+                if (anchor >= 0) {
                     // ---- the atoms of the placed residue
-                    const int anchor = 31 - __clz(same);
                     const bool by_number = sa.ignore_chain == 2;
                     if (lane < mw) st.mask[lane] = masks[(int64_t)g * mw + lane];
                     __syncwarp();
@@ -4493,7 +4588,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                         const float4 x = valid ? kx[pos] : make_float4(0.f, 0.f, 0.f, 0.f);
                         const int32_t an = valid ? cv.nh_pos[abase + pos] : 0;
                         for (int p = beg; p < end; p++) {
-                            unsigned exact = 0;
+                            Mask exact = 0;
                             const bool near = valid && test(exyz[p], x, rule_p, thr_p, lev, exact);
                             const unsigned m = __ballot_sync(FULL_MASK, near);
                             if (!m) continue;
@@ -4547,23 +4642,22 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                         for (int j = lev, e = beg + i; j >= 0; j--, e = eparent[e]) r.atom[j] = eatom[e];
                     }
                     __syncwarp();
-                    if (lane == lev) lcur = lend;
+                    lcur.set(lev, lev_end);
                     spilled = true;
-                } else if (lane == lev) {
-                    lmax = (end - beg) / 2;
+                } else {
+                    lmax.set(lev, (end - beg) / 2);
                 }
                 continue;
             }
-            F += Fc;
+            F.add(lev + 1, Fc);
             rech += crech;
-            if (lane == lev) lcur = end;
+            lcur.set(lev, end);
             if (lev + 1 < n - 1) {
                 if (nend > top) {
                     lev++;
-                    if (lane == lev) {
-                        lbeg = lcur = top;
-                        lend = nend;
-                    }
+                    lbeg.set(lev, top);
+                    lcur.set(lev, top);
+                    lend.set(lev, nend);
                     top = nend;
                 }
                 continue;
@@ -4576,20 +4670,19 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                 for (int e = lane; e < top; e += 32) efirst[e] = 0xFFFF;
                 __syncwarp();
                 for (int l = n - 1; l >= 1; l--) {
-                    const int e0 = l == n - 1 ? top : __shfl_sync(FULL_MASK, lbeg, l);
-                    const int e1 = l == n - 1 ? nend : __shfl_sync(FULL_MASK, lend, l);
+                    const int e0 = l == n - 1 ? top : lbeg.get(l), e1 = l == n - 1 ? nend : lend.get(l);
                     for (int e = e0 + lane; e < e1; e += 32)
                         if (l == n - 1 || efirst[e] != 0xFFFF) efirst[eparent[e]] = (uint16_t)e;
                     __syncwarp();
                     bool other = false;
                     for (int e = e0 + lane; e < e1; e += 32)
                         if (l == n - 1 || efirst[e] != 0xFFFF) other |= efirst[eparent[e]] != (uint16_t)e;
-                    if (__any_sync(FULL_MASK, other)) branch |= 1u << l;
+                    if (__any_sync(FULL_MASK, other)) branch |= Mask(1) << l;
                 }
                 int live = 0;
-                const int seeds = __shfl_sync(FULL_MASK, lend, 0);
+                const int seeds = lend.get(0);
                 for (int e = lane; e < seeds; e += 32) live += efirst[e] != 0xFFFF ? 1 : 0;
-                if (__reduce_add_sync(FULL_MASK, live) > 1) branch |= 1u;
+                if (__reduce_add_sync(FULL_MASK, live) > 1) branch |= Mask(1);
             }
             int64_t rb = 0;
             int ui = -1;
@@ -4638,7 +4731,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
         }
         if (!kd_needed && !outgrown && rows > 0) {
             // rows in several segments part anywhere
-            if (n_seg > 1 || spilled || sub) branch = n == 32 ? ~0u : (1u << n) - 1u;
+            if (n_seg > 1 || spilled || sub) branch = n == NL ? ~Mask(0) : (Mask(1) << n) - 1;
         }
         if (!HEAVY) {
             if (lane == 0 && seg >= 0 && seg < out.capacity) fw.units[seg].branch = branch;
@@ -4647,7 +4740,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
             const int it = hp.first + blk;
             const int before = atomicExch(&fw.item_head[it], seg);
             if (seg0 < out.capacity) fw.units[seg0].next = before;
-            atomicOr(&fw.item_branch[it], branch);
+            atomicOr(&fw.item_branch[it], (unsigned long long)branch);
         }
         // rows without a hit among them that end the stream by themselves
         const bool ended = HEAVY && !sub && !spilled && sa.max_candidates >= 0 && rows >= sa.max_candidates + 2ll &&
@@ -4682,17 +4775,26 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                 }
             }
             if (!kd_needed || HEAVY) {
-                const long long Fp = __shfl_up_sync(FULL_MASK, F, 1);
-                const unsigned long long bexp =
-                    lane >= 1 && lane < n ? (unsigned long long)(4LL * lane * Fp + (4LL * (lane + 1) + 16) * F) : 0ull;
+                unsigned long long part = 0, comp = 0, bexp = 0;
+                for (int w = 0; w < W; w++) {
+                    const int l = lane + 32 * w;
+                    long long before = __shfl_up_sync(FULL_MASK, F.v[w], 1);
+                    if (w > 0) {
+                        const long long y = __shfl_sync(FULL_MASK, F.v[w - 1], 31);
+                        if (lane == 0) before = y;
+                    }
+                    part += (unsigned long long)F.v[w];
+                    if (l == n - 1) comp = (unsigned long long)F.v[w];
+                    if (l >= 1 && l < n) bexp += (unsigned long long)(4LL * l * before + (4LL * (l + 1) + 16) * F.v[w]);
+                }
                 if (HEAVY) {
                     // per pair: counted unless another item hands the pair to k_search
                     auto add = [&](int k, unsigned long long v) {
                         for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
                         if (lane == 0 && v) atomicAdd(&fw.heavy_stats[4 * (int64_t)hidx + k], v);
                     };
-                    add(0, (unsigned long long)F);
-                    add(1, lane == n - 1 ? (unsigned long long)F : 0ull);
+                    add(0, part);
+                    add(1, comp);
                     add(2, bexp);
                     add(3, rech);
                     if (lane == 0 && sub) atomicAdd(&fw.results[hp.first + blk].x, rows);
@@ -4700,8 +4802,8 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, PJG_FREE_MIN_BLOCKS)
                         fw.results[hp.first + blk] = make_int2(rows, (any_hit || spilled ? 1 : 0) | (ended ? 2 : 0));
                 } else {
                     if (lane == 0 && rows > 0) out.pair_rows[pair] = rows;
-                    a_part += (unsigned long long)F;
-                    if (lane == n - 1) a_comp += (unsigned long long)F;
+                    a_part += part;
+                    a_comp += comp;
                     a_bexp += bexp;
                     a_rech += rech;
                 }
@@ -4761,23 +4863,26 @@ __global__ void k_free_requests(TemplateView tv, CandView cd, int32_t reorder, L
 // Lists of the levels at which the rows of a pending unit part, warp per unit.
 __global__ void k_pending_requests(int64_t n_pending, TemplateView tv, CandView cd, int32_t reorder, LeafDemand dm,
                                    FreeWork fw) {
+    __shared__ int32_t order[8][64], sig[8][64];
     const int lane = lane_id();
     const int T = tv.n_templates, G = cd.n_sigs;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t x = warp; x < n_pending; x += nwarps) {
         const RowUnit u = fw.units[fw.pending[x]];
-        const uint32_t branch = u.item >= 0 ? fw.item_branch[u.item] : u.branch;
+        const unsigned long long branch = u.item >= 0 ? fw.item_branch[u.item] : u.branch;
         const int s = u.pair / T, t = u.pair % T;
         const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
-        int c = INT_MAX;
-        int64_t w = 0;
-        if (lane < n) {
-            w = (int64_t)s * G + tv.sig[ab + lane];
-            c = cd.count[w];
+        const int64_t wb = (int64_t)s * G;
+        __syncwarp();
+        level_order(tv, cd, ab, n, wb, reorder, order[threadIdx.x >> 5], sig[threadIdx.x >> 5]);
+        __syncwarp();
+        for (int l0 = 0; l0 < n; l0 += 32) {
+            const int l = l0 + lane;
+            const bool want = l > 0 && l < n && ((branch >> l) & 1ull);
+            const int64_t w = want ? wb + sig[threadIdx.x >> 5][l] : wb;
+            request_list_warp(dm, want, w, want ? cd.count[w] : 0);
         }
-        const int rank = level_rank(n, c, reorder);
-        request_list_warp(dm, lane < n && rank > 0 && ((branch >> rank) & 1u), w, c);
     }
 }
 
@@ -4845,7 +4950,7 @@ struct UnitWarp {
     unsigned long long key[UNIT_ROWS];
     int32_t cur[UNIT_ROWS], atom[UNIT_ROWS], row[UNIT_ROWS];
     int32_t slot_atom[UNIT_SLOTS], slot_rank[UNIT_SLOTS];
-    int32_t order[32], sig[32];
+    int32_t order[64], sig[64];
 };
 
 // place of atom a in the candidate list of signature g: residue names in the
@@ -4883,17 +4988,8 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
         const int s = u.pair / T, t = u.pair % T;
         const int ab = tv.atom_begin[t], n = tv.atom_begin[t + 1] - ab;
         const int64_t abase = cv.atom_base[s], wb = (int64_t)s * G;
-        int c = INT_MAX, sg = 0;
-        if (lane < n) {
-            sg = tv.sig[ab + lane];
-            c = cd.count[wb + sg];
-        }
-        const int rank = level_rank(n, c, reorder);
         __syncwarp();
-        if (lane < n) {
-            U.order[rank] = lane;
-            U.sig[rank] = sg;
-        }
+        level_order(tv, cd, ab, n, wb, reorder, U.order, U.sig);
         int at = 0;
         for (int q = w; q >= 0;) {
             const RowUnit v = fw.units[q];
@@ -4903,8 +4999,8 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
         }
         for (int i = lane; i < R; i += 32) U.cur[i] = 0;
         __syncwarp();
-        for (unsigned left = u.item >= 0 ? fw.item_branch[u.item] : u.branch; left; left &= left - 1) {
-            const int l = __ffs(left) - 1;
+        for (unsigned long long left = u.item >= 0 ? fw.item_branch[u.item] : u.branch; left; left &= left - 1) {
+            const int l = __ffsll((long long)left) - 1;
             const int k = U.order[l], g = U.sig[l];
             if (l == 0) {
                 for (int i = lane; i < R; i += 32)
@@ -5002,7 +5098,7 @@ struct DirectWarp {
     int32_t mem[2][MAXM];      // the nodes' atoms, children in the other buffer
     uint32_t rk[MAXM];         // ranks of the node being split
     alignas(16) int32_t bins[128];
-    int32_t order[32], sig[32];
+    int32_t order[64], sig[64];
     int4 stack[32];            // nodes to split: first entry, entries, depth | buffer << 8, number
 };
 
@@ -5041,26 +5137,22 @@ __global__ void __launch_bounds__(WARPS * 32)
         const int64_t abase = cv.atom_base[s], wb = (int64_t)s * G;
         // ranks are below the structure's atoms: the shift to 128 bins of them
         const int shift = max(0, 32 - __clz(cv.atom_count[s]) - 7);
-        const uint32_t branch = u.item >= 0 ? fw.item_branch[u.item] : u.branch;
-        int c = INT_MAX, sg = 0;
-        if (lane < n) {
-            sg = tv.sig[ab + lane];
-            c = cd.count[wb + sg];
-        }
-        const int rank = level_rank(n, c, reorder);
-        const bool parts = lane < n && rank > 0 && ((branch >> rank) & 1u);  // this atom's level parts rows
+        const unsigned long long branch = u.item >= 0 ? fw.item_branch[u.item] : u.branch;
+        __syncwarp();
+        level_order(tv, cd, ab, n, wb, reorder, U.order, U.sig);
+        __syncwarp();
+        // the longest list whose level parts rows
+        int most = 0;
+        for (int l = lane; l < n; l += 32)
+            if (l > 0 && ((branch >> l) & 1ull)) most = max(most, cd.count[wb + U.sig[l]]);
+        most = __reduce_max_sync(FULL_MASK, most);
         bool pending = R > UNIT_ROWS;
-        if (!LONG && !pending && __any_sync(FULL_MASK, parts && c > DIRECT_MAX)) {
-            if (R <= DIRECT_LONG_ROWS && !__any_sync(FULL_MASK, parts && c > DIRECT_LONG)) {
+        if (!LONG && !pending && most > DIRECT_MAX) {
+            if (R <= DIRECT_LONG_ROWS && most <= DIRECT_LONG) {
                 if (lane == 0) fw.long_units[atomicAdd(fw.n_long_units, 1ull)] = w;
                 continue;
             }
             pending = true;
-        }
-        __syncwarp();
-        if (lane < n) {
-            U.order[rank] = lane;
-            U.sig[rank] = sg;
         }
         if (!pending) {
             int at = 0;
@@ -5074,8 +5166,8 @@ __global__ void __launch_bounds__(WARPS * 32)
         }
         __syncwarp();
         const int q0 = cv.nh_begin[cv.bucket_begin[s]];
-        for (unsigned left = pending ? 0u : branch; left && !pending; left &= left - 1) {
-            const int l = __ffs(left) - 1;
+        for (unsigned long long left = pending ? 0ull : branch; left && !pending; left &= left - 1) {
+            const int l = __ffsll((long long)left) - 1;
             const int k = U.order[l], g = U.sig[l];
             if (l == 0) {
                 for (int i = lane; i < R; i += 32)
@@ -5304,7 +5396,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
     k_unit_order_large(ChunkView cv, TemplateView tv, CandView cd, SigView sv, const int32_t *res_place,
                        int32_t reorder, FreeWork fw, CompleteRows out) {
-    __shared__ int32_t order[32], sig[32], leaf[UNIT_LARGE_THREADS];
+    __shared__ int32_t order[64], sig[64], leaf[UNIT_LARGE_THREADS];
     __shared__ long long region;
     const int T = tv.n_templates, G = cd.n_sigs, tid = threadIdx.x;
     const int64_t total = (int64_t)*fw.n_large_units;
@@ -5318,16 +5410,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
         const int64_t abase = cv.atom_base[s], wb = (int64_t)s * G;
         __syncthreads();
         if (tid < 32) {
-            int c = INT_MAX, sg = 0;
-            if (tid < n) {
-                sg = tv.sig[ab + tid];
-                c = cd.count[wb + sg];
-            }
-            const int rank = level_rank(n, c, reorder);
-            if (tid < n) {
-                order[rank] = tid;
-                sig[rank] = sg;
-            }
+            level_order(tv, cd, ab, n, wb, reorder, order, sig);
             if (tid == 0) region = (long long)atomicAdd(fw.scratch_used, (unsigned long long)R);
         }
         __syncthreads();
@@ -5345,8 +5428,8 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
             q = u.item >= 0 ? v.next : -1;
         }
         __syncthreads();
-        for (unsigned left = u.item >= 0 ? fw.item_branch[u.item] : u.branch; left; left &= left - 1) {
-            const int l = __ffs(left) - 1;
+        for (unsigned long long left = u.item >= 0 ? fw.item_branch[u.item] : u.branch; left; left &= left - 1) {
+            const int l = __ffsll((long long)left) - 1;
             const int k = order[l], g = sig[l];
             const int m = cd.count[wb + g];
             const int32_t *la = l == 0 ? nullptr : cd.leaf_atom + cd.leaf_offset[wb + g];
@@ -5900,7 +5983,7 @@ void launch_axis_ranks(cudaStream_t st, int32_t n_structures, int32_t max_atoms,
 }
 
 void launch_demand_levels(cudaStream_t st, int blocks, const TemplateView &tv, const CandView &cd, int32_t n_pairs,
-                          int32_t max_level, int32_t reorder, const LeafDemand &dm) {
+                          int32_t max_level, int32_t reorder, int32_t whole_over, const LeafDemand &dm) {
     // (also with max_level 0: the pairs of templates over 32 atoms request
     // every list here)
     // thread per pair
@@ -5909,7 +5992,7 @@ void launch_demand_levels(cudaStream_t st, int blocks, const TemplateView &tv, c
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n_pairs + 255) / 256, (int64_t)sms * 8));
-    if (n_pairs > 0) k_demand_levels<<<g, 256, 0, st>>>(tv, cd, n_pairs, max_level, reorder, dm);
+    if (n_pairs > 0) k_demand_levels<<<g, 256, 0, st>>>(tv, cd, n_pairs, max_level, reorder, whole_over, dm);
 }
 
 void launch_list_keys(cudaStream_t st, int blocks, int32_t n_sigs, const int32_t *count, const int64_t *offset,
@@ -6036,23 +6119,27 @@ cudaError_t launch_search_free(cudaStream_t st, bool fp32, const ChunkView &cv, 
                                const CandView &cd, const FreeView &fv, const SearchArgs &sa, int32_t *item_counter,
                                const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
                                const LeafDemand &dm, const FreeWork &fw) {
-    auto kern = fp32 ? k_search_free<true, false> : k_search_free<false, false>;
-    const int smem = (int)sizeof(FreeState<FREE_CAP>) * FREE_WARPS;
+    const bool wide = fw.n_wide > 0;  // this launch: the templates of 33 to 64 atoms
+    auto kern = wide ? (fp32 ? k_search_free<true, false, 64> : k_search_free<false, false, 64>)
+                     : (fp32 ? k_search_free<true, false, 32> : k_search_free<false, false, 32>);
+    const int smem = (int)(wide ? sizeof(FreeState<FREE_CAP, 64>) : sizeof(FreeState<FREE_CAP, 32>)) * FREE_WARPS;
+    const int64_t items = wide ? (int64_t)cv.n_structures * fw.n_wide : sa.n_pairs;
     int64_t grid = 0, resident = 0;
-    cudaError_t e = free_grid((const void *)kern, smem, sa.n_pairs, &grid, &resident);
+    cudaError_t e = free_grid((const void *)kern, smem, items, &grid, &resident);
     if (e != cudaSuccess) return e;
     SearchArgs fa = sa;
     // a pair takes microseconds: several a queue step once every resident
     // warp has tens of them
-    fa.pair_grain = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, sa.n_pairs / (resident * FREE_WARPS * 16)));
+    fa.pair_grain = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, items / (resident * FREE_WARPS * 16)));
     kern<<<(int)grid, FREE_WARPS * 32, smem, st>>>(cv, tv, cd, fv, fa, item_counter, scanned, out, counters, dm, fw);
     return cudaGetLastError();
 }
 
 cudaError_t heavy_warps(bool fp32, int64_t n_items, int64_t *warps) {
-    auto kern = fp32 ? k_search_free<true, true> : k_search_free<false, true>;
+    auto kern = fp32 ? k_search_free<true, true, 32> : k_search_free<false, true, 32>;
     int64_t grid = 0, resident = 0;
-    cudaError_t e = free_grid((const void *)kern, (int)sizeof(FreeState<1>) * FREE_WARPS, n_items, &grid, &resident);
+    cudaError_t e =
+        free_grid((const void *)kern, (int)sizeof(FreeState<1, 32>) * FREE_WARPS, n_items, &grid, &resident);
     *warps = grid * FREE_WARPS;
     return e;
 }
@@ -6061,11 +6148,16 @@ cudaError_t launch_search_heavy(cudaStream_t st, bool fp32, int64_t warps, const
                                 const TemplateView &tv, const CandView &cd, const FreeView &fv, const SearchArgs &sa,
                                 int32_t *item_counter, const CompleteRows &out, unsigned long long *counters,
                                 const LeafDemand &dm, const FreeWork &fw) {
-    auto kern = fp32 ? k_search_free<true, true> : k_search_free<false, true>;
+    const bool wide = fw.n_wide > 0;
+    auto kern = wide ? (fp32 ? k_search_free<true, true, 64> : k_search_free<false, true, 64>)
+                     : (fp32 ? k_search_free<true, true, 32> : k_search_free<false, true, 32>);
+    const int smem = (int)(wide ? sizeof(FreeState<1, 64>) : sizeof(FreeState<1, 32>)) * FREE_WARPS;
+    cudaError_t e = cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
     SearchArgs fa = sa;
     fa.pair_grain = 1;
-    kern<<<(int)(warps / FREE_WARPS), FREE_WARPS * 32, (int)sizeof(FreeState<1>) * FREE_WARPS, st>>>(
-        cv, tv, cd, fv, fa, item_counter, nullptr, out, counters, dm, fw);
+    kern<<<(int)(warps / FREE_WARPS), FREE_WARPS * 32, smem, st>>>(cv, tv, cd, fv, fa, item_counter, nullptr, out,
+                                                                   counters, dm, fw);
     return cudaGetLastError();
 }
 
@@ -6135,19 +6227,19 @@ void launch_unit_order(cudaStream_t st, int64_t n_pending, const ChunkView &cv, 
 cudaError_t launch_search_large(cudaStream_t st, const ChunkView &cv, const TemplateView &tv, const CandView &cd,
                                 const SearchArgs &sa, const int32_t *large, int32_t n_large, int32_t *item_counter,
                                 const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
-                                const int32_t *lstate) {
-    if (n_large <= 0 || cv.n_structures <= 0) return cudaSuccess;
+                                const int32_t *lstate, const Suspended *left, int32_t n_left) {
+    if (n_large <= 0 || cv.n_structures <= 0 || (left && n_left <= 0)) return cudaSuccess;
     const size_t smem = (size_t)large_warp_bytes(tv.max_atoms) * LARGE_WARPS;
     cudaError_t e = cudaFuncSetAttribute(k_search_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t items = (int64_t)cv.n_structures * n_large;
+    const int64_t items = left ? n_left : (int64_t)cv.n_structures * n_large;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((items + LARGE_WARPS - 1) / LARGE_WARPS,
                                                                  (int64_t)std::max(sms, 1) * 4));
     k_search_large<<<grid, LARGE_WARPS * 32, smem, st>>>(cv, tv, cd, sa, large, n_large, item_counter, scanned, out,
-                                                         counters, lstate);
+                                                         counters, lstate, left, n_left);
     return cudaGetLastError();
 }
 

@@ -291,7 +291,7 @@ struct RowUnit {
     int32_t heavy;                     // index of its HeavyPair (-1: none)
     int32_t item;                      // its item in `results` (-1: none)
     int32_t next;                      // the item's next segment (-1: none)
-    uint32_t branch;                   // levels at which the pair's rows part
+    unsigned long long branch;         // levels at which the pair's rows part
 };
 
 // An entry of an item whose children outgrew the frontier: searched as an
@@ -299,7 +299,7 @@ struct RowUnit {
 struct SpilledEntry {
     int32_t heavy, block;              // heavy pair and item it belongs to
     int32_t level;                     // its level; atoms of levels 0 .. level
-    int32_t atom[32];
+    int32_t atom[64];
 };
 
 // Worklists of the order-free search.
@@ -311,11 +311,13 @@ struct FreeWork {
     const int2 *items;                 // (heavy pair, block), block by block
     int32_t n_items;
     int32_t item_seeds;
+    const int32_t *wide;               // templates of 33 to 64 atoms (n_wide > 0:
+    int32_t n_wide;                    //   the launch takes their pairs alone)
     int2 *results;                     // per item: rows (-1: not finished), flags
                                        //   (1: a hit among them, 2: the stream ends)
     unsigned long long *heavy_stats;   // [4 * heavy pairs] partials, complete, bytes, rechecks
     int32_t *item_head;                // per item: its list of segments (-1: no rows)
-    uint32_t *item_branch;             //   levels at which its rows part
+    unsigned long long *item_branch;   //   levels at which its rows part
     const int64_t *item_base;          //   rows of the pair before it
     float4 *arena_xyz;                 // frontiers of the items being searched,
     int32_t *arena_atom;               //   HEAVY_CAP entries a warp
@@ -435,9 +437,10 @@ void launch_list_share(cudaStream_t st, int blocks, const ChunkView &cv, int32_t
                        const ListShare &ls, unsigned long long *counters);
 
 // requests (LeafDemand) the lists of levels 1 .. max_level of every pair
-// of the chunk that has no empty candidate list
+// of the chunk that has no empty candidate list, and every list of the
+// templates of more than whole_over (>= 32) atoms
 void launch_demand_levels(cudaStream_t st, int blocks, const TemplateView &tv, const CandView &cd, int32_t n_pairs,
-                          int32_t max_level, int32_t reorder, const LeafDemand &dm);
+                          int32_t max_level, int32_t reorder, int32_t whole_over, const LeafDemand &dm);
 // the pairs whose cost bucket is above the level that leaves at most
 // `target` pairs above it: flags and list (n_heavy), from the buckets the
 // level demand wrote (bins: 66 counters, zeroed by the caller)
@@ -520,12 +523,13 @@ cudaError_t launch_search(cudaStream_t st, int grid, bool wide, bool fp32, const
                           const LeafDemand &dm);
 
 // k_search_large over the pairs (chunk structure x templates `large`) of
-// the templates with more than 32 atoms; item_counter zeroed by the caller;
+// the templates with more than 32 atoms, or over the pairs of such templates
+// among `left`; item_counter zeroed by the caller;
 // lstate: per-list leaf-order state (nullptr: every list ordered)
 cudaError_t launch_search_large(cudaStream_t st, const ChunkView &cv, const TemplateView &tv, const CandView &cd,
                                 const SearchArgs &sa, const int32_t *large, int32_t n_large, int32_t *item_counter,
                                 const int32_t *scanned, const CompleteRows &out, unsigned long long *counters,
-                                const int32_t *lstate);
+                                const int32_t *lstate, const Suspended *left = nullptr, int32_t n_left = 0);
 
 // every hit atom in its template's frame (out[3 * k + d] for hit atom k)
 void launch_superposed_atoms(cudaStream_t st, int64_t n_hits, int64_t n_atoms, const int32_t *structure,

@@ -233,3 +233,59 @@ def test_long_lists_replayed():
     res, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=2.0, distance_cutoff=1.0,
                        max_dynamic_distance=1.0)
     assert ref["hits"]["count"] > 0 and res.stats()["leaf_exact"] > 0
+
+
+def _cut(spec, atoms):
+    for k in ("xyz", "res_seq", "chain", "weight", "code", "resnames", "names"):
+        setattr(spec, k, getattr(spec, k)[:atoms])
+    return spec
+
+
+@pytest.mark.parametrize("atoms", [32, 33, 63, 64, 65])
+@pytest.mark.parametrize("kw", [dict(), dict(mode="fp64"), dict(ignore_chain=2), dict(max_candidates=1),
+                                dict(best_match=True, max_candidates=4), dict(reorder=False)])
+def test_levels_of_two_lanes(atoms, kw):
+    """Templates around 32 and 64 atoms (one level a lane, two, more than
+    that), with lists on both sides of the first frontier's room, beside
+    ordinary ones."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(38, [150, 300])
+    specs = [_cut(s, atoms) for s in _templates(38, structs, 4, lo=22, hi=23, radius=16.0)]
+    specs += [_cut(s, atoms) for s in _templates(38, structs, 2, lo=17, hi=18, radius=16.0, permissive=True,
+                                                 atoms_per_res=4)]
+    specs += _templates(40, structs, 6)
+    pt = W.pack_templates(specs)
+    assert (np.diff(pt.atom_offset) == atoms).sum() >= 2
+    _, ref = compare(pt, W.pack(structs), rmsd_threshold=2.0, distance_cutoff=1.6, max_dynamic_distance=1.6, **kw)
+    assert (np.diff(ref["hits"]["atom_offset"]) > 32).any() or atoms == 32
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(max_candidates=20), dict(best_match=True, max_candidates=1000)])
+def test_spilled_entries_of_two_lane_levels(kw):
+    """As test_spilled_entries with templates of 36 atoms."""
+    from pyjess_gb300 import workloads as W
+
+    rng = np.random.default_rng(7)
+    structs = W.make_structures([rng], [60], [1])
+    specs = [W.make_template(rng, structs[0], 9, modes=(3,), mode_p=(1.0,), radius=14.0, atoms_per_res=4)
+             for _ in range(2)]
+    compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=2.0, distance_cutoff=2.0,
+            max_dynamic_distance=2.0, **kw)
+
+
+@pytest.mark.parametrize("atoms", [5, 33])
+@pytest.mark.parametrize("max_candidates", [0, 3])
+def test_entry_that_cannot_be_split(atoms, max_candidates):
+    """Any atom of any residue at any distance: one seed has more children
+    than a frontier holds, so the pair goes to the searches in order."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(39, [1250])
+    names = sorted({bytes(x) for x in structs[0]["name"]})
+    spec = _templates(39, structs, 1, lo=atoms, hi=atoms + 1, radius=40.0, permissive=True, atoms_per_res=1)[0]
+    spec.names = [list(names) for _ in spec.names]
+    assert len(spec.code) == atoms
+    _, ref = compare(W.pack_templates([spec]), W.pack(structs), rmsd_threshold=1e3, distance_cutoff=200.0,
+                     max_dynamic_distance=200.0, max_candidates=max_candidates, best_match=True)
+    assert ref["hits"]["count"] == 1
