@@ -5531,9 +5531,9 @@ __global__ void k_order_counts(int64_t n_pairs, int32_t T, const int32_t *pair_r
 //    warning), but the template's stream ends at the first row whose
 //    ordinal is M+1 past the previous hit (or the template start).
 // A pair of at most AUTOMATON_LANE_ROWS rows by one thread; longer ones are
-// listed for k_automaton_long, a warp each, 32 rows a step (dense pairs have
-// tens of thousands of rows: 60 pairs of 5,000 rows took one thread each
-// 12.3 ms).
+// listed for k_automaton_long, a warp each, 32 rows a step with the next step's
+// values loaded ahead (60 pairs of 5,000 rows: 0.36 ms; 2.6 with one row
+// after the other and no load ahead, 12.3 by one thread a pair).
 constexpr int AUTOMATON_LANE_ROWS = 16;
 
 __global__ void k_automaton(int64_t n_pairs, int32_t T, const int32_t *atom_begin, const int32_t *cnt_q,
@@ -5635,12 +5635,20 @@ __global__ void k_automaton_long(int32_t T, const int32_t *atom_begin, const int
         double cur = INFINITY;  // best: the minimum so far and its row
         int64_t b = -1;
         bool stop = false;
+        // (the next step's values loaded ahead)
+        double r_next = lane < cn ? rr.rmsd[o + lane] : INFINITY;
+        int nan_next = lane < cn ? rr.nan_rot[o + lane] : 0;
         for (int64_t k0 = 0; k0 < cn; k0 += 32) {
             const int64_t k = k0 + lane;
             const bool valid = k < cn;
-            const double r = valid ? rr.rmsd[o + k] : INFINITY;
+            const double r = r_next;
+            const int nr = nan_next;
+            if (k + 32 < cn) {
+                r_next = rr.rmsd[o + k + 32];
+                nan_next = rr.nan_rot[o + k + 32];
+            }
             const bool pass = !stop && valid && r <= thr;
-            const bool nan_rot = pass && rr.nan_rot[o + k] != 0;
+            const bool nan_rot = pass && nr != 0;
             bool hv = false, wv = false;
             if (best) {
                 const bool in = pass && (M < 0 || k <= (int64_t)M + 1);
@@ -5670,24 +5678,37 @@ __global__ void k_automaton_long(int32_t T, const int32_t *atom_begin, const int
                 hv = pass && !nan_rot;
                 wv = nan_rot;
             } else {
-                // the passing rows one after the other (the stream may end
-                // at any of them)
+                // the stream ends at the first passing row that has M + 1
+                // rows or more between it and the last hit (or the start);
+                // it is a hit itself at M + 1 exactly
                 const unsigned pm = __ballot_sync(FULL_MASK, pass), nm = __ballot_sync(FULL_MASK, nan_rot);
-                for (unsigned left = pm; left && !stop; left &= left - 1) {
-                    const int ln = __ffs(left) - 1;
-                    const int64_t kk = k0 + ln;
-                    if (lane == ln) np++;
-                    if (kk > base + M + 1) {
-                        stop = true;
-                        break;
+                if (pm && !nm) {
+                    const unsigned before = pm & ((1u << lane) - 1u);
+                    const int64_t from = before ? k0 + 32 - __clz(before) : base;
+                    const unsigned ends = __ballot_sync(FULL_MASK, pass && k > from + M);
+                    const int last = ends ? __ffs(ends) - 1 : 31;
+                    if (pass && lane <= last) np++;
+                    hv = pass && lane <= last && k <= from + M + 1;
+                    base = k0 + 32 - __clz(pm);
+                    stop = ends != 0;
+                } else {
+                    // undefined rotations: one row after the other
+                    for (unsigned left = pm; left && !stop; left &= left - 1) {
+                        const int ln = __ffs(left) - 1;
+                        const int64_t kk = k0 + ln;
+                        if (lane == ln) np++;
+                        if (kk > base + M + 1) {
+                            stop = true;
+                            break;
+                        }
+                        const bool undef = (nm >> ln) & 1u;
+                        if (lane == ln) {
+                            wv = undef;
+                            hv = !undef;
+                        }
+                        if (kk == base + M + 1) stop = true;
+                        if (!undef) base = kk + 1;
                     }
-                    const bool nr = (nm >> ln) & 1u;
-                    if (lane == ln) {
-                        wv = nr;
-                        hv = !nr;
-                    }
-                    if (kk == base + M + 1) stop = true;
-                    if (!nr) base = kk + 1;
                 }
             }
             if (valid) {

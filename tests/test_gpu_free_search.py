@@ -289,3 +289,17 @@ def test_entry_that_cannot_be_split(atoms, max_candidates):
     _, ref = compare(W.pack_templates([spec]), W.pack(structs), rmsd_threshold=1e3, distance_cutoff=200.0,
                      max_dynamic_distance=200.0, max_candidates=max_candidates, best_match=True)
     assert ref["hits"]["count"] == 1
+
+
+@pytest.mark.parametrize("max_candidates", [0, 1, 4, 30, 31, 32, 33, 63, 200])
+@pytest.mark.parametrize("threshold", [0.75, 1.2])
+def test_streams_cut_within_a_step(max_candidates, threshold):
+    """Streams of hundreds of rows of which some pass, cut after gaps around
+    the 32 rows a warp takes a step."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(41, [120, 70])
+    specs = _templates(41, structs, 12, lo=2, hi=4, permissive=True)
+    _, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=threshold, distance_cutoff=2.5,
+                     max_dynamic_distance=2.5, max_candidates=max_candidates)
+    assert ref["hits"]["count"] > 0
