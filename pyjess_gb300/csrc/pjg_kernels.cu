@@ -3992,8 +3992,9 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
 // the search in order took 214 ms with 12.6 M lists put in leaf order.
 //
 // Templates of 33 to 64 atoms have instances of their own (NL = 64 levels,
-// two a lane); larger ones go to k_search_large (24 structures x 24 such templates in 120: 12 ms in
-// order with every list of theirs ordered up front, 0.6 ms here).
+// two a lane); larger ones go to k_search_large.  24 such templates among 120
+// against 24 structures: 12 ms in order with every list of theirs ordered up
+// front, 0.6 ms here.
 template <int CAP, int NL>
 struct FreeState {
     float4 xyz[CAP];            // frontier entries of every level: point and key,
@@ -4247,6 +4248,12 @@ __device__ __forceinline__ void level_order(const TemplateView &tv, const CandVi
         }
     }
 }
+
+// Parents tested together against a step of a whole list, in items: 384 pairs
+// with lists of 2,000 to 5,000 take 13.7 ms with 1, 11.2 with 4, 11.4 with 8;
+// 1,000 x 4,000 13.8 / 13.0 / 13.7.  The first instance, whose entries are in
+// shared memory, gains nothing from it (29.8 -> 31 to 34 ms).
+constexpr int HEAVY_PARENTS = 4;
 
 template <bool FP32, bool HEAVY, int NL>
 __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCKS : 2)
@@ -4587,6 +4594,34 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                     for_list(cv, masks + (int64_t)g * mw, mw, q0, st.sq, [&](bool valid, int pos) {
                         const float4 x = valid ? kx[pos] : make_float4(0.f, 0.f, 0.f, 0.f);
                         const int32_t an = valid ? cv.nh_pos[abase + pos] : 0;
+                        if (HEAVY) {
+                            // several parents' tests in flight (their entries
+                            // are in global memory); queued one a lane at a time
+                            for (int p0 = beg; p0 < end; p0 += HEAVY_PARENTS) {
+                                unsigned near = 0;
+#pragma unroll
+                                for (int u = 0; u < HEAVY_PARENTS; u++) {
+                                    Mask exact = 0;
+                                    if (valid && p0 + u < end &&
+                                        test(exyz[min(p0 + u, end - 1)], x, rule_p, thr_p, lev, exact))
+                                        near |= 1u << u;
+                                }
+                                for (unsigned m; (m = __ballot_sync(FULL_MASK, near != 0)) != 0; near &= near - 1) {
+                                    if (near) {
+                                        const int qi = queued + __popc(m & lt);
+                                        st.cq[qi] = an;
+                                        st.pq[qi] = (uint16_t)(p0 + __ffs(near) - 1);
+                                    }
+                                    queued += __popc(m);
+                                    __syncwarp();
+                                    if (queued >= 32) {
+                                        run_batch(32);
+                                        if (full || kd_needed) return false;
+                                    }
+                                }
+                            }
+                            return true;
+                        }
                         for (int p = beg; p < end; p++) {
                             Mask exact = 0;
                             const bool near = valid && test(exyz[p], x, rule_p, thr_p, lev, exact);
