@@ -9,7 +9,8 @@
 //                       from the per-bucket histograms of atom names
 //   k_candidates        the lists themselves, in candidate (ResIndex) order
 //   k_scan_*            exclusive scans of list lengths and row counts
-//   k_axis_ranks        per-structure axis ranks (once, at upload)
+//   k_rank_tiles, k_axis_ranks
+//                       per-structure axis ranks (once, at upload)
 //   k_demand_levels     requests the kd leaf order of the lists a pair
 //                       reaches first
 //   k_list_keys, k_list_reps, k_list_share
@@ -22,16 +23,19 @@
 //   k_leaf_sorted<M>    kd leaf order by sorted-axis splits, with a qselect
 //                       replay of tied nodes
 //   k_leaf_exact<M>     the literal qselect sequence, for the rest
-//   k_sig_kinds         atom kinds each signature's list takes
-//   k_search_free       every pair without any order (two instances: whole
-//                       pairs, items of seeds of heavy pairs)
-//   k_unit_order, k_unit_order_large
+//   k_sig_kinds, k_list_kinds
+//                       atom kinds that each signature's list takes, in each
+//                       structure, and the list's length
+//   k_search_free       every pair without any order (whole pairs, items of
+//                       seeds of heavy pairs; 32 or 64 levels)
+//   k_unit_order_direct, k_unit_order, k_unit_order_large
 //                       the rows found without order put in the reference's
 //   k_search            persistent warp per pair, order-preserving
 //                       depth-first-over-tiles frontier expansion: the plain
 //                       mode, explicit leaf levels, and the few pairs the
 //                       order-free search leaves
-//                       (k_search_large: templates over 32 atoms)
+//                       (k_search_large: templates over 64 atoms, and those
+//                       over 32 that the order-free search leaves)
 //   k_superpose         thread per complete row, FP64 covariance and
 //                       quaternion eigen-solve
 //   k_order_counts, k_automaton, k_automaton_long, k_gather_hits
@@ -3986,7 +3990,7 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
 // passed the parent's own test) are queued with their parents, 32 a batch.
 //
 // Bound by issue slots and the latency of the pair's dependent loads.
-// Measured on 1,000 structures x 4,000 templates: 29 + 13 ms for the two
+// Measured on 1,000 structures x 4,000 templates: 29.8 + 13.0 ms for the two
 // instances (with FREE_CAP 192 26 + 18; without the queue, and with the
 // kinds of a list looked up 32 at a time instead of read as a mask, 44 + 22);
 // the search in order took 214 ms with 12.6 M lists put in leaf order.
@@ -5103,32 +5107,36 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
 // level are told apart by splitting only the kd nodes that hold two of them,
 // from the root down.  A node's left child is the half with the smaller axis
 // ranks, whatever the rest of the tree looks like: found by a histogram of the
-// rank's high bits for a node of more than 32 atoms; a node of at most 32 is taken apart
-// down to its leaves at once (an atom a lane, per axis the mask of the atoms
-// below it; a lane's place in its node is then a popcount).  A tie at a median
+// rank's high bits for a node of more than 32 atoms; a node of at most 32 is
+// taken apart down to its leaves at once (an atom a lane, per axis the mask of
+// the atoms below it; a lane's place in its node is then a popcount).  A tie at a median
 // boundary, where qselect's arrangement decides, leaves the unit to the leaf
 // order (its lists are requested and the unit listed in fw.pending), and so do
 // large units and long lists with many rows (dense templates: few lists,
 // shared by many units).  Splits along a path halve, so a level costs about
 // two passes over its list.
 //
-// Two instances by list length (shared memory a warp holds): units whose
-// lists have at most DIRECT_MAX entries, and, passed on by the first, lists of
-// up to DIRECT_LONG with at most DIRECT_LONG_ROWS rows.
-// Measured on 1,000 structures x 4,000 templates: 8.8 and 8.9 ms, and 11 ms
-// for the 62,000 lists left to the leaf order, where ordering every such list
-// (0.84 M) and ranking the rows by them took 42 and 9 ms.  With 3,000
-// templates against one protein: 0.35 ms instead of 1.9 ms.
+// Two instances by the shared memory a warp holds, which sets the warps an SM
+// has: units of at most DIRECT_ROWS rows whose lists have at most DIRECT_MAX
+// entries (24 warps; 20 for 128 rows, 12 for 256), and, passed on by the
+// first, more rows, and lists of up to DIRECT_LONG with at most
+// DIRECT_LONG_ROWS rows (7 warps).
+// Measured on 1,000 structures x 4,000 templates: 5.9 and 9.7 ms (DIRECT_ROWS
+// 128 6.8 and 9.2, 256 9.7 and 9.0), and 11 ms for the 62,000 lists left to the
+// leaf order, where ordering every such list (0.84 M) and ranking the rows by
+// them took 42 and 9 ms.  With 3,000 templates against one protein: 0.35 ms
+// instead of 1.9 ms.
 constexpr int DIRECT_MAX = 512, DIRECT_LONG = 2048;
 constexpr int DIRECT_WARPS = 4, DIRECT_LONG_WARPS = 1;
 constexpr int DIRECT_LONG_ROWS = 32;
+constexpr int DIRECT_ROWS = 64;
 
-template <int MAXM>
+template <int MAXM, int ROWS>
 struct DirectWarp {
-    unsigned long long key[UNIT_ROWS];
-    int32_t cur[UNIT_ROWS], atom[UNIT_ROWS], row[UNIT_ROWS];
-    uint32_t code[UNIT_ROWS];  // path from the root: a bit a split, 0 right (reported first)
-    uint16_t node[UNIT_ROWS];  // node the row's atom is in
+    unsigned long long key[ROWS];
+    int32_t cur[ROWS], atom[ROWS], row[ROWS];
+    uint32_t code[ROWS];       // path from the root: a bit a split, 0 right (reported first)
+    uint16_t node[ROWS];       // node the row's atom is in
     uint16_t sq[32];
     int32_t mem[2][MAXM];      // the nodes' atoms, children in the other buffer
     uint32_t rk[MAXM];         // ranks of the node being split
@@ -5137,13 +5145,13 @@ struct DirectWarp {
     int4 stack[32];            // nodes to split: first entry, entries, depth | buffer << 8, number
 };
 
-template <int MAXM, int WARPS>
+template <int MAXM, int ROWS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
     k_unit_order_direct(ChunkView cv, TemplateView tv, CandView cd, SigView sv, FreeView fv, const int32_t *res_place,
                         int32_t reorder, FreeWork fw, CompleteRows out) {
     extern __shared__ __align__(16) unsigned char direct_smem[];
     constexpr bool LONG = MAXM > DIRECT_MAX;
-    DirectWarp<MAXM> &U = reinterpret_cast<DirectWarp<MAXM> *>(direct_smem)[threadIdx.x >> 5];
+    DirectWarp<MAXM, ROWS> &U = reinterpret_cast<DirectWarp<MAXM, ROWS> *>(direct_smem)[threadIdx.x >> 5];
     const int lane = lane_id();
     const unsigned lt = (1u << lane) - 1u;
     const int T = tv.n_templates, G = cd.n_sigs;
@@ -5182,8 +5190,8 @@ __global__ void __launch_bounds__(WARPS * 32)
             if (l > 0 && ((branch >> l) & 1ull)) most = max(most, cd.count[wb + U.sig[l]]);
         most = __reduce_max_sync(FULL_MASK, most);
         bool pending = R > UNIT_ROWS;
-        if (!LONG && !pending && most > DIRECT_MAX) {
-            if (R <= DIRECT_LONG_ROWS && most <= DIRECT_LONG) {
+        if (!LONG && !pending && (most > DIRECT_MAX || R > ROWS)) {
+            if (most <= DIRECT_MAX || (R <= DIRECT_LONG_ROWS && most <= DIRECT_LONG)) {
                 if (lane == 0) fw.long_units[atomicAdd(fw.n_long_units, 1ull)] = w;
                 continue;
             }
@@ -6264,11 +6272,11 @@ cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const Chu
                                                                          out);
         return cudaGetLastError();
     };
-    cudaError_t e = launch(k_unit_order_direct<DIRECT_MAX, DIRECT_WARPS>,
-                           (int)sizeof(DirectWarp<DIRECT_MAX>) * DIRECT_WARPS, DIRECT_WARPS, n_units);
+    cudaError_t e = launch(k_unit_order_direct<DIRECT_MAX, DIRECT_ROWS, DIRECT_WARPS>,
+                           (int)sizeof(DirectWarp<DIRECT_MAX, DIRECT_ROWS>) * DIRECT_WARPS, DIRECT_WARPS, n_units);
     if (e == cudaSuccess)
-        e = launch(k_unit_order_direct<DIRECT_LONG, DIRECT_LONG_WARPS>,
-                   (int)sizeof(DirectWarp<DIRECT_LONG>) * DIRECT_LONG_WARPS, DIRECT_LONG_WARPS, n_units);
+        e = launch(k_unit_order_direct<DIRECT_LONG, UNIT_ROWS, DIRECT_LONG_WARPS>,
+                   (int)sizeof(DirectWarp<DIRECT_LONG, UNIT_ROWS>) * DIRECT_LONG_WARPS, DIRECT_LONG_WARPS, n_units);
     return e;
 }
 

@@ -303,3 +303,18 @@ def test_streams_cut_within_a_step(max_candidates, threshold):
     _, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=threshold, distance_cutoff=2.5,
                      max_dynamic_distance=2.5, max_candidates=max_candidates)
     assert ref["hits"]["count"] > 0
+
+
+@pytest.mark.parametrize("reach", [1.2, 1.6, 1.9, 2.2])
+def test_units_of_dozens_of_rows(reach):
+    """Pairs of 2 to 300 rows (every row a hit) in lists of up to 120 entries:
+    units on both sides of the rows that each instance holds."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(42, [60, 80, 100, 120], chains=1)
+    specs = _templates(42, structs, 100, lo=2, hi=4, permissive=True)
+    _, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=10.0, distance_cutoff=reach,
+                     max_dynamic_distance=reach)
+    h = ref["hits"]
+    rows = np.unique(h["structure"].astype(np.int64) * len(specs) + h["template"], return_counts=True)[1]
+    assert (rows > 1).any() and (reach < 1.6 or (rows > 64).any())
