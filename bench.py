@@ -12,7 +12,7 @@ FP32-guarded distance tests with FP64 recheck.
   e2e         the same metric through the C ABI with host buffers: per step
               pjg_templates_create + pjg_structures_create (H2D), pjg_query,
               pjg_results_copy (D2H), wall clock
-  roofline    k_search (the expansion kernel): algorithmic expansion bytes /
+  roofline    k_search_free (the expansion kernel): algorithmic expansion bytes /
               kernel time against the measured HBM copy bandwidth
   cpu_baseline  the CPU oracle (a port of the reference's algorithm) on the
               host cores, on a bounded sample of the same workload
@@ -311,6 +311,7 @@ def search_profile(args):
     os.environ["PJG_LIB_VARIANT"] = variant
     from pyjess_gb300 import _build, _native
 
+    os.environ.setdefault("PJG_LEAF_LEVELS", "4")  # k_search takes the pairs of a query ordered up front
     _build.build(variant=variant)
     _native.init(dist_env()[2])
     wl = workload(args)
@@ -421,26 +422,26 @@ def main():
     s0 = stats[-1]
     hits_per_s = s0["hits"] * world * args.steps / (total_ms / 1e3)
 
-    # ---- roofline of the expansion kernel (k_search)
+    # ---- roofline of the expansion kernel (k_search_free, both instances)
     peaks, peak_kind = measured_peaks()
     exp_ms = sum(s["ms_expansion"] for s in stats)
     exp_bytes = sum(s["bytes_expansion"] for s in stats)
     achieved = exp_bytes / (exp_ms / 1e3) / 1e9 if exp_ms > 0 else 0.0
     peak = float(peaks["hbm_gbs"])
     traffic, issue = None, None
-    tpath = os.path.join(ROOT, "profiles", "k_search_traffic.json")
+    tpath = os.path.join(ROOT, "profiles", "k_search_free_traffic.json")
     if os.path.exists(tpath):
         with open(tpath) as f:
             tr = json.load(f)
-        # the resource that binds k_search: issue slots (ncu, same capture)
+        # the resource that binds k_search_free: issue slots (ncu, same capture)
         if tr.get("issue_active_frac") is not None:
             issue = {"frac": tr["issue_active_frac"], "frac_first_round": tr.get("issue_active_frac_first_round"),
                      "warp_inst_per_partial": tr.get("warp_inst_per_partial"),
                      "source": "ncu smsp__issue_active.avg.pct_of_peak_sustained_active and sm__inst_executed.sum "
-                               "of the k_search launches of a 20 x 5,000 query (profiles/k_search_traffic.json)"}
+                               "of the k_search_free launches of a 20 x 5,000 query (profiles/k_search_free_traffic.json)"}
         # DRAM bytes per algorithmic expansion byte, measured by ncu over the
-        # k_search launches of one query of a smaller case, times the
-        # expansion bytes of an average launch of this workload
+        # k_search_free launches of one query of a smaller case, times the
+        # expansion bytes of an average search round of this workload
         if tr.get("dram_per_expansion_byte"):
             launches_k = max(1, sum(s["search_rounds"] for s in stats))
             traffic = tr["dram_per_expansion_byte"] * exp_bytes / launches_k
@@ -549,7 +550,7 @@ def main():
         "batched_over_plain": value / plain["value"] if plain else None,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if peak else None, "traffic": traffic,
-                     "kernel": "k_search", "peak_kind": peak_kind, "issue_slots": issue,
+                     "kernel": "k_search_free", "peak_kind": peak_kind, "issue_slots": issue,
                      "bytes_expansion_per_step": exp_bytes / args.steps,
                      "ms_expansion_per_step": exp_ms / args.steps},
         "stage_ms": {"candidates": s0["ms_candidates"], "expansion": s0["ms_expansion"],
