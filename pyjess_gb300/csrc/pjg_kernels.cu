@@ -5435,7 +5435,10 @@ __global__ void __launch_bounds__(WARPS * 32)
 // Block per unit of more rows (a seed of a flexible template can have
 // thousands): the rows kept sorted as far as the levels taken tell them
 // apart, row[p] at position p of class cls[p] (the position where its class
-// begins), so a level compares a row with its own class only.
+// begins), so a level compares a row with its own class only: the class's end
+// by bisection, so that the keys' loads do not wait for each other (31,853
+// pairs with items of thousands of rows: 1.4 ms; 4.5 with the class looked up
+// row by row).
 __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
     k_unit_order_large(ChunkView cv, TemplateView tv, CandView cd, SigView sv, const int32_t *res_place,
                        int32_t reorder, FreeWork fw, CompleteRows out) {
@@ -5503,8 +5506,16 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
             for (int p = tid; p < R; p += blockDim.x) {
                 const int c0 = cls[p];
                 const unsigned long long mine = key[p];
+                // the end of the class, then its keys with loads in flight
+                int end = R;
+                for (int in = p; end - in > 1;) {
+                    const int mid = (in + end) >> 1;
+                    if (cls[mid] == c0) in = mid;
+                    else end = mid;
+                }
                 int before = 0;
-                for (int q = c0; q < R && cls[q] == c0; q++) before += key[q] < mine ? 1 : 0;
+#pragma unroll 8
+                for (int q = c0; q < end; q++) before += key[q] < mine ? 1 : 0;
                 const int c1 = c0 + before;
                 const int to = c1 + atomicAdd(&fill[c1], 1);
                 row2[to] = row[p];
