@@ -52,7 +52,8 @@ enum {
     PJG_MODE_PLAIN_FP64 = 0,
     /* all pairs in one launch sequence; distance tests in FP32 on
      * centroid-relative coordinates with a guard band, anything inside the
-     * band rechecked in FP64 with the reference's operation order. */
+     * band rechecked in FP64 with the reference's operation order
+     * (templates of more than 64 atoms: every test in FP64). */
     PJG_MODE_BATCHED_FP32 = 1,
     /* all pairs in one launch sequence, FP64 distance tests. */
     PJG_MODE_BATCHED_FP64 = 2

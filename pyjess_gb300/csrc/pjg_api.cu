@@ -1429,7 +1429,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         if (bound > g) g = bound;
         CUDA_TRY(dalloc(d_params, (size_t)std::max<int64_t>(tp->n_params, 1), st));
         launch_params(st, T, tp->d_atom_begin, tp->d_param_begin, tp->d_dist, tp->d_weight,
-                      P->distance_cutoff, P->max_dynamic_distance, g, d_params.p);
+                      P->distance_cutoff, P->max_dynamic_distance, g, fp32, d_params.p);
         launches++;
         CUDA_TRY(cudaGetLastError());
     }

@@ -77,7 +77,7 @@ __device__ __forceinline__ uint64_t global_ns() {
 // 0, squares a*a and b*b, box half-width b.
 
 __global__ void k_params(int n_templates, const int32_t *atom_begin, const int32_t *param_begin,
-                         const double *dist, const double *weight, double r, double s, double g,
+                         const double *dist, const double *weight, double r, double s, double g, bool fp32,
                          AnnulusParam *out) {
     int t = blockIdx.x;
     if (t >= n_templates) return;
@@ -109,6 +109,12 @@ __global__ void k_params(int n_templates, const int32_t *atom_begin, const int32
         P.thr.y = __double2float_ru(ahi * ahi);
         P.thr.z = blo > 0.0 ? __double2float_rd(blo * blo) : -1.0f;
         P.thr.w = __double2float_ru(bhi * bhi);
+        if (!fp32) {
+            // no FP32 bounds to test a distance with: such a test would reject
+            // every point (the outer one still culls blocks)
+            P.thr.x = P.thr.y = INFINITY;
+            P.thr.z = -1.0f;
+        }
         P.pad = 0.0;
         out[base + idx] = P;
     }
@@ -3986,6 +3992,10 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32)
 // children than HEAVY_CAP has room for, and points whose decision needs the
 // kd-tree (outside an annulus box by rounding).
 //
+// The FP64 mode tests every distance in FP64 (annulus64), the rules alone on
+// the FP32 entries: 61 structures x 1,003 templates 11.4 ms a pass, where an
+// FP32 screen, which that mode rules out, took 6.3 to 7.2.
+//
 // Every test of a chain runs on a full warp: candidates (of a residue, or that
 // passed the parent's own test) are queued with their parents, 32 a batch.
 //
@@ -4490,28 +4500,31 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                 }
                 anchor = __reduce_max_sync(FULL_MASK, anchor);
                 __syncwarp();
-                // the lanes' tests at one chain entry
+                // the lanes' tests at one chain entry (FP64 mode: the rule; the
+                // distance by annulus64)
                 auto test = [&](const float4 &e, const float4 &x, const int4 &r, const float4 &th, int j,
                                 Mask &exact) -> bool {
                     const int32_t d = __float_as_int(e.w) ^ __float_as_int(x.w);
+                    const bool ok = (d & r.x) == 0 && ((d & r.y) | r.z) != 0;
+                    if (!FP32) return ok;
                     const float dx = e.x - x.x, dy = e.y - x.y, dz = e.z - x.z;
                     const float d2 = dx * dx + dy * dy + dz * dz;
-                    const bool ok = (d & r.x) == 0 && ((d & r.y) | r.z) != 0 && !(d2 < th.x || d2 > th.w);
-                    if (!FP32 || !(d2 >= th.y && d2 <= th.z)) exact |= Mask(1) << j;
-                    return ok;
+                    if (!(d2 >= th.y && d2 <= th.z)) exact |= Mask(1) << j;
+                    return ok && !(d2 < th.x || d2 > th.w);
                 };
                 // candidates that passed: inconclusive ones decided in FP64,
-                // the others appended as children
-                auto accept = [&](bool pass, Mask exact, int p, int32_t an, const float4 &x) {
-                    if (__any_sync(FULL_MASK, pass && exact)) {
-                        int v = 1;
+                // the others appended as children (outside: not in every
+                // annulus box)
+                auto accept = [&](bool pass, Mask exact, bool outside, int p, int32_t an, const float4 &x) {
+                    if (FP32 && __any_sync(FULL_MASK, pass && exact)) {
                         if (pass && exact) {
-                            if (FP32) crech += __popcll((unsigned long long)exact);
-                            v = free_decide(eatom, eparent, st.order, exact, lev, p, an, xyz64, prm, n, qn);
+                            crech += __popcll((unsigned long long)exact);
+                            const int v = free_decide(eatom, eparent, st.order, exact, lev, p, an, xyz64, prm, n, qn);
                             pass = v != 0;
+                            outside = v == 2;
                         }
-                        if (__any_sync(FULL_MASK, v == 2)) kd_needed = true;
                     }
+                    if (__any_sync(FULL_MASK, pass && outside)) kd_needed = true;
                     const unsigned m = __ballot_sync(FULL_MASK, pass);
                     const int np = __popc(m);
                     Fc += np;
@@ -4538,15 +4551,22 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                     const int p = pass ? st.pq[queued + lane] : 0;
                     const int32_t an = pass ? st.cq[queued + lane] : 0;
                     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                    bool outside = false;
                     if (pass) {
                         x = cv.xyz32[abase + an];
-                        for (int j = lev, e = p; j >= 0; j--, e = eparent[e])
-                            if (!test(exyz[e], x, st.rule[j], st.thr[j], j, exact)) {
-                                pass = false;
-                                break;
+                        double x64[3];
+                        for (int i = 0; i < 3 && !FP32; i++) x64[i] = xyz64[3 * (int64_t)an + i];
+                        for (int j = lev, e = p; j >= 0; j--, e = eparent[e]) {
+                            pass = test(exyz[e], x, st.rule[j], st.thr[j], j, exact);
+                            if (!FP32 && pass) {
+                                bool inb;
+                                pass = annulus64(xyz64 + 3 * (int64_t)eatom[e], x64, prm[st.order[j] * n + qn], &inb);
+                                outside |= !inb;
                             }
+                            if (!pass) break;
+                        }
                     }
-                    accept(pass, exact, p, an, x);
+                    accept(pass, exact, outside, p, an, x);
                     __syncwarp();
                 };
                 if (anchor >= 0) {
@@ -4595,21 +4615,27 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                     // those that pass the parent's own test are queued
                     const float4 thr_p = st.thr[lev];
                     const int4 rule_p = st.rule[lev];
+                    const AnnulusParam &prm_p = prm[st.order[lev] * n + qn];
                     for_list(cv, masks + (int64_t)g * mw, mw, q0, st.sq, [&](bool valid, int pos) {
                         const float4 x = valid ? kx[pos] : make_float4(0.f, 0.f, 0.f, 0.f);
                         const int32_t an = valid ? cv.nh_pos[abase + pos] : 0;
+                        double x64[3] = {};
+                        if (!FP32 && valid)
+                            for (int i = 0; i < 3; i++) x64[i] = xyz64[3 * (int64_t)an + i];
+                        auto near_parent = [&](int p) -> bool {
+                            Mask exact = 0;
+                            if (!test(exyz[p], x, rule_p, thr_p, lev, exact)) return false;
+                            bool inb;
+                            return FP32 || annulus64(xyz64 + 3 * (int64_t)eatom[p], x64, prm_p, &inb);
+                        };
                         if (HEAVY) {
                             // several parents' tests in flight (their entries
                             // are in global memory); queued one a lane at a time
                             for (int p0 = beg; p0 < end; p0 += HEAVY_PARENTS) {
                                 unsigned near = 0;
 #pragma unroll
-                                for (int u = 0; u < HEAVY_PARENTS; u++) {
-                                    Mask exact = 0;
-                                    if (valid && p0 + u < end &&
-                                        test(exyz[min(p0 + u, end - 1)], x, rule_p, thr_p, lev, exact))
-                                        near |= 1u << u;
-                                }
+                                for (int u = 0; u < HEAVY_PARENTS; u++)
+                                    if (valid && p0 + u < end && near_parent(min(p0 + u, end - 1))) near |= 1u << u;
                                 for (unsigned m; (m = __ballot_sync(FULL_MASK, near != 0)) != 0; near &= near - 1) {
                                     if (near) {
                                         const int qi = queued + __popc(m & lt);
@@ -4627,8 +4653,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                             return true;
                         }
                         for (int p = beg; p < end; p++) {
-                            Mask exact = 0;
-                            const bool near = valid && test(exyz[p], x, rule_p, thr_p, lev, exact);
+                            const bool near = valid && near_parent(p);
                             const unsigned m = __ballot_sync(FULL_MASK, near);
                             if (!m) continue;
                             if (near) {
@@ -5839,8 +5864,10 @@ __global__ void k_gather_hits(int64_t n_rows, int32_t T, int32_t structure_base,
 // Launchers
 
 void launch_params(cudaStream_t st, int n_templates, const int32_t *atom_begin, const int32_t *param_begin,
-                   const double *dist, const double *weight, double r, double s, double g, AnnulusParam *out) {
-    if (n_templates > 0) k_params<<<n_templates, 256, 0, st>>>(n_templates, atom_begin, param_begin, dist, weight, r, s, g, out);
+                   const double *dist, const double *weight, double r, double s, double g, bool fp32,
+                   AnnulusParam *out) {
+    if (n_templates > 0)
+        k_params<<<n_templates, 256, 0, st>>>(n_templates, atom_begin, param_begin, dist, weight, r, s, g, fp32, out);
 }
 
 void launch_candidates(cudaStream_t st, int blocks, bool fill, const ChunkView &cv, const SigView &sv,

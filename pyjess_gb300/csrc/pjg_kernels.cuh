@@ -376,7 +376,8 @@ size_t search_state_bytes();
 // Host-side launchers (the kernels themselves live in pjg_kernels.cu).
 
 void launch_params(cudaStream_t st, int n_templates, const int32_t *atom_begin, const int32_t *param_begin,
-                   const double *dist, const double *weight, double r, double s, double g, AnnulusParam *out);
+                   const double *dist, const double *weight, double r, double s, double g, bool fp32,
+                   AnnulusParam *out);
 
 // fill == false: list lengths of every list of the chunk; fill == true: the
 // lists themselves, of every list (work == nullptr) or of the lists in

@@ -54,6 +54,17 @@ def test_scattered_residues(mode, ignore):
     assert ref["hits"]["count"] > 0
 
 
+@pytest.mark.parametrize("ignore", [0, 2])
+def test_fp64_mode_near_annulus_bounds(ignore):
+    """Atoms within 1e-6 A of annulus boundaries in FP64 mode, whose annuli
+    hold no FP32 bounds to reject a point with: the oracle's hits."""
+    from pyjess_gb300 import workloads as W
+
+    wl = W.config(3, n_structures=20, n_templates=200)
+    res, ref = compare(wl.templates, wl.structures, mode="fp64", ignore_chain=ignore, **wl.params)
+    assert ref["hits"]["count"] > 0 and res.stats()["fp64_rechecks"] == 0
+
+
 @pytest.mark.parametrize("kw", [dict(), dict(best_match=True), dict(max_candidates=0), dict(max_candidates=5),
                                 dict(max_candidates=300), dict(best_match=True, max_candidates=7),
                                 dict(reorder=False), dict(reorder=False, max_candidates=40)])
