@@ -4263,6 +4263,23 @@ __device__ __forceinline__ void level_order(const TemplateView &tv, const CandVi
     }
 }
 
+// An item's result, read by other items of its pair while it is written: one
+// 8-byte access each way, so that rows and flags are of one moment.
+__device__ __forceinline__ int2 load_result(const int2 *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return make_int2((int)(unsigned)v, (int)(v >> 32));
+}
+__device__ __forceinline__ void store_result(int2 *p, int2 r) {
+    const unsigned long long v = (unsigned)r.x | ((unsigned long long)(unsigned)r.y << 32);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ int load_flag(const int32_t *p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // Parents tested together against a step of a whole list, in items: 384 pairs
 // with lists of 2,000 to 5,000 take 13.7 ms with 1, 11.2 with 4, 11.4 with 8;
 // 1,000 x 4,000 13.8 / 13.0 / 13.7.  The first instance, whose entries are in
@@ -4318,7 +4335,10 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                 blk = it.y;
             }
             hp = fw.heavy[hidx];
-            if (hp.failed) continue;
+            // (read by one lane: another warp may set it at this moment)
+            int failed = 0;
+            if (lane == 0) failed = load_flag(&fw.heavy[hidx].failed);
+            if (__shfl_sync(FULL_MASK, failed, 0)) continue;
         }
         const int pair = HEAVY      ? hp.pair
                          : NL == 32 ? item
@@ -4334,15 +4354,16 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
         // rows (best_match), or, right before it, that many rows without a
         // hit among them, or one of them ended the stream
         if (HEAVY && !sub && sa.max_candidates >= 0 && blk > 0) {
-            const volatile int2 *res = fw.results + hp.first;
+            const int2 *res = fw.results + hp.first;
             long long sum = 0;
             bool end = false;
             for (int x0 = ((blk - 1) / 32) * 32; x0 >= 0; x0 -= 32) {
                 const int x = x0 + lane;
                 int r = -1, f = 0;
                 if (x < blk) {
-                    r = res[x].x;
-                    f = res[x].y;
+                    const int2 v = load_result(res + x);
+                    r = v.x;
+                    f = v.y;
                 }
                 const bool done = x < blk && r >= 0;
                 end |= __any_sync(FULL_MASK, done && (f & 2));
@@ -4363,7 +4384,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                 if (!more) break;
             }
             if (end || sum >= (long long)sa.max_candidates + 2) {
-                if (lane == 0) fw.results[hp.first + blk] = make_int2(0, 2);
+                if (lane == 0) store_result(&fw.results[hp.first + blk], make_int2(0, 2));
                 continue;
             }
         }
@@ -4863,7 +4884,8 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                     add(3, rech);
                     if (lane == 0 && sub) atomicAdd(&fw.results[hp.first + blk].x, rows);
                     if (lane == 0 && !sub)
-                        fw.results[hp.first + blk] = make_int2(rows, (any_hit || spilled ? 1 : 0) | (ended ? 2 : 0));
+                        store_result(&fw.results[hp.first + blk],
+                                     make_int2(rows, (any_hit || spilled ? 1 : 0) | (ended ? 2 : 0)));
                 } else {
                     if (lane == 0 && rows > 0) out.pair_rows[pair] = rows;
                     a_part += part;

@@ -302,6 +302,22 @@ def test_entry_that_cannot_be_split(atoms, max_candidates):
     assert ref["hits"]["count"] == 1
 
 
+def test_cut_items_give_the_same_stream_every_time():
+    """Hundreds of items of a pair in flight, each asking the ones before it
+    whether it is still wanted: the oracle's cut stream in every run."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(45, [1500, 1300])
+    specs = _templates(45, structs, 6, lo=2, hi=4, permissive=True)
+    pt, ps = W.pack_templates(specs), W.pack(structs)
+    kw = dict(rmsd_threshold=1.0, distance_cutoff=1.2, max_dynamic_distance=1.2, max_candidates=40)
+    _, ref = compare(pt, ps, **kw)
+    want = hit_keys(ref["hits"])
+    assert len(want) > 0
+    for _ in range(20):
+        assert hit_keys(gpu_query(pt, ps, **kw).arrays()) == want
+
+
 @pytest.mark.parametrize("max_candidates", [0, 1, 4, 30, 31, 32, 33, 63, 200])
 @pytest.mark.parametrize("threshold", [0.75, 1.2])
 def test_streams_cut_within_a_step(max_candidates, threshold):
