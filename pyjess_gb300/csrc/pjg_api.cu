@@ -2228,7 +2228,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         fw.row_key = d_row_key.p;
                         fw.row_scratch = d_row_scratch.p;
                         fw.large_units = d_large_units.p;
-                        launch_unit_order(st, (int64_t)free_n[6], cv, tv, cd, sv, sp->d_res_place, P->reorder, fw, cr);
+                        launch_unit_order(st, (int64_t)free_n[6], cv, tv, cd, sv, sp->d_res_place, P->reorder,
+                                          sa.budget_ns, d_counters.p, fw, cr);
                         launches++;
                         CUDA_TRY(cudaGetLastError());
                     }

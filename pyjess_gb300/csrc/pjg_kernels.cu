@@ -5485,14 +5485,36 @@ __global__ void __launch_bounds__(WARPS * 32)
 // begins), so a level compares a row with its own class only: the class's end
 // by bisection, so that the keys' loads do not wait for each other (31,853
 // pairs with items of thousands of rows: 1.4 ms; 4.5 with the class looked up
-// row by row).
+// row by row).  A level with a class of more than UNIT_COUNT_MAX rows is
+// merge-sorted instead: a row counting its class is quadratic (580,000 rows in
+// one class: 133 ms, 52 s counted; 33,750: 5.2 and 177 ms; 6,574: 0.5 and 1.7).
+// The time budget is polled at every level, merge pass and block of leaves.
+constexpr int UNIT_COUNT_MAX = 4096;
+
 __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
     k_unit_order_large(ChunkView cv, TemplateView tv, CandView cd, SigView sv, const int32_t *res_place,
-                       int32_t reorder, FreeWork fw, CompleteRows out) {
+                       int32_t reorder, uint64_t budget_ns, unsigned long long *counters, FreeWork fw,
+                       CompleteRows out) {
     __shared__ int32_t order[64], sig[64], leaf[UNIT_LARGE_THREADS];
     __shared__ long long region;
+    __shared__ int most, over;
     const int T = tv.n_templates, G = cd.n_sigs, tid = threadIdx.x;
     const int64_t total = (int64_t)*fw.n_large_units;
+    uint64_t t_start = 0;
+    if (tid == 0) {
+        t_start = global_ns();
+        over = 0;
+    }
+    // (by every thread; a barrier on both sides)
+    auto out_of_time = [&]() -> bool {
+        __syncthreads();
+        if (tid == 0 && global_ns() - t_start > budget_ns) {
+            over = 1;
+            atomicMax(&counters[C_ERROR], 3ull);
+        }
+        __syncthreads();
+        return over != 0;
+    };
     for (int64_t x = blockIdx.x; x < total; x += gridDim.x) {
         const int head = fw.large_units[x];
         const RowUnit u = fw.units[head];
@@ -5520,12 +5542,13 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
             at += v.count;
             q = u.item >= 0 ? v.next : -1;
         }
-        __syncthreads();
         for (unsigned long long left = u.item >= 0 ? fw.item_branch[u.item] : u.branch; left; left &= left - 1) {
             const int l = __ffsll((long long)left) - 1;
             const int k = order[l], g = sig[l];
             const int m = cd.count[wb + g];
             const int32_t *la = l == 0 ? nullptr : cd.leaf_atom + cd.leaf_offset[wb + g];
+            if (out_of_time()) return;
+            if (tid == 0) most = 0;
             for (int p = tid; p < R; p += blockDim.x) {
                 const int32_t a = out.atoms[(int64_t)row[p] * out.stride + k];
                 key[p] = l == 0 ? candidate_place(cv, sv, res_place, g, abase, a) : (unsigned long long)(uint32_t)a;
@@ -5535,7 +5558,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
                 // atoms (bit 63 set once replaced) by their leaf ranks, the list
                 // through shared memory
                 for (int k0 = 0; k0 < m; k0 += blockDim.x) {
-                    __syncthreads();
+                    if (out_of_time()) return;
                     if (k0 + tid < m) leaf[tid] = la[k0 + tid];
                     __syncthreads();
                     const int kn = min((int)blockDim.x, m - k0);
@@ -5550,6 +5573,62 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
                 }
             }
             __syncthreads();
+            // the largest class
+            for (int p = tid; p < R; p += blockDim.x)
+                if (p + 1 == R || cls[p + 1] != cls[p]) atomicMax(&most, p + 1 - cls[p]);
+            __syncthreads();
+            if (most > UNIT_COUNT_MAX) {
+                // by (class, key): the first level taken has one class, a leaf
+                // rank and a class share 63 bits at the others
+                if (l > 0)
+                    for (int p = tid; p < R; p += blockDim.x)
+                        key[p] = ((unsigned long long)(uint32_t)cls[p] << 32) | (uint32_t)key[p];
+                int32_t *src = row2, *dst = cls2;  // positions, sorted in runs
+                for (int p = tid; p < R; p += blockDim.x) src[p] = p;
+                for (int lw = 0; (1ll << lw) < R; lw++) {  // runs of 2^lw
+                    if (out_of_time()) return;
+                    for (int p = tid; p < R; p += blockDim.x) {
+                        // p's place among its run and the sibling run, equal
+                        // keys of the left run first
+                        const int run = p >> lw;
+                        const long long sib = (long long)(run ^ 1) << lw;
+                        const bool right = run & 1;
+                        const int i = src[p];
+                        const unsigned long long mine = key[i];
+                        const int from = (int)min(sib, (long long)R);
+                        int lo = from, hi = (int)min(sib + (1ll << lw), (long long)R);
+                        while (lo < hi) {
+                            const int mid = lo + ((hi - lo) >> 1);
+                            const unsigned long long v = key[src[mid]];
+                            if (v < mine || (right && v == mine)) lo = mid + 1;
+                            else hi = mid;
+                        }
+                        dst[(right ? p - (1 << lw) : p) + (lo - from)] = i;
+                    }
+                    int32_t *y = src;
+                    src = dst;
+                    dst = y;
+                }
+                __syncthreads();
+                // new classes (where a row's key begins) and the rows in order
+                for (int p = tid; p < R; p += blockDim.x) {
+                    const unsigned long long mine = key[src[p]];
+                    int lo = 0, hi = p;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (key[src[mid]] < mine) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    fill[p] = lo;
+                    dst[p] = row[src[p]];
+                }
+                __syncthreads();
+                for (int p = tid; p < R; p += blockDim.x) {
+                    cls[p] = fill[p];
+                    row[p] = dst[p];
+                }
+                continue;
+            }
             for (int p = tid; p < R; p += blockDim.x) {
                 const int c0 = cls[p];
                 const unsigned long long mine = key[p];
@@ -5575,6 +5654,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
             row2 = x1;
             cls2 = x2;
         }
+        __syncthreads();
         for (int p = tid; p < R; p += blockDim.x) out.ordinal[row[p]] = ord0 + p;
     }
 }
@@ -6342,10 +6422,12 @@ cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const Chu
 
 void launch_unit_order(cudaStream_t st, int64_t n_pending, const ChunkView &cv, const TemplateView &tv,
                        const CandView &cd, const SigView &sv, const int32_t *res_place, int32_t reorder,
-                       const FreeWork &fw, const CompleteRows &out) {
+                       uint64_t budget_ns, unsigned long long *counters, const FreeWork &fw,
+                       const CompleteRows &out) {
     const int64_t blocks = std::min<int64_t>((n_pending + UNIT_WARPS - 1) / UNIT_WARPS, 152 * 16);
     k_unit_order<<<(int)blocks, UNIT_WARPS * 32, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
-    k_unit_order_large<<<152 * 4, UNIT_LARGE_THREADS, 0, st>>>(cv, tv, cd, sv, res_place, reorder, fw, out);
+    k_unit_order_large<<<152 * 4, UNIT_LARGE_THREADS, 0, st>>>(cv, tv, cd, sv, res_place, reorder, budget_ns, counters,
+                                                              fw, out);
 }
 
 cudaError_t launch_search_large(cudaStream_t st, const ChunkView &cv, const TemplateView &tv, const CandView &cd,

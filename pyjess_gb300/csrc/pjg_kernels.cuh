@@ -511,7 +511,8 @@ void launch_pending_requests(cudaStream_t st, int64_t n_pending, const TemplateV
                              int32_t reorder, const LeafDemand &dm, const FreeWork &fw);
 void launch_unit_order(cudaStream_t st, int64_t n_pending, const ChunkView &cv, const TemplateView &tv,
                        const CandView &cd, const SigView &sv, const int32_t *res_place, int32_t reorder,
-                       const FreeWork &fw, const CompleteRows &out);
+                       uint64_t budget_ns, unsigned long long *counters, const FreeWork &fw,
+                       const CompleteRows &out);
 
 // culling blocks per list: ceil(count / CULL_BLK)
 void launch_block_counts(cudaStream_t st, int64_t n, const int32_t *count, int32_t *nblk);

@@ -285,6 +285,48 @@ def test_spilled_entries_of_two_lane_levels(kw):
             max_dynamic_distance=2.0, **kw)
 
 
+def _one_seed_any_pair(seed, atoms):
+    """One structure and a template of four atoms: the first two have one
+    candidate, the others any atom at any distance, so the pair has one item
+    and nearly atoms^2 rows."""
+    from pyjess_gb300 import workloads as W
+
+    s = _structures(seed, [atoms // 4])[0]
+    spec = _templates(seed, [s], 1, lo=4, hi=5, radius=60.0, permissive=True, atoms_per_res=1)[0]
+    for k in ("xyz", "name", "resname", "res_seq", "chain", "serial"):
+        s[k] = np.array(s[k][:atoms])
+    names = sorted({bytes(x) for x in s["name"]})
+    s["name"][0], s["name"][20] = np.frombuffer(b"_ZZ__YY_", np.uint8).reshape(2, 4)
+    s["chain"][:] = s["chain"][0]
+    spec.chain, spec.res_seq = [bytes(s["chain"][0])] * 4, [1, 2, 3, 4]
+    spec.names = [[b"_ZZ_"], [b"_YY_"], names, names]
+    return W.pack_templates([spec]), W.pack([s])
+
+
+@pytest.mark.parametrize("atoms", [36, 84, 85, 112])
+def test_classes_around_the_largest_counted(atoms):
+    """Units whose rows all part at one level, of 370 to 8,302 rows: on
+    both sides of the largest class that is counted row by row."""
+    pt, ps = _one_seed_any_pair(46, atoms)
+    _, ref = compare(pt, ps, rmsd_threshold=100.0, distance_cutoff=300.0, max_dynamic_distance=300.0)
+    rows = ref["stats"]["complete"]
+    assert ref["hits"]["count"] > 256 and (rows > 4096) == (atoms > 84)
+
+
+def test_unit_of_half_a_million_rows():
+    """One class of hundreds of thousands of rows: ordered within a second
+    (each row against every other would take ten)."""
+    import time
+
+    pt, ps = _one_seed_any_pair(47, 780)
+    kw = dict(rmsd_threshold=7.0, distance_cutoff=300.0, max_dynamic_distance=300.0)
+    res, ref = compare(pt, ps, **kw)
+    assert ref["hits"]["count"] > 100 and ref["stats"]["complete"] > 500000
+    t0 = time.perf_counter()
+    gpu_query(pt, ps, **kw)
+    assert time.perf_counter() - t0 < 2.0
+
+
 @pytest.mark.parametrize("atoms", [5, 33])
 @pytest.mark.parametrize("max_candidates", [0, 3])
 def test_entry_that_cannot_be_split(atoms, max_candidates):
