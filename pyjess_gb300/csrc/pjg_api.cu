@@ -2138,8 +2138,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         CUDA_TRY(read_back());
                         // entries whose children outgrew the frontier, level
                         // by level at most as deep as a template
-                        for (int pass = 0; free_n[5] > 0; pass++) {
-                            if (pass > 40) {
+                        for (int pass = 0; free_n[5] > 0 && hz[C_ERROR] == 0; pass++) {
+                            if (pass > std::min(tp->nmax, 64)) {
                                 status = fail(PJG_ERR_CAPACITY, "spilled entries did not converge");
                                 goto done;
                             }
@@ -2213,7 +2213,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     dm.resume = next_out;
                     dm.n_resume = (int32_t)ns;
                     dm.pool_in = pool_next;
-                    if (!spare) {
+                    if (round == 0 && free_chunk) {
                         CUDA_TRY(dalloc(d_susp_b, (size_t)n_pairs, st));
                         spare = d_susp_b.p;
                     }
