@@ -1373,14 +1373,29 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     FreeView fv{sp->n_kinds, (sp->n_kinds + 31) / 32, sp->d_kind_name, sp->d_kind_res, nullptr,
                 (sp->max_local_kinds + 31) / 32, nullptr, sp->d_nh_kind, sp->d_kxyz, sp->d_res_pos, sp->d_res_kind,
                 sp->d_res_range};
-    const bool free_first = P->mode != PJG_MODE_PLAIN_FP64 && demand_levels == TUNING_DEFAULTS.leaf_levels &&
+    bool free_first = P->mode != PJG_MODE_PLAIN_FP64 && demand_levels == TUNING_DEFAULTS.leaf_levels &&
                             !getenv("PJG_LEAF_LEVELS") && sp->max_local_kinds <= FREE_MAX_KINDS &&
                             (int64_t)G * fv.kind_words <= (1ll << 28);
     // few enough atoms and signatures for one chunk whatever the lists hold:
     // their total is not read back (order-free search: the lists are filled on
     // demand, and then their total is)
     constexpr int64_t LEAST_ENTRIES = 48ll << 20;
-    const bool few_entries = free_first && sp->N * (int64_t)G <= LEAST_ENTRIES && !getenv("PJG_ENTRY_BUDGET");
+    bool few_entries = free_first && sp->N * (int64_t)G <= LEAST_ENTRIES && !getenv("PJG_ENTRY_BUDGET");
+    // the lists' kind masks (up to 128 B a list, as the structure of the most
+    // kinds needs) of the whole set in the pass that counts the lists, when
+    // they take no more than mask_budget bytes; else chunk by chunk, so many
+    // structures at a time (1,000 x 4,000 pairs: 0.2 GB and 3.0 ms in one pass)
+    int64_t mask_budget = 2ll << 30;
+    if (const char *v = getenv("PJG_MASK_BUDGET"))
+        if (atoll(v) > 0) mask_budget = atoll(v);
+    const int64_t mask_bytes = 4ll * G * fv.mask_words;  // a structure's
+    bool masks_whole = free_first && (double)mask_bytes * S <= (double)mask_budget;
+    // most structures a chunk may take for the order-free search's buffers: by
+    // the masks, and for now (smaller once they did not fit, growing again)
+    int mask_cap = INT32_MAX;
+    if (free_first && !masks_whole)
+        mask_cap = (int)std::max<int64_t>(1, std::min<int64_t>(INT32_MAX, mask_budget / std::max<int64_t>(mask_bytes, 1)));
+    int free_cap = mask_cap;
     std::vector<int64_t> totals(S);
 
     if (T == 0 || S == 0) {
@@ -1460,12 +1475,21 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                    tp->d_resnames, tp->d_partner_begin, tp->d_partner_res, tp->d_partner_name};
         int blocks = (int)std::min<int64_t>((W + 7) / 8, (int64_t)sm_count() * 32);
         if (free_first) {
-            CUDA_TRY(dalloc(d_sig_bits, (size_t)G * fv.kind_words, st));
-            CUDA_TRY(dalloc(d_kind_masks, (size_t)W * fv.mask_words, st));
+            // (no room for the signatures' kinds: the search in order)
+            cudaError_t e = dalloc(d_sig_bits, (size_t)G * fv.kind_words, st);
+            if (e == cudaSuccess && masks_whole) e = dalloc(d_kind_masks, (size_t)W * fv.mask_words, st);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                free_first = few_entries = false;
+                free_cap = mask_cap = INT32_MAX;
+            } else {
+                CUDA_TRY(e);
+            }
+        }
+        if (free_first) {
             fv.sig_bits = d_sig_bits.p;
-            fv.kind_masks = d_kind_masks.p;
             launch_sig_kinds(st, sv, fv, d_sig_bits.p);
-            launch_list_kinds(st, cv, sv, fv, d_count.p, d_scanned.p, d_kind_masks.p);
+            launch_list_kinds(st, cv, sv, fv, d_count.p, d_scanned.p, masks_whole ? d_kind_masks.p : nullptr);
             launches++;
         } else {
             launch_candidates(st, std::max(blocks, 1), false, cv, sv, d_count.p, d_scanned.p, nullptr, nullptr);
@@ -1571,7 +1595,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         while (s0 < S) {
             int s1 = s0;
             int64_t entries = 0;
-            while (s1 < S && (s1 == s0 || (entries + totals[s1] <= ENTRY_BUDGET && s1 - s0 < chunk_cap))) {
+            while (s1 < S && (s1 == s0 || (entries + totals[s1] <= ENTRY_BUDGET && s1 - s0 < std::min(chunk_cap, free_cap)))) {
                 entries += totals[s1];
                 s1++;
             }
@@ -1593,10 +1617,23 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                        tp->d_resnames, tp->d_partner_begin, tp->d_partner_res, tp->d_partner_name};
             int32_t *cnt_c = d_count.p + (int64_t)s0 * G;
             int32_t *scn_c = d_scanned.p + (int64_t)s0 * G;
-            if (free_first) fv.kind_masks = d_kind_masks.p + (int64_t)s0 * G * fv.mask_words;
             CUDA_TRY(cudaEventRecord(ev[1], st));
             const int64_t n_pairs = (int64_t)Sc * T;
-            const bool free_chunk = free_first && n_pairs <= INT32_MAX - (1 << 20);
+            bool free_chunk = free_first && n_pairs <= INT32_MAX - (1 << 20);
+            if (free_chunk && masks_whole) {
+                fv.kind_masks = d_kind_masks.p + (int64_t)s0 * G * fv.mask_words;
+            } else if (free_chunk) {
+                const cudaError_t e = dalloc(d_kind_masks, (size_t)Wc * fv.mask_words, st);
+                if (e == cudaErrorMemoryAllocation) {
+                    cudaGetLastError();
+                    free_chunk = false;
+                } else {
+                    CUDA_TRY(e);
+                    fv.kind_masks = d_kind_masks.p;
+                    launch_list_kinds(st, cv, sv, fv, cnt_c, scn_c, d_kind_masks.p);
+                    launches++;
+                }
+            }
             int64_t leaf_filled = 0;  // leaf entries of the lists ordered so far
             const int fill_blocks = std::max(1, (int)std::min<int64_t>((Wc + 7) / 8, (int64_t)sm_count() * 32));
             TemplateView tv{T, tp->nmax, tp->d_atom_begin, tp->d_sig, tp->d_pos, tp->d_key, tp->d_param_begin,

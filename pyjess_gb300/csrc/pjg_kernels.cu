@@ -4105,8 +4105,8 @@ __global__ void k_sig_kinds(SigView sv, FreeView fv, uint32_t *sig_bits) {
 }
 
 // Lists of the order-free search: thread per (structure, signature), the
-// local kinds of the structure that the list takes (a bit each, kind_masks)
-// and the list's length, the sum of their atoms; `scanned` as
+// local kinds of the structure that the list takes (a bit each, kind_masks;
+// nullptr: lengths only) and the list's length, the sum of their atoms; `scanned` as
 // k_candidate_counts.  The threads of a warp share a structure, so its kinds
 // are read once for all; their signatures' bits are staged in shared memory.
 constexpr int LIST_KINDS_THREADS = 128;
@@ -4138,7 +4138,7 @@ __global__ void __launch_bounds__(LIST_KINDS_THREADS)
                     cnt += cv.nh_count[q];
                 }
             }
-            masks[w * fv.mask_words + i] = m;
+            if (masks) masks[w * fv.mask_words + i] = m;
         }
         int sc = 0;
         const int code = sv.code[g];

@@ -327,6 +327,32 @@ def test_unit_of_half_a_million_rows():
     assert time.perf_counter() - t0 < 2.0
 
 
+@pytest.mark.parametrize("structures_a_chunk", [1, 3])
+def test_kind_masks_of_a_chunk(monkeypatch, structures_a_chunk):
+    """A set with a structure of a thousand atom kinds, whose kind masks do
+    not fit a small limit: the masks chunk by chunk."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(49, [200, 90, 150, 300, 120, 60, 110])
+    s, m = structs[2], 800
+    rng = np.random.default_rng(49)
+    extra = {"xyz": s["xyz"][rng.integers(len(s["xyz"]), size=m)] + rng.normal(scale=3.0, size=(m, 3)),
+             "name": np.frombuffer(b"".join(b"X%03d" % i for i in range(m)), np.uint8).reshape(m, 4),
+             "resname": np.tile(np.frombuffer(b"LIG\0", np.uint8), (m, 1)),
+             "res_seq": np.arange(900, 900 + m, dtype=np.int32), "chain": np.tile(s["chain"][:1], (m, 1)),
+             "serial": np.arange(9000, 9000 + m, dtype=np.int32)}
+    for k, v in extra.items():
+        s[k] = np.ascontiguousarray(np.concatenate([s[k], v]))
+    pt, ps = W.pack_templates(_templates(49, structs, 40)), W.pack(structs)
+    kinds = len(np.unique(np.concatenate([s["resname"], s["name"]], 1), axis=0))
+    lists = len({(int(c), pt.names[a:b].tobytes(), pt.resnames[e:f].tobytes())
+                 for c, a, b, e, f in zip(pt.code, pt.name_offset, pt.name_offset[1:], pt.resname_offset,
+                                          pt.resname_offset[1:])})
+    monkeypatch.setenv("PJG_MASK_BUDGET", str(structures_a_chunk * lists * 4 * -(-kinds // 32)))
+    res, ref = compare(pt, ps, **PARAMS)
+    assert ref["hits"]["count"] > 0 and res.stats()["chunks"] == -(-len(structs) // structures_a_chunk)
+
+
 @pytest.mark.parametrize("atoms", [5, 33])
 @pytest.mark.parametrize("max_candidates", [0, 3])
 def test_entry_that_cannot_be_split(atoms, max_candidates):
