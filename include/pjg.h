@@ -149,8 +149,9 @@ typedef struct {
                                         with no leaf order yet (rerun)     */
     int32_t search_rounds;           /* search launches                    */
     int32_t row_splits;              /* chunks redone on fewer structures
-                                        because their complete rows did
-                                        not fit in memory                  */
+                                        because their complete rows, or
+                                        the items of their pairs, did not
+                                        fit in memory                      */
     int64_t leaf_shared;             /* of leaf_lists: lists of the same
                                         atoms as another list of their
                                         structure, sharing its leaf order  */

@@ -1149,6 +1149,10 @@ cudaError_t scan_exclusive(const T *in, int64_t n, int64_t *out, std::vector<DBu
     return cudaGetLastError();
 }
 
+// bytes of an item's arrays: its place and result, rows before it, its list of
+// segments, its levels, its counting bins
+constexpr double ITEM_BYTES = 8 + 8 + 8 + 4 + 8 + 8;
+
 // places in a query's block of counters: the statistics (Counter), the lists
 // requested in a chunk, then what an attempt at a chunk's search adds up
 enum : int {
@@ -1394,7 +1398,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     // the masks, and for now (smaller once they did not fit, growing again)
     int mask_cap = INT32_MAX;
     if (free_first && !masks_whole)
-        mask_cap = (int)std::max<int64_t>(1, std::min<int64_t>(INT32_MAX, mask_budget / std::max<int64_t>(mask_bytes, 1)));
+        mask_cap = (int)std::max<int64_t>(
+            1, std::min<int64_t>(INT32_MAX, mask_budget / std::max<int64_t>(mask_bytes, 1)));
     int free_cap = mask_cap;
     std::vector<int64_t> totals(S);
 
@@ -1546,8 +1551,11 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
         // (grown with a quarter of headroom) and the per-row stages after the
         // search (superposition, automaton, compaction and the hits they may
         // append)
-        const double row_buf_bytes = 12.0 + 4.0 * stride + (cut_inline ? 8.0 : 0.0);
-        const double row_stage_bytes = 360.0 + 4.0 * stride;
+        // (order-free search: a unit a row, and for the units put in order by
+        // their lists' leaves a key, five words of scratch and three places)
+        const double row_buf_bytes = 12.0 + 4.0 * stride + (cut_inline ? 8.0 : 0.0) +
+                                     (free_first ? (double)sizeof(RowUnit) : 0.0);
+        const double row_stage_bytes = 360.0 + 4.0 * stride + (free_first ? 40.0 : 0.0);
         // memory a chunk's rows may use: free device memory, memory the
         // stream-ordered pool holds unused, and the row buffers and per-row
         // arrays of the previous chunk (reused)
@@ -1565,6 +1573,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             }
             cudaGetLastError();
             a += (double)(d_c_pair.n * 4 + d_c_ord.n * 8 + d_c_atoms.n * 4 + d_c_rmsd.n * 8);
+            a += (double)(d_units.n * sizeof(RowUnit) + d_row_key.n * 8 + d_row_scratch.n * 4 + d_pending.n * 4 +
+                          d_large_units.n * 4);
             a += (double)(d_r_rmsd.n * 8 + d_r_rot.n * 8 + d_r_cen.n * 8 + d_r_nan.n * 4 + d_r_src.n * 8 +
                           d_r_hit.n * 4 + d_r_warn.n * 4 + d_r_hatoms.n * 4 + d_r_hidx.n * 8 + d_r_widx.n * 8 +
                           d_r_aidx.n * 8);
@@ -1586,6 +1596,15 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             bound_cap = (int)std::max(1.0, std::min((double)max_chunk, (double)row_budget() / per));
             chunk_cap = bound_cap;
         }
+        // items a chunk may hold: their arrays in an eighth of the memory its
+        // rows may use (PJG_ITEM_BUDGET sets it)
+        auto item_budget = [&](int64_t n) -> int64_t {
+            const char *v = getenv("PJG_ITEM_BUDGET");
+            if (v && atoll(v) > 0) return atoll(v);
+            if (n <= 1 << 22) return INT32_MAX;
+            return std::min<int64_t>(INT32_MAX, (int64_t)(row_memory() / 8 / ITEM_BYTES));
+        };
+        int ordered_from = -1;  // a structure searched in order: alone it outgrows the order-free search
         int s0 = 0;
         int64_t c_cap = 1 << 20;
         CUDA_TRY(dalloc(d_c_pair, c_cap, st));
@@ -1619,7 +1638,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             int32_t *scn_c = d_scanned.p + (int64_t)s0 * G;
             CUDA_TRY(cudaEventRecord(ev[1], st));
             const int64_t n_pairs = (int64_t)Sc * T;
-            bool free_chunk = free_first && n_pairs <= INT32_MAX - (1 << 20);
+            bool free_chunk = free_first && n_pairs <= INT32_MAX - (1 << 20) && s0 != ordered_from;
             if (free_chunk && masks_whole) {
                 fv.kind_masks = d_kind_masks.p + (int64_t)s0 * G * fv.mask_words;
             } else if (free_chunk) {
@@ -2003,6 +2022,16 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             // redone on half its structures
             bool split = false;
             bool invalid_rows = false;  // rows of pairs that k_search took over
+            // set when the order-free search's own buffers cannot be held: the
+            // chunk is redone on fewer structures (free_fit of them), a single
+            // structure in order
+            bool free_full = false;
+            double free_fit = 0.5;
+            auto no_room = [&](cudaError_t e) -> bool {
+                if (e != cudaErrorMemoryAllocation) return false;
+                cudaGetLastError();
+                return free_full = true;
+            };
             for (int attempt = 0; attempt < 8; attempt++) {
                 if (attempt > 0)
                     CUDA_TRY(cudaMemsetAsync(d_z.p + ZC_ATTEMPT, 0,
@@ -2034,8 +2063,10 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                                                  st));
                     CUDA_TRY(cudaEventRecord(ev[6], st));
                     if (round == 0 && free_chunk) {
-                        CUDA_TRY(dalloc(d_units, (size_t)c_cap, st));
-                        CUDA_TRY(dalloc(d_heavy_pairs, (size_t)n_pairs, st));
+                        cudaError_t er = dalloc(d_units, (size_t)c_cap, st);
+                        if (er == cudaSuccess) er = dalloc(d_heavy_pairs, (size_t)n_pairs, st);
+                        if (no_room(er)) break;
+                        CUDA_TRY(er);
                         fw.item_seeds = P->max_candidates >= 0        ? FREE_ITEM_CUT
                                         : n_pairs <= FREE_FEW_PAIRS ? FREE_ITEM_FEW
                                                                     : FREE_ITEM;
@@ -2114,24 +2145,31 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         const int64_t ns1 = (int64_t)ns;
                         const int64_t ni = (int64_t)free_n[2];
                         const int64_t nbins = (sp->max_atoms + fw.item_seeds - 1) / fw.item_seeds;
-                        if (ni > INT32_MAX) {
-                            status = fail(PJG_ERR_CAPACITY, "too many items in one chunk");
-                            goto done;
+                        const int64_t most_items = item_budget(ni);
+                        if (ni > most_items) {
+                            free_full = true;
+                            free_fit = 0.9 * (double)most_items / (double)ni;
+                            break;
                         }
                         int64_t warps = 0;
-                        CUDA_TRY(heavy_warps(fp32, ni, &warps));
-                        CUDA_TRY(dalloc(d_bins, 2 * (size_t)nbins, st));
-                        CUDA_TRY(dalloc(d_bin_off, (size_t)nbins, st));
-                        CUDA_TRY(dalloc(d_items, (size_t)ni, st));
-                        CUDA_TRY(dalloc(d_results, (size_t)ni, st));
-                        CUDA_TRY(dalloc(d_item_base, (size_t)ni, st));
-                        CUDA_TRY(dalloc(d_item_head, (size_t)ni, st));
-                        CUDA_TRY(dalloc(d_item_branch, (size_t)ni, st));
-                        CUDA_TRY(dalloc(d_spill_a, SPILL_CAP, st));
-                        CUDA_TRY(dalloc(d_heavy_stats, 4 * (size_t)nh, st));
-                        CUDA_TRY(dalloc(d_arena_xyz, (size_t)warps * HEAVY_CAP, st));
-                        CUDA_TRY(dalloc(d_arena_atom, (size_t)warps * HEAVY_CAP, st));
-                        CUDA_TRY(dalloc(d_arena_parent, 2 * (size_t)warps * HEAVY_CAP, st));
+                        cudaError_t er = heavy_warps(fp32, ni, &warps);
+                        auto room = [&](auto &buf, int64_t n) {
+                            if (er == cudaSuccess) er = dalloc(buf, (size_t)n, st);
+                        };
+                        room(d_bins, 2 * nbins);
+                        room(d_bin_off, nbins);
+                        room(d_items, ni);
+                        room(d_results, ni);
+                        room(d_item_base, ni);
+                        room(d_item_head, ni);
+                        room(d_item_branch, ni);
+                        room(d_spill_a, SPILL_CAP);
+                        room(d_heavy_stats, 4 * (int64_t)nh);
+                        room(d_arena_xyz, warps * HEAVY_CAP);
+                        room(d_arena_atom, warps * HEAVY_CAP);
+                        room(d_arena_parent, 2 * warps * HEAVY_CAP);
+                        if (no_room(er)) break;
+                        CUDA_TRY(er);
                         CUDA_TRY(cudaMemsetAsync(d_bins.p, 0, 2 * (size_t)nbins * sizeof(int32_t), st));
                         CUDA_TRY(cudaMemsetAsync(d_results.p, 0xFF, (size_t)ni * sizeof(int2), st));
                         CUDA_TRY(cudaMemsetAsync(d_item_head.p, 0xFF, (size_t)ni * sizeof(int32_t), st));
@@ -2182,15 +2220,17 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                             }
                             fw.n_items = (int32_t)free_n[5];
                             if (pass > 0) std::swap(d_spill_a, d_spill_b);
-                            CUDA_TRY(dalloc(d_spill_b, SPILL_CAP, st));
+                            CUDA_TRY(heavy_warps(fp32, fw.n_items, &warps));
+                            room(d_spill_b, SPILL_CAP);
+                            room(d_arena_xyz, warps * HEAVY_CAP);
+                            room(d_arena_atom, warps * HEAVY_CAP);
+                            room(d_arena_parent, 2 * warps * HEAVY_CAP);
+                            if (no_room(er)) break;
+                            CUDA_TRY(er);
                             fw.spilled_in = d_spill_a.p;
                             fw.spilled_out = d_spill_b.p;
                             CUDA_TRY(cudaMemsetAsync(fw.n_spilled, 0, sizeof(unsigned long long), st));
                             CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
-                            CUDA_TRY(heavy_warps(fp32, fw.n_items, &warps));
-                            CUDA_TRY(dalloc(d_arena_xyz, (size_t)warps * HEAVY_CAP, st));
-                            CUDA_TRY(dalloc(d_arena_atom, (size_t)warps * HEAVY_CAP, st));
-                            CUDA_TRY(dalloc(d_arena_parent, 2 * (size_t)warps * HEAVY_CAP, st));
                             fw.arena_xyz = d_arena_xyz.p;
                             fw.arena_atom = d_arena_atom.p;
                             fw.arena_parent = d_arena_parent.p;
@@ -2201,6 +2241,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                             CUDA_TRY(cudaGetLastError());
                             CUDA_TRY(read_back());
                         }
+                        if (free_full) break;
                         launch_heavy_rows(st, nh, fw, d_item_base.p, d_pair_rows.p, d_counters.p);
                         launches++;
                         if ((int64_t)ns > ns1) {
@@ -2216,7 +2257,9 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     if (round == 0 && free_chunk && free_n[0] && (int64_t)nc <= c_cap) {
                         // the rows found without order, in the reference's;
                         // units it leaves wait for their lists' leaf order
-                        CUDA_TRY(dalloc(d_pending, 2 * (size_t)free_n[0], st));
+                        const cudaError_t er = dalloc(d_pending, 2 * (size_t)free_n[0], st);
+                        if (no_room(er)) break;
+                        CUDA_TRY(er);
                         fw.pending = d_pending.p;
                         fw.long_units = d_pending.p + free_n[0];
                         CUDA_TRY(launch_unit_order_direct(st, (int64_t)free_n[0], cv, tv, cd, sv, fv, sp->d_res_place,
@@ -2257,11 +2300,14 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     std::swap(next_out, spare);
                     std::swap(pool_next, pool_spare);
                 }
+                if (free_full) break;
                 if ((int64_t)nc <= c_cap) {
                     if (free_chunk && free_n[6]) {
-                        CUDA_TRY(dalloc(d_row_key, (size_t)nc, st));
-                        CUDA_TRY(dalloc(d_row_scratch, 5 * (size_t)nc, st));
-                        CUDA_TRY(dalloc(d_large_units, (size_t)free_n[6], st));
+                        cudaError_t er = dalloc(d_row_key, (size_t)nc, st);
+                        if (er == cudaSuccess) er = dalloc(d_row_scratch, 5 * (size_t)nc, st);
+                        if (er == cudaSuccess) er = dalloc(d_large_units, (size_t)free_n[6], st);
+                        if (no_room(er)) break;
+                        CUDA_TRY(er);
                         fw.row_key = d_row_key.p;
                         fw.row_scratch = d_row_scratch.p;
                         fw.large_units = d_large_units.p;
@@ -2308,6 +2354,17 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     CUDA_TRY(cudaMemcpyAsync(d_counters.p, snap, sizeof snap, cudaMemcpyHostToDevice, st));
                     CUDA_TRY(cudaStreamSynchronize(st));
                 }
+            }
+            if (free_full) {
+                if (Sc > 1) free_cap = std::max(1, std::min(Sc / 2, (int)(free_fit * Sc)));
+                else ordered_from = s0;
+                chunks--;
+                row_splits++;
+                search_rounds = search_rounds0;
+                suspensions = suspensions0;
+                ms_search = ms_search_chunk0;
+                CUDA_TRY(cudaMemcpyAsync(d_counters.p, d_z.p + ZC_CHUNK, stats_bytes, cudaMemcpyDeviceToDevice, st));
+                continue;
             }
             CUDA_TRY(cudaEventRecord(ev[3], st));
             {
@@ -2422,6 +2479,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     chunk_cap = max_chunk;
                 }
                 chunk_cap = std::max(chunk_cap, std::min(bound_cap, max_chunk));
+                free_cap = free_cap < mask_cap / 2 ? 2 * free_cap : mask_cap;
             }
             s0 = s1;
         }

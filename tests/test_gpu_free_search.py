@@ -327,6 +327,23 @@ def test_unit_of_half_a_million_rows():
     assert time.perf_counter() - t0 < 2.0
 
 
+@pytest.mark.parametrize("budget", ["1", "60"])
+@pytest.mark.parametrize("kw", [dict(), dict(max_candidates=5), dict(best_match=True, max_candidates=7)])
+def test_more_items_than_room(monkeypatch, budget, kw):
+    """Chunks with more items than there is room for are redone on fewer
+    structures, a single structure in order: nothing is refused."""
+    from pyjess_gb300 import workloads as W
+
+    monkeypatch.setenv("PJG_ITEM_BUDGET", budget)
+    structs = _structures(48, [900, 60, 1500, 700, 800])
+    specs = _templates(48, structs, 24, hi=5)
+    specs += [_cut(t, 34) for t in _templates(48, structs, 2, lo=12, hi=13, radius=16.0)]
+    res, ref = compare(W.pack_templates(specs), W.pack(structs), rmsd_threshold=1.6, distance_cutoff=2.2,
+                       max_dynamic_distance=2.2, **kw)
+    st = res.stats()
+    assert ref["hits"]["count"] > 0 and st["row_splits"] > 0 and st["chunks"] > 1
+
+
 @pytest.mark.parametrize("structures_a_chunk", [1, 3])
 def test_kind_masks_of_a_chunk(monkeypatch, structures_a_chunk):
     """A set with a structure of a thousand atom kinds, whose kind masks do
