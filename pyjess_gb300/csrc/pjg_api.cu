@@ -206,15 +206,92 @@ struct Scratch {
     }
 };
 
-// a handle's or a result's device block back to its device's pool
-void free_block(void *block, int device) {
-    if (!block) return;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev != device) cudaSetDevice(device);
-    cudaFreeAsync(block, nullptr);
-    if (dev != device) cudaSetDevice(dev);
-}
+// Memory of handles and results (and of the arrays a structure upload needs
+// meanwhile): a pool of their own on each device, which keeps OBJECT_KEEP bytes
+// beyond the live blocks for the next ones and gives the rest back to the
+// device: at the next wait of any stream, and as soon as a block of
+// OBJECT_PROMPT bytes is freed.  (The pool of the queries' buffers keeps up to
+// half the device.)
+constexpr size_t OBJECT_KEEP = 256 << 20, OBJECT_PROMPT = 64 << 20;
+
+struct ObjectPool {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long ctx = 0;  // the context it belongs to
+    size_t live = 0;             // bytes of its blocks
+    uint64_t threshold = 0;      // what it may hold (set anew when live has
+};                               //   moved by a quarter of OBJECT_KEEP)
+std::mutex g_object_mutex;
+ObjectPool g_object_pool[256];   // guarded by g_object_mutex
+
+struct Block {
+    void *p = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+    unsigned long long ctx = 0;
+
+    cudaError_t alloc(size_t n, cudaStream_t st) {
+        bytes = std::max<size_t>(n, 1);
+        ctx = current_context_id();
+        cudaError_t e = cudaGetDevice(&device);
+        if (e != cudaSuccess) return e;
+        if (device >= 256) return cudaErrorInvalidDevice;
+        std::lock_guard<std::mutex> g(g_object_mutex);
+        ObjectPool &o = g_object_pool[device];
+        if (!o.pool || o.ctx != ctx) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            o = ObjectPool{};
+            e = cudaMemPoolCreate(&o.pool, &props);
+            if (e != cudaSuccess) return e;
+            o.ctx = ctx;
+        }
+        e = cudaMallocFromPoolAsync(&p, bytes, o.pool, st);
+        if (e == cudaErrorMemoryAllocation) {
+            // what the queries' pool holds unused may make the room
+            cudaGetLastError();
+            cudaMemPool_t q;
+            if (cudaDeviceGetDefaultMemPool(&q, device) == cudaSuccess) cudaMemPoolTrimTo(q, 0);
+            e = cudaMallocFromPoolAsync(&p, bytes, o.pool, st);
+        }
+        if (e != cudaSuccess) {
+            p = nullptr;
+            return e;
+        }
+        o.live += bytes;
+        limit(o);
+        return e;
+    }
+    // in the order of `st` (nullptr: now); nothing to do once its context is gone
+    void free(cudaStream_t st = nullptr) {
+        if (!p) return;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev != device) cudaSetDevice(device);
+        if (current_context_id() == ctx) {
+            cudaFreeAsync(p, st);
+            if (bytes >= OBJECT_PROMPT && !st) cudaStreamSynchronize(nullptr);
+            std::lock_guard<std::mutex> g(g_object_mutex);
+            ObjectPool &o = g_object_pool[device];
+            if (o.pool && o.ctx == ctx) {
+                o.live -= bytes;
+                limit(o);
+                if (bytes >= OBJECT_PROMPT && !st) cudaMemPoolTrimTo(o.pool, o.live + OBJECT_KEEP);
+            }
+        }
+        if (dev != device) cudaSetDevice(dev);
+        p = nullptr;
+    }
+
+private:
+    static void limit(ObjectPool &o) {
+        const uint64_t most = o.live + OBJECT_KEEP;
+        if (o.threshold <= most + OBJECT_KEEP / 4 && most <= o.threshold + OBJECT_KEEP / 4) return;
+        o.threshold = most;
+        cudaMemPoolSetAttribute(o.pool, cudaMemPoolAttrReleaseThreshold, &o.threshold);
+    }
+};
 
 constexpr size_t IDLE_MAX = 8, CACHE_MAX = 64 << 20;
 std::mutex g_scratch_mutex;
@@ -240,6 +317,7 @@ Scratch *acquire_scratch(int device, cudaError_t *e) {
     if (*e == cudaSuccess) return x;
     x->destroy();
     delete x;
+    cudaGetLastError();  // (reported here; a later call does not meet it)
     return nullptr;
 }
 
@@ -313,23 +391,20 @@ struct Upload {
         items.push_back({(void **)dst, nullptr, std::max<size_t>(n, 1) * sizeof(T), total});
         total += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
     }
-    // allocates *block and fills it on x's stream (arrays with a source
+    // allocates `block` and fills it on x's stream (arrays with a source
     // first, so that they share one copy)
-    cudaError_t run(void **block, Scratch *x) {
-        cudaError_t e = cudaMallocAsync(block, std::max<size_t>(total, 1), x->st);
-        if (e != cudaSuccess) {
-            *block = nullptr;
-            return e;
-        }
+    cudaError_t run(Block *block, Scratch *x) {
+        cudaError_t e = block->alloc(total, x->st);
+        if (e != cudaSuccess) return e;
         size_t filled = 0;
         for (const Item &it : items) {
-            *it.dst = (char *)*block + it.at;
+            *it.dst = (char *)block->p + it.at;
             if (it.src) filled = it.at + it.bytes;
         }
         if (filled <= Scratch::PINNED) {
             for (const Item &it : items)
                 if (it.src) std::memcpy(x->pinned + it.at, it.src, it.bytes);
-            return cudaMemcpyAsync(*block, x->pinned, filled, cudaMemcpyHostToDevice, x->st);
+            return cudaMemcpyAsync(block->p, x->pinned, filled, cudaMemcpyHostToDevice, x->st);
         }
         for (const Item &it : items)
             if (it.src && e == cudaSuccess)
@@ -384,7 +459,7 @@ struct pjg_templates {
     // of them, those of at most 64 (order-free search) and the larger ones
     std::vector<int32_t> large, wide, huge;
     int32_t *d_large = nullptr, *d_wide = nullptr, *d_huge = nullptr;
-    void *block = nullptr;  // the device arrays
+    Block block;            // the device arrays
     bool counted = false;   // a live handle
 };
 
@@ -419,7 +494,7 @@ struct pjg_structures {
     uint16_t *d_res_kind = nullptr;
     int4 *d_res_range = nullptr;
     int device = 0;
-    void *block = nullptr;  // the device arrays
+    Block block;            // the device arrays
     bool counted = false;   // a live handle
 };
 
@@ -432,14 +507,44 @@ struct HitStore {
     int64_t *ordinal = nullptr, *atom_offset = nullptr, *warn_before = nullptr;
     double *rmsd = nullptr, *rot = nullptr, *centres = nullptr;
 
-    void *block = nullptr;                            // the arrays
+    Block block;                                      // the arrays
 
-    // room for `h` more hits, `a` more atoms, `w` more warnings
+    // room for `h` more hits, `a` more atoms, `w` more warnings: twice what
+    // there is, or, where that cannot be had, what is needed
     cudaError_t reserve(int64_t h, int64_t a, int64_t w, cudaStream_t st) {
-        if (block && hits + h <= cap_h && atoms + a <= cap_a && warns + w <= cap_w) return cudaSuccess;
+        if (block.p && hits + h <= cap_h && atoms + a <= cap_a && warns + w <= cap_w) return cudaSuccess;
         auto bigger = [](int64_t need, int64_t cap) { return need <= cap ? cap : std::max<int64_t>(need, 2 * cap); };
-        const int64_t nh = bigger(hits + h, cap_h), na = bigger(atoms + a, cap_a), nw = bigger(warns + w, cap_w);
-        HitStore old = *this;
+        int64_t nh = bigger(hits + h, cap_h), na = bigger(atoms + a, cap_a), nw = bigger(warns + w, cap_w);
+        Block fresh;
+        Upload lay = layout(nh, na, nw);
+        cudaError_t e = fresh.alloc(lay.total, st);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            nh = hits + h;
+            na = atoms + a;
+            nw = warns + w;
+            lay = layout(nh, na, nw);
+            e = fresh.alloc(lay.total, st);
+        }
+        if (e != cudaSuccess) return e;
+        // (what each array holds, in the order of layout)
+        const int64_t used[] = {4 * hits, 4 * hits, 8 * hits, 8 * hits, 72 * hits, 48 * hits, 8 * hits,
+                                4 * atoms, 4 * warns, 8 * warns};
+        for (size_t i = 0; i < lay.items.size(); i++) {
+            const Upload::Item &it = lay.items[i];
+            char *to = (char *)fresh.p + it.at;
+            if (e == cudaSuccess && block.p && used[i] > 0)
+                e = cudaMemcpyAsync(to, *it.dst, (size_t)used[i], cudaMemcpyDeviceToDevice, st);
+            *it.dst = to;
+        }
+        block.free(st);
+        block = fresh;
+        cap_h = nh;
+        cap_a = na;
+        cap_w = nw;
+        return e;
+    }
+    Upload layout(int64_t nh, int64_t na, int64_t nw) {
         Upload lay;
         lay.room(&structure, (size_t)nh);
         lay.room(&tpl, (size_t)nh);
@@ -451,34 +556,7 @@ struct HitStore {
         lay.room(&atoms_, (size_t)na);
         lay.room(&warn_structure, (size_t)nw);
         lay.room(&warn_before, (size_t)nw);
-        void *b = nullptr;
-        cudaError_t e = cudaMallocAsync(&b, std::max<size_t>(lay.total, 1), st);
-        if (e != cudaSuccess) {
-            old.block = nullptr;  // (still this store's)
-            return e;
-        }
-        for (const Upload::Item &it : lay.items) *it.dst = (char *)b + it.at;
-        block = b;
-        cap_h = nh;
-        cap_a = na;
-        cap_w = nw;
-        auto keep = [&](void *to, const void *from, int64_t bytes) {
-            if (e == cudaSuccess && from && bytes > 0)
-                e = cudaMemcpyAsync(to, from, (size_t)bytes, cudaMemcpyDeviceToDevice, st);
-        };
-        keep(structure, old.structure, 4 * hits);
-        keep(tpl, old.tpl, 4 * hits);
-        keep(ordinal, old.ordinal, 8 * hits);
-        keep(rmsd, old.rmsd, 8 * hits);
-        keep(rot, old.rot, 72 * hits);
-        keep(centres, old.centres, 48 * hits);
-        keep(atom_offset, old.atom_offset, 8 * hits);
-        keep(atoms_, old.atoms_, 4 * atoms);
-        keep(warn_structure, old.warn_structure, 4 * warns);
-        keep(warn_before, old.warn_before, 8 * warns);
-        if (old.block) cudaFreeAsync(old.block, st);
-        old.block = nullptr;
-        return e;
+        return lay;
     }
     // the segment view at the current ends
     HitSegment tail() const {
@@ -486,9 +564,7 @@ struct HitStore {
                           centres + 6 * hits, atom_offset + hits, atoms_ + atoms, warn_structure + warns,
                           warn_before + warns};
     }
-    ~HitStore() {
-        if (block) cudaFreeAsync(block, nullptr);
-    }
+    ~HitStore() { block.free(); }
 };
 
 struct pjg_results {
@@ -798,7 +874,7 @@ pjg_status pjg_templates_create(const pjg_template_set *set, pjg_templates **out
 
 void pjg_templates_destroy(pjg_templates *h) {
     if (!h) return;
-    free_block(h->block, h->device);
+    h->block.free();
     if (h->counted) handle_destroyed();
     delete h;
 }
@@ -1056,21 +1132,18 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
     if (e == cudaSuccess) {
         // axis ranks of every atom (the leaf-order sorted-axis path), and the
         // residue order and kind-ordered points of the order-free search
-        DBuf<unsigned long long> tile_key;
-        DBuf<uint16_t> tile_idx;
-        t_cache = &x->cache;
-        e = dalloc(tile_key, 4 * n1, x->st);
-        if (e == cudaSuccess) e = dalloc(tile_idx, 4 * n1, x->st);
+        Block tiles;
+        e = tiles.alloc((sizeof(unsigned long long) + sizeof(uint16_t)) * 4 * n1, x->st);
         if (e == cudaSuccess) {
-            launch_axis_ranks(x->st, S, h->max_atoms, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key.p, tile_idx.p,
-                              h->d_lrank, h->d_urank,
+            unsigned long long *tile_key = (unsigned long long *)tiles.p;
+            uint16_t *tile_idx = (uint16_t *)(tile_key + 4 * n1);
+            launch_axis_ranks(x->st, S, h->max_atoms, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key,
+                              tile_idx, h->d_lrank, h->d_urank,
                               ResidueOrder{h->d_xyz32, h->d_nh_pos, d_local_kind, h->d_kxyz, h->d_res_pos,
                                            h->d_res_kind, h->d_res_range, h->d_sorted, h->d_res_place});
             e = cudaGetLastError();
         }
-        dfree(tile_key, x->st);
-        dfree(tile_idx, x->st);
-        t_cache = nullptr;
+        tiles.free(x->st);
         const cudaError_t e2 = cudaStreamSynchronize(x->st);
         if (e == cudaSuccess) e = e2;
     }
@@ -1091,7 +1164,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
 
 void pjg_structures_destroy(pjg_structures *h) {
     if (!h) return;
-    free_block(h->block, h->device);
+    h->block.free();
     if (h->counted) handle_destroyed();
     delete h;
 }
