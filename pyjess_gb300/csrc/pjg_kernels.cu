@@ -6545,7 +6545,7 @@ void launch_gather_hits(cudaStream_t st, int64_t n_rows, int32_t n_templates, in
 //
 // Bound by the FP64 pipe (about 30 operations an atom for the covariance,
 // the rest for the 4 x 4 eigen-solve): a thread per row keeps every lane of
-// it busy.  Measured at 300,000 rows of 12 atoms: 0.41 ms; 9.58 ms with a
+// it busy.  Measured at 300,000 rows of 12 atoms: 0.40 ms; 9.58 ms with a
 // warp per row (one lane in the eigen-solve) and the compaction in one block.
 
 static __device__ __align__(256) uint32_t g_noalloc_words[PJG_NOALLOC_MAX_ROWS / 32];
@@ -6553,33 +6553,102 @@ static __device__ __align__(256) uint32_t g_noalloc_words[PJG_NOALLOC_MAX_ROWS /
 constexpr int SUPERPOSE_ROWS_THREADS = 64;  // small blocks: a few thousand rows already reach every SM
 constexpr int COMPACT_THREADS = 256;        // a block compacts 32 words (1,024 rows)
 
+// K sums over up to 32 atoms, as a tree: in a group of four atoms the even and
+// the odd ones, their sum, then the groups in pairs (as many roundings as a
+// warp's butterfly; two running sums lost up to 1.7 times as much in the
+// centres of 17 to 32 atoms).  add(v, k) adds atom k's terms to v.
+template <int K, typename Add>
+__device__ __forceinline__ void tree_sum(int n, double (&out)[K], Add add) {
+    double s0[K], s1[K], s2[K], v[K], w[K];  // s: sums of one, two and four groups to the left
+    // group g's sum in v merged with what stands to its left
+    auto merge = [&](int g) {
+#pragma unroll
+        for (int q = 0; q < K; q++) v[q] += w[q];
+        if (g & 1) {
+#pragma unroll
+            for (int q = 0; q < K; q++) v[q] += s0[q];
+            if (g & 2) {
+#pragma unroll
+                for (int q = 0; q < K; q++) v[q] += s1[q];
+                if (g & 4) {
+#pragma unroll
+                    for (int q = 0; q < K; q++) v[q] += s2[q];
+                } else {
+#pragma unroll
+                    for (int q = 0; q < K; q++) s2[q] = v[q];
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < K; q++) s1[q] = v[q];
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < K; q++) s0[q] = v[q];
+        }
+    };
+    auto zero = [&]() {
+#pragma unroll
+        for (int q = 0; q < K; q++) v[q] = w[q] = 0.0;
+    };
+    const int whole = n >> 2, rest = n & 3;
+    for (int g = 0; g < whole; g++) {
+        zero();
+        add(v, 4 * g);
+        add(w, 4 * g + 1);
+        add(v, 4 * g + 2);
+        add(w, 4 * g + 3);
+        merge(g);
+    }
+    if (rest) {
+        zero();
+        add(v, 4 * whole);
+        if (rest > 1) add(w, 4 * whole + 1);
+        if (rest > 2) add(v, 4 * whole + 2);
+        merge(whole);
+    }
+    const int groups = (n + 3) >> 2;  // (eight: all in v)
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        double r = groups == 8 ? v[q] : 0.0;
+        if (groups & 1) r = s0[q];
+        if (groups & 2) r = s1[q] + r;
+        if (groups & 4) r = s2[q] + r;
+        out[q] = r;
+    }
+}
+
 __global__ void __launch_bounds__(SUPERPOSE_ROWS_THREADS)
     k_superpose_rows(const double *mol_xyz, const double *tpl_xyz, int32_t n_rows, int32_t n, double rmsd_threshold,
                      double *rmsd_out, double *rot_out, double *cen_out, uint32_t *words) {
     __shared__ double cb[3];      // template centroid
     __shared__ double tb[32][3];  // centred template atoms
+    __shared__ double sumB;       // their square sum
     if (threadIdx.x < 3) {
-        double acc = 0.0;
-        for (int k = 0; k < n; k++) acc += tpl_xyz[3 * k + threadIdx.x];
-        cb[threadIdx.x] = acc / (double)n;
+        double c[1];
+        tree_sum(n, c, [&](double (&v)[1], int k) { v[0] += tpl_xyz[3 * k + threadIdx.x]; });
+        cb[threadIdx.x] = c[0] / (double)n;
     }
     __syncthreads();
     for (int q = threadIdx.x; q < 3 * n; q += blockDim.x) tb[q / 3][q % 3] = tpl_xyz[q] - cb[q % 3];
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int k = threadIdx.x;
+        const double sb = warp_sum(k < n ? tb[k][0] * tb[k][0] + tb[k][1] * tb[k][1] + tb[k][2] * tb[k][2] : 0.0);
+        if (k == 0) sumB = sb;
+    }
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool pass = false;
     if (i < n_rows) {
         const double *x = mol_xyz + i * 3 * n;
+        double ca[3], P[2][9] = {}, pA[2] = {}, S[9];
+        tree_sum(n, ca, [&](double (&v)[3], int k) {
+            for (int d = 0; d < 3; d++) v[d] += x[3 * k + d];
+        });
+        for (int d = 0; d < 3; d++) ca[d] /= (double)n;
         // two partial sums each (even and odd atoms): shorter dependence
-        // chains, and rounding nearer a tree's than a chain's
-        double ca[3], cp[2][3] = {}, P[2][9] = {}, pA[2] = {}, pB[2] = {}, S[9];
-#pragma unroll 2
-        for (int k = 0; k < n; k += 2)
-            for (int d = 0; d < 3; d++) {
-                cp[0][d] += x[3 * k + d];
-                if (k + 1 < n) cp[1][d] += x[3 * k + 3 + d];
-            }
-        for (int d = 0; d < 3; d++) ca[d] = (cp[0][d] + cp[1][d]) / (double)n;
+        // chains.  (As a tree they are no nearer to the exact fit and 7% of
+        // the time dearer.)
 #pragma unroll 2
         for (int k = 0; k < n; k += 2)
 #pragma unroll
@@ -6589,12 +6658,11 @@ __global__ void __launch_bounds__(SUPERPOSE_ROWS_THREADS)
                              a2 = x[3 * (k + h) + 2] - ca[2];
                 const double b0 = tb[k + h][0], b1 = tb[k + h][1], b2 = tb[k + h][2];
                 pA[h] += a0 * a0 + a1 * a1 + a2 * a2;
-                pB[h] += b0 * b0 + b1 * b1 + b2 * b2;
                 P[h][0] += a0 * b0; P[h][1] += a0 * b1; P[h][2] += a0 * b2;
                 P[h][3] += a1 * b0; P[h][4] += a1 * b1; P[h][5] += a1 * b2;
                 P[h][6] += a2 * b0; P[h][7] += a2 * b1; P[h][8] += a2 * b2;
             }
-        const double sumA = pA[0] + pA[1], sumB = pB[0] + pB[1];
+        const double sumA = pA[0] + pA[1];
         for (int q = 0; q < 9; q++) S[q] = P[0][q] + P[1][q];
         double rmsd = 0.0, R[9];
         bool bad = false;

@@ -138,3 +138,28 @@ def test_superpose_noalloc_row_edges(rows, atoms):
     if rows and atoms >= 4:  # (well separated singular values: a defined rotation)
         ok = (sv[:, 1] + sign[:, 2] * sv[:, 2]) > 1e-3 * sv[:, 0]
         assert np.abs(rot.cpu().numpy().reshape(rows, 3, 3) - R)[ok].max() <= ROT_TOL
+
+
+@pytest.mark.parametrize("atoms", [5, 12, 17, 31, 32])
+def test_superpose_noalloc_centres_are_tree_sums(atoms):
+    """One coordinate of 1 among ones of 2^-53, which a running sum loses one
+    by one: the centres are within the roundings of a tree of the atoms (five
+    additions on the way of any of them, then the division)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    L = _bind()
+    u = 2.0 ** -53
+    mol = np.full((atoms, atoms, 3), u)  # row r: the 1 at atom r
+    mol[np.arange(atoms), np.arange(atoms)] = 1.0
+    exact = (1 + (atoms - 1) * 2.0 ** -53) / atoms  # (in units of the last place: the roundings below cover its own)
+    dev = torch.device("cuda")
+    d = [torch.tensor(mol.reshape(-1), device=dev), torch.tensor(mol[0].reshape(-1), device=dev)]
+    rmsd, rot, cen = (torch.zeros(k * atoms, dtype=torch.float64, device=dev) for k in (1, 9, 6))
+    idx, count = (torch.zeros(k, dtype=torch.int32, device=dev) for k in (atoms, 1))
+    st = L.pjg_superpose_noalloc(d[0].data_ptr(), d[1].data_ptr(), atoms, atoms, 1.0, rmsd.data_ptr(), rot.data_ptr(),
+                                 cen.data_ptr(), idx.data_ptr(), count.data_ptr(), None)
+    assert st == 0, L.pjg_noalloc_last_error()
+    torch.cuda.synchronize()
+    err = np.abs(cen.cpu().numpy().reshape(atoms, 6) - exact).max()
+    assert err <= (5 * u * (1 + atoms * u) + 2 * u) / atoms, err * atoms / u
