@@ -6622,7 +6622,6 @@ __global__ void __launch_bounds__(SUPERPOSE_ROWS_THREADS)
                      double *rmsd_out, double *rot_out, double *cen_out, uint32_t *words) {
     __shared__ double cb[3];      // template centroid
     __shared__ double tb[32][3];  // centred template atoms
-    __shared__ double sumB;       // their square sum
     if (threadIdx.x < 3) {
         double c[1];
         tree_sum(n, c, [&](double (&v)[1], int k) { v[0] += tpl_xyz[3 * k + threadIdx.x]; });
@@ -6631,12 +6630,9 @@ __global__ void __launch_bounds__(SUPERPOSE_ROWS_THREADS)
     __syncthreads();
     for (int q = threadIdx.x; q < 3 * n; q += blockDim.x) tb[q / 3][q % 3] = tpl_xyz[q] - cb[q % 3];
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const int k = threadIdx.x;
-        const double sb = warp_sum(k < n ? tb[k][0] * tb[k][0] + tb[k][1] * tb[k][1] + tb[k][2] * tb[k][2] : 0.0);
-        if (k == 0) sumB = sb;
-    }
-    __syncthreads();
+    // (by each warp: no third barrier)
+    const int b = lane_id();
+    const double sumB = warp_sum(b < n ? tb[b][0] * tb[b][0] + tb[b][1] * tb[b][1] + tb[b][2] * tb[b][2] : 0.0);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool pass = false;
     if (i < n_rows) {
