@@ -403,6 +403,40 @@ def test_cut_items_give_the_same_stream_every_time():
         assert hit_keys(gpu_query(pt, ps, **kw).arrays()) == want
 
 
+@pytest.mark.parametrize("mode", ["fp32", "fp64"])
+def test_pair_handed_over_after_rows_of_it_were_written(mode):
+    """Twelve ligands, ten of them alone among 30 atoms and the last two in a
+    cluster of 8,500: the first item of the pair writes its rows, the second
+    meets entries with more children than a frontier holds, and the pair goes
+    to the search in order.  Rows and counters are those of one search."""
+    from pyjess_gb300 import workloads as W
+
+    rng = np.random.default_rng(53)
+    ball = lambda n: (lambda v: v / np.linalg.norm(v, axis=1)[:, None] * rng.uniform(2, 28, (n, 1)))(
+        rng.normal(size=(n, 3)))
+    centres = np.zeros((12, 3))
+    centres[:10, 0] = 1000.0 * np.arange(1, 11)
+    centres[10:] = [[0.4, 0.0, 0.0], [-0.4, 0.3, 0.1]]
+    ligand = np.array([[0.0, 0.0, 0.0], [1.5, 0.0, 0.2], [0.1, 1.4, 0.3]])
+    xyz = np.concatenate([(centres[:, None] + ligand).reshape(-1, 3)] + [centres[i] + ball(30) for i in range(10)] +
+                         [ball(8500)])
+    n = len(xyz)
+    raw = lambda parts, width: np.frombuffer(b"".join(parts), np.uint8).reshape(-1, width).copy()
+    s = {"xyz": np.round(xyz, 3), "name": raw([b"_ZZ__YY__XX_"] * 12 + [b"_CA_"] * (n - 36), 4),
+         "resname": raw([b"LIG\0"] * 36 + [b"ALA\0"] * (n - 36), 4), "chain": raw([b" A"] * n, 2),
+         "res_seq": np.concatenate([np.repeat(np.arange(1, 13), 3), np.arange(100, 100 + n - 36)]).astype(np.int32),
+         "serial": np.arange(1, n + 1, dtype=np.int32)}
+    spec = W.TemplateSpec(code=[0] * 4, res_seq=[1, 1, 1, 2], chain=[b" A"] * 4,
+                          xyz=[*ligand, np.array([9.0, 8.0, 7.0])], weight=[0.0] * 4,
+                          names=[[b"_ZZ_"], [b"_YY_"], [b"_XX_"], [b"_CA_"]],
+                          resnames=[[b"LIG\0"]] * 3 + [[b"ALA\0"]])
+    res, ref = compare(W.pack_templates([spec]), W.pack([s]), mode=mode, rmsd_threshold=5.0, distance_cutoff=20.0,
+                       max_dynamic_distance=20.0)
+    st = res.stats()
+    assert ref["stats"]["complete"] > 17000 and 0 < ref["hits"]["count"] < ref["stats"]["complete"]
+    assert st["search_rounds"] == 2 and st["suspensions"] == 1
+
+
 @pytest.mark.parametrize("max_candidates", [0, 1, 4, 30, 31, 32, 33, 63, 200])
 @pytest.mark.parametrize("threshold", [0.75, 1.2])
 def test_streams_cut_within_a_step(max_candidates, threshold):

@@ -347,6 +347,25 @@ def test_heavy_pairs_first(monkeypatch, heavy):
     compare(wl.templates, wl.structures, mode="fp32", **wl.params)
 
 
+@pytest.mark.parametrize("heavy", ["1", "0"])
+def test_heavy_pairs_first_in_the_search_in_order(monkeypatch, heavy):
+    """As test_heavy_pairs_first with the levels to order chosen, so that the
+    search in order takes the pairs (its cost histogram and heavy list, two
+    launches more than without)."""
+    from pyjess_gb300 import workloads as W
+
+    monkeypatch.setenv("PJG_HEAVY_PER_WARP", "1")
+    monkeypatch.setenv("PJG_LEAF_LEVELS", "4")
+    monkeypatch.setenv("PJG_HEAVY_FIRST", heavy)
+    wl = W.config(3, n_structures=70, n_templates=300)
+    res, _ = compare(wl.templates, wl.structures, mode="fp32", **wl.params)
+    launches = res.stats()["launches"]
+    monkeypatch.setenv("PJG_HEAVY_FIRST", "0")
+    other = gpu_query(wl.templates, wl.structures, mode="fp32", **wl.params)
+    assert hit_keys(other.arrays()) == hit_keys(res.arrays())
+    assert launches - other.stats()["launches"] == (2 if heavy == "1" else 0)
+
+
 @pytest.mark.parametrize("levels", [3, 10])
 def test_leaf_order_up_front_levels_without_reorder(monkeypatch, levels):
     """Template atoms taken in their own order (reorder=False) with 3 and
