@@ -258,21 +258,23 @@ void pjg_results_destroy(pjg_results *r);
  * (pyjess_gb300/tune.py) measures them on a sample of a workload and sets
  * the fastest.  Process-wide: each pjg_query reads the values in force when
  * it starts.  A field of 0 keeps the built-in default.
- *   leaf_levels    levels (after level 0) whose candidate lists are put in
- *                  kd leaf order before the search; deeper lists when a
- *                  pair first reaches them (default 4; -1 every list up
- *                  front; the plain FP64 mode always orders every list).
- *                  At the default the batched modes search every pair
+ *   leaf_levels    0 (the default): the batched modes search every pair
  *                  without any order first and order only the lists that
- *                  tell a pair's rows apart; another value searches every
- *                  pair in order
+ *                  tell a pair's rows apart.  Another value searches every
+ *                  pair in order: the levels (after level 0) whose candidate
+ *                  lists are put in kd leaf order before the search, deeper
+ *                  lists when a pair first reaches them (-1 every list up
+ *                  front, as the plain FP64 mode always does; -1 .. 64).
+ *                  block_min, tile_cap, leaf_rank_max and leaf_reach act on
+ *                  the searches in order alone
  *   block_min      shortest list the search expands one parent at a time
  *                  with block culling (shorter lists: lanes over (parent,
  *                  candidate) pairs) (default 64, 1 .. 65535)
  *   tile_cap       most entries of a frontier tile (default 4096, 32 ..
  *                  16384)
  *   pair_grain     (structure, template) pairs a search warp takes from the
- *                  work queue at a time (default 1, 1 .. 64)
+ *                  work queue at a time (default 1, 1 .. 64; without order at
+ *                  least so many, up to 16 where there are pairs enough)
  *   leaf_rank_max  longest tie-free list put in leaf order by the
  *                  leaf-order kernel's instance with the smallest buffers
  *                  (longer lists: the instances for up to 512 and 1024

@@ -1293,7 +1293,10 @@ void write_search_profile(const unsigned long long *d_prof, cudaStream_t st, con
 
 namespace {
 std::mutex g_tuning_mutex;
-constexpr pjg_tuning TUNING_DEFAULTS = {4, 64, 4096, 1, LEAF_RANK_MAX, -1};
+// (leaf_levels 0: the order-free search first; what it leaves, and chunks it
+// does not take, are searched in order with ORDER_LEVELS)
+constexpr pjg_tuning TUNING_DEFAULTS = {0, 64, 4096, 1, LEAF_RANK_MAX, -1};
+constexpr int ORDER_LEVELS = 4;
 pjg_tuning g_tuning = TUNING_DEFAULTS;
 
 pjg_tuning current_tuning() {
@@ -1440,7 +1443,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     // up front: with one structure a chunk, the host round trip of each
     // extra search round costs more than the ordering it saves.
     const pjg_tuning tune = current_tuning();
-    int demand_levels = P->mode == PJG_MODE_PLAIN_FP64 ? -1 : tune.leaf_levels;
+    int demand_levels = P->mode == PJG_MODE_PLAIN_FP64 ? -1 : tune.leaf_levels ? tune.leaf_levels : ORDER_LEVELS;
     {
         const char *v = getenv("PJG_LEAF_LEVELS");
         if (v && *v && P->mode != PJG_MODE_PLAIN_FP64) demand_levels = atoi(v);
@@ -1450,7 +1453,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     FreeView fv{sp->n_kinds, (sp->n_kinds + 31) / 32, sp->d_kind_name, sp->d_kind_res, nullptr,
                 (sp->max_local_kinds + 31) / 32, nullptr, sp->d_nh_kind, sp->d_kxyz, sp->d_res_pos, sp->d_res_kind,
                 sp->d_res_range};
-    bool free_first = P->mode != PJG_MODE_PLAIN_FP64 && demand_levels == TUNING_DEFAULTS.leaf_levels &&
+    bool free_first = P->mode != PJG_MODE_PLAIN_FP64 && tune.leaf_levels == 0 &&
                             !getenv("PJG_LEAF_LEVELS") && sp->max_local_kinds <= FREE_MAX_KINDS &&
                             (int64_t)G * fv.kind_words <= (1ll << 28);
     // few enough atoms and signatures for one chunk whatever the lists hold:

@@ -6333,8 +6333,9 @@ cudaError_t launch_search_free(cudaStream_t st, bool fp32, const ChunkView &cv, 
     if (e != cudaSuccess) return e;
     SearchArgs fa = sa;
     // a pair takes microseconds: several a queue step once every resident
-    // warp has tens of them
-    fa.pair_grain = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, items / (resident * FREE_WARPS * 16)));
+    // warp has tens of them, no fewer than asked for
+    fa.pair_grain = (int32_t)std::max<int64_t>(sa.pair_grain,
+                                               std::min<int64_t>(16, items / (resident * FREE_WARPS * 16)));
     kern<<<(int)grid, FREE_WARPS * 32, smem, st>>>(cv, tv, cd, fv, fa, item_counter, scanned, out, counters, dm, fw);
     return cudaGetLastError();
 }

@@ -1,8 +1,9 @@
 """Autotuner of the GPU search's execution knobs (``pjg_tuning``).
 
 A batched query moves work between its kernels through a few knobs that
-change no result: how many levels of candidate lists get their kd leaf
-order before the search (the rest on demand, at the price of suspending
+change no result: whether pairs are searched without any order first (the
+default) or in order, and then how many levels of candidate lists get their kd
+leaf order before the search (the rest on demand, at the price of suspending
 and resuming the pairs that reach them), the list length from which the
 search expands one parent at a time with block culling, the frontier tile
 capacity, how many pairs a search warp takes from the work queue at once,
@@ -32,12 +33,12 @@ import time
 
 import numpy as np
 
-DEFAULTS = {"leaf_levels": 4, "block_min": 64, "tile_cap": 4096, "pair_grain": 1, "leaf_rank_max": 256,
+DEFAULTS = {"leaf_levels": 0, "block_min": 64, "tile_cap": 4096, "pair_grain": 1, "leaf_rank_max": 256,
             "leaf_reach": -1}
 # candidate values per knob, searched in this order
 SPACE = {
     "leaf_reach": [-1, 1, 2, 3],
-    "leaf_levels": [1, 2, 3, 4, 5, 6, -1],
+    "leaf_levels": [0, 1, 2, 3, 4, 5, 6, -1],
     "block_min": [32, 48, 64, 96, 128, 192],
     "pair_grain": [1, 2, 4, 8],
     "tile_cap": [1024, 2048, 4096, 8192],

@@ -54,6 +54,28 @@ def test_every_tuning_gives_the_oracle_hits(tuning):
         assert gs[key] == ref["stats"][key], key
 
 
+def test_every_count_of_levels_can_be_chosen():
+    """leaf_levels 0 is the order-free search, every other value a search in
+    order, 4 among them; what get_tuning returns sets the same again."""
+    from pyjess_gb300 import _native, workloads
+    from test_gpu_parity import gpu_query
+
+    wl = workloads.config(3, n_structures=30, n_templates=300)
+    lists = {}
+    try:
+        for levels in (0, 3, 4, 5):
+            _native.set_tuning({"leaf_levels": levels})
+            assert _native.get_tuning()["leaf_levels"] == levels
+            _native.set_tuning(_native.get_tuning())
+            res = gpu_query(wl.templates, wl.structures, **wl.params)
+            lists[levels] = res.stats()["leaf_lists"]
+    finally:
+        _native.set_tuning(None)
+    # (every order has the lists its pairs reach, the order-free search those
+    # that tell rows apart)
+    assert 10 * lists[0] < min(lists[k] for k in (3, 4, 5))
+
+
 def test_autotune_sample_and_cache(tmp_path):
     from oracle import oracle
     from pyjess_gb300 import _native, tune, workloads
