@@ -48,6 +48,24 @@ def test_cache_roundtrip_and_bad_files(tmp_path):
     assert tune.lookup("GPU A", "key1", path) is None
 
 
+def test_entries_of_another_search_are_measured_anew(tmp_path):
+    """A cache written for a search in order (no search named in it) would
+    choose that search for every later query."""
+    path = tmp_path / "tuning.json"
+    old = {"tuning": dict(tune.DEFAULTS, leaf_levels=3), "ms": 1.0}
+    path.write_text(json.dumps({"GPU A": {"key1": old, "key2": dict(old, search="other")}}))
+    assert tune.lookup("GPU A", "key1", path) is None and tune.lookup("GPU A", "key2", path) is None
+    tune.store("GPU A", "key1", old, path)
+    assert tune.lookup("GPU A", "key1", path)["tuning"] == old["tuning"]
+
+
+def test_differences_within_the_noise_change_nothing():
+    best, t, _ = tune.coordinate_descent(lambda cfg: 10.0 if cfg == tune.DEFAULTS else 9.9)
+    assert best == tune.DEFAULTS and t == 10.0
+    best, t, _ = tune.coordinate_descent(lambda cfg: 9.0 if cfg["pair_grain"] == 4 else 10.0)
+    assert best == dict(tune.DEFAULTS, pair_grain=4) and t == 9.0
+
+
 def test_cache_path_from_environment(tmp_path, monkeypatch):
     monkeypatch.setenv(tune.CACHE_ENV, str(tmp_path / "c.json"))
     assert tune.cache_path() == tmp_path / "c.json"
