@@ -122,7 +122,10 @@ typedef struct {
                                         queries whose hits outgrow memory */
 } pjg_query_params;
 
-/* Per-query counters and device timings (milliseconds, CUDA events). */
+/* Per-query counters and device timings (milliseconds, CUDA events).  With
+ * max_candidates the batched modes stop a pair by blocks of seeds: partials,
+ * complete, passing and bytes_expansion may then count work past the exact row
+ * at which its stream ends, the same in every run. */
 typedef struct {
     int64_t pairs;                   /* template x structure pairs         */
     int64_t candidate_entries;       /* sum of candidate-list lengths      */

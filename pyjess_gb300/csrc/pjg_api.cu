@@ -1223,8 +1223,8 @@ cudaError_t scan_exclusive(const T *in, int64_t n, int64_t *out, std::vector<DBu
 }
 
 // bytes of an item's arrays: its place and result, rows before it, its list of
-// segments, its levels, its counting bins
-constexpr double ITEM_BYTES = 8 + 8 + 8 + 4 + 8 + 8;
+// segments, its levels, its counting bins, its counters
+constexpr double ITEM_BYTES = 8 + 8 + 8 + 4 + 8 + 8 + 32;
 
 // places in a query's block of counters: the statistics (Counter), the lists
 // requested in a chunk, then what an attempt at a chunk's search adds up
@@ -1234,8 +1234,9 @@ enum : int {
     ZC_ATTEMPT,
     ZC_ROWS = ZC_ATTEMPT,
     ZC_FREE,            // units, heavy pairs, their items, scratch, large units,
-                        // spilled entries, units left to the leaf order, long units
-    ZC_NWORK = ZC_FREE + 8,
+                        // spilled entries, units left to the leaf order, long
+                        // units, items to search in order
+    ZC_NWORK = ZC_FREE + 9,
     ZC_NSUSP,
     ZC_POOL,
     ZC_ITEM,            // the work queue (32 bits)
@@ -1384,7 +1385,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
     DBuf<uint32_t> d_sig_bits, d_kind_masks;
     DBuf<RowUnit> d_units;
     DBuf<HeavyPair> d_heavy_pairs;
-    DBuf<unsigned long long> d_heavy_stats, d_row_key;
+    DBuf<unsigned long long> d_item_stats, d_row_key;
     DBuf<int2> d_items, d_results;
     DBuf<int64_t> d_item_base, d_bin_off;
     DBuf<int32_t> d_bins, d_arena_atom, d_row_scratch, d_item_head, d_large_units, d_long_pairs, d_pending;
@@ -2097,7 +2098,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
             // set when the chunk's complete rows cannot be held: the chunk is
             // redone on half its structures
             bool split = false;
-            bool invalid_rows = false;  // rows of pairs that k_search took over
+            bool invalid_rows = false;  // rows without a place: of pairs k_search took over, past a cut
             // set when the order-free search's own buffers cannot be held: the
             // chunk is redone on fewer structures (free_fit of them), a single
             // structure in order
@@ -2124,8 +2125,8 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                 dm.n_resume = 0;
                 dm.pool_in = nullptr;
                 // units, heavy pairs, their items, (scratch, large units,) spilled entries,
-                // units left to the leaf order
-                unsigned long long free_n[8] = {};
+                // units left to the leaf order, long units, items to search in order
+                unsigned long long free_n[9] = {};
                 FreeWork fw{};
                 Suspended *next_out = d_susp_a.p, *spare = d_susp_b.p;
                 unsigned char *pool_next = d_pool_a.p, *pool_spare = d_pool_b.p;
@@ -2151,6 +2152,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         fw.n_spilled = d_free_n.p + 5;
                         fw.n_pending = d_free_n.p + 6;
                         fw.n_long_units = d_free_n.p + 7;
+                        fw.n_failed = d_free_n.p + 8;
                         fw.units = d_units.p;
                         fw.n_units = d_free_n.p;
                         fw.heavy = d_heavy_pairs.p;
@@ -2194,7 +2196,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         ns = dm.state || free_chunk ? hz[ZC_NSUSP] : 0;
                         used = hz[ZC_LEAF_USED];
                         if (round == 0)
-                            for (int i = 0; i < 8; i++) free_n[i] = hz[ZC_FREE + i];
+                            for (int i = 0; i < 9; i++) free_n[i] = hz[ZC_FREE + i];
                         float m = 0.f;
                         if (e == cudaSuccess) e = cudaEventElapsedTime(&m, ev[6], ev[7]);
                         ms_search += m;
@@ -2240,7 +2242,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         room(d_item_head, ni);
                         room(d_item_branch, ni);
                         room(d_spill_a, SPILL_CAP);
-                        room(d_heavy_stats, 4 * (int64_t)nh);
+                        room(d_item_stats, 4 * ni);
                         room(d_arena_xyz, warps * HEAVY_CAP);
                         room(d_arena_atom, warps * HEAVY_CAP);
                         room(d_arena_parent, 2 * warps * HEAVY_CAP);
@@ -2250,7 +2252,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         CUDA_TRY(cudaMemsetAsync(d_results.p, 0xFF, (size_t)ni * sizeof(int2), st));
                         CUDA_TRY(cudaMemsetAsync(d_item_head.p, 0xFF, (size_t)ni * sizeof(int32_t), st));
                         CUDA_TRY(cudaMemsetAsync(d_item_branch.p, 0, (size_t)ni * sizeof(unsigned long long), st));
-                        CUDA_TRY(cudaMemsetAsync(d_heavy_stats.p, 0, 4 * (size_t)nh * sizeof(unsigned long long), st));
+                        CUDA_TRY(cudaMemsetAsync(d_item_stats.p, 0, 4 * (size_t)ni * sizeof(unsigned long long), st));
                         CUDA_TRY(cudaMemsetAsync(d_pair_counter.p, 0, sizeof(int32_t), st));
                         launch_heavy_bins(st, nh, d_heavy_pairs.p, d_bins.p);
                         CUDA_TRY(scan_exclusive(d_bins.p, nbins, d_bin_off.p, scan_tmp, st));
@@ -2258,7 +2260,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                         fw.items = d_items.p;
                         fw.n_items = (int32_t)ni;
                         fw.results = d_results.p;
-                        fw.heavy_stats = d_heavy_stats.p;
+                        fw.item_stats = d_item_stats.p;
                         fw.item_base = d_item_base.p;
                         fw.arena_xyz = d_arena_xyz.p;
                         fw.arena_atom = d_arena_atom.p;
@@ -2318,17 +2320,25 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                             CUDA_TRY(read_back());
                         }
                         if (free_full) break;
-                        launch_heavy_rows(st, nh, fw, d_item_base.p, d_pair_rows.p, d_counters.p);
+                        launch_heavy_rows(st, nh, fw, sa, d_item_base.p, d_pair_rows.p, dm, d_counters.p);
                         launches++;
+                        CUDA_TRY(cudaGetLastError());
+                        // (rows of items past the cut, and of pairs that go to
+                        // k_search, have no place)
+                        invalid_rows = invalid_rows || P->max_candidates >= 0 || free_n[8];
+                        if (free_n[8]) {
+                            const double ms0 = ms_search;
+                            CUDA_TRY(read_back());
+                            ms_search = ms0;
+                        }
                         if ((int64_t)ns > ns1) {
                             // pairs that an item left to k_search (their level-0
                             // lists are filled)
                             launch_free_requests(st, tv, cd, P->reorder, dm, nullptr, 0, dm.suspended, (int32_t)ns1,
                                                  (int32_t)ns);
                             launches++;
-                            invalid_rows = true;
+                            CUDA_TRY(cudaGetLastError());
                         }
-                        CUDA_TRY(cudaGetLastError());
                     }
                     if (round == 0 && free_chunk && free_n[0] && (int64_t)nc <= c_cap) {
                         // the rows found without order, in the reference's;
@@ -2491,7 +2501,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
                     launch_superpose(st, blocks, cv, tv, cr, rr);
                     CUDA_TRY(dalloc(d_long_pairs, (size_t)std::min<int64_t>(n_pairs, rows), st));
                     if (invalid_rows) {
-                        // (rows of a pair that k_search took over have no slot)
+                        // (rows of a pair that k_search took over, or past a cut, have no slot)
                         CUDA_TRY(cudaMemsetAsync(d_r_hit.p, 0, (size_t)rows * sizeof(int32_t), st));
                         CUDA_TRY(cudaMemsetAsync(d_r_warn.p, 0, (size_t)rows * sizeof(int32_t), st));
                         CUDA_TRY(cudaMemsetAsync(d_r_hatoms.p, 0, (size_t)rows * sizeof(int32_t), st));
@@ -2610,7 +2620,7 @@ extern "C" pjg_status pjg_query(const pjg_templates *tp, const pjg_structures *s
 done:
     if (st) {
         dfree(d_sig_bits, st); dfree(d_kind_masks, st); dfree(d_units, st); dfree(d_heavy_pairs, st);
-        dfree(d_heavy_stats, st); dfree(d_row_key, st); dfree(d_items, st); dfree(d_results, st);
+        dfree(d_item_stats, st); dfree(d_row_key, st); dfree(d_items, st); dfree(d_results, st);
         dfree(d_item_base, st); dfree(d_bin_off, st); dfree(d_bins, st); dfree(d_arena_atom, st);
         dfree(d_row_scratch, st); dfree(d_arena_xyz, st); dfree(d_arena_parent, st); dfree(d_item_head, st);
         dfree(d_large_units, st); dfree(d_long_pairs, st); dfree(d_pending, st); dfree(d_item_branch, st); dfree(d_spill_a, st);

@@ -4106,8 +4106,8 @@ __global__ void k_sig_kinds(SigView sv, FreeView fv, uint32_t *sig_bits) {
 
 // Lists of the order-free search: thread per (structure, signature), the
 // local kinds of the structure that the list takes (a bit each, kind_masks;
-// nullptr: lengths only) and the list's length, the sum of their atoms; `scanned` as
-// k_candidate_counts.  The threads of a warp share a structure, so its kinds
+// nullptr: lengths only) and the list's length, the sum of their atoms;
+// `scanned` as k_candidate_counts.  The threads of a warp share a structure, so its kinds
 // are read once for all; their signatures' bits are staged in shared memory.
 constexpr int LIST_KINDS_THREADS = 128;
 constexpr int LIST_KINDS_WORDS = 16;  // signature words staged (more: read from global memory)
@@ -4263,6 +4263,16 @@ __device__ __forceinline__ void level_order(const TemplateView &tv, const CandVi
     }
 }
 
+// a pair to search from its start
+__device__ __forceinline__ Suspended whole_pair(int pair) {
+    Suspended sp;
+    sp.pair = pair;
+    sp.pad = 0;
+    sp.skip = 0;
+    sp.state = -1;
+    return sp;
+}
+
 // An item's result, read by other items of its pair while it is written: one
 // 8-byte access each way, so that rows and flags are of one moment.
 __device__ __forceinline__ int2 load_result(const int2 *p) {
@@ -4335,10 +4345,13 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                 blk = it.y;
             }
             hp = fw.heavy[hidx];
-            // (read by one lane: another warp may set it at this moment)
+            // items after one that has to be searched in order are not wanted
+            // (none is without a cut); read by one lane: another warp may set
+            // it at this moment
             int failed = 0;
-            if (lane == 0) failed = load_flag(&fw.heavy[hidx].failed);
-            if (__shfl_sync(FULL_MASK, failed, 0)) continue;
+            if (lane == 0) failed = load_flag(&fw.heavy[hidx].failed_item);
+            failed = __shfl_sync(FULL_MASK, failed, 0);
+            if (sa.max_candidates < 0 ? failed != INT_MAX : blk >= failed) continue;
         }
         const int pair = HEAVY      ? hp.pair
                          : NL == 32 ? item
@@ -4430,7 +4443,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
         int rows = 0, any_hit = 0;
         // rows written: last segment, its levels at which rows part, segments
         int seg = -1, seg0 = -1, n_seg = 0;
-        bool spilled = false;
+        bool spilled = false, outgrew = false;
         Mask branch = 0;
         PerLevel<long long, W> F;  // partial assignments
         F.fill(0);
@@ -4708,6 +4721,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                     kd_needed = true;
                     continue;
                 }
+                outgrew = true;
                 const int np = lev_end - beg;
                 unsigned long long at = ~0ull;
                 if (lane == 0) {
@@ -4828,7 +4842,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
             atomicOr(&fw.item_branch[it], (unsigned long long)branch);
         }
         // rows without a hit among them that end the stream by themselves
-        const bool ended = HEAVY && !sub && !spilled && sa.max_candidates >= 0 && rows >= sa.max_candidates + 2ll &&
+        const bool ended = HEAVY && !sub && !outgrew && sa.max_candidates >= 0 && rows >= sa.max_candidates + 2ll &&
                            (sa.best_match || !any_hit);
         if (!HEAVY && outgrown && !kd_needed) {
             // in items of seeds
@@ -4837,29 +4851,21 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                 h.pair = pair;
                 h.blocks = (m0 + fw.item_seeds - 1) / fw.item_seeds;
                 h.first = (int32_t)atomicAdd(fw.n_heavy + 1, (unsigned long long)h.blocks);
-                h.failed = 0;
+                h.failed_item = INT_MAX;
+                h.cut = 0;
                 fw.heavy[atomicAdd(fw.n_heavy, 1ull)] = h;
             }
         } else {
             if (kd_needed) {
-                // in order, by k_search
-                int won = 1;
-                if (HEAVY) {
-                    if (lane == 0) won = atomicExch(&fw.heavy[hidx].failed, 1) == 0;
-                    won = __shfl_sync(FULL_MASK, won, 0);
-                }
-                if (won) {
-                    if (lane == 0) {
-                        Suspended sp;
-                        sp.pair = pair;
-                        sp.pad = 0;
-                        sp.skip = 0;
-                        sp.state = -1;
-                        dm.suspended[atomicAdd(dm.n_suspended, 1ull)] = sp;
-                    }
+                // in order, by k_search (an item: if it counts, k_heavy_rows)
+                if (lane == 0 && HEAVY) {
+                    atomicMin(&fw.heavy[hidx].failed_item, blk);
+                    atomicAdd(fw.n_failed, 1ull);
+                } else if (lane == 0) {
+                    dm.suspended[atomicAdd(dm.n_suspended, 1ull)] = whole_pair(pair);
                 }
             }
-            if (!kd_needed || HEAVY) {
+            if (!kd_needed) {
                 unsigned long long part = 0, comp = 0, bexp = 0;
                 for (int w = 0; w < W; w++) {
                     const int l = lane + 32 * w;
@@ -4873,10 +4879,10 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                     if (l >= 1 && l < n) bexp += (unsigned long long)(4LL * l * before + (4LL * (l + 1) + 16) * F.v[w]);
                 }
                 if (HEAVY) {
-                    // per pair: counted unless another item hands the pair to k_search
+                    // per item: counted if the item is
                     auto add = [&](int k, unsigned long long v) {
                         for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
-                        if (lane == 0 && v) atomicAdd(&fw.heavy_stats[4 * (int64_t)hidx + k], v);
+                        if (lane == 0 && v) atomicAdd(&fw.item_stats[4 * (int64_t)(hp.first + blk) + k], v);
                     };
                     add(0, part);
                     add(1, comp);
@@ -4885,7 +4891,7 @@ __global__ void __launch_bounds__(FREE_WARPS * 32, NL == 32 ? PJG_FREE_MIN_BLOCK
                     if (lane == 0 && sub) atomicAdd(&fw.results[hp.first + blk].x, rows);
                     if (lane == 0 && !sub)
                         store_result(&fw.results[hp.first + blk],
-                                     make_int2(rows, (any_hit || spilled ? 1 : 0) | (ended ? 2 : 0)));
+                                     make_int2(rows, (any_hit || outgrew ? 1 : 0) | (ended ? 2 : 0)));
                 } else {
                     if (lane == 0 && rows > 0) out.pair_rows[pair] = rows;
                     a_part += part;
@@ -4988,35 +4994,68 @@ __global__ void k_heavy_items(int32_t n_heavy, const HeavyPair *heavy, const int
             items[bin_begin[b] + atomicAdd(&bin_fill[b], 1)] = make_int2(i, b);
 }
 
-// Warp per heavy pair: rows before each of its items, the pair's rows and
-// its share of the counters (a pair handed to k_search counts there).
-__global__ void k_heavy_rows(int32_t n_heavy, const HeavyPair *heavy, const int2 *results, int64_t *item_base,
-                             const unsigned long long *heavy_stats, int32_t *pair_rows,
-                             unsigned long long *counters) {
+// Warp per heavy pair: its items that count, the rows before each of them, the
+// pair's rows and its share of the counters.  With max_candidates the items up
+// to the first whose predecessors end the stream by themselves: the rule by
+// which an item skips itself, over all results before it, so that neither rows
+// nor counters depend on which items were in flight.  A pair of which an item
+// that counts has to be searched in order goes to k_search, and counts there.
+__global__ void k_heavy_rows(int32_t n_heavy, HeavyPair *heavy, const int2 *results, int64_t *item_base,
+                             const unsigned long long *item_stats, int32_t max_candidates, int32_t best_match,
+                             int32_t *pair_rows, LeafDemand dm, unsigned long long *counters) {
     const int lane = lane_id();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    unsigned long long sum = 0;
+    const long long enough = (long long)max_candidates + 2;
+    unsigned long long sum[4] = {};
     for (int i = warp; i < n_heavy; i += nwarps) {
         const HeavyPair h = heavy[i];
-        if (h.failed) continue;
+        int cut = h.blocks;
+        if (max_candidates >= 0) {
+            long long run = 0;  // rows since the last item with a hit (best_match: all)
+            for (int b0 = 0; b0 < h.blocks && cut == h.blocks; b0 += 32) {
+                const int2 r = b0 + lane < h.blocks ? results[h.first + b0 + lane] : make_int2(0, 0);
+                for (int j = 0; j < min(32, h.blocks - b0); j++) {
+                    if (run >= enough) {
+                        cut = b0 + j;
+                        break;
+                    }
+                    const int rows = max(__shfl_sync(FULL_MASK, r.x, j), 0), flags = __shfl_sync(FULL_MASK, r.y, j);
+                    run = !best_match && (flags & 1) ? 0 : run + rows;
+                }
+            }
+        }
+        if (h.failed_item < cut) {
+            if (lane == 0) {
+                heavy[i].cut = 0;
+                dm.suspended[atomicAdd(dm.n_suspended, 1ull)] = whole_pair(h.pair);
+            }
+            continue;
+        }
         long long carry = 0;
-        for (int b0 = 0; b0 < h.blocks; b0 += 32) {
+        for (int b0 = 0; b0 < cut; b0 += 32) {
             const int b = b0 + lane;
-            const long long r = b < h.blocks ? max(results[h.first + b].x, 0) : 0;
+            const long long r = b < cut ? max(results[h.first + b].x, 0) : 0;
             long long incl = r;
             for (int o = 1; o < 32; o <<= 1) {
                 const long long y = __shfl_up_sync(FULL_MASK, incl, o);
                 if (lane >= o) incl += y;
             }
-            if (b < h.blocks) item_base[h.first + b] = carry + incl - r;
+            if (b < cut) {
+                item_base[h.first + b] = carry + incl - r;
+                for (int k = 0; k < 4; k++) sum[k] += item_stats[4 * (int64_t)(h.first + b) + k];
+            }
             carry += __shfl_sync(FULL_MASK, incl, 31);
         }
-        if (lane == 0) pair_rows[h.pair] = (int32_t)carry;
-        if (lane < 4) sum += heavy_stats[4 * (int64_t)i + lane];
+        if (lane == 0) {
+            heavy[i].cut = cut;
+            pair_rows[h.pair] = (int32_t)carry;
+        }
     }
-    if (lane < 4 && sum)
-        atomicAdd(&counters[lane == 0 ? C_PARTIALS : lane == 1 ? C_COMPLETE : lane == 2 ? C_BYTES_EXP : C_RECHECK],
-                  sum);
+    for (int k = 0; k < 4; k++) {
+        for (int o = 16; o; o >>= 1) sum[k] += __shfl_xor_sync(FULL_MASK, sum[k], o);
+        if (lane == 0 && sum[k])
+            atomicAdd(&counters[k == 0 ? C_PARTIALS : k == 1 ? C_COMPLETE : k == 2 ? C_BYTES_EXP : C_RECHECK], sum[k]);
+    }
 }
 
 // The places of a unit's rows (a pair's, or an item's) in the pair's stream.
@@ -5167,7 +5206,7 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
 // has: units of at most DIRECT_ROWS rows whose lists have at most DIRECT_MAX
 // entries (24 warps; 20 for 128 rows, 12 for 256), and, passed on by the
 // first, more rows, and lists of up to DIRECT_LONG with at most
-// DIRECT_LONG_ROWS rows (7 warps).
+// DIRECT_LONG_ROWS rows (6 warps).
 // Measured on 1,000 structures x 4,000 templates: 5.9 and 9.7 ms (DIRECT_ROWS
 // 128 6.8 and 9.2, 256 9.7 and 9.0), and 11 ms for the 62,000 lists left to the
 // leaf order, where ordering every such list (0.84 M) and ranking the rows by
@@ -5209,8 +5248,9 @@ __global__ void __launch_bounds__(WARPS * 32)
         const int w = LONG ? fw.long_units[x] : (int)x;
         const RowUnit u = fw.units[w];
         if (!LONG) {
-            if (u.heavy >= 0 && fw.heavy[u.heavy].failed) {
-                for (int i = lane; i < u.count; i += 32) out.pair[u.row_base + i] = -1;  // k_search's rows count
+            if (u.heavy >= 0 && u.item - fw.heavy[u.heavy].first >= fw.heavy[u.heavy].cut) {
+                // (past the cut, or k_search's rows count)
+                for (int i = lane; i < u.count; i += 32) out.pair[u.row_base + i] = -1;
                 continue;
             }
             // (a segment that does not lead its unit's list is not a unit)
@@ -6390,10 +6430,11 @@ void launch_heavy_items(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy
     k_heavy_items<<<(n_heavy + 255) / 256, 256, 0, st>>>(n_heavy, heavy, bin_begin, bin_fill, items);
 }
 
-void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int64_t *item_base, int32_t *pair_rows,
-                       unsigned long long *counters) {
+void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, const SearchArgs &sa, int64_t *item_base,
+                       int32_t *pair_rows, const LeafDemand &dm, unsigned long long *counters) {
     k_heavy_rows<<<std::min((n_heavy + 7) / 8, 152 * 8), 256, 0, st>>>(n_heavy, fw.heavy, fw.results, item_base,
-                                                                     fw.heavy_stats, pair_rows, counters);
+                                                                     fw.item_stats, sa.max_candidates, sa.best_match,
+                                                                     pair_rows, dm, counters);
 }
 
 cudaError_t launch_unit_order_direct(cudaStream_t st, int64_t n_units, const ChunkView &cv, const TemplateView &tv,
@@ -6544,9 +6585,9 @@ void launch_gather_hits(cudaStream_t st, int64_t n_rows, int32_t n_templates, in
 // Each call writes the word of every row it later reads, so nothing carries
 // over from one call to the next.
 //
-// Bound by the FP64 pipe (about 30 operations an atom for the covariance,
-// the rest for the 4 x 4 eigen-solve): a thread per row keeps every lane of
-// it busy.  Measured at 300,000 rows of 12 atoms: 0.40 ms; 9.58 ms with a
+// Bound by the FP64 pipe, 88% of whose peak it issues (about 25 operations an
+// atom for the covariance, the rest for the 4 x 4 eigen-solve): a thread per
+// row keeps every lane of it busy.  Measured at 300,000 rows of 12 atoms: 0.40 ms; 9.58 ms with a
 // warp per row (one lane in the eigen-solve) and the compaction in one block.
 
 static __device__ __align__(256) uint32_t g_noalloc_words[PJG_NOALLOC_MAX_ROWS / 32];

@@ -278,7 +278,8 @@ struct HeavyPair {
     int32_t pair;
     int32_t blocks;                    // items
     int32_t first;                     // its first item in `results`
-    int32_t failed;                    // handed to k_search
+    int32_t failed_item;               // first item that has to be searched in order (INT_MAX: none)
+    int32_t cut;                       // items that count (k_heavy_rows; 0: the pair goes to k_search)
 };
 
 // Rows of the order-free search whose order among each other is still to be
@@ -315,7 +316,8 @@ struct FreeWork {
     int32_t n_wide;                    //   the launch takes their pairs alone)
     int2 *results;                     // per item: rows (-1: not finished), flags
                                        //   (1: a hit among them, 2: the stream ends)
-    unsigned long long *heavy_stats;   // [4 * heavy pairs] partials, complete, bytes, rechecks
+    unsigned long long *n_failed;      // items that have to be searched in order
+    unsigned long long *item_stats;    // [4 * items] partials, complete, bytes, rechecks
     int32_t *item_head;                // per item: its list of segments (-1: no rows)
     unsigned long long *item_branch;   //   levels at which its rows part
     const int64_t *item_base;          //   rows of the pair before it
@@ -412,8 +414,11 @@ void launch_leaf_order(cudaStream_t st, int blocks, const ChunkView &cv, int32_t
 // the same for few lists (at most LEAF_FEW_ENTRIES entries in all), requested
 // for ties or long units by the order-free search: one launch of the
 // sorted-axis split for every length (as long as its longest list) instead of
-// seven that a tied list would pass through (annotating a protein with 3,000
-// templates, 199 lists: 0.24 ms in 5 launches, 1.0 ms in 19)
+// seven that a tied list would pass through.  Time of a query's lists and row
+// ordering with all requests in one launch set / in the other: 74 lists (9,000
+// entries) 0.70 / 0.98 ms, 421 (0.16 M) 1.31 / 2.62, 5,371 (1.9 M) 4.04 / 5.41,
+// 17,871 (7.7 M) 13.6 / 15.6, 55,636 (21 M) 30.7 / 28.2, 155,139 (61 M)
+// 86.2 / 76.7: the line lies between 7.7 M and 21 M entries
 constexpr int64_t LEAF_FEW_ENTRIES = 8 << 20;
 constexpr int LEAF_FEW_LAUNCHES = 5;
 void launch_leaf_order_few(cudaStream_t st, const ChunkView &cv, int32_t n_sigs, const int32_t *count,
@@ -493,8 +498,8 @@ cudaError_t launch_search_heavy(cudaStream_t st, bool fp32, int64_t warps, const
 void launch_heavy_bins(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy, int32_t *bins);
 void launch_heavy_items(cudaStream_t st, int32_t n_heavy, const HeavyPair *heavy, const int64_t *bin_begin,
                         int32_t *bin_fill, int2 *items);
-void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, int64_t *item_base, int32_t *pair_rows,
-                       unsigned long long *counters);
+void launch_heavy_rows(cudaStream_t st, int32_t n_heavy, const FreeWork &fw, const SearchArgs &sa, int64_t *item_base,
+                       int32_t *pair_rows, const LeafDemand &dm, unsigned long long *counters);
 // the units' rows in the reference's order (out.ordinal): without lists in
 // leaf order where that can be done (the others in fw.pending), then those by
 // their lists' leaf order

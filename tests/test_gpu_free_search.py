@@ -327,6 +327,25 @@ def test_unit_of_half_a_million_rows():
     assert time.perf_counter() - t0 < 2.0
 
 
+@pytest.mark.parametrize("kw", [dict(max_candidates=0), dict(max_candidates=40), dict(max_candidates=700),
+                                dict(best_match=True, max_candidates=40), dict(best_match=True, max_candidates=700)])
+def test_cut_streams_count_the_same_every_time(kw):
+    """Items past a pair's cut may or may not have been in flight when its
+    earlier ones ended the stream: the counters are of the items before it."""
+    from pyjess_gb300 import _native, workloads as W
+    from pyjess_gb300._abi import QueryParams
+
+    structs = _structures(45, [1500, 1300, 1400, 1200])
+    specs = _templates(45, structs, 12, lo=2, hi=4, permissive=True)
+    T, S = _native.Templates(W.pack_templates(specs)), _native.Structures(W.pack(structs))
+    P = QueryParams(rmsd_threshold=1.0, distance_cutoff=1.2, max_dynamic_distance=1.2, ignore_chain=0,
+                    max_candidates=kw["max_candidates"], best_match=int(kw.get("best_match", False)), reorder=1,
+                    mode=_native.MODE_BATCHED_FP32)
+    counters = {tuple(_native.query(T, S, P).stats()[k] for k in (
+        "partials", "complete", "passing", "hits", "bytes_expansion", "fp64_rechecks")) for _ in range(12)}
+    assert len(counters) == 1
+
+
 @pytest.mark.parametrize("budget", ["1", "60"])
 @pytest.mark.parametrize("kw", [dict(), dict(max_candidates=5), dict(best_match=True, max_candidates=7)])
 def test_more_items_than_room(monkeypatch, budget, kw):
