@@ -927,34 +927,30 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
         std::vector<uint32_t> hname;  // distinct atom names of each bucket, sorted
         std::vector<int32_t> hcount, hbegin{0};
         std::vector<int32_t> hoff;    // start of each distinct name's atoms in nh_pos (structure-local)
-        std::vector<int32_t> hkind;   // its kind (distinct residue and atom name of the set)
+        std::vector<int32_t> hkind;   // its kind (distinct residue and atom name), in the numbers of
+        int thread = 0;               //   the host thread that met it
         double radius = 0.0;
         int64_t bad = -1;  // first atom with a non-finite coordinate
     };
     std::vector<Buckets> bk(std::max(S, 0));
-    // kinds of the set, numbered as the host threads meet them (each thread
-    // keeps the ones it has seen, so the shared table is rarely locked)
-    using KindMap = std::unordered_map<uint64_t, int32_t>;
-    KindMap kinds_all;
-    std::vector<uint32_t> kind_name, kind_res;
-    std::mutex kinds_mutex;
-    auto kind_of = [&](uint32_t res, uint32_t nm, KindMap &seen) -> int32_t {
-        const uint64_t key = ((uint64_t)res << 32) | nm;
-        auto it = seen.find(key);
-        if (it != seen.end()) return it->second;
-        std::lock_guard<std::mutex> g(kinds_mutex);
-        auto ins = kinds_all.emplace(key, (int32_t)kind_name.size());
-        if (ins.second) {
-            kind_name.push_back(nm);
-            kind_res.push_back(res);
+    // kinds of the set: each host thread numbers those it meets, the numbers
+    // are joined afterwards (a table shared by the threads, locked for each new
+    // kind, made an upload of 16 structures 0.8 ms longer)
+    struct ThreadKinds {
+        std::unordered_map<uint64_t, int32_t> number;
+        std::vector<uint64_t> key;
+        int32_t of(uint32_t res, uint32_t nm) {
+            const uint64_t k = ((uint64_t)res << 32) | nm;
+            auto ins = number.emplace(k, (int32_t)key.size());
+            if (ins.second) key.push_back(k);
+            return ins.first->second;
         }
-        seen.emplace(key, ins.first->second);
-        return ins.first->second;
     };
-    auto prepare = [&](int s, KindMap &seen) {
+    auto prepare = [&](int s, ThreadKinds &seen, int thread) {
         const int64_t b0 = base[s];
         const int n = count[s];
         Buckets &B = bk[s];
+        B.thread = thread;
         for (int i = 0; i < n && B.bad < 0; i++)
             for (int d = 0; d < 3; d++)
                 if (!std::isfinite(set->xyz[3 * (b0 + i) + d])) B.bad = i;
@@ -1033,7 +1029,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
                 if (i == 0 || nm[i] != nm[i - 1]) {
                     B.hname.push_back(nm[i]);
                     B.hcount.push_back(0);
-                    B.hkind.push_back(kind_of(B.name[k], nm[i], seen));
+                    B.hkind.push_back(seen.of(B.name[k], nm[i]));
                 }
                 B.hcount.back()++;
             }
@@ -1056,16 +1052,16 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
             }
         }
     };
+    const int nthreads = (int)std::max<unsigned>(1, std::min<unsigned>(32, std::thread::hardware_concurrency()));
+    std::vector<ThreadKinds> met((size_t)std::max(1, std::min(nthreads, S)));
     {
-        const int nthreads = (int)std::max<unsigned>(1, std::min<unsigned>(32, std::thread::hardware_concurrency()));
         std::atomic<int> next{0};
-        auto worker = [&]() {
-            KindMap seen;
-            for (int s; (s = next.fetch_add(1)) < S;) prepare(s, seen);
+        auto worker = [&](int i) {
+            for (int s; (s = next.fetch_add(1)) < S;) prepare(s, met[i], i);
         };
         std::vector<std::thread> pool;
-        for (int i = 1; i < std::min(nthreads, S); i++) pool.emplace_back(worker);
-        worker();
+        for (int i = 1; i < (int)met.size(); i++) pool.emplace_back(worker, i);
+        worker(0);
         for (auto &th : pool) th.join();
     }
     for (int s = 0; s < S; s++)
@@ -1073,6 +1069,16 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
             delete h;
             return fail(PJG_ERR_INVALID, "structure %d atom %lld: non-finite coordinate", s, (long long)bk[s].bad);
         }
+    // the kinds' numbers in the set, per thread and its own number
+    ThreadKinds all;
+    std::vector<std::vector<int32_t>> kind_of(met.size());
+    for (size_t i = 0; i < met.size(); i++)
+        for (uint64_t k : met[i].key) kind_of[i].push_back(all.of((uint32_t)(k >> 32), (uint32_t)k));
+    std::vector<uint32_t> kind_name, kind_res;
+    for (uint64_t k : all.key) {
+        kind_name.push_back((uint32_t)k);
+        kind_res.push_back((uint32_t)(k >> 32));
+    }
     std::vector<int32_t> nh_begin{0}, nh_count, nh_off, nh_kind;
     std::vector<uint32_t> nh_name;
     for (int s = 0; s < S; s++) {
@@ -1081,7 +1087,7 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
         nh_name.insert(nh_name.end(), B.hname.begin(), B.hname.end());
         nh_count.insert(nh_count.end(), B.hcount.begin(), B.hcount.end());
         nh_off.insert(nh_off.end(), B.hoff.begin(), B.hoff.end());
-        nh_kind.insert(nh_kind.end(), B.hkind.begin(), B.hkind.end());
+        for (int32_t k : B.hkind) nh_kind.push_back(kind_of[(size_t)B.thread][(size_t)k]);
         h->max_local_kinds = std::max(h->max_local_kinds, (int32_t)B.hname.size());
     }
     h->n_kinds = (int32_t)kind_name.size();

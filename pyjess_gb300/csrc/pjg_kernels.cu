@@ -1641,11 +1641,12 @@ __global__ void k_leaf_exact(ChunkView cv, int32_t n_sigs, const int32_t *count,
 //
 // Two kernels, so that one structure spreads over the chip: a block sorts a
 // tile of RANK_TILE atoms of one axis in shared memory, then a thread per
-// (atom, axis) sums binary searches over the sorted tiles.  Bound by their
-// latency for a single structure (8,000 atoms: 310 us with one block an axis
-// and tiles of 2,048, 75 us now).
+// (atom, axis) sums binary searches over the sorted tiles, whose number the
+// tile's size keeps small.  With tiles of 512 atoms an upload of 14,825 atoms
+// took 0.86 ms (0.82 now), 256 structures 5.6 ms (5.3), 2,000 33.0 (31.9).
 
-constexpr int RANK_TILE = 512;
+constexpr int RANK_TILE = 2048;
+constexpr int RANK_SORT_THREADS = RANK_TILE / 2;  // a pair each
 constexpr int RANK_THREADS = 256;
 
 __device__ __forceinline__ unsigned long long order_key(double x) {
@@ -1665,7 +1666,7 @@ __device__ __forceinline__ unsigned long long rank_key(const double *xyz64, cons
     return a < 3 ? order_key(xyz64[3 * i + a]) : residue_key(__float_as_int(ro.xyz32[i].w));
 }
 
-__global__ void __launch_bounds__(RANK_THREADS)
+__global__ void __launch_bounds__(RANK_SORT_THREADS)
     k_rank_tiles(const int64_t *atom_base, const int32_t *atom_count, const double *xyz64, int64_t n_atoms,
                  unsigned long long *tile_key, uint16_t *tile_idx, ResidueOrder ro) {
     __shared__ unsigned long long key[RANK_TILE];
@@ -1675,13 +1676,12 @@ __global__ void __launch_bounds__(RANK_THREADS)
     const int n = atom_count[s];
     for (int t0 = blockIdx.z * RANK_TILE; t0 < n; t0 += gridDim.z * RANK_TILE) {
         const int tn = min(RANK_TILE, n - t0);
-        for (int i = threadIdx.x; i < RANK_TILE; i += RANK_THREADS) {
+        for (int i = threadIdx.x; i < RANK_TILE; i += RANK_SORT_THREADS) {
             key[i] = i < tn ? rank_key(xyz64, ro, b0 + t0 + i, a) : ~0ull;
             idx[i] = (uint16_t)i;
         }
         __syncthreads();
         // bitonic sort by (key, idx), a pair a thread
-        static_assert(RANK_TILE == 2 * RANK_THREADS, "one pair a thread");
         for (int k = 2; k <= RANK_TILE; k <<= 1) {
             for (int j = k >> 1; j > 0; j >>= 1) {
                 const int q = threadIdx.x, lj = __ffs(j) - 1;
@@ -1700,7 +1700,7 @@ __global__ void __launch_bounds__(RANK_THREADS)
                 __syncthreads();
             }
         }
-        for (int i = threadIdx.x; i < tn; i += RANK_THREADS) {
+        for (int i = threadIdx.x; i < tn; i += RANK_SORT_THREADS) {
             tile_key[a * n_atoms + b0 + t0 + i] = key[i];
             tile_idx[a * n_atoms + b0 + t0 + i] = idx[i];
         }
@@ -6217,12 +6217,13 @@ void launch_axis_ranks(cudaStream_t st, int32_t n_structures, int32_t max_atoms,
     if (n_structures <= 0) return;
     // enough blocks a structure for the longest one, up to a few waves of the
     // chip in all
-    const int64_t tiles = ((int64_t)max_atoms + RANK_TILE - 1) / RANK_TILE;
-    const unsigned z = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>({tiles, 65535, std::max<int64_t>(1, 152 * 64 / ((int64_t)n_structures * 4))}));
-    k_rank_tiles<<<dim3((unsigned)n_structures, 4, z), RANK_THREADS, 0, st>>>(atom_base, atom_count, xyz64, n_atoms,
-                                                                             tile_key, tile_idx, ro);
-    k_axis_ranks<<<dim3((unsigned)n_structures, 4, 2 * z), RANK_THREADS, 0, st>>>(
+    const int64_t most = std::max<int64_t>(1, 152 * 64 / ((int64_t)n_structures * 4));
+    auto depth = [&](int atoms, int64_t at_most) -> unsigned {
+        return (unsigned)std::max<int64_t>(1, std::min<int64_t>(((int64_t)max_atoms + atoms - 1) / atoms, at_most));
+    };
+    k_rank_tiles<<<dim3((unsigned)n_structures, 4, depth(RANK_TILE, most)), RANK_SORT_THREADS, 0, st>>>(
+        atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, ro);
+    k_axis_ranks<<<dim3((unsigned)n_structures, 4, depth(RANK_THREADS, 2 * most)), RANK_THREADS, 0, st>>>(
         atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, lrank, urank, ro);
 }
 

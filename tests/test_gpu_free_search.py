@@ -232,6 +232,24 @@ def test_structures_around_a_rank_tile(atoms):
     compare(W.pack_templates(specs), W.pack(structs), **PARAMS)
 
 
+@pytest.mark.parametrize("atoms", [2047, 2048, 2049, 4097])
+def test_structures_of_several_rank_tiles(atoms):
+    """As test_structures_around_a_rank_tile around multiples of the 2,048
+    atoms of a tile, 20 structures at a time (names met by several host
+    threads)."""
+    from pyjess_gb300 import workloads as W
+
+    structs = _structures(54, [atoms // 6] * 2 + [40] * 18)
+    specs = _templates(54, structs, 20, hi=4)
+    for i, s in enumerate(structs[:2]):
+        for k in ("xyz", "name", "resname", "res_seq", "chain", "serial"):
+            s[k] = np.ascontiguousarray(s[k][:atoms])
+        assert len(s["xyz"]) == atoms
+        if i:
+            s["xyz"] = np.round(s["xyz"] / 0.25) * 0.25
+    compare(W.pack_templates(specs), W.pack(structs), **PARAMS)
+
+
 def test_long_lists_replayed():
     """Backbone lists of 4,300 entries with ties (the exact replay in 192 KB of
     shared memory)."""
