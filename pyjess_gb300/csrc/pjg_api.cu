@@ -207,19 +207,22 @@ struct Scratch {
 };
 
 // Memory of handles and results (and of the arrays a structure upload needs
-// meanwhile): a pool of their own on each device, which keeps OBJECT_KEEP bytes
-// beyond the live blocks for the next ones and gives the rest back to the
-// device: at the next wait of any stream, and as soon as a block of
-// OBJECT_PROMPT bytes is freed.  (The pool of the queries' buffers keeps up to
-// half the device.)
-constexpr size_t OBJECT_KEEP = 256 << 20, OBJECT_PROMPT = 64 << 20;
+// meanwhile): a pool of their own on each device, which keeps a 64th of the
+// device (PJG_OBJECT_KEEP bytes) beyond the live blocks for the next ones and
+// gives the rest back to the device: at the next wait of any stream, and as
+// soon as a block of OBJECT_PROMPT bytes is freed.  (Mapping memory anew costs:
+// a query of 10 M pairs with 2.2 GB of hits took 218.8 ms with 256 MiB kept,
+// 211.0 with 4.4 GB.  The pool of the queries' buffers keeps up to half the
+// device.)
+constexpr size_t OBJECT_PROMPT = 64 << 20;
 
 struct ObjectPool {
     cudaMemPool_t pool = nullptr;
     unsigned long long ctx = 0;  // the context it belongs to
     size_t live = 0;             // bytes of its blocks
+    size_t keep = 0;             // bytes it keeps beyond them
     uint64_t threshold = 0;      // what it may hold (set anew when live has
-};                               //   moved by a quarter of OBJECT_KEEP)
+};                               //   moved by a quarter of `keep`)
 std::mutex g_object_mutex;
 ObjectPool g_object_pool[256];   // guarded by g_object_mutex
 
@@ -246,7 +249,11 @@ struct Block {
             e = cudaMemPoolCreate(&o.pool, &props);
             if (e != cudaSuccess) return e;
             o.ctx = ctx;
+            size_t fb = 0, tb = 0;
+            o.keep = cudaMemGetInfo(&fb, &tb) == cudaSuccess ? tb / 64 : 256 << 20;
         }
+        if (const char *v = getenv("PJG_OBJECT_KEEP"))
+            if (atoll(v) > 0) o.keep = (size_t)atoll(v);
         e = cudaMallocFromPoolAsync(&p, bytes, o.pool, st);
         if (e == cudaErrorMemoryAllocation) {
             // what the queries' pool holds unused may make the room
@@ -277,7 +284,7 @@ struct Block {
             if (o.pool && o.ctx == ctx) {
                 o.live -= bytes;
                 limit(o);
-                if (bytes >= OBJECT_PROMPT && !st) cudaMemPoolTrimTo(o.pool, o.live + OBJECT_KEEP);
+                if (bytes >= OBJECT_PROMPT && !st) cudaMemPoolTrimTo(o.pool, o.live + o.keep);
             }
         }
         if (dev != device) cudaSetDevice(dev);
@@ -286,8 +293,8 @@ struct Block {
 
 private:
     static void limit(ObjectPool &o) {
-        const uint64_t most = o.live + OBJECT_KEEP;
-        if (o.threshold <= most + OBJECT_KEEP / 4 && most <= o.threshold + OBJECT_KEEP / 4) return;
+        const uint64_t most = o.live + o.keep;
+        if (o.threshold <= most + o.keep / 4 && most <= o.threshold + o.keep / 4) return;
         o.threshold = most;
         cudaMemPoolSetAttribute(o.pool, cudaMemPoolAttrReleaseThreshold, &o.threshold);
     }

@@ -22,7 +22,7 @@ def _tiled(copies):
                           res_seq=tile(one.res_seq), serial=tile(one.serial))
 
 
-def test_dropped_handles_and_results_leave_the_device():
+def test_dropped_handles_and_results_leave_the_device(monkeypatch):
     """A result and a structure handle of about a gigabyte each: once
     dropped, other programs of the device can have their memory (the queries'
     own buffers are kept)."""
@@ -31,6 +31,7 @@ def test_dropped_handles_and_results_leave_the_device():
     from pyjess_gb300 import _native, workloads as W
     from pyjess_gb300._abi import QueryParams
 
+    monkeypatch.setenv("PJG_OBJECT_KEEP", str(256 << 20))
     one, many = _tiled(3000)
     rng = np.random.default_rng(52)
     donor = W.make_structures([np.random.default_rng(51)], [300], [2])[0]
