@@ -5528,7 +5528,9 @@ __global__ void __launch_bounds__(WARPS * 32)
 // row by row).  A level with a class of more than UNIT_COUNT_MAX rows is
 // merge-sorted instead: a row counting its class is quadratic (580,000 rows in
 // one class: 133 ms, 52 s counted; 33,750: 5.2 and 177 ms; 6,574: 0.5 and 1.7).
-// The time budget is polled at every level, merge pass and block of leaves.
+// The time budget is polled at every level, merge pass and block of leaves;
+// once it is spent the rows keep the order they have (each its own place: the
+// stages that follow read every place of a pair before the query fails).
 constexpr int UNIT_COUNT_MAX = 4096;
 
 __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
@@ -5548,7 +5550,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
     // (by every thread; a barrier on both sides)
     auto out_of_time = [&]() -> bool {
         __syncthreads();
-        if (tid == 0 && global_ns() - t_start > budget_ns) {
+        if (tid == 0 && !over && global_ns() - t_start > budget_ns) {
             over = 1;
             atomicMax(&counters[C_ERROR], 3ull);
         }
@@ -5587,7 +5589,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
             const int k = order[l], g = sig[l];
             const int m = cd.count[wb + g];
             const int32_t *la = l == 0 ? nullptr : cd.leaf_atom + cd.leaf_offset[wb + g];
-            if (out_of_time()) return;
+            if (out_of_time()) break;
             if (tid == 0) most = 0;
             for (int p = tid; p < R; p += blockDim.x) {
                 const int32_t a = out.atoms[(int64_t)row[p] * out.stride + k];
@@ -5598,7 +5600,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
                 // atoms (bit 63 set once replaced) by their leaf ranks, the list
                 // through shared memory
                 for (int k0 = 0; k0 < m; k0 += blockDim.x) {
-                    if (out_of_time()) return;
+                    if (out_of_time()) break;
                     if (k0 + tid < m) leaf[tid] = la[k0 + tid];
                     __syncthreads();
                     const int kn = min((int)blockDim.x, m - k0);
@@ -5613,6 +5615,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
                 }
             }
             __syncthreads();
+            if (over) break;
             // the largest class
             for (int p = tid; p < R; p += blockDim.x)
                 if (p + 1 == R || cls[p + 1] != cls[p]) atomicMax(&most, p + 1 - cls[p]);
@@ -5626,7 +5629,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
                 int32_t *src = row2, *dst = cls2;  // positions, sorted in runs
                 for (int p = tid; p < R; p += blockDim.x) src[p] = p;
                 for (int lw = 0; (1ll << lw) < R; lw++) {  // runs of 2^lw
-                    if (out_of_time()) return;
+                    if (out_of_time()) break;
                     for (int p = tid; p < R; p += blockDim.x) {
                         // p's place among its run and the sibling run, equal
                         // keys of the left run first
@@ -5650,6 +5653,7 @@ __global__ void __launch_bounds__(UNIT_LARGE_THREADS)
                     dst = y;
                 }
                 __syncthreads();
+                if (over) break;
                 // new classes (where a row's key begins) and the rows in order
                 for (int p = tid; p < R; p += blockDim.x) {
                     const unsigned long long mine = key[src[p]];
@@ -5975,7 +5979,9 @@ __global__ void k_gather_hits(int64_t n_rows, int32_t T, int32_t structure_base,
     const bool h = hit[d] != 0, w = warn[d] != 0;
     if (!h && !w) return;
     const int64_t i = rr.src[d];
+    if (i < 0 || i >= n_rows) return;  // (a place no row took: the query has an error)
     const int pair = in.pair[i];
+    if (pair < 0) return;
     const int s = pair / T, t = pair % T;
     const int64_t q = (int64_t)s * T + (T - 1 - t);
     if (h) {

@@ -42,3 +42,20 @@ def test_time_budget_returns_timeout_and_library_stays_usable(monkeypatch):
     assert res["count"] == ref["count"] > 0
     assert hit_keys(res) == hit_keys(ref)
     check_rmsd(res, ref, wl.templates, wl.structures)
+
+
+def test_time_budget_spent_in_the_row_order(monkeypatch):
+    """A unit of 580,000 rows: found within the budget, ordered in several
+    times as much.  The ordering stops by itself, with every row at a place of
+    its own, and the next query is answered."""
+    from test_gpu_free_search import _one_seed_any_pair
+    from test_gpu_parity import compare, gpu_query
+
+    pt, ps = _one_seed_any_pair(47, 780)
+    kw = dict(rmsd_threshold=7.0, distance_cutoff=300.0, max_dynamic_distance=300.0)
+    monkeypatch.setenv("PJG_KERNEL_BUDGET_S", "0.02")
+    with pytest.raises(RuntimeError, match="timeout"):
+        gpu_query(pt, ps, **kw)
+    monkeypatch.delenv("PJG_KERNEL_BUDGET_S")
+    _, ref = compare(pt, ps, **kw)
+    assert ref["hits"]["count"] > 100
