@@ -176,7 +176,7 @@ struct Scratch {
 
     cudaError_t create(int dev) {
         device = dev;
-        ctx = current_context_id();
+        ctx = bound_context_id(dev);
         cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         for (auto &v : ev)
             if (e == cudaSuccess) e = cudaEventCreate(&v);
@@ -234,10 +234,10 @@ struct Block {
 
     cudaError_t alloc(size_t n, cudaStream_t st) {
         bytes = std::max<size_t>(n, 1);
-        ctx = current_context_id();
         cudaError_t e = cudaGetDevice(&device);
         if (e != cudaSuccess) return e;
         if (device >= 256) return cudaErrorInvalidDevice;
+        ctx = bound_context_id(device);
         std::lock_guard<std::mutex> g(g_object_mutex);
         ObjectPool &o = g_object_pool[device];
         if (!o.pool || o.ctx != ctx) {
@@ -276,7 +276,7 @@ struct Block {
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev != device) cudaSetDevice(device);
-        if (current_context_id() == ctx) {
+        if (bound_context_id(device) == ctx) {
             cudaFreeAsync(p, st);
             if (bytes >= OBJECT_PROMPT && !st) cudaStreamSynchronize(nullptr);
             std::lock_guard<std::mutex> g(g_object_mutex);
@@ -307,7 +307,7 @@ int g_handles = 0;               // live template and structure handles (guarded
 
 // a scratch of the current device, idle; nullptr with *e set on failure
 Scratch *acquire_scratch(int device, cudaError_t *e) {
-    const unsigned long long ctx = current_context_id();
+    const unsigned long long ctx = bound_context_id(device);
     *e = cudaSuccess;
     {
         std::lock_guard<std::mutex> g(g_scratch_mutex);
@@ -355,14 +355,14 @@ void handle_destroyed() {
         std::lock_guard<std::mutex> g(g_scratch_mutex);
         if (--g_handles == 0) out.swap(g_idle);
     }
-    const unsigned long long ctx = out.empty() ? 0 : current_context_id();
     int dev = 0;
     if (!out.empty()) cudaGetDevice(&dev);
+    const unsigned long long ctx = out.empty() ? 0 : bound_context_id(dev);
     for (Scratch *x : out) {
         // (another device's or context's: dropped with its context)
         if (x->device != dev) {
             cudaSetDevice(x->device);
-            if (current_context_id() == x->ctx) x->destroy();
+            if (bound_context_id(x->device) == x->ctx) x->destroy();
             cudaSetDevice(dev);
         } else if (x->ctx == ctx) {
             x->destroy();

@@ -6802,6 +6802,12 @@ unsigned long long current_context_id() {
     if (!get_current || !get_id || get_current(&ctx) != 0 || !ctx || get_id(ctx, &id) != 0) return 0;
     return id;
 }
+
+unsigned long long bound_context_id(int device) {
+    const unsigned long long id = current_context_id();
+    if (id != 0 || cudaSetDevice(device) != cudaSuccess || cudaFree(nullptr) != cudaSuccess) return id;
+    return current_context_id();
+}
 }  // namespace pjg
 
 namespace {

@@ -371,6 +371,9 @@ struct HitSegment {
 // unique id of the calling thread's current CUDA context (0 if unknown; ids
 // are never reused)
 unsigned long long current_context_id();
+// the same for `device`, whose primary context is made the thread's first if it
+// has none yet (a thread that has not used CUDA)
+unsigned long long bound_context_id(int device);
 
 // bytes of k_search's per-warp pair state (shared memory, before the tiles)
 size_t search_state_bytes();
