@@ -1641,12 +1641,13 @@ __global__ void k_leaf_exact(ChunkView cv, int32_t n_sigs, const int32_t *count,
 //
 // Two kernels, so that one structure spreads over the chip: a block sorts a
 // tile of RANK_TILE atoms of one axis in shared memory, then a thread per
-// (atom, axis) sums binary searches over the sorted tiles, whose number the
-// tile's size keeps small.  With tiles of 512 atoms an upload of 14,825 atoms
-// took 0.86 ms (0.82 now), 256 structures 5.6 ms (5.3), 2,000 33.0 (31.9).
-
-constexpr int RANK_TILE = 2048;
-constexpr int RANK_SORT_THREADS = RANK_TILE / 2;  // a pair each
+// (atom, axis) sums binary searches over the sorted tiles.  Tiles of 512 atoms
+// spread a small set over the chip, tiles of 2,048 keep the sums of a larger
+// one short: uploads with the one / the other, one structure of 2,350 atoms
+// 172 / 188 us, 4,687 atoms 447 / 444, 14,825 atoms 856 / 817, 256 structures
+// 5.57 / 5.20 ms, 2,000 32.8 / 31.8 ms.
+constexpr int RANK_FEW = 512, RANK_MANY = 2048;
+constexpr int64_t RANK_FEW_ATOMS = 4096;  // most atoms of a set sorted in the smaller tiles
 constexpr int RANK_THREADS = 256;
 
 __device__ __forceinline__ unsigned long long order_key(double x) {
@@ -1666,7 +1667,8 @@ __device__ __forceinline__ unsigned long long rank_key(const double *xyz64, cons
     return a < 3 ? order_key(xyz64[3 * i + a]) : residue_key(__float_as_int(ro.xyz32[i].w));
 }
 
-__global__ void __launch_bounds__(RANK_SORT_THREADS)
+template <int RANK_TILE>
+__global__ void __launch_bounds__(RANK_TILE / 2)
     k_rank_tiles(const int64_t *atom_base, const int32_t *atom_count, const double *xyz64, int64_t n_atoms,
                  unsigned long long *tile_key, uint16_t *tile_idx, ResidueOrder ro) {
     __shared__ unsigned long long key[RANK_TILE];
@@ -1676,7 +1678,7 @@ __global__ void __launch_bounds__(RANK_SORT_THREADS)
     const int n = atom_count[s];
     for (int t0 = blockIdx.z * RANK_TILE; t0 < n; t0 += gridDim.z * RANK_TILE) {
         const int tn = min(RANK_TILE, n - t0);
-        for (int i = threadIdx.x; i < RANK_TILE; i += RANK_SORT_THREADS) {
+        for (int i = threadIdx.x; i < RANK_TILE; i += RANK_TILE / 2) {
             key[i] = i < tn ? rank_key(xyz64, ro, b0 + t0 + i, a) : ~0ull;
             idx[i] = (uint16_t)i;
         }
@@ -1700,7 +1702,7 @@ __global__ void __launch_bounds__(RANK_SORT_THREADS)
                 __syncthreads();
             }
         }
-        for (int i = threadIdx.x; i < tn; i += RANK_SORT_THREADS) {
+        for (int i = threadIdx.x; i < tn; i += RANK_TILE / 2) {
             tile_key[a * n_atoms + b0 + t0 + i] = key[i];
             tile_idx[a * n_atoms + b0 + t0 + i] = idx[i];
         }
@@ -1708,6 +1710,7 @@ __global__ void __launch_bounds__(RANK_SORT_THREADS)
     }
 }
 
+template <int RANK_TILE>
 __global__ void __launch_bounds__(RANK_THREADS)
     k_axis_ranks(const int64_t *atom_base, const int32_t *atom_count, const double *xyz64, int64_t n_atoms,
                  const unsigned long long *tile_key, const uint16_t *tile_idx, uint32_t *lrank, uint32_t *urank,
@@ -6227,10 +6230,14 @@ void launch_axis_ranks(cudaStream_t st, int32_t n_structures, int32_t max_atoms,
     auto depth = [&](int atoms, int64_t at_most) -> unsigned {
         return (unsigned)std::max<int64_t>(1, std::min<int64_t>(((int64_t)max_atoms + atoms - 1) / atoms, at_most));
     };
-    k_rank_tiles<<<dim3((unsigned)n_structures, 4, depth(RANK_TILE, most)), RANK_SORT_THREADS, 0, st>>>(
-        atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, ro);
-    k_axis_ranks<<<dim3((unsigned)n_structures, 4, depth(RANK_THREADS, 2 * most)), RANK_THREADS, 0, st>>>(
-        atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, lrank, urank, ro);
+    auto launch = [&](auto tiles, auto ranks, int tile) {
+        tiles<<<dim3((unsigned)n_structures, 4, depth(tile, most)), tile / 2, 0, st>>>(
+            atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, ro);
+        ranks<<<dim3((unsigned)n_structures, 4, depth(RANK_THREADS, 2 * most)), RANK_THREADS, 0, st>>>(
+            atom_base, atom_count, xyz64, n_atoms, tile_key, tile_idx, lrank, urank, ro);
+    };
+    if (n_atoms <= RANK_FEW_ATOMS) launch(k_rank_tiles<RANK_FEW>, k_axis_ranks<RANK_FEW>, RANK_FEW);
+    else launch(k_rank_tiles<RANK_MANY>, k_axis_ranks<RANK_MANY>, RANK_MANY);
 }
 
 void launch_demand_levels(cudaStream_t st, int blocks, const TemplateView &tv, const CandView &cd, int32_t n_pairs,
