@@ -1145,10 +1145,15 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
     if (e == cudaSuccess) {
         // axis ranks of every atom (the leaf-order sorted-axis path), and the
         // residue order and kind-ordered points of the order-free search
+        // (the sorted tiles: a kept block where one is large enough)
+        const size_t tile_bytes = (sizeof(unsigned long long) + sizeof(uint16_t)) * 4 * n1;
+        DBuf<unsigned long long> kept;
         Block tiles;
-        e = tiles.alloc((sizeof(unsigned long long) + sizeof(uint16_t)) * 4 * n1, x->st);
+        t_cache = &x->cache;
+        const bool small = BlockCache::class_of(tile_bytes) >= 0;
+        e = small ? dalloc(kept, tile_bytes / sizeof(unsigned long long) + 1, x->st) : tiles.alloc(tile_bytes, x->st);
         if (e == cudaSuccess) {
-            unsigned long long *tile_key = (unsigned long long *)tiles.p;
+            unsigned long long *tile_key = small ? kept.p : (unsigned long long *)tiles.p;
             uint16_t *tile_idx = (uint16_t *)(tile_key + 4 * n1);
             launch_axis_ranks(x->st, S, h->max_atoms, h->d_atom_base, h->d_atom_count, h->d_xyz64, N, tile_key,
                               tile_idx, h->d_lrank, h->d_urank,
@@ -1157,6 +1162,8 @@ pjg_status pjg_structures_create(const pjg_structure_set *set, pjg_structures **
             e = cudaGetLastError();
         }
         tiles.free(x->st);
+        dfree(kept, x->st);
+        t_cache = nullptr;
         const cudaError_t e2 = cudaStreamSynchronize(x->st);
         if (e == cudaSuccess) e = e2;
     }
